@@ -1,0 +1,98 @@
+"""GPU parity of the register-tile kernel (three tokens and more, every format it takes) against the CPU oracle.
+
+Sizes sit at the edges of its tiles: eight tokens per MMA column group, 16 or 32 rows per warp, 1 to 8 slices of K per
+CTA, one to eight token groups per tile, rows that start at any even address.  Bound: 1e-5 relative L2 and the reference
+harnesses' |a - e| <= 1e-4 + 2e-3 |e|: integer sums are exact, only the order of the fp32 additions differs.
+"""
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+
+from helpers import TQ1_POWERS, activations, reference_tolerance_ok, rel_l2, tables, weights
+
+pytestmark = pytest.mark.gpu
+
+FORMATS = ["Q4_0", "Q8_0", "Q2_K", "Q3_K", "Q4_K", "Q5_K", "Q6_K", "IQ2_XXS", "TQ1_0"]
+
+
+@pytest.fixture(scope="module")
+def torch():
+    import torch
+
+    if not torch.cuda.is_available():
+        pytest.fail("these tests need a CUDA device; there is no CPU fallback to test")
+    return torch
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from weft_b200.runtime.driver import Toolchain, last_error, load_library
+
+    lib = load_library(Toolchain().resolve().compiler)
+    assert lib.weft_b200_init(0) == 0, last_error(lib)
+    lib.weft_b200_mul_mat_shard.argtypes = [ctypes.c_int, ctypes.c_int] + [ctypes.c_void_p] * 7 + [ctypes.c_size_t] * 4 + [ctypes.c_uint]
+    return lib
+
+
+class Problem:
+    def __init__(self, torch, oracle, golden, name, m, n, k):
+        rng = np.random.default_rng(m * 7 + n * 3 + k)
+        self.fmt, self.m, self.n, self.k = oracle.FORMAT_IDS[name], m, n, k
+        w, x = weights(self.fmt, rng, n, k), activations(rng, m, k)
+        grid, signs = tables(golden)
+        self.want, self.want_xq = oracle.mul_mat(self.fmt, w, x, n, k, m, rule=1, grid=grid, signs=signs)
+        self.w, self.x = torch.from_numpy(w).cuda(), torch.from_numpy(x).cuda()
+        self.grid, self.signs = torch.from_numpy(grid).cuda(), torch.from_numpy(signs).cuda()
+        self.powers = torch.from_numpy(TQ1_POWERS.view(np.int32)).cuda()
+        self.xq = torch.zeros(self.want_xq.shape, dtype=torch.uint8, device="cuda")
+        self.y = torch.full((m, n), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+
+    def run(self, lib, flags=0):
+        assert lib.weft_b200_mul_mat_shard(self.fmt, 1, self.w.data_ptr(), None if flags else self.x.data_ptr(), self.xq.data_ptr(), self.grid.data_ptr(),
+                                           self.signs.data_ptr(), self.powers.data_ptr(), self.y.data_ptr(), self.n, self.k, self.m, self.n, flags) == 0
+
+    def check(self):
+        got = self.y.cpu().numpy()
+        assert np.array_equal(self.xq.cpu().numpy(), self.want_xq)
+        assert rel_l2(got, self.want) <= 1e-5
+        assert reference_tolerance_ok(got, self.want)
+
+
+@pytest.mark.parametrize("name", FORMATS)
+@pytest.mark.parametrize("mnk", [(3, 1, 256), (3, 17, 512), (8, 300, 1792), (9, 129, 4096), (17, 515, 2304), (40, 64, 2560), (65, 1000, 768), (77, 33, 4352), (136, 700, 512)])
+def test_batch_shapes(torch, lib, oracle, golden, name, mnk):
+    problem = Problem(torch, oracle, golden, name, *mnk)
+    problem.run(lib)
+    problem.check()
+    first = problem.y.clone()                      # the caller's records instead of X: the same planes, the same bits
+    problem.y.fill_(float("nan"))
+    torch.cuda.synchronize()
+    problem.run(lib, flags=1)
+    assert torch.equal(problem.y, first)
+
+
+def test_batch_workspace_is_per_stream_and_per_capture(torch, lib, oracle, golden):
+    """A captured call keeps working while calls of another size run on another stream in between."""
+    small, large = Problem(torch, oracle, golden, "Q4_K", 5, 200, 1024), Problem(torch, oracle, golden, "Q6_K", 60, 300, 2048)
+    side, other, graph = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    lib.weft_b200_set_async(1)
+    try:
+        lib.weft_b200_set_stream(ctypes.c_void_p(side.cuda_stream))
+        with torch.cuda.graph(graph, stream=side):
+            small.run(lib)
+        lib.weft_b200_set_stream(ctypes.c_void_p(other.cuda_stream))
+        for _ in range(3):
+            graph.replay()
+            large.run(lib)
+        assert lib.weft_b200_synchronize() == 0
+    finally:
+        lib.weft_b200_set_stream(None)
+        lib.weft_b200_set_async(0)
+    torch.cuda.synchronize()
+    small.check()
+    large.check()
+    del graph

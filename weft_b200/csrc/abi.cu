@@ -260,8 +260,8 @@ int do_quantize(int act, const float *X, uint8_t *Y, size_t M, size_t K) {
     return call.finish();
 }
 
-// mode 0: GEMV per activation row; mode 1: tensor-core contraction when the shape allows, else GEMV.
-int do_mul_mat(int fmt, int mode, const void *W, const float *X, void *Xq, const int8_t *grid, const int8_t *signs,
+// One path for the decode and the tiled symbols: what runs is chosen by the number of token rows, the format and the shape.
+int do_mul_mat(int fmt, const void *W, const float *X, void *Xq, const int8_t *grid, const int8_t *signs,
                const uint32_t *powers, float *Y, size_t N, size_t K, size_t M, size_t ldy, unsigned flags, bool vec_dot_only,
                const GatherArgs *gather = nullptr) {
     std::lock_guard<std::recursive_mutex> guard(g.lock);
@@ -278,9 +278,8 @@ int do_mul_mat(int fmt, int mode, const void *W, const float *X, void *Xq, const
     if ((fmt == F_Q6_K || fmt == F_IQ1_M) && (reinterpret_cast<uintptr_t>(w) & 1u) && call.realign(&w, N * row_bytes(fmt, K))) return 1;
     if (!have_xq && call.map(X, M * K * sizeof(float), true, false, &x)) return 1;
     // Decode quantizes X inside the GEMV (its first CTA stores the records, nobody loads them again), so a pinned Xq can
-    // be written in place; a call that may take the tensor-core path or the separate quantize kernel reads Xq back.
-    const bool may_contract = mode == 1 && M >= 32 && K % 256 == 0;
-    const bool xq_in_place = !have_xq && !may_contract && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    // be written in place; a batch may take a path that reads Xq back.
+    const bool xq_in_place = !have_xq && M < 3 && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     if (call.map(Xq, M * row_bytes(act, K), have_xq, !have_xq, &xq, xq_in_place)) return 1;
     if (codebook_bytes(fmt) && (call.map(grid, codebook_bytes(fmt), true, false, &gr) || (has_sign_table(fmt) && call.map(signs, 1024, true, false, &sg)))) return 1;
     if (fmt == F_TQ1_0 && call.map(powers, 20, true, false, &pw)) return 1;
@@ -293,29 +292,33 @@ int do_mul_mat(int fmt, int mode, const void *W, const float *X, void *Xq, const
         (reinterpret_cast<uintptr_t>(y) & 3u) || (x && (reinterpret_cast<uintptr_t>(x) & 3u)))
         return fail("a buffer does not meet its Encoding alignment");
     const int sms = g.prop.multiProcessorCount;
-    const bool by_blocks = mode == 1 && prefill_blocks_supported(fmt, (long long)N, (long long)K, (long long)M, w, xq);
-    const bool by_codebook = mode == 1 && gr && sg && prefill_codebook_supported(fmt, (long long)N, (long long)K, (long long)M, w, xq);
-    const bool to_prefill = by_blocks || by_codebook || (mode == 1 && (prefill_supported(fmt, (long long)N, (long long)K, (long long)M, w, xq) ||
-                                                                       prefill_pair_supported(fmt, (long long)N, (long long)K, (long long)M, w, xq)));
-    // decode: the GEMV's own prologue quantizes X (one launch) when the fp32 rows allow 16-byte loads
-    const bool fuse_quantize = !have_xq && !to_prefill && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-    if (!have_xq && !fuse_quantize &&
-        launched(launch_quantize(act, (const float *)x, xq, (long long)M, (long long)K, sms, g.stream), "activation quantize"))
-        return 1;
-    if (to_prefill) {
-        PrefillArgs pa{fmt, w, xq, (const uint32_t *)pw, (float *)y, (long long)N, (long long)K, (long long)M, (long long)ldy, g.status_dev};
-        const bool pair = prefill_pair_supported(fmt, (long long)N, (long long)K, (long long)M, w, xq);
-        if (launched(by_codebook ? launch_prefill_codebook(pa, (const int8_t *)gr, (const int8_t *)sg, sms, g.stream) : by_blocks ? launch_prefill_blocks(pa, sms, g.stream) : pair ? launch_prefill_pair(pa, sms, g.stream) : launch_prefill(pa, sms, g.stream), "prefill mul_mat",
-                     pair ? prefill_pair_launches(fmt) : 1)) return 1;   // the pair paths launch their plane kernel first
-        if (gather && launched(launch_gather_push(*gather, (long long)M, (long long)N, (long long)ldy, g.status_dev, sms, g.stream), "peer all-gather")) return 1;
+    const bool pair = prefill_pair_supported(fmt, (long long)N, (long long)K, (long long)M, w, xq);
+    const TileArgs ta{fmt, w, have_xq ? nullptr : (const float *)x, xq, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw,
+                      (float *)y, (long long)N, (long long)K, (long long)M, (long long)ldy};
+    bool gathered = false;
+    if (!pair && tile_supported(ta)) {
+        // a batch of tokens: register tiles, the weights read once per tile of tokens; their first kernel quantizes X
+        uint8_t *planes = nullptr;
+        CU(workspace(tile_plane_bytes(ta), g.stream, &planes));
+        if (launched(launch_tile(ta, planes, sms, g.stream), "batched mul_mat", 2)) return 1;
     } else {
-        GemvArgs ga{fmt, w, xq, fuse_quantize ? (const float *)x : nullptr, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw,
-                    (float *)y, (long long)N, (long long)K, (long long)M, (long long)ldy, g.status_dev, y_on_host};
-        const bool fused = gather && gemv_gathers(ga);
-        if (fused) ga.gather = *gather;
-        if (launched(launch_gemv(ga, sms, g.stream), "decode mul_mat")) return 1;
-        if (gather && !fused && launched(launch_gather_push(*gather, (long long)M, (long long)N, (long long)ldy, g.status_dev, sms, g.stream), "peer all-gather")) return 1;
+        // decode: the GEMV's own prologue quantizes X (one launch) when the fp32 rows allow 16-byte loads
+        const bool fuse_quantize = !have_xq && !pair && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+        if (!have_xq && !fuse_quantize &&
+            launched(launch_quantize(act, (const float *)x, xq, (long long)M, (long long)K, sms, g.stream), "activation quantize"))
+            return 1;
+        if (pair) {
+            const PrefillArgs pa{fmt, w, xq, (const uint32_t *)pw, (float *)y, (long long)N, (long long)K, (long long)M, (long long)ldy, g.status_dev};
+            if (launched(launch_prefill_pair(pa, sms, g.stream), "prefill mul_mat", prefill_pair_launches(fmt))) return 1;   // its plane kernel first
+        } else {
+            GemvArgs ga{fmt, w, xq, fuse_quantize ? (const float *)x : nullptr, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw,
+                        (float *)y, (long long)N, (long long)K, (long long)M, (long long)ldy, g.status_dev, y_on_host};
+            gathered = gather && gemv_gathers(ga);
+            if (gathered) ga.gather = *gather;
+            if (launched(launch_gemv(ga, sms, g.stream), "decode mul_mat")) return 1;
+        }
     }
+    if (gather && !gathered && launched(launch_gather_push(*gather, (long long)M, (long long)N, (long long)ldy, g.status_dev, sms, g.stream), "peer all-gather")) return 1;
     return call.finish();
 }
 
@@ -418,10 +421,10 @@ int weft_b200_mma_peak(int mode, double *tera_ops) {
 // ---- vec_dot
 #define VEC_DOT(name, fmt, TABLE_PARAMS, GRID, SIGNS, POWERS)                                                          \
     int name(const uint8_t *W, const uint8_t *X TABLE_PARAMS, float *Y, size_t K) {                                   \
-        return do_mul_mat(fmt, 0, W, nullptr, const_cast<uint8_t *>(X), GRID, SIGNS, POWERS, Y, 1, K, 1, 1, 0, true); \
+        return do_mul_mat(fmt, W, nullptr, const_cast<uint8_t *>(X), GRID, SIGNS, POWERS, Y, 1, K, 1, 1, 0, true); \
     }                                                                                                                  \
     int name##_rows(const uint8_t *W, const uint8_t *X TABLE_PARAMS, float *Y, size_t N, size_t K) {                  \
-        return do_mul_mat(fmt, 0, W, nullptr, const_cast<uint8_t *>(X), GRID, SIGNS, POWERS, Y, N, K, 1, N, 0, true); \
+        return do_mul_mat(fmt, W, nullptr, const_cast<uint8_t *>(X), GRID, SIGNS, POWERS, Y, N, K, 1, N, 0, true); \
     }
 #define NO_TABLES
 #define IQ_TABLES , const int8_t *grid, const int8_t *signs
@@ -478,50 +481,50 @@ int q8_0_quantize_rows(const float *X, uint8_t *Y, size_t M, size_t K) { return 
 int q8_K_quantize_rows(const float *X, uint8_t *Y, size_t M, size_t K) { return do_quantize(F_Q8_K, X, Y, M, K); }
 
 // ---- mul_mat
-#define MUL_MAT(name, fmt, mode, TABLE_PARAMS, GRID, SIGNS, POWERS)                                                    \
+#define MUL_MAT(name, fmt, TABLE_PARAMS, GRID, SIGNS, POWERS)                                                    \
     int name(const uint8_t *W, const float *X, uint8_t *Xq TABLE_PARAMS, float *Y, size_t N, size_t K, size_t M) {    \
-        return do_mul_mat(fmt, mode, W, X, Xq, GRID, SIGNS, POWERS, Y, N, K, M, N, 0, false);                         \
+        return do_mul_mat(fmt, W, X, Xq, GRID, SIGNS, POWERS, Y, N, K, M, N, 0, false);                         \
     }
-MUL_MAT(production_mul_mat_q4_0_decode, F_Q4_0, 0, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q8_0_decode, F_Q8_0, 0, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q4_k_decode, F_Q4_K, 0, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q2_k_decode, F_Q2_K, 0, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q3_k_decode, F_Q3_K, 0, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q5_k_decode, F_Q5_K, 0, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q6_k_decode, F_Q6_K, 0, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_iq2_xxs_decode, F_IQ2_XXS, 0, IQ_TABLES, grid, signs, nullptr)
-MUL_MAT(production_mul_mat_tq1_0_decode, F_TQ1_0, 0, TQ_TABLES, nullptr, nullptr, powers)
+MUL_MAT(production_mul_mat_q4_0_decode, F_Q4_0, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q8_0_decode, F_Q8_0, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q4_k_decode, F_Q4_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q2_k_decode, F_Q2_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q3_k_decode, F_Q3_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q5_k_decode, F_Q5_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q6_k_decode, F_Q6_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_iq2_xxs_decode, F_IQ2_XXS, IQ_TABLES, grid, signs, nullptr)
+MUL_MAT(production_mul_mat_tq1_0_decode, F_TQ1_0, TQ_TABLES, nullptr, nullptr, powers)
 // same functions under the names of the reference's alternative lowering plans (examples/kernels/mul_mat/
 // tq1_0_lane16_decode.py:10-23, q3_k_predecoded_scales_decode.py:10-21, q3_k_predecoded_scales.py:10-61)
-MUL_MAT(production_mul_mat_tq1_0_lane16_decode, F_TQ1_0, 0, TQ_TABLES, nullptr, nullptr, powers)
-MUL_MAT(production_mul_mat_q3_k_predecoded_scales_decode, F_Q3_K, 0, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q3_k_predecoded_scales, F_Q3_K, 1, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q4_0, F_Q4_0, 1, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q8_0, F_Q8_0, 1, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q4_k_staged, F_Q4_K, 1, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q2_k, F_Q2_K, 1, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q3_k, F_Q3_K, 1, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q5_k, F_Q5_K, 1, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_q6_k, F_Q6_K, 1, NO_TABLES, nullptr, nullptr, nullptr)
-MUL_MAT(production_mul_mat_tq1_0, F_TQ1_0, 1, TQ_TABLES, nullptr, nullptr, powers)
-MUL_MAT(production_mul_mat_iq2_xxs_staged, F_IQ2_XXS, 1, IQ_TABLES, grid, signs, nullptr)
-MUL_MAT(production_mul_mat_iq2_xxs, F_IQ2_XXS, 1, IQ_TABLES, grid, signs, nullptr)
+MUL_MAT(production_mul_mat_tq1_0_lane16_decode, F_TQ1_0, TQ_TABLES, nullptr, nullptr, powers)
+MUL_MAT(production_mul_mat_q3_k_predecoded_scales_decode, F_Q3_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q3_k_predecoded_scales, F_Q3_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q4_0, F_Q4_0, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q8_0, F_Q8_0, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q4_k_staged, F_Q4_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q2_k, F_Q2_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q3_k, F_Q3_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q5_k, F_Q5_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_q6_k, F_Q6_K, NO_TABLES, nullptr, nullptr, nullptr)
+MUL_MAT(production_mul_mat_tq1_0, F_TQ1_0, TQ_TABLES, nullptr, nullptr, powers)
+MUL_MAT(production_mul_mat_iq2_xxs_staged, F_IQ2_XXS, IQ_TABLES, grid, signs, nullptr)
+MUL_MAT(production_mul_mat_iq2_xxs, F_IQ2_XXS, IQ_TABLES, grid, signs, nullptr)
 // IQ2_XS (examples/kernels/mul_mat/iq2_xs.py:27-33, iq2_xs_staged.py:30-36) and IQ3_XXS (iq3_xxs.py:11-17): the GEMV per
 // token row at any token count
-MUL_MAT(production_mul_mat_iq2_xs, F_IQ2_XS, 1, IQ_TABLES, grid, signs, nullptr)
-MUL_MAT(production_mul_mat_iq2_xs_staged, F_IQ2_XS, 1, IQ_TABLES, grid, signs, nullptr)
-MUL_MAT(production_mul_mat_iq3_xxs, F_IQ3_XXS, 1, IQ_TABLES, grid, signs, nullptr)
+MUL_MAT(production_mul_mat_iq2_xs, F_IQ2_XS, IQ_TABLES, grid, signs, nullptr)
+MUL_MAT(production_mul_mat_iq2_xs_staged, F_IQ2_XS, IQ_TABLES, grid, signs, nullptr)
+MUL_MAT(production_mul_mat_iq3_xxs, F_IQ3_XXS, IQ_TABLES, grid, signs, nullptr)
 // IQ2_S (examples/kernels/mul_mat/iq2_s.py:10-16, iq2_s_staged.py:29-35) and IQ3_S (iq3_s.py:10-16): one table argument
-MUL_MAT(production_mul_mat_iq2_s, F_IQ2_S, 1, GRID_ONLY, grid, nullptr, nullptr)
-MUL_MAT(production_mul_mat_iq2_s_staged, F_IQ2_S, 1, GRID_ONLY, grid, nullptr, nullptr)
-MUL_MAT(production_mul_mat_iq3_s, F_IQ3_S, 1, GRID_ONLY, grid, nullptr, nullptr)
+MUL_MAT(production_mul_mat_iq2_s, F_IQ2_S, GRID_ONLY, grid, nullptr, nullptr)
+MUL_MAT(production_mul_mat_iq2_s_staged, F_IQ2_S, GRID_ONLY, grid, nullptr, nullptr)
+MUL_MAT(production_mul_mat_iq3_s, F_IQ3_S, GRID_ONLY, grid, nullptr, nullptr)
 // IQ1_S (examples/kernels/mul_mat/iq1_s.py:9-15, iq1_s_decode.py:10-16) and IQ1_M (iq1_m.py:10-17, iq1_m_decode.py:10-17,
 // iq1_m_lane16_decode.py:10-17)
-MUL_MAT(production_mul_mat_iq1_s, F_IQ1_S, 1, GRID_ONLY, grid, nullptr, nullptr)
-MUL_MAT(production_mul_mat_iq1_s_decode, F_IQ1_S, 0, GRID_ONLY, grid, nullptr, nullptr)
-MUL_MAT(production_mul_mat_iq1_m, F_IQ1_M, 1, IQ1M_TABLES, grid, nullptr, reinterpret_cast<const uint32_t *>(f16_bits))
-MUL_MAT(production_mul_mat_iq1_m_decode, F_IQ1_M, 0, IQ1M_TABLES, grid, nullptr, reinterpret_cast<const uint32_t *>(f16_bits))
-MUL_MAT(production_mul_mat_iq1_m_lane16_decode, F_IQ1_M, 0, IQ1M_TABLES, grid, nullptr, reinterpret_cast<const uint32_t *>(f16_bits))
+MUL_MAT(production_mul_mat_iq1_s, F_IQ1_S, GRID_ONLY, grid, nullptr, nullptr)
+MUL_MAT(production_mul_mat_iq1_s_decode, F_IQ1_S, GRID_ONLY, grid, nullptr, nullptr)
+MUL_MAT(production_mul_mat_iq1_m, F_IQ1_M, IQ1M_TABLES, grid, nullptr, reinterpret_cast<const uint32_t *>(f16_bits))
+MUL_MAT(production_mul_mat_iq1_m_decode, F_IQ1_M, IQ1M_TABLES, grid, nullptr, reinterpret_cast<const uint32_t *>(f16_bits))
+MUL_MAT(production_mul_mat_iq1_m_lane16_decode, F_IQ1_M, IQ1M_TABLES, grid, nullptr, reinterpret_cast<const uint32_t *>(f16_bits))
 
 // ---- persistent interleaved layout Q4K_I[16]: artifact functions and the kernels that consume it
 static size_t q4ki_packed_size(size_t rows, size_t K) { return K % 256 == 0 && rows % 16 == 0 ? rows * (K / 256) * 144 : 0; }
@@ -542,7 +545,7 @@ static int q4ki_pack(const uint8_t *source, uint8_t *target, size_t rows, size_t
 size_t q4_k_q8_k_gemv_W_packed_size(size_t M, size_t K) { return q4ki_packed_size(M, K); }
 int q4_k_q8_k_gemv_W_pack(const uint8_t *source, uint8_t *target, size_t M, size_t K) { return q4ki_pack(source, target, M, K); }
 int q4_k_q8_k_gemv(const uint8_t *W, const uint8_t *X, float *Y, size_t M, size_t K) {
-    return do_mul_mat(F_Q4_K_I16, 0, W, nullptr, const_cast<uint8_t *>(X), nullptr, nullptr, nullptr, Y, M, K, 1, M, 0, true);
+    return do_mul_mat(F_Q4_K_I16, W, nullptr, const_cast<uint8_t *>(X), nullptr, nullptr, nullptr, Y, M, K, 1, M, 0, true);
 }
 // The reference's two other statements of this GEMV (four 16-bit partial groups per sub-block; a 32-bit contraction
 // per sub-block) differ in the vector plan only: same layout, same integer sums, same float op tree
@@ -551,14 +554,14 @@ int q4_k_q8_k_gemv(const uint8_t *W, const uint8_t *X, float *Y, size_t M, size_
     size_t name##_W_packed_size(size_t M, size_t K) { return q4ki_packed_size(M, K); }                                \
     int name##_W_pack(const uint8_t *source, uint8_t *target, size_t M, size_t K) { return q4ki_pack(source, target, M, K); } \
     int name(const uint8_t *W, const uint8_t *X, float *Y, size_t M, size_t K) {                                       \
-        return do_mul_mat(F_Q4_K_I16, 0, W, nullptr, const_cast<uint8_t *>(X), nullptr, nullptr, nullptr, Y, M, K, 1, M, 0, true); \
+        return do_mul_mat(F_Q4_K_I16, W, nullptr, const_cast<uint8_t *>(X), nullptr, nullptr, nullptr, Y, M, K, 1, M, 0, true); \
     }
 Q4KI_GEMV_ALIAS(q4_k_q8_k_gemv_groups4)
 Q4KI_GEMV_ALIAS(q4_k_q8_k_gemv_contract)
 size_t production_mul_mat_q4_k_persistent_W_packed_size(size_t N, size_t K) { return q4ki_packed_size(N, K); }
 int production_mul_mat_q4_k_persistent_W_pack(const uint8_t *source, uint8_t *target, size_t N, size_t K) { return q4ki_pack(source, target, N, K); }
 int production_mul_mat_q4_k_persistent(const uint8_t *W, const float *X, uint8_t *Xq, float *Y, size_t M, size_t K, size_t N) {
-    return do_mul_mat(F_Q4_K_I16, 0, W, X, Xq, nullptr, nullptr, nullptr, Y, N, K, M, N, 0, false);
+    return do_mul_mat(F_Q4_K_I16, W, X, Xq, nullptr, nullptr, nullptr, Y, N, K, M, N, 0, false);
 }
 
 // Steps i .. i + count - 1 of a chain as one grouped launch: same activations, same K, one activation row, Q4_K
@@ -612,7 +615,7 @@ int weft_b200_mul_mat_chain(const weft_b200_mul_mat_step *steps, size_t count) {
         if (s.format != F_Q4_0 && s.format != F_Q8_0 && s.format != F_Q2_K && s.format != F_Q3_K && s.format != F_Q4_K && s.format != F_Q5_K &&
             s.format != F_Q6_K && s.format != F_IQ2_XXS && s.format != F_TQ1_0)  /* chains: the formats of the first version */
             return fail("step %zu: unknown weight format id %d", i, s.format);
-        if (do_mul_mat(s.format, 0, s.W, s.X, s.Xq, s.grid, s.signs, s.powers, s.Y, s.N, s.K, s.M, s.N, s.flags, false)) return 1;
+        if (do_mul_mat(s.format, s.W, s.X, s.Xq, s.grid, s.signs, s.powers, s.Y, s.N, s.K, s.M, s.N, s.flags, false)) return 1;
     }
     return 0;
 }
@@ -695,7 +698,7 @@ int weft_b200_mul_mat_shard_gather(int format, int mode, const uint8_t *W_local,
             ga.stage[r] = static_cast<uint2 *>(stage_ranks[r]);
         }
     }
-    return do_mul_mat(format, mode, W_local, X, Xq, grid, signs, powers, ga.y[rank], N_local, K, M, N, flags, false, &ga);
+    return do_mul_mat(format, W_local, X, Xq, grid, signs, powers, ga.y[rank], N_local, K, M, N, flags, false, &ga);
 }
 
 int weft_b200_mul_mat_shard(int format, int mode, const uint8_t *W_local, const float *X, uint8_t *Xq,
@@ -704,7 +707,7 @@ int weft_b200_mul_mat_shard(int format, int mode, const uint8_t *W_local, const 
     if (format != F_Q4_0 && format != F_Q8_0 && format != F_Q2_K && format != F_Q3_K && format != F_Q4_K && format != F_Q5_K && format != F_Q6_K && format != F_IQ2_XXS && format != F_IQ2_XS && format != F_IQ3_XXS && format != F_IQ2_S && format != F_IQ3_S && format != F_IQ1_S && format != F_IQ1_M && format != F_TQ1_0 && format != F_Q4_K_I16)
         return fail("unknown weight format id %d", format);
     if (mode != 0 && mode != 1) return fail("mode must be 0 (decode) or 1 (prefill)");
-    return do_mul_mat(format, mode, W_local, X, Xq, grid, signs, powers, Y_columns, N_local, K, M, ldy, flags, false);
+    return do_mul_mat(format, W_local, X, Xq, grid, signs, powers, Y_columns, N_local, K, M, ldy, flags, false);
 }
 
 }  // extern "C"

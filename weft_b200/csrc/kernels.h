@@ -73,23 +73,31 @@ struct PrefillArgs {
     long long n, k, m, ldy;
     int *status;
 };
-// tcgen05 int8 tensor-core path; returns cudaErrorNotSupported for shapes it does not take.
-cudaError_t launch_prefill(const PrefillArgs &a, int sm_count, cudaStream_t stream);
-bool prefill_supported(int fmt, long long n, long long k, long long m, const void *w, const void *xq);
-// The same contraction on CTA pairs (256 tokens per tile, tcgen05 cta_group::2): Q4_K with more than 128 tokens.
+// tcgen05 int8 contraction on CTA pairs (256 tokens per tile, cta_group::2): Q4_K and TQ1_0 with more than 128 tokens.
 cudaError_t launch_prefill_pair(const PrefillArgs &a, int sm_count, cudaStream_t stream);
 bool prefill_pair_supported(int fmt, long long n, long long k, long long m, const void *w, const void *xq);
 int prefill_pair_launches(int fmt);   // kernels one launch_prefill_pair call puts on the stream (the plane kernel counts)
 
-// Q4_0 / Q8_0 x Q8_0 with more than a few tokens: one K = 32 contraction per 32-element block (both operands carry a
-// scale per block), accumulators rotating through tensor memory, scales applied in the epilogue.
-cudaError_t launch_prefill_blocks(const PrefillArgs &a, int sm_count, cudaStream_t stream);
-bool prefill_blocks_supported(int fmt, long long n, long long k, long long m, const void *w, const void *xq);
+// More than one token row: the register-tile kernel (tile.cuh) behind the kernel that quantizes X into its planes.
+struct TileArgs {
+    int fmt;
+    const void *w;           // (n, k) records, 16-byte aligned
+    const float *x;          // (m, k) fp32 activations, or NULL: xq already holds the records
+    const void *xq;          // (m, k) Q8_0 / Q8_K records; written when x is given
+    const int8_t *grid, *signs;
+    const uint32_t *powers;
+    float *y;                // (m, ldy)
+    long long n, k, m, ldy;
+};
+bool tile_supported(const TileArgs &a);
+size_t tile_plane_bytes(const TileArgs &a);
+cudaError_t launch_tile(const TileArgs &a, uint8_t *planes, int sm_count, cudaStream_t stream);   // two kernels
+template <int FMT> cudaError_t launch_tile_kernel(const TileArgs &a, const uint8_t *planes, int sm_count, cudaStream_t stream);
 
-// IQ2_XXS x Q8_K with more than a few tokens: one contraction per 32-element group (integer scale 2 s + 1 per group),
-// combined in integers in the epilogue; grid int8[256][8] and signs int8[128][8] (+1 / -1) in device memory.
-cudaError_t launch_prefill_codebook(const PrefillArgs &a, const int8_t *grid, const int8_t *signs, int sm_count, cudaStream_t stream);
-bool prefill_codebook_supported(int fmt, long long n, long long k, long long m, const void *w, const void *xq);
+// Device memory for a call's activation planes, valid for the work it puts on `stream` (workspace.cu); the generation
+// changes whenever memory handed out earlier outside a capture is gone.
+cudaError_t workspace(size_t bytes, cudaStream_t stream, uint8_t **out);
+unsigned long long workspace_generation();
 
 // Bare tcgen05.mma issue loop on every SM (mode 0: kind::i8, one CTA per SM; 1: kind::i8 on CTA pairs; 2: kind::f16):
 // spans_dev receives the nanoseconds each issuing CTA took; *ops_per_launch the operations the whole launch performs.

@@ -1082,29 +1082,6 @@ bool prefill_pair_supported(int fmt, long long n, long long k, long long m, cons
            (reinterpret_cast<uintptr_t>(w) & 15u) == 0 && (reinterpret_cast<uintptr_t>(xq) & 3u) == 0;
 }
 
-// The planes of the latest call: one device allocation that only ever grows.  Calls are serialised by the
-// library and run on one stream, so the next call's plane kernel starts after this call's contraction has ended.  A
-// larger request gets a new allocation; the previous ones stay until the process ends, because work already queued (or a
-// captured graph) may still name them.
-struct PlaneScratch {
-    uint8_t *base = nullptr;
-    size_t bytes = 0;
-};
-static PlaneScratch g_planes;
-
-static cudaError_t reserve_planes(size_t bytes, uint8_t **out) {
-    if (bytes > g_planes.bytes) {
-        uint8_t *fresh = nullptr;
-        const size_t want = (bytes + bytes / 4 + 255) & ~size_t(255);
-        const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&fresh), want);
-        if (e != cudaSuccess) return e;
-        g_planes.base = fresh;
-        g_planes.bytes = want;
-    }
-    *out = g_planes.base;
-    return cudaSuccess;
-}
-
 // The register trade assumes the allocation the kernel was compiled with: a build with another one must not run
 static cudaError_t check_launch_registers(const void *kernel, int expected) {
     cudaFuncAttributes attr;
@@ -1139,7 +1116,7 @@ static cudaError_t launch_prefill_pair_tq1(const PrefillArgs &a, int sm_count, c
     p.xd_pitch = (a.m + 63) & ~63LL;
     const size_t code_bytes = ((size_t)a.m * (size_t)a.k + 255) & ~size_t(255);
     uint8_t *planes = nullptr;
-    e = reserve_planes(code_bytes + (size_t)p.nb * (size_t)p.xd_pitch * sizeof(float), &planes);
+    e = workspace(code_bytes + (size_t)p.nb * (size_t)p.xd_pitch * sizeof(float), stream, &planes);
     if (e != cudaSuccess) return e;
     p.xd = reinterpret_cast<const float *>(planes + code_bytes);
     {
@@ -1190,7 +1167,7 @@ static cudaError_t launch_prefill_pair_q4k_planes(const PrefillArgs &a, int sm_c
     const size_t code_bytes = ((size_t)a.m * (size_t)a.k + 255) & ~size_t(255);
     const size_t xd_bytes = ((size_t)p.nb * (size_t)p.xd_pitch * sizeof(float) + 255) & ~size_t(255);
     uint8_t *planes = nullptr;
-    e = reserve_planes(code_bytes + xd_bytes + (size_t)a.m * (size_t)p.nb * 32, &planes);
+    e = workspace(code_bytes + xd_bytes + (size_t)a.m * (size_t)p.nb * 32, stream, &planes);
     if (e != cudaSuccess) return e;
     p.xd = reinterpret_cast<const float *>(planes + code_bytes);
     uint8_t *mins = planes + code_bytes + xd_bytes;

@@ -1,0 +1,162 @@
+// Host side of the register-tile kernel (tile.cuh) and the kernel that quantizes activations into its planes.
+#include "tile.cuh"
+
+#include <algorithm>
+
+namespace weft {
+
+// ------------------------------------------------------------------ activation planes
+// One warp per (token, 256-element block): quantizes the fp32 values (same bodies as the standalone quantizers), stores the
+// caller's records, and writes the codes in fragment order with the scales and sums the tile kernel needs.  Without X the
+// caller's records are the source.  HBM/L2-bound: 4 bytes in, 1.14 out to the records and 1.02 - 1.27 to the planes.
+template <int FMT, bool FROM_X, bool A16>
+__global__ void __launch_bounds__(256) tile_planes_kernel(const float *__restrict__ x, uint8_t *__restrict__ xq, uint8_t *__restrict__ planes, int m, int nb) {
+    using F = TileFormat<FMT>;
+    __shared__ __align__(16) uint32_t s_codes[8][64];
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long unit = (long long)blockIdx.x * 8 + warp;
+    if (unit >= (long long)m * nb) return;
+    const int token = (int)(unit / nb), block = (int)(unit - (long long)token * nb), n = token & 7;
+    uint8_t *group = planes + ((long long)(token >> 3) * nb + block) * F::GROUP;
+    uint32_t q0, q1;
+    int sum = 0;                                  // Q8_K: of the lane pair's 16 codes (the record's bsum)
+    float d;
+    if constexpr (F::PAIR32) {
+        uint8_t *rec = xq + (unit * 8 + (lane >> 2)) * 34;
+        if constexpr (FROM_X) {
+            float v[8];
+            load8<A16>(x + unit * 256 + 8 * lane, v);
+            int sum32;
+            q8_0_warp(v, q0, q1, sum32, d);
+            store_q8_0(rec, lane & 3, q0, q1, d);
+            d = __half2float(__float2half_rn(d));
+        } else {
+            q0 = ld_u32_a2(rec + 2 + 8 * (lane & 3));
+            q1 = ld_u32_a2(rec + 6 + 8 * (lane & 3));
+            d = half_at(rec);
+        }
+        if ((lane & 3) == 0) *reinterpret_cast<float *>(group + 2048 + 32 * (lane >> 2) + 4 * n) = d;
+    } else {
+        uint8_t *rec = xq + unit * 292;
+        if constexpr (FROM_X) {
+            float v[8];
+            load8<A16>(x + unit * 256 + 8 * lane, v);
+            q8_k_warp(v, q0, q1, sum, d);
+            store_q8_k(rec, lane, q0, q1, sum, d);
+        } else {
+            q0 = *reinterpret_cast<const uint32_t *>(rec + 4 + 8 * lane);
+            q1 = *reinterpret_cast<const uint32_t *>(rec + 8 + 8 * lane);
+            sum = *reinterpret_cast<const int16_t *>(rec + 260 + (lane & ~1));
+            d = *reinterpret_cast<const float *>(rec);
+        }
+        if (lane == 0) *reinterpret_cast<float *>(group + 2048 + 4 * n) = d;
+        if constexpr (F::MINS > 0) {              // sums as 64 h + l, two exact f16 limbs: lane t of the fragment column holds two sums
+#pragma unroll
+            for (int q = 0; q < F::MINS; ++q) {
+                int s[2];
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const int at = F::MINS == 1 ? 8 * (lane & 3) + 4 * i : 16 * q + 4 * (lane & 3) + 2 * i;      // lane that holds the sum
+                    s[i] = __shfl_sync(0xffffffffu, sum, at);
+                    if (F::MINS == 1) s[i] += __shfl_sync(0xffffffffu, sum, at + 2);
+                }
+                const __half2 l = __floats2half2_rn((float)(s[0] & 63), (float)(s[1] & 63)), h = __floats2half2_rn((float)(s[0] >> 6), (float)(s[1] >> 6));
+                if (lane < 4)
+                    *reinterpret_cast<uint2 *>(group + 2048 + 32 + 256 * q + (n * 4 + lane) * 8) =
+                        make_uint2(*reinterpret_cast<const uint32_t *>(&l), *reinterpret_cast<const uint32_t *>(&h));
+            }
+        }
+        if constexpr (FMT == F_TQ1_0) {
+            int total = dp4a_ss(q0, 0x01010101u, dp4a_ss(q1, 0x01010101u, 0));
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+            if (lane == 0) *reinterpret_cast<int *>(group + 2048 + 32 + 4 * n) = -total;
+        }
+    }
+    s_codes[warp][2 * lane] = q0;
+    s_codes[warp][2 * lane + 1] = q1;
+    __syncwarp();
+    if (lane < 16) {
+        const int j = lane >> 2, t = lane & 3;
+        uint32_t out[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {             // word i of the lane: groups 2j (low, high), 2j + 1 (low, high)
+            const int g = 2 * j + (i >> 1), half = i & 1;
+            if constexpr (F::ORDER == ORDER_NATURAL) out[i] = s_codes[warp][8 * g + 2 * t + half];
+            else if constexpr (F::ORDER == ORDER_SPLIT16) out[i] = s_codes[warp][8 * g + 4 * half + t];
+            else {
+                const int word = 2 * g + half, e = tl_ternary_element(word, t), stride = tl_ternary_stride(word);
+                const uint8_t *c = reinterpret_cast<const uint8_t *>(s_codes[warp]) + e;
+                out[i] = (uint32_t)c[0] | ((uint32_t)c[stride] << 8) | ((uint32_t)c[2 * stride] << 16) | ((uint32_t)c[3 * stride] << 24);
+            }
+        }
+        *reinterpret_cast<uint4 *>(group + 512 * j + (n * 4 + t) * 16) = make_uint4(out[0], out[1], out[2], out[3]);
+    }
+}
+
+template <int FMT>
+static cudaError_t launch_planes(const TileArgs &a, uint8_t *planes, cudaStream_t stream) {
+    const int nb = (int)(a.k / 256);
+    const unsigned grid = (unsigned)((a.m * nb + 7) / 8);
+    uint8_t *xq = static_cast<uint8_t *>(const_cast<void *>(a.xq));
+    if (!a.x) tile_planes_kernel<FMT, false, false><<<grid, 256, 0, stream>>>(nullptr, xq, planes, (int)a.m, nb);
+    else if (reinterpret_cast<uintptr_t>(a.x) & 15u) tile_planes_kernel<FMT, true, false><<<grid, 256, 0, stream>>>(a.x, xq, planes, (int)a.m, nb);
+    else tile_planes_kernel<FMT, true, true><<<grid, 256, 0, stream>>>(a.x, xq, planes, (int)a.m, nb);
+    return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------ dispatch
+
+static bool tile_format(int fmt) {
+    return fmt == F_Q4_0 || fmt == F_Q8_0 || fmt == F_Q2_K || fmt == F_Q3_K || fmt == F_Q4_K || fmt == F_Q5_K || fmt == F_Q6_K || fmt == F_IQ2_XXS || fmt == F_TQ1_0;
+}
+static int tile_group_bytes(int fmt) {
+    switch (fmt) {
+    case F_Q4_0: return TileFormat<F_Q4_0>::GROUP;
+    case F_Q8_0: return TileFormat<F_Q8_0>::GROUP;
+    case F_Q2_K: return TileFormat<F_Q2_K>::GROUP;
+    case F_Q3_K: return TileFormat<F_Q3_K>::GROUP;
+    case F_Q4_K: return TileFormat<F_Q4_K>::GROUP;
+    case F_Q5_K: return TileFormat<F_Q5_K>::GROUP;
+    case F_Q6_K: return TileFormat<F_Q6_K>::GROUP;
+    case F_IQ2_XXS: return TileFormat<F_IQ2_XXS>::GROUP;
+    default: return TileFormat<F_TQ1_0>::GROUP;
+    }
+}
+
+bool tile_supported(const TileArgs &a) {
+    // From three tokens on: up to there a GEMV per token row, which reads the matrix each time, is as quick (two tokens,
+    // 14336 x 4096: Q4_K 13.6 us against 16 us, Q6_K 20 against 24; three: 19.6 and 28.9 against the same).
+    // 16-byte copies of weight rows need a 16-byte aligned matrix; sizes within a tile are 32-bit in the kernel
+    return tile_format(a.fmt) && a.m >= 3 && a.m <= (1 << 20) && a.k % 256 == 0 && a.k / 256 <= (1 << 20) && (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0;
+}
+
+size_t tile_plane_bytes(const TileArgs &a) { return (size_t)((a.m + 7) / 8) * (size_t)(a.k / 256) * tile_group_bytes(a.fmt); }
+
+cudaError_t launch_tile(const TileArgs &a, uint8_t *planes, int sm_count, cudaStream_t stream) {
+    cudaError_t e;
+    switch (a.fmt) {
+    case F_Q4_0: e = launch_planes<F_Q4_0>(a, planes, stream); break;
+    case F_Q8_0: e = launch_planes<F_Q8_0>(a, planes, stream); break;
+    case F_Q4_K: case F_Q5_K: e = launch_planes<F_Q4_K>(a, planes, stream); break;
+    case F_Q2_K: e = launch_planes<F_Q2_K>(a, planes, stream); break;
+    case F_Q3_K: case F_Q6_K: e = launch_planes<F_Q6_K>(a, planes, stream); break;
+    case F_IQ2_XXS: e = launch_planes<F_IQ2_XXS>(a, planes, stream); break;
+    default: e = launch_planes<F_TQ1_0>(a, planes, stream); break;
+    }
+    if (e != cudaSuccess) return e;
+    switch (a.fmt) {
+    case F_Q4_0: return launch_tile_kernel<F_Q4_0>(a, planes, sm_count, stream);
+    case F_Q8_0: return launch_tile_kernel<F_Q8_0>(a, planes, sm_count, stream);
+    case F_Q2_K: return launch_tile_kernel<F_Q2_K>(a, planes, sm_count, stream);
+    case F_Q3_K: return launch_tile_kernel<F_Q3_K>(a, planes, sm_count, stream);
+    case F_Q4_K: return launch_tile_kernel<F_Q4_K>(a, planes, sm_count, stream);
+    case F_Q5_K: return launch_tile_kernel<F_Q5_K>(a, planes, sm_count, stream);
+    case F_Q6_K: return launch_tile_kernel<F_Q6_K>(a, planes, sm_count, stream);
+    case F_IQ2_XXS: return launch_tile_kernel<F_IQ2_XXS>(a, planes, sm_count, stream);
+    default: return launch_tile_kernel<F_TQ1_0>(a, planes, sm_count, stream);
+    }
+}
+
+}  // namespace weft

@@ -1,0 +1,782 @@
+// mul_mat for more than one token row: Y[m, n] = vec_dot(W[n], Xq[m]) as int8 tensor-core tiles whose results stay in
+// registers (mma.sync m16n8k32 / m16n8k16), for every format of the path that a batch of tokens is multiplied with.
+// (Same functions as prefill.cu and the decode GEMVs; examples/kernels/mul_mat/*.py of the reference.)
+//
+// What it is for: from 2 tokens up to the sizes the CTA-pair kernels of prefill_pair.cu take.  A weight record carries
+// an integer scale per 16 or 32 elements, so a product can be accumulated on the tensor core over 16 or 32 elements only
+// before the scale has to be applied.  With tensor-memory accumulators that is a round trip per group or two int8 limbs
+// per weight; a register accumulator costs one integer multiply-add per value, which runs beside the next MMA (measured on
+// this device: m16n8k32 int8 at 0.5 per clock and SM alone, 0.49 with four multiply-adds behind each).
+//
+// A warp owns 32 weight rows (two m16 tiles).  Per 256-element block it unpacks the rows' records from shared memory
+// straight into MMA fragments, once, and applies them to every group of eight tokens of the CTA's tile.  The eight warps
+// of a CTA are `wr` row groups times `wk` slices of K (blocks are dealt to the slices in turn; the slices' sums meet in
+// shared memory at the end of a tile): few tokens or few rows leave the chip idle unless K is cut as well.
+//
+// Weights are read once per token tile by 16-byte cp.async into a ring of stages.  Rows of formats whose record is not a
+// multiple of 16 bytes start at any even address: the copy takes the 16-byte window around the record and the reader
+// shifts.  Activations come from planes in fragment order that tile_planes_kernel writes while it quantizes: 2048 bytes
+// of codes per (eight tokens, block) plus the scales and the operand of the min term, so a fragment is one 16-byte
+// shared-memory load for two 32-element groups.
+#pragma once
+
+#include "gemv_units.cuh"
+#include "kernels.h"
+
+#include <algorithm>
+#include <type_traits>
+
+namespace weft {
+
+constexpr int TL_WARPS = 8, TL_THREADS = TL_WARPS * 32;
+constexpr int TL_SMEM = 227 * 1024;
+
+constexpr int tl_gcd(int a, int b) { return b ? tl_gcd(b, a % b) : a; }
+
+// Order of a block's 256 codes inside the fragments.  Lane t of a quad holds, of every 32-element group,
+//   NATURAL: elements 8t .. 8t+7;   SPLIT16: 4t .. 4t+3 and 16+4t .. 16+4t+3 (one MMA of K = 16 per sub-group of 16);
+//   TERNARY: the sixteen four-element words in the order in which TQ1_0 digits come out of a record (tl_ternary_element).
+enum TileOrder { ORDER_NATURAL = 0, ORDER_SPLIT16 = 1, ORDER_TERNARY = 2 };
+
+template <int FMT> struct TileFormat {
+    static constexpr int UNIT = unit_bytes(FMT);
+    static constexpr int GRAIN = tl_gcd(UNIT, 16);               // rows start at a multiple of this
+    static constexpr bool SHIFTED = GRAIN != 16;
+    static constexpr int PIECES = (UNIT + 16 - GRAIN + 15) / 16;  // 16-byte copies per row and block
+    static constexpr int PITCH = PIECES * 16;                     // rows in shared memory, in the order of the copies
+    static constexpr bool SUB16 = FMT == F_Q2_K || FMT == F_Q3_K || FMT == F_Q6_K;     // a scale per 16 elements
+    static constexpr bool PAIR32 = FMT == F_Q4_0 || FMT == F_Q8_0;                     // an f16 scale per 32 on both sides
+    static constexpr int ORDER = FMT == F_TQ1_0 ? ORDER_TERNARY : (SUB16 || PAIR32) ? ORDER_SPLIT16 : ORDER_NATURAL;
+    static constexpr int MINS = (FMT == F_Q4_K || FMT == F_Q5_K) ? 1 : FMT == F_Q2_K ? 2 : 0;   // K = 16 MMAs of the min term
+    // per (eight tokens, block), behind the codes: PAIR32 f32 d[8 groups][8 tokens]; else f32 d[8 tokens], then the min
+    // operands (256 bytes each) or, TQ1_0, i32 -sum of the codes [8 tokens]
+    static constexpr int AUX = PAIR32 ? 256 : 32 + 256 * MINS + (FMT == F_TQ1_0 ? 32 : 0);
+    static constexpr int GROUP = 2048 + AUX;                     // bytes of the plane per (eight tokens, block)
+    static constexpr int TABLES = FMT == F_IQ2_XXS ? (256 + 128) * 128 : 0;   // shared-memory bytes of the striped codebooks
+};
+
+// CTAs per SM: narrow tiles have few independent MMAs per step, so a second CTA hides what one waits for
+constexpr int tl_ctas(int nt, int mt) { return mt == 2 ? 1 : nt == 1 ? 3 : 2; }
+
+struct TileParams {
+    const uint8_t *w;
+    const uint8_t *planes;       // [(m + 7) / 8][nb] groups
+    const int8_t *grid, *signs;  // IQ2_XXS
+    const uint32_t *powers;      // TQ1_0
+    float *y;
+    long long n, ldy, row_bytes, w_bytes;
+    int m, nb;                   // tokens, blocks per row
+    int wk;                      // slices of K (1, 2, 4, 8); 8 / wk row groups
+    int row_tiles, token_tiles, tiles, steps, stages;
+};
+
+// Word i (0..15) of lane t in ORDER_TERNARY: the element of its first code, and the stride to the next three.
+__host__ __device__ constexpr int tl_ternary_element(int i, int t) {
+    return i < 5 ? 32 * i + 8 * t : i < 8 ? 160 + 16 * (i - 5) + 4 * t : i < 13 ? 32 * (i - 8) + 8 * t + 4 : i < 15 ? 160 + 16 * (i - 10) + 4 * t : 240 + t;
+}
+__host__ __device__ constexpr int tl_ternary_stride(int i) { return i < 15 ? 1 : 4; }
+
+// ------------------------------------------------------------------ instructions
+
+__device__ __forceinline__ void mma_k32(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, int c0, int c1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%10,%11,%10,%11};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c0), "r"(c1));
+}
+__device__ __forceinline__ void mma_k32_add(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
+        : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ void mma_k16(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t b) {
+    asm("mma.sync.aligned.m16n8k16.row.col.s32.s8.s8.s32 {%0,%1,%2,%3},{%4,%5},{%6},{%7,%7,%7,%7};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a0), "r"(a1), "r"(b), "r"(0));
+}
+__device__ __forceinline__ void mma_f16_add(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
+        : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// two fp32 operations per instruction, each rounded as the scalar one
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+    return d;
+}
+__device__ __forceinline__ void fma2_into(float &c0, float &c1, float2 a, float2 b) {
+    const float2 d = fma2(a, b, make_float2(c0, c1));
+    c0 = d.x; c1 = d.y;
+}
+// 16 bytes global -> shared, of which `valid` (0..16) exist; the rest reads as zero
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src, int valid) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid) : "memory");
+}
+__device__ __forceinline__ void cp16(uint32_t dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
+
+// ------------------------------------------------------------------ weight rows in shared memory
+
+// Four bytes at an even address: two aligned loads and a shift.
+struct EvenWords {
+    const uint8_t *base;
+    uint32_t shift;
+    __device__ __forceinline__ explicit EvenWords(const uint8_t *p) {
+        const uintptr_t a = reinterpret_cast<uintptr_t>(p);
+        base = p - (a & 2u);
+        shift = (uint32_t)(a & 2u) * 8u;
+    }
+    __device__ __forceinline__ uint32_t at(int offset) const {
+        return __funnelshift_r(*reinterpret_cast<const uint32_t *>(base + offset), *reinterpret_cast<const uint32_t *>(base + offset + 4), shift);
+    }
+};
+// The same where the parity of the address is known (rows on 16-byte boundaries).
+template <bool ODD>
+__device__ __forceinline__ uint32_t word_at(const uint8_t *p) {
+    if (!ODD) return *reinterpret_cast<const uint32_t *>(p);
+    return __byte_perm(*reinterpret_cast<const uint32_t *>(p - 2), *reinterpret_cast<const uint32_t *>(p + 2), 0x5432);
+}
+
+// u - OFFSET in every byte, as int8, for 0 <= u and OFFSET < 64
+template <int OFFSET>
+__device__ __forceinline__ uint32_t bytes_minus(uint32_t u) { return (u + (0x80u - OFFSET) * 0x01010101u) ^ 0x80808080u; }
+
+// g * s for codebook bytes g and sign bytes given as masks (0xff: -1): complement and add one, without carries between bytes
+__device__ __forceinline__ uint32_t signed_bytes(uint32_t g, uint32_t mask) {
+    const uint32_t t = g ^ mask;
+    return ((t & 0x7f7f7f7fu) + (mask & 0x01010101u)) ^ (t & 0x80808080u);
+}
+
+__device__ __forceinline__ float half_at(const uint8_t *p) { return half_bits_to_float(ld_u16(p)); }
+
+// two bytes (0..63) of `v` at bit `shift` as an f16 pair
+__device__ __forceinline__ uint32_t bytes_to_half2(uint32_t v, uint32_t shift) {
+    const uint32_t biased = __byte_perm(v >> shift, 0x64646464u, 0x4140);      // {1024 + m0, 1024 + m1}
+    const __half2 h = __hsub2(*reinterpret_cast<const __half2 *>(&biased), __half2(__ushort_as_half(0x6400), __ushort_as_half(0x6400)));
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+__device__ __forceinline__ uint32_t half2_times_64(uint32_t v) {
+    const __half2 h = __hmul2(*reinterpret_cast<const __half2 *>(&v), __half2(__ushort_as_half(0x5400), __ushort_as_half(0x5400)));
+    return *reinterpret_cast<const uint32_t *>(&h);
+}
+
+// What a warp keeps of its 16 MT rows for half a block (128 elements: four 32-element groups).
+template <int FMT, int MT>
+struct TileHalf {
+    static constexpr int SCALES = TileFormat<FMT>::SUB16 ? 8 : 4;
+    uint32_t a[MT][4][4];                // [m16 tile][group][fragment]: {row r low, row r + 8 low, row r high, row r + 8 high}
+    int sc[MT][2][SCALES];               // [m16 tile][row r / r + 8][group or sub-group]: integer scales
+    float dw[MT][2][4];                  // PAIR32: the f16 scale of every group
+};
+// ... and for the whole block
+template <int FMT, int MT>
+struct TileBlock {
+    float d[MT][2], dmin[MT][2];
+    uint32_t mins[MT][TileFormat<FMT>::MINS ? TileFormat<FMT>::MINS : 1][4];   // A fragments of the min term
+};
+
+// One row's part of half `H` of a block: codes into fragment registers `lo` (elements of the low words) and `hi`.
+// `p` is the record (unit) in shared memory, t the lane's place in its quad, `copy` the lane's codebook copy.
+template <int FMT, int H>
+__device__ __forceinline__ void unpack_half(const uint8_t *p, int t, const uint8_t *s_grid, const uint8_t *s_neg, int copy, bool plain_powers,
+                                            const uint32_t (&powers)[5], uint32_t (&lo)[4], uint32_t (&hi)[4], int (&sc)[TileFormat<FMT>::SUB16 ? 8 : 4], float (&dw)[4]) {
+    if constexpr (FMT == F_Q4_K || FMT == F_Q5_K) {
+        constexpr int QS = FMT == F_Q4_K ? 16 : 48;
+        uint2 fifth = make_uint2(0, 0);
+        if constexpr (FMT == F_Q5_K) fifth = *reinterpret_cast<const uint2 *>(p + 16 + 8 * t);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const uint2 q = *reinterpret_cast<const uint2 *>(p + QS + 32 * (2 * H + j) + 8 * t);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                uint32_t l = (q.x >> (4 * e)) & 0x0f0f0f0fu, h = (q.y >> (4 * e)) & 0x0f0f0f0fu;
+                if constexpr (FMT == F_Q5_K) {
+                    const int g = 4 * H + 2 * j + e;
+                    l |= (g <= 4 ? fifth.x << (4 - g) : fifth.x >> (g - 4)) & 0x10101010u;
+                    h |= (g <= 4 ? fifth.y << (4 - g) : fifth.y >> (g - 4)) & 0x10101010u;
+                }
+                lo[2 * j + e] = l;
+                hi[2 * j + e] = h;
+            }
+        }
+        const uint4 head = *reinterpret_cast<const uint4 *>(p);
+        const uint32_t s = H == 0 ? head.y & 0x3f3f3f3fu : (head.w & 0x0f0f0f0fu) | (((head.y >> 6) & 0x03030303u) << 4);
+#pragma unroll
+        for (int g = 0; g < 4; ++g) sc[g] = (int)byte_of(s, g);
+    } else if constexpr (FMT == F_Q6_K) {
+        const EvenWords w(p);
+        const uint32_t s0 = w.at(192 + 8 * H), s1 = w.at(196 + 8 * H);
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const uint32_t l0 = w.at(64 * H + 16 * s + 4 * t), l1 = w.at(64 * H + 32 + 16 * s + 4 * t), top = w.at(128 + 32 * H + 16 * s + 4 * t);
+            uint32_t (&out)[4] = s ? hi : lo;
+            out[0] = bytes_minus<32>((l0 & 0x0f0f0f0fu) | ((top << 4) & 0x30303030u));
+            out[1] = bytes_minus<32>((l1 & 0x0f0f0f0fu) | ((top << 2) & 0x30303030u));
+            out[2] = bytes_minus<32>(((l0 >> 4) & 0x0f0f0f0fu) | (top & 0x30303030u));
+            out[3] = bytes_minus<32>(((l1 >> 4) & 0x0f0f0f0fu) | ((top >> 2) & 0x30303030u));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sc[i] = (int)(int8_t)((i < 4 ? s0 : s1) >> (8 * (i & 3)));
+    } else if constexpr (FMT == F_Q3_K) {
+        const EvenWords w(p);
+        uint32_t packed[4];
+        q3k_unpack_scales(w.at(96), w.at(100), w.at(104), packed);
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const uint32_t q = w.at(32 + 32 * H + 16 * s + 4 * t), mask = w.at(16 * s + 4 * t);
+            uint32_t (&out)[4] = s ? hi : lo;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const int bit = 4 * H + g;
+                out[g] = bytes_minus<4>(((q >> (2 * g)) & 0x03030303u) | ((bit <= 2 ? mask << (2 - bit) : mask >> (bit - 2)) & 0x04040404u));
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sc[i] = (int)byte_of(packed[2 * H + (i >> 2)], i & 3) - 32;
+    } else if constexpr (FMT == F_Q2_K) {
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(p);       // 84-byte records: rows start on 4-byte boundaries
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const uint32_t q = w[4 + 8 * H + 4 * s + t];
+            uint32_t (&out)[4] = s ? hi : lo;
+#pragma unroll
+            for (int g = 0; g < 4; ++g) out[g] = (q >> (2 * g)) & 0x03030303u;
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) sc[i] = (int)(byte_of(w[2 * H + (i >> 2)], i & 3) & 15u);
+    } else if constexpr (FMT == F_Q4_0) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const uint8_t *r = p + 18 * (4 * H + g);
+            const uint32_t q = g & 1 ? word_at<false>(r + 2 + 4 * t) : word_at<true>(r + 2 + 4 * t);
+            lo[g] = bytes_minus<8>(q & 0x0f0f0f0fu);
+            hi[g] = bytes_minus<8>((q >> 4) & 0x0f0f0f0fu);
+            dw[g] = half_at(r);
+        }
+    } else if constexpr (FMT == F_Q8_0) {
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const uint8_t *r = p + 34 * (4 * H + g);
+            lo[g] = g & 1 ? word_at<false>(r + 2 + 4 * t) : word_at<true>(r + 2 + 4 * t);
+            hi[g] = g & 1 ? word_at<false>(r + 18 + 4 * t) : word_at<true>(r + 18 + 4 * t);
+            dw[g] = half_at(r);
+        }
+    } else if constexpr (FMT == F_IQ2_XXS) {
+        const EvenWords w(p + 2);
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const uint32_t index = w.at(8 * (4 * H + g)), meta = w.at(8 * (4 * H + g) + 4);
+            const uint2 grid = *reinterpret_cast<const uint2 *>(s_grid + ((index >> (8 * t)) & 255u) * 128 + 8 * copy);
+            const uint2 neg = *reinterpret_cast<const uint2 *>(s_neg + ((meta >> (7 * t)) & 127u) * 128 + 8 * copy);
+            lo[g] = signed_bytes(grid.x, neg.x);
+            hi[g] = signed_bytes(grid.y, neg.y);
+            sc[g] = (int)(2u * (meta >> 28) + 1u);
+        }
+    } else if constexpr (FMT == F_TQ1_0) {
+        // words of digits in ORDER_TERNARY.  Half 0: the five digits of record bytes 8t..8t+3, digits 0..2 of bytes 32+4t..+3;
+        // half 1: the five of bytes 8t+4..8t+7, digits 3, 4 of bytes 32+4t..+3, the four of byte 48 + t
+        const EvenWords w(p);
+        constexpr uint32_t M = 0x00ff00ffu;
+        uint32_t out[8];
+        const uint32_t five = w.at(8 * t + 4 * H), rest = w.at(32 + 4 * t);
+        uint32_t e = five & M, o = (five >> 8) & M;
+#pragma unroll
+        for (int n = 0; n < 5; ++n) {
+            if (!plain_powers) { e = ((five & M) * powers[n]) & M; o = (((five >> 8) & M) * powers[n]) & M; }
+            const uint32_t te = e * 3u, to = o * 3u;
+            out[n] = __byte_perm(te, to, 0x7351);
+            if (plain_powers) { e = te & M; o = to & M; }
+        }
+        e = rest & M; o = (rest >> 8) & M;
+        if (H == 1) { e = (e * powers[3]) & M; o = (o * powers[3]) & M; }
+#pragma unroll
+        for (int n = 0; n < 3 - H; ++n) {
+            if (!plain_powers) { e = ((rest & M) * powers[3 * H + n]) & M; o = (((rest >> 8) & M) * powers[3 * H + n]) & M; }
+            const uint32_t te = e * 3u, to = o * 3u;
+            out[5 + n] = __byte_perm(te, to, 0x7351);
+            if (plain_powers) { e = te & M; o = to & M; }
+        }
+        if (H == 1) {
+            const uint32_t q = p[48 + t];
+            uint32_t digits = 0;
+#pragma unroll
+            for (int n = 0; n < 4; ++n) digits |= ((((q * powers[n]) & 255u) * 3u) >> 8) << (8 * n);
+            out[7] = digits;
+        }
+#pragma unroll
+        for (int g = 0; g < 4; ++g) { lo[g] = out[2 * g]; hi[g] = out[2 * g + 1]; }
+    }
+    (void)sc; (void)dw;
+}
+
+// The f16 scale(s) of a row's record, and its part of the min term's A fragments ({m | 64 m} over K = 16).
+template <int FMT>
+__device__ __forceinline__ void unpack_block(const uint8_t *p, int t, float &d, float &dmin, uint32_t (&low)[TileFormat<FMT>::MINS ? TileFormat<FMT>::MINS : 1],
+                                             uint32_t (&high)[TileFormat<FMT>::MINS ? TileFormat<FMT>::MINS : 1]) {
+    if constexpr (FMT == F_Q4_K || FMT == F_Q5_K) {
+        const uint4 head = *reinterpret_cast<const uint4 *>(p);
+        d = half_bits_to_float(head.x);
+        dmin = half_bits_to_float(head.x >> 16);
+        const uint32_t m = t < 2 ? head.z & 0x3f3f3f3fu : ((head.w >> 4) & 0x0f0f0f0fu) | (((head.z >> 6) & 0x03030303u) << 4);
+        low[0] = bytes_to_half2(m, 16 * (t & 1));
+        high[0] = half2_times_64(low[0]);
+    } else if constexpr (FMT == F_Q2_K) {
+        const uint32_t *w = reinterpret_cast<const uint32_t *>(p);
+        d = half_bits_to_float(w[20]);
+        dmin = half_bits_to_float(w[20] >> 16);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            low[q] = bytes_to_half2((w[2 * q + (t >> 1)] >> 4) & 0x0f0f0f0fu, 16 * (t & 1));
+            high[q] = half2_times_64(low[q]);
+        }
+    } else if constexpr (FMT == F_Q6_K) d = half_at(p + 208);
+    else if constexpr (FMT == F_Q3_K) d = half_at(p + 108);
+    else if constexpr (FMT == F_IQ2_XXS) d = 0.125f * half_at(p);     // the factor 1/8 of the format, a power of two
+    else if constexpr (FMT == F_TQ1_0) d = half_at(p + 52);
+    (void)dmin; (void)low; (void)high;
+}
+
+// ------------------------------------------------------------------ the kernel
+
+// Where tile number `index` lies: token tiles of the same rows follow each other, so that CTAs running at the same time
+// read the same weights.
+struct TilePlace { long long row0; int group0, live; };
+
+template <int NT>
+__device__ __forceinline__ TilePlace tile_place(const TileParams &p, int index, int tile_rows) {
+    TilePlace r;
+    const int row_tile = index / p.token_tiles, token_tile = index - row_tile * p.token_tiles;
+    r.row0 = (long long)row_tile * tile_rows;
+    r.group0 = token_tile * NT;
+    r.live = min(NT, (p.m + 7) / 8 - r.group0);
+    return r;
+}
+
+// One half of a block for every token group of the tile.  `stage` is the (eight tokens, block) groups in shared memory.
+template <int FMT, int NT, int MT, int H>
+__device__ __forceinline__ void tile_half(const uint8_t *stage, int lane, const TileHalf<FMT, MT> &wt, const TileBlock<FMT, MT> &blk, float (&acc)[NT][MT][4]) {
+    using F = TileFormat<FMT>;
+    constexpr int MAGIC = 0x4b400000;                        // 1.5 * 2^23 as bits: integer accumulators that start here are floats
+    const int t = lane & 3;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt) {
+        const uint8_t *group = stage + nt * F::GROUP;
+        const uint4 q0 = *reinterpret_cast<const uint4 *>(group + 1024 * H + 16 * lane), q1 = *reinterpret_cast<const uint4 *>(group + 1024 * H + 512 + 16 * lane);
+        const uint32_t b[4][2] = {{q0.x, q0.y}, {q0.z, q0.w}, {q1.x, q1.y}, {q1.z, q1.w}};
+        if constexpr (F::PAIR32) {
+            // acc += (isum * d_w) * d_x per group.  isum * d_w is one fused multiply-add on the biased accumulator: the product
+            // bias * d_w has 13 significant bits, so the sum is isum * d_w rounded once
+#pragma unroll
+            for (int g = 0; g < 4; ++g) {
+                const float2 dx = *reinterpret_cast<const float2 *>(group + 2048 + 32 * (4 * H + g) + 8 * t);
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) {
+                    int d[4];
+                    mma_k32(d, wt.a[mt][g], b[g][0], b[g][1], MAGIC, MAGIC);
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        const float dw = wt.dw[mt][e][g], back = -12582912.0f * dw;
+                        const float2 v = fma2(make_float2(__int_as_float(d[2 * e]), __int_as_float(d[2 * e + 1])), make_float2(dw, dw), make_float2(back, back));
+                        fma2_into(acc[nt][mt][2 * e], acc[nt][mt][2 * e + 1], v, dx);
+                    }
+                }
+            }
+        } else {
+            const float2 xd = *reinterpret_cast<const float2 *>(group + 2048 + 8 * t);
+            int2 bias = make_int2(0, 0);
+            if constexpr (FMT == F_TQ1_0)
+                if (H == 0) bias = *reinterpret_cast<const int2 *>(group + 2048 + 32 + 8 * t);
+            float msum[MT][4] = {};
+            if constexpr (F::MINS > 0 && H == 1) {
+#pragma unroll
+                for (int q = 0; q < F::MINS; ++q) {
+                    const uint2 m = *reinterpret_cast<const uint2 *>(group + 2048 + 32 + 256 * q + 8 * lane);
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt) mma_f16_add(msum[mt], blk.mins[mt][q], m.x, m.y);
+                }
+            }
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt) {
+                int isum[4] = {0, 0, 0, 0};
+                if constexpr (FMT == F_TQ1_0) {              // one scale per block: the groups accumulate on the tensor core
+                    mma_k32(isum, wt.a[mt][0], b[0][0], b[0][1], bias.x, bias.y);
+#pragma unroll
+                    for (int g = 1; g < 4; ++g) mma_k32_add(isum, wt.a[mt][g], b[g][0], b[g][1]);
+                } else {
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        int d[4];
+                        if constexpr (F::SUB16) {
+#pragma unroll
+                            for (int s = 0; s < 2; ++s) {
+                                mma_k16(d, wt.a[mt][g][2 * s], wt.a[mt][g][2 * s + 1], b[g][s]);
+#pragma unroll
+                                for (int c = 0; c < 4; ++c) isum[c] += wt.sc[mt][c >> 1][2 * g + s] * d[c];
+                            }
+                        } else {
+                            mma_k32(d, wt.a[mt][g], b[g][0], b[g][1], 0, 0);
+#pragma unroll
+                            for (int c = 0; c < 4; ++c) isum[c] += wt.sc[mt][c >> 1][g] * d[c];
+                        }
+                    }
+                }
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {                 // rows r and r + 8, the lane's two tokens side by side
+                    float2 v = mul2(make_float2((float)isum[2 * e], (float)isum[2 * e + 1]), make_float2(blk.d[mt][e], blk.d[mt][e]));
+                    if constexpr (F::MINS > 0 && H == 1)
+                        v = fma2(make_float2(msum[mt][2 * e], msum[mt][2 * e + 1]), make_float2(-blk.dmin[mt][e], -blk.dmin[mt][e]), v);
+                    fma2_into(acc[nt][mt][2 * e], acc[nt][mt][2 * e + 1], xd, v);
+                }
+            }
+        }
+    }
+}
+
+template <int FMT, int NT, int MT>
+__global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const TileParams p) {
+    using F = TileFormat<FMT>;
+    constexpr int TL_ROWS = 16 * MT;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, t = lane & 3;
+    const int wk = p.wk, wr = TL_WARPS / wk, slice = warp / wr, row_group = warp - slice * wr;
+    const int tile_rows = wr * TL_ROWS;
+    uint8_t *s_tables = smem;
+    uint8_t *ring = smem + F::TABLES;
+    // With one token group every warp keeps its own copy of the slice's group behind its rows and never meets the others
+    // before the end of a tile: the step's barrier was a fifth of the time at eight tokens, the second copy comes from L2.
+    constexpr bool PRIVATE = NT == 1;
+    constexpr int OWN = TL_ROWS * F::PITCH + F::GROUP;         // PRIVATE: bytes of a stage per warp
+    const int w_stage = TL_WARPS * TL_ROWS * F::PITCH, stage_bytes = PRIVATE ? TL_WARPS * OWN : w_stage + wk * NT * F::GROUP;
+    const int own_rows = warp * (PRIVATE ? OWN : TL_ROWS * F::PITCH);
+    uint8_t *s_sums = ring + (size_t)p.stages * stage_bytes;   // only with wk > 1
+
+    asm volatile("griddepcontrol.launch_dependents;");
+
+    // ---- copies of one step of a tile.  A warp brings its own 32 rows: piece i * 32 + lane of them, in the order in which they
+    // lie in shared memory, so that the destination is an immediate offset
+    constexpr int COPIES = (TL_ROWS * F::PIECES + 31) / 32;
+    uint32_t offsets[F::SHIFTED ? 1 : COPIES];               // of the lane's pieces from the warp's first row
+    const uint8_t *w_first = nullptr;                         // the warp's first row of the tile being filled
+    uint32_t w_skew = 0;                                      // SHIFTED: that row's offset from a 16-byte boundary
+    int w_last = 0;                                           // index of the last row the warp may read
+    const uint32_t row_bytes = (uint32_t)p.row_bytes;
+    auto enter_tile = [&](const TilePlace &place) {
+        long long first = place.row0 + row_group * TL_ROWS;
+        if (first >= p.n) first = p.n - 1;                    // a warp beyond the last row copies and computes that row
+        w_last = (int)min((long long)TL_ROWS - 1, p.n - 1 - first);
+        const long long start = first * p.row_bytes;
+        w_skew = F::SHIFTED ? (uint32_t)start & 15u : 0u;
+        w_first = p.w + (start - w_skew);
+        if (!F::SHIFTED)
+#pragma unroll
+            for (int i = 0; i < COPIES; ++i) {
+                const int piece = i * 32 + lane, row = piece / F::PIECES;
+                offsets[i] = (uint32_t)min(row, w_last) * row_bytes + 16u * (uint32_t)(piece - row * F::PIECES);
+            }
+    };
+    auto copy_weights = [&](int step, uint8_t *stage) {
+        const int block = step * wk + slice;
+        if (block >= p.nb) return;
+        const uint32_t dst = smem_addr(stage + own_rows) + 16 * lane;
+        if constexpr (!F::SHIFTED) {
+            const uint8_t *src = w_first + (uint32_t)block * (uint32_t)F::UNIT;
+#pragma unroll
+            for (int i = 0; i < COPIES; ++i)
+                if ((i + 1) * 32 <= TL_ROWS * F::PIECES || i * 32 + lane < TL_ROWS * F::PIECES) cp16(dst + 512 * i, src + offsets[i]);
+        } else {
+            const long long left = p.w_bytes - (w_first - p.w);          // bytes of the matrix from w_first on
+            const bool ends = left < (long long)(w_last + 1) * row_bytes + 32;   // the matrix may end inside a 16-byte window
+            int row = lane / F::PIECES, piece = lane - row * F::PIECES;
+            const uint32_t base = w_skew + (uint32_t)block * (uint32_t)F::UNIT;
+#pragma unroll
+            for (int i = 0; i < COPIES; ++i) {
+                if ((i + 1) * 32 > TL_ROWS * F::PIECES && i * 32 + lane >= TL_ROWS * F::PIECES) break;
+                const uint32_t at = ((base + (uint32_t)min(row, w_last) * row_bytes) & ~15u) + 16u * piece;
+                if (!ends) cp16(dst + 512 * i, w_first + at);
+                else cp16(dst + 512 * i, w_first + ((long long)at < left ? at : 0u), (int)max(0LL, min(16LL, left - at)));
+                row += 32 / F::PIECES;
+                piece += 32 % F::PIECES;
+                if (piece >= F::PIECES) { piece -= F::PIECES; ++row; }
+            }
+        }
+    };
+    auto copy_tokens = [&](const TilePlace &place, int step, uint8_t *stage) {
+        constexpr int PIECES = F::GROUP / 16;
+        if constexpr (PRIVATE) {
+            const int block = step * wk + slice;
+            if (block >= p.nb) return;
+            const uint32_t dst = smem_addr(stage + own_rows + TL_ROWS * F::PITCH) + 16 * lane;
+            const uint8_t *src = p.planes + ((long long)place.group0 * p.nb + block) * F::GROUP + 16 * lane;
+#pragma unroll
+            for (int i = 0; i < (PIECES + 31) / 32; ++i)
+                if ((i + 1) * 32 <= PIECES || i * 32 + lane < PIECES) cp16(dst + 512 * i, src + 512 * i);
+        } else {
+        for (int unit = warp; unit < wk * place.live; unit += TL_WARPS) {        // (slice, token group): GROUP contiguous bytes
+            const int kg = unit / place.live, nt = unit - kg * place.live, block = step * wk + kg;
+            if (block >= p.nb) break;
+            const uint32_t dst = smem_addr(stage + w_stage + (kg * NT + nt) * F::GROUP) + 16 * lane;
+            const uint8_t *src = p.planes + ((long long)(place.group0 + nt) * p.nb + block) * F::GROUP + 16 * lane;
+#pragma unroll
+            for (int i = 0; i < (PIECES + 31) / 32; ++i)
+                if ((i + 1) * 32 <= PIECES || i * 32 + lane < PIECES) cp16(dst + 512 * i, src + 512 * i);
+        }
+        }
+    };
+
+    // ---- fill the ring: weights first, they do not depend on the kernel that makes the planes
+    int fill_tile = blockIdx.x, fill_step = 0;
+    const int ahead = p.stages - 1;
+    {
+        int tile = fill_tile, step = 0;
+        enter_tile(tile_place<NT>(p, tile, tile_rows));
+        for (int s = 0; s < ahead && tile < p.tiles; ++s) {
+            copy_weights(step, ring + (size_t)s * stage_bytes);
+            if (++step == p.steps) { step = 0; tile += gridDim.x; if (tile < p.tiles) enter_tile(tile_place<NT>(p, tile, tile_rows)); }
+        }
+    }
+    uint32_t powers[5] = {1, 3, 9, 27, 81};
+    bool plain_powers = true;
+    if constexpr (FMT == F_TQ1_0) {
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const uint32_t v = p.powers[i] & 255u;
+            plain_powers &= v == powers[i];
+            powers[i] = v;
+        }
+    }
+    if constexpr (FMT == F_IQ2_XXS) {
+        stage_iq2_tables_striped(p.grid, p.signs, s_tables, s_tables + 256 * 128);
+        __syncthreads();
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    TilePlace fill_place = tile_place<NT>(p, fill_tile, tile_rows);
+    for (int s = 0; s < ahead; ++s) {
+        if (fill_tile < p.tiles) {
+            copy_tokens(fill_place, fill_step, ring + (size_t)s * stage_bytes);
+            if (++fill_step == p.steps) { fill_step = 0; fill_tile += gridDim.x; if (fill_tile < p.tiles) fill_place = tile_place<NT>(p, fill_tile, tile_rows); }
+        }
+        cp_commit();
+    }
+
+    float acc[NT][MT][4];
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[nt][mt][c] = 0.0f;
+
+    int slot = 0, fill_slot = ahead;
+    for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
+        const TilePlace place = tile_place<NT>(p, tile, tile_rows);
+        uint32_t skew[MT][2];                                   // SHIFTED: low bits of the rows' byte offsets
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                const long long n = place.row0 + row_group * TL_ROWS + 16 * mt + 8 * e + r;
+                skew[mt][e] = (uint32_t)(n >= p.n ? p.n - 1 : n) * row_bytes;
+            }
+        for (int step = 0; step < p.steps; ++step) {
+            if (p.stages == 2) cp_wait<0>(); else if (p.stages == 3) cp_wait<1>(); else if (p.stages == 4) cp_wait<2>(); else cp_wait<4>();
+            if constexpr (PRIVATE) __syncwarp(); else __syncthreads();   // this step has landed for all its readers; the oldest slot is free
+            if (fill_tile < p.tiles) {
+                uint8_t *stage = ring + (size_t)fill_slot * stage_bytes;
+                copy_weights(fill_step, stage);
+                copy_tokens(fill_place, fill_step, stage);
+                if (++fill_step == p.steps) {
+                    fill_step = 0;
+                    fill_tile += gridDim.x;
+                    if (fill_tile < p.tiles) { fill_place = tile_place<NT>(p, fill_tile, tile_rows); enter_tile(fill_place); }
+                }
+            }
+            cp_commit();
+            if (++fill_slot == p.stages) fill_slot = 0;
+            const uint8_t *stage = ring + (size_t)slot * stage_bytes;
+            if (++slot == p.stages) slot = 0;
+            const int block = step * wk + slice;
+            if (block >= p.nb) continue;
+            const uint8_t *tokens = PRIVATE ? stage + own_rows + TL_ROWS * F::PITCH : stage + w_stage + slice * NT * F::GROUP;
+            const uint8_t *rows[MT][2];
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    rows[mt][e] = stage + own_rows + (16 * mt + 8 * e + r) * F::PITCH;
+                    if (F::SHIFTED) rows[mt][e] += (skew[mt][e] + (uint32_t)block * (uint32_t)F::UNIT) & 15u;
+                }
+            TileBlock<FMT, MT> blk;
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    constexpr int Q = F::MINS ? F::MINS : 1;
+                    uint32_t low[Q] = {}, high[Q] = {};
+                    if constexpr (!F::PAIR32) unpack_block<FMT>(rows[mt][e], t, blk.d[mt][e], blk.dmin[mt][e], low, high);
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) { blk.mins[mt][q][e] = low[q]; blk.mins[mt][q][2 + e] = high[q]; }
+                }
+            auto half = [&](auto h) {
+                constexpr int H = decltype(h)::value;
+                TileHalf<FMT, MT> wt;
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                    for (int e = 0; e < 2; ++e) {
+                        uint32_t lo[4], hi[4];
+                        unpack_half<FMT, H>(rows[mt][e], t, s_tables, s_tables + 256 * 128, lane & 15, plain_powers, powers, lo, hi, wt.sc[mt][e], wt.dw[mt][e]);
+#pragma unroll
+                        for (int g = 0; g < 4; ++g) { wt.a[mt][g][e] = lo[g]; wt.a[mt][g][2 + e] = hi[g]; }
+                    }
+                tile_half<FMT, NT, MT, H>(tokens, lane, wt, blk, acc);
+            };
+            half(std::integral_constant<int, 0>{});
+            half(std::integral_constant<int, 1>{});
+        }
+
+        // ---- the slices' sums meet in shared memory, two token groups at a time: [slice][token][row]
+        if (wk > 1) {
+            constexpr int AT_ONCE = NT > 1 ? 2 : 1;
+            const int pitch = tile_rows + 4;                   // the four quads of a row of lanes store to different banks
+            float *sums = reinterpret_cast<float *>(s_sums);
+#pragma unroll
+            for (int nt0 = 0; nt0 < NT; nt0 += AT_ONCE) {
+#pragma unroll
+                for (int i = 0; i < AT_ONCE; ++i)
+                    if (nt0 + i < NT)
+#pragma unroll
+                        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                            for (int c = 0; c < 4; ++c)
+                                sums[((slice * AT_ONCE + i) * 8 + 2 * t + (c & 1)) * pitch + row_group * TL_ROWS + 16 * mt + 8 * (c >> 1) + r] = acc[nt0 + i][mt][c];
+                __syncthreads();
+                for (int i = tid; i < AT_ONCE * 8 * tile_rows; i += TL_THREADS) {
+                    const int token_in = i / tile_rows, row = i - token_in * tile_rows, token = (place.group0 + nt0) * 8 + token_in;
+                    const long long n = place.row0 + row;
+                    if (token >= p.m || n >= p.n || nt0 * 8 + token_in >= NT * 8) continue;
+                    float total = 0.0f;
+                    for (int k = 0; k < wk; ++k) total += sums[(k * AT_ONCE * 8 + token_in) * pitch + row];
+                    p.y[(long long)token * p.ldy + n] = total;
+                }
+                __syncthreads();
+            }
+        } else
+        {
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const int token = (place.group0 + nt) * 8 + 2 * t + c;
+                    if (token >= p.m) continue;
+                    float *y = p.y + (long long)token * p.ldy;
+#pragma unroll
+                    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const long long n = place.row0 + row_group * TL_ROWS + 16 * mt + 8 * e + r;
+                            if (n < p.n) y[n] = acc[nt][mt][2 * e + c];
+                        }
+                }
+            }
+        }
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[nt][mt][c] = 0.0f;
+    }
+    cp_wait<0>();
+}
+
+// ------------------------------------------------------------------ launch
+
+// How a launch is cut: token groups per tile, slices of K per CTA, ring stages.
+struct TilePlan { int nt, mt, wk, stages; double cost; };
+
+constexpr int tl_sum_bytes(int nt, int mt, int wk) { return wk > 1 ? wk * (nt > 1 ? 16 : 8) * (TL_WARPS / wk * 16 * mt + 4) * 4 : 0; }
+template <int FMT> constexpr int tl_stage_bytes(int nt, int mt, int wk) { return TL_WARPS * 16 * mt * TileFormat<FMT>::PITCH + (nt == 1 ? TL_WARPS : wk * nt) * TileFormat<FMT>::GROUP; }
+
+template <int FMT, int NT, int MT>
+cudaError_t launch_tile_plan(const TileArgs &a, const uint8_t *planes, const TilePlan &plan, int sm_count, cudaStream_t stream) {
+    using F = TileFormat<FMT>;
+    TileParams p{};
+    p.w = static_cast<const uint8_t *>(a.w);
+    p.planes = planes;
+    p.grid = a.grid; p.signs = a.signs; p.powers = a.powers;
+    p.y = a.y;
+    p.n = a.n; p.ldy = a.ldy;
+    p.nb = (int)(a.k / 256);
+    p.row_bytes = (long long)p.nb * F::UNIT;
+    p.w_bytes = p.row_bytes * a.n;
+    p.m = (int)a.m;
+    p.wk = plan.wk;
+    p.stages = plan.stages;
+    const int tile_rows = TL_WARPS / plan.wk * 16 * MT;
+    p.row_tiles = (int)((a.n + tile_rows - 1) / tile_rows);
+    p.token_tiles = (int)(((a.m + 7) / 8 + NT - 1) / NT);
+    p.tiles = p.row_tiles * p.token_tiles;
+    p.steps = (p.nb + plan.wk - 1) / plan.wk;
+    const int smem = F::TABLES + plan.stages * tl_stage_bytes<FMT>(NT, MT, plan.wk) + tl_sum_bytes(NT, MT, plan.wk);
+    cudaError_t e = grant_dynamic_smem(reinterpret_cast<const void *>(tile_kernel<FMT, NT, MT>), smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)std::min(p.tiles, sm_count * std::max(1, std::min(tl_ctas(NT, MT), 228 * 1024 / (smem + 1024)))));
+    cfg.blockDim = dim3(TL_THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, tile_kernel<FMT, NT, MT>, p);
+}
+
+// Picks the cut with the least estimated time.  A step of a CTA that has an SM to itself takes about 1.1 + 0.3 nt
+// microseconds (32 rows per warp), a pair of CTAs with 16 rows per warp together 0.9 + 0.29 nt, three with one token group
+// 2.0 (fitted to Q4_K, 8 to 512 tokens; twice the MMAs per group with a scale per 16 elements); the slices' sums cost a
+// little per tile.  What decides is how full the last round of the grid is and how long K is kept in one piece.
+template <int FMT>
+TilePlan tile_plan(const TileArgs &a, int sm_count) {
+    using F = TileFormat<FMT>;
+    const long long groups = (a.m + 7) / 8, nb = a.k / 256;
+    const double base = F::SUB16 ? 1.6 : 1.0, slope = F::SUB16 ? 1.7 : 1.0;
+    TilePlan best{0, 0, 0, 0, 0.0};
+    for (int mt = 1; mt <= 2; ++mt)
+        for (int nt = 1; nt <= 8 && nt <= groups; ++nt)
+            for (int wk : {1, 2, 4, 8}) {
+                const int stage = tl_stage_bytes<FMT>(nt, mt, wk), fixed = F::TABLES + tl_sum_bytes(nt, mt, wk);
+                int ctas = tl_ctas(nt, mt), stages = 0;
+                for (; ctas > 0 && stages < 2; --ctas) stages = (TL_SMEM / ctas - 1024 - fixed) / stage;
+                ++ctas;
+                stages = stages >= 6 ? 6 : stages >= 4 ? 4 : stages;
+                if (stages < 2 || (wk > nb && wk > 1)) continue;
+                const int tile_rows = TL_WARPS / wk * 16 * mt;
+                const long long tiles = ((a.n + tile_rows - 1) / tile_rows) * ((groups + nt - 1) / nt), steps = (nb + wk - 1) / wk;
+                const double step = mt == 2 ? (F::PAIR32 ? 1.4 : 1.1) * base + 0.3 * slope * nt : ctas == 3 ? 2.0 * base : 0.9 * base + 0.29 * slope * nt;
+                const double rounds = std::max(0.7, (double)((tiles + sm_count - 1) / sm_count) / ctas);
+                const double cost = (mt == 2 ? std::max(1.0, rounds) : rounds) * ((double)steps * step + 0.5 + (wk > 1 ? 0.2 * nt : 0.0));
+                if (!best.nt || cost < best.cost) best = TilePlan{nt, mt, wk, stages, cost};
+            }
+    return best;
+}
+
+template <int FMT>
+cudaError_t launch_tile_kernel(const TileArgs &a, const uint8_t *planes, int sm_count, cudaStream_t stream) {
+    const TilePlan plan = tile_plan<FMT>(a, sm_count);
+#define TL_CASE(NT, MT) case (NT) * 4 + (MT): return launch_tile_plan<FMT, NT, MT>(a, planes, plan, sm_count, stream)
+    switch (plan.nt * 4 + plan.mt) {
+    TL_CASE(1, 1); TL_CASE(2, 1); TL_CASE(3, 1); TL_CASE(4, 1); TL_CASE(5, 1); TL_CASE(6, 1); TL_CASE(7, 1); TL_CASE(8, 1);
+    TL_CASE(1, 2); TL_CASE(2, 2); TL_CASE(3, 2); TL_CASE(4, 2); TL_CASE(5, 2); TL_CASE(6, 2); TL_CASE(7, 2); TL_CASE(8, 2);
+    default: return cudaErrorNotSupported;
+    }
+#undef TL_CASE
+}
+
+}  // namespace weft

@@ -1,0 +1,136 @@
+// Device memory that a call needs between its own kernels (the activation planes of the batch kernels).
+//
+// Outside a capture every stream has one buffer, which grows: the calls of a stream follow each other, so the next call's
+// first kernel starts after the previous call's last one has read it.  A handful of streams is remembered; a further one
+// takes the place of the longest unused, whose work is waited for first.
+//
+// A captured call may be replayed at any time and on any stream, so a capture gets memory of its own: one buffer per
+// captured graph and size, tied to the graph by a user object.  When the graph and everything instantiated from it are
+// gone the buffer goes to a free list that the next capture or the next growing stream takes from.
+//
+// Callers hold the library's lock.
+#include "kernels.h"
+
+#include <mutex>
+#include <vector>
+
+namespace weft {
+
+namespace {
+
+struct Buffer { uint8_t *base; size_t bytes; int device; };
+struct StreamBuffer { cudaStream_t stream; int device; Buffer buffer; unsigned long long used; };
+struct CaptureBuffer { unsigned long long id; Buffer buffer; };
+
+constexpr size_t kStreams = 8, kFree = 8;
+std::vector<StreamBuffer> g_streams;
+std::vector<CaptureBuffer> g_captures;      // of the captures still being recorded, newest last
+unsigned long long g_clock = 0, g_generation = 0;
+
+std::mutex g_returned_lock;                 // the user object's callback runs on a thread of the driver's
+std::vector<Buffer> g_returned;
+
+void give_back(void *p) {                   // no CUDA calls are allowed here
+    Buffer *b = static_cast<Buffer *>(p);
+    std::lock_guard<std::mutex> guard(g_returned_lock);
+    g_returned.push_back(*b);
+    delete b;
+}
+
+// A buffer of at least `bytes`: a returned one that fits without being four times too large, or a new allocation.
+cudaError_t obtain(size_t bytes, int device, Buffer *out) {
+    {
+        std::lock_guard<std::mutex> guard(g_returned_lock);
+        for (size_t i = 0; i < g_returned.size(); ++i)
+            if (g_returned[i].device == device && g_returned[i].bytes >= bytes && g_returned[i].bytes / 4 <= bytes) {
+                *out = g_returned[i];
+                g_returned.erase(g_returned.begin() + i);
+                return cudaSuccess;
+            }
+    }
+    const size_t want = (bytes + bytes / 4 + 65535) & ~size_t(65535);
+    // an allocation is legal while this thread captures, in the relaxed mode
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    uint8_t *base = nullptr;
+    const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&base), want);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return e;
+    *out = Buffer{base, want, device};
+    return cudaSuccess;
+}
+
+void drop_surplus() {                       // outside a capture: keep a few returned buffers, free the rest
+    std::vector<Buffer> surplus;
+    {
+        std::lock_guard<std::mutex> guard(g_returned_lock);
+        while (g_returned.size() > kFree) { surplus.push_back(g_returned.front()); g_returned.erase(g_returned.begin()); }
+    }
+    for (const Buffer &b : surplus) cudaFree(b.base);
+}
+
+}  // namespace
+
+unsigned long long workspace_generation() { return g_generation; }
+
+cudaError_t workspace(size_t bytes, cudaStream_t stream, uint8_t **out) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return e;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    e = cudaStreamGetCaptureInfo(stream, &status, &id, &graph);
+    if (e != cudaSuccess) return e;
+    if (status == cudaStreamCaptureStatusActive) {
+        for (const CaptureBuffer &c : g_captures)
+            if (c.id == id && c.buffer.bytes >= bytes) { *out = c.buffer.base; return cudaSuccess; }
+        Buffer b;
+        e = obtain(bytes, device, &b);
+        if (e != cudaSuccess) return e;
+        cudaUserObject_t object;
+        Buffer *owned = new Buffer(b);
+        e = cudaUserObjectCreate(&object, owned, give_back, 1, cudaUserObjectNoDestructorSync);
+        if (e != cudaSuccess) { give_back(owned); return e; }
+        e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
+        if (e != cudaSuccess) { cudaUserObjectRelease(object, 1); return e; }
+        if (g_captures.size() >= kStreams) g_captures.erase(g_captures.begin());
+        g_captures.push_back(CaptureBuffer{id, b});
+        *out = b.base;
+        return cudaSuccess;
+    }
+    drop_surplus();
+    StreamBuffer *mine = nullptr;
+    for (StreamBuffer &s : g_streams)
+        if (s.stream == stream && s.device == device) mine = &s;
+    if (!mine) {
+        if (g_streams.size() >= kStreams) {
+            size_t oldest = 0;
+            for (size_t i = 1; i < g_streams.size(); ++i)
+                if (g_streams[i].used < g_streams[oldest].used) oldest = i;
+            e = cudaDeviceSynchronize();    // its stream may be gone by now; what it left behind is not
+            if (e != cudaSuccess) return e;
+            cudaFree(g_streams[oldest].buffer.base);
+            g_streams.erase(g_streams.begin() + oldest);
+            ++g_generation;
+        }
+        g_streams.push_back(StreamBuffer{stream, device, Buffer{nullptr, 0, device}, 0});
+        mine = &g_streams.back();
+    }
+    mine->used = ++g_clock;
+    if (mine->buffer.bytes < bytes) {
+        if (mine->buffer.base) {            // the stream's earlier work may still read the old one
+            e = cudaStreamSynchronize(stream);
+            if (e != cudaSuccess) return e;
+            cudaFree(mine->buffer.base);
+            mine->buffer = Buffer{nullptr, 0, device};
+            ++g_generation;
+        }
+        e = obtain(bytes, device, &mine->buffer);
+        if (e != cudaSuccess) return e;
+    }
+    *out = mine->buffer.base;
+    return cudaSuccess;
+}
+
+}  // namespace weft
