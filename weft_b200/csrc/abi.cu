@@ -11,8 +11,11 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <list>
 #include <map>
 #include <mutex>
+#include <string>
+#include <unordered_map>
 #include <vector>
 
 using namespace weft;
@@ -45,6 +48,8 @@ struct State {
     std::map<uintptr_t, Resident> resident;   // keyed by host base address
     uint8_t *arena = nullptr;                 // staging for host-pointer arguments; grows, never shrinks
     size_t arena_bytes = 0;
+    uint8_t *bounce = nullptr, *bounce_dev = nullptr;   // pinned, mapped: small host arguments in pageable memory pass through it
+    cudaStream_t capture_stream = nullptr;              // graphs of repeated calls are recorded here
 };
 State g;
 
@@ -89,22 +94,86 @@ int device_status() {
                                            : s == ST_TMEM_ALLOC ? "tensor memory allocation failed" : "unknown status");
 }
 
+int launched(cudaError_t e, const char *what, unsigned count = 1) {
+    if (e != cudaSuccess) return fail("%s launch failed: %s", what, cudaGetErrorString(e));
+    g.launches += count;
+    return 0;
+}
+
+// ---- graphs of repeated calls
+// A synchronous call costs a launch and a wait whatever the kernel does: 8.9 us here for one empty kernel, 10.9 for two.
+// Replaying an instantiated graph costs 6.4 and 7.1, and nothing that prepares a launch (tensor maps, occupancy queries)
+// is done again.  Programs make the same calls over and over (the same layer on the same buffers, once per token), so a
+// call that has been seen kSeenBefore times with the same arguments is captured, and replayed from then on.  What is
+// kept is the launch, not its result: kernels, sizes and addresses, which are the key; every argument is looked up and
+// checked anew before the key is formed.  The least recently used entry makes room.  Everything runs under g.lock.
+constexpr unsigned kSeenBefore = 3;
+constexpr size_t kGraphs = 1024;
+
+class Key {
+  public:
+    template <typename... T> void add(T... values) { (put(values), ...); }
+    std::string text() const { return std::string(reinterpret_cast<const char *>(words_), n_ * sizeof(uint64_t)); }
+    bool fits() const { return fits_; }
+
+  private:
+    void put(const void *p) { put((uint64_t)reinterpret_cast<uintptr_t>(p)); }
+    template <typename T> void put(T v) { put((uint64_t)v); }
+    void put(uint64_t v) { if (n_ < kWords) words_[n_++] = v; else fits_ = false; }
+    static constexpr size_t kWords = 192;
+    uint64_t words_[kWords];
+    size_t n_ = 0;
+    bool fits_ = true;
+};
+
+struct GraphEntry { std::string key; cudaGraphExec_t exec = nullptr; unsigned launches = 0, seen = 0; bool unfit = false; };
+
+class GraphCache {
+  public:
+    // The entry of a key, made on first sight; the caller's call counts as one more sighting.
+    GraphEntry &find(std::string &&key) {
+        auto it = index_.find(key);
+        if (it != index_.end()) {
+            entries_.splice(entries_.begin(), entries_, it->second);
+            return entries_.front();
+        }
+        if (entries_.size() >= kGraphs) {
+            if (entries_.back().exec) cudaGraphExecDestroy(entries_.back().exec);
+            index_.erase(entries_.back().key);
+            entries_.pop_back();
+        }
+        entries_.emplace_front();
+        entries_.front().key = key;
+        index_.emplace(std::move(key), entries_.begin());
+        return entries_.front();
+    }
+
+  private:
+    std::list<GraphEntry> entries_;      // most recently used first
+    std::unordered_map<std::string, std::list<GraphEntry>::iterator> index_;
+};
+GraphCache g_graphs;
+
 // One argument of a call: where the caller's bytes live and where the kernel will find them.
 struct Arg {
-    const void *user = nullptr;
+    void *user = nullptr;      // written host argument whose bytes have to reach the caller after the call
     void *dev = nullptr;
-    void *mapped = nullptr;    // the user's buffer as the device sees it, when it is pinned and mapped host memory
+    void *mapped = nullptr;    // host memory as the device sees it: the user's own when pinned, else a slice of the bounce buffer
+    void *bounce = nullptr;    // host address of that slice
     size_t bytes = 0;
     bool written = false, overflow = false;
 };
 
-// Host arguments up to this size in pinned, mapped memory move by a copy kernel instead of the copy engine.
+// Host arguments up to this size move by a copy kernel through pinned, mapped memory instead of the copy engine.
 constexpr size_t kKernelCopyMax = size_t(1) << 18;
+constexpr size_t kBounceBytes = size_t(1) << 20;
 
 // Host-pointer arguments are staged in one device arena owned by the library (256-byte aligned slices).
 // An argument that does not fit gets a one-off allocation, and the arena is regrown after the call so
-// that the same call fits next time.  Calls that stage anything always end with a stream synchronize,
-// so the arena is free again when the next call starts.
+// that the same call fits next time.  Small arguments in ordinary (pageable) memory pass through a pinned bounce
+// buffer of the library's: the driver's own path for pageable copies waits for each of them.
+// Calls that stage anything always end with a stream synchronize, so arena and bounce buffer are free again when the
+// next call starts.
 class Call {
   public:
     ~Call() {
@@ -112,8 +181,8 @@ class Call {
             if (a.overflow && a.dev) { cudaStreamSynchronize(g.stream); cudaFree(a.dev); }
     }
     // Returns the device address for `ptr` (bytes long). read: copy in when host; written: copy back.
-    // direct: a written host argument in pinned, mapped memory that the kernels only ever store to (never read back)
-    // is handed to them as it is -- their stores go to the caller's buffer, no staging slice and no copy back.
+    // direct: a written host argument that the kernels only ever store to (never read back) is handed to them in mapped
+    // memory -- their stores go to the caller's pinned buffer (or the bounce buffer), no staging slice and no copy back.
     int map(const void *ptr, size_t bytes, bool read, bool written, void **out, bool direct = false) {
         *out = nullptr;
         direct_ = false;
@@ -141,14 +210,24 @@ class Call {
             }
         }
         Arg arg;
-        arg.user = ptr; arg.bytes = bytes; arg.written = written;
-        if (attr.type == cudaMemoryTypeHost && attr.devicePointer && bytes <= kKernelCopyMax) arg.mapped = attr.devicePointer;
-        if (direct && written && !read && arg.mapped) { *out = arg.mapped; direct_ = true; return 0; }
+        arg.user = const_cast<void *>(ptr); arg.bytes = bytes; arg.written = written;
+        if (bytes <= kKernelCopyMax) {
+            if (attr.type == cudaMemoryTypeHost && attr.devicePointer) arg.mapped = attr.devicePointer;
+            else if (bounce_slice(arg)) return 1;
+        }
+        if (arg.bounce && read) memcpy(arg.bounce, ptr, bytes);
+        if (direct && written && !read && arg.mapped) {
+            *out = arg.mapped;
+            direct_ = true;
+            args_.push_back(arg);
+            return 0;
+        }
         if (slice(arg)) return 1;
         if (read) {
-            if (arg.mapped) CU(launch_copy_bytes(arg.dev, arg.mapped, bytes, g.stream));
-            else CU(cudaMemcpyAsync(arg.dev, ptr, bytes, cudaMemcpyHostToDevice, g.stream));
+            if (arg.mapped) before_.push_back(Copy{arg.dev, arg.mapped, bytes});
+            else { repeatable_ = false; CU(cudaMemcpyAsync(arg.dev, ptr, bytes, cudaMemcpyHostToDevice, g.stream)); }
         }
+        if (written && arg.mapped) after_.push_back(Copy{arg.mapped, arg.dev, bytes});
         *out = arg.dev;
         return 0;
     }
@@ -159,19 +238,87 @@ class Call {
         arg.bytes = bytes;
         if (slice(arg)) return 1;
         any_host_ = true;   // the slice is reused by the next call: end this one with a synchronize
+        repeatable_ = false;
+        if (issue_before(g.stream)) return 1;   // the argument may itself be on its way to the device
         CU(cudaMemcpyAsync(arg.dev, *dev, bytes, cudaMemcpyDeviceToDevice, g.stream));
         *dev = arg.dev;
         return 0;
     }
-    // Copy written host arguments back and decide whether to wait.
+    static bool on_device(const void *ptr) {
+        cudaPointerAttributes attr{};
+        if (cudaPointerGetAttributes(&attr, ptr) != cudaSuccess) { cudaGetLastError(); return false; }
+        return attr.type == cudaMemoryTypeDevice || attr.type == cudaMemoryTypeManaged;
+    }
+    void not_repeatable() { repeatable_ = false; }
+
+    // Issues the call: staged copies in, what `enqueue(stream)` puts on the stream, copies back.  `key` holds everything
+    // that decides what enqueue does.  A call that waits anyway may be replayed from a graph.
+    template <typename F> int issue(Key &key, F &&enqueue) {
+        if (repeatable_ && (any_host_ || !g.async)) {
+            for (const Copy &c : before_) key.add(c.dst, c.src, c.bytes);
+            key.add(~uint64_t(0));
+            for (const Copy &c : after_) key.add(c.dst, c.src, c.bytes);
+            key.add((const void *)g.stream, workspace_generation());
+            if (key.fits()) {
+                GraphEntry &entry = g_graphs.find(key.text());
+                if (!entry.exec && !entry.unfit && ++entry.seen > kSeenBefore) capture(entry, enqueue);
+                if (entry.exec) {
+                    CU(cudaGraphLaunch(entry.exec, g.stream));
+                    g.launches += entry.launches;
+                    return finish();
+                }
+            }
+        }
+        if (issue_before(g.stream) || enqueue(g.stream) || issue_after(g.stream)) return 1;
+        return finish();
+    }
+
+    // true when the latest map() handed the kernels mapped host memory
+    bool direct() const { return direct_; }
+
+  private:
+    struct Copy { void *dst; const void *src; size_t bytes; };
+
+    int issue_before(cudaStream_t stream) {
+        for (const Copy &c : before_)
+            if (launched(launch_copy_bytes(c.dst, c.src, c.bytes, stream), "argument copy", 0)) return 1;
+        before_.clear();
+        return 0;
+    }
+    int issue_after(cudaStream_t stream) {
+        for (const Copy &c : after_)
+            if (launched(launch_copy_bytes(c.dst, c.src, c.bytes, stream), "result copy", 0)) return 1;
+        return 0;
+    }
+    template <typename F> void capture(GraphEntry &entry, F &&enqueue) {
+        entry.unfit = true;                       // unless everything below succeeds
+        // a stream of the library's own: others may be enqueuing on the caller's at this moment
+        if (!g.capture_stream && cudaStreamCreateWithFlags(&g.capture_stream, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); return; }
+        const unsigned long long launches = g.launches;
+        const std::vector<Copy> before = before_;
+        if (cudaStreamBeginCapture(g.capture_stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) { cudaGetLastError(); return; }
+        const int failed = issue_before(g.capture_stream) || enqueue(g.capture_stream) || issue_after(g.capture_stream);
+        before_ = before;
+        cudaGraph_t graph = nullptr;
+        const cudaError_t e = cudaStreamEndCapture(g.capture_stream, &graph);
+        if (!failed && e == cudaSuccess && cudaGraphInstantiate(&entry.exec, graph, 0) == cudaSuccess) {
+            entry.launches = (unsigned)(g.launches - launches);
+            entry.unfit = false;
+        } else {
+            entry.exec = nullptr;
+            cudaGetLastError();
+        }
+        g.launches = launches;
+        if (graph) cudaGraphDestroy(graph);
+    }
+    // Copy large written host arguments back and decide whether to wait.
     int finish() {
         for (Arg &a : args_)
-            if (a.written) {
-                if (a.mapped) CU(launch_copy_bytes(a.mapped, a.dev, a.bytes, g.stream));
-                else CU(cudaMemcpyAsync(const_cast<void *>(a.user), a.dev, a.bytes, cudaMemcpyDeviceToHost, g.stream));
-            }
+            if (a.written && !a.mapped) CU(cudaMemcpyAsync(a.user, a.dev, a.bytes, cudaMemcpyDeviceToHost, g.stream));
         if (any_host_ || !g.async) {
             CU(cudaStreamSynchronize(g.stream));
+            for (Arg &a : args_)
+                if (a.written && a.bounce) memcpy(a.user, a.bounce, a.bytes);
             if (wanted_ > g.arena_bytes) {   // make the next identical call fit
                 if (g.arena) cudaFree(g.arena);
                 g.arena = nullptr;
@@ -184,12 +331,19 @@ class Call {
         }
         return 0;
     }
-
-    // true when the latest map() handed the caller's pinned buffer to the kernels as it is
-    bool direct() const { return direct_; }
-
-  private:
-    bool direct_ = false;
+    // A slice of the bounce buffer; without one left the argument moves by the copy engine.
+    int bounce_slice(Arg &arg) {
+        if (!g.bounce) {
+            CU(cudaHostAlloc(reinterpret_cast<void **>(&g.bounce), kBounceBytes, cudaHostAllocMapped | cudaHostAllocPortable));
+            CU(cudaHostGetDevicePointer(reinterpret_cast<void **>(&g.bounce_dev), g.bounce, 0));
+        }
+        const size_t offset = (bounced_ + 255) & ~size_t(255);
+        if (offset + arg.bytes > kBounceBytes) return 0;
+        bounced_ = offset + arg.bytes;
+        arg.bounce = g.bounce + offset;
+        arg.mapped = g.bounce_dev + offset;
+        return 0;
+    }
     int slice(Arg &arg) {
         const size_t offset = (used_ + 255) & ~size_t(255);
         wanted_ = ((wanted_ + 255) & ~size_t(255)) + arg.bytes;
@@ -199,25 +353,21 @@ class Call {
         } else {
             CU(cudaMalloc(&arg.dev, arg.bytes));
             arg.overflow = true;
+            repeatable_ = false;
         }
         args_.push_back(arg);
         return 0;
     }
     std::vector<Arg> args_;
-    size_t used_ = 0, wanted_ = 0;
-    bool any_host_ = false;
+    std::vector<Copy> before_, after_;
+    size_t used_ = 0, wanted_ = 0, bounced_ = 0;
+    bool any_host_ = false, direct_ = false, repeatable_ = true;
 };
 
 size_t row_bytes(int fmt, size_t k) { return k / record_elements(fmt) * record_bytes(fmt); }
 
 int check_k(int fmt, size_t k) {
     if (k % record_elements(fmt)) return fail("K = %zu does not contain complete %d-element records", k, record_elements(fmt));
-    return 0;
-}
-
-int launched(cudaError_t e, const char *what, unsigned count = 1) {
-    if (e != cudaSuccess) return fail("%s launch failed: %s", what, cudaGetErrorString(e));
-    g.launches += count;
     return 0;
 }
 
@@ -239,10 +389,13 @@ int do_dequantize(int fmt, const void *W, const int8_t *grid, const int8_t *sign
     if (fmt == F_TQ1_0 && call.map(powers, 20, true, false, &pw)) return 1;
     if (fmt == F_IQ1_M && call.map(powers, 65536 * sizeof(float), true, false, &pw)) return 1;   // the caller's float[65536] table of f16 bit patterns
     if (call.map(Y, N * K * sizeof(float), false, true, &y)) return 1;
-    if (launched(launch_dequantize(fmt, w, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw, (float *)y,
-                                   (long long)(N * K), g.prop.multiProcessorCount, g.stream), "row_dequantize"))
-        return 1;
-    return call.finish();
+    const long long elements = (long long)(N * K);
+    Key key;
+    key.add(1, fmt, w, gr, sg, pw, y, elements);
+    return call.issue(key, [&](cudaStream_t stream) {
+        return launched(launch_dequantize(fmt, w, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw, (float *)y, elements,
+                                          g.prop.multiProcessorCount, stream), "row_dequantize");
+    });
 }
 
 int do_quantize(int act, const float *X, uint8_t *Y, size_t M, size_t K) {
@@ -255,71 +408,104 @@ int do_quantize(int act, const float *X, uint8_t *Y, size_t M, size_t K) {
     if (call.map(Y, M * row_bytes(act, K), false, true, &y)) return 1;
     if ((reinterpret_cast<uintptr_t>(y) & (act == F_Q8_K ? 3u : 1u)) || (reinterpret_cast<uintptr_t>(x) & 3u))
         return fail("activation buffers do not meet their Encoding alignment");
-    if (launched(launch_quantize(act, (const float *)x, y, (long long)M, (long long)K, g.prop.multiProcessorCount, g.stream), "quantize"))
-        return 1;
-    return call.finish();
+    Key key;
+    key.add(2, act, x, y, M, K);
+    return call.issue(key, [&](cudaStream_t stream) {
+        return launched(launch_quantize(act, (const float *)x, y, (long long)M, (long long)K, g.prop.multiProcessorCount, stream), "quantize");
+    });
 }
 
-// One path for the decode and the tiled symbols: what runs is chosen by the number of token rows, the format and the shape.
+// One mul_mat with its arguments where the kernels find them, and which kernels run.  One path for the decode and the tiled
+// symbols: what runs is chosen by the number of token rows, the format and the shape.
+struct MulMat {
+    enum Path { NOTHING, GEMV, PAIR, TILES };
+    int fmt = 0, act = 0;
+    Path path = NOTHING;
+    void *w = nullptr, *x = nullptr, *xq = nullptr, *y = nullptr, *gr = nullptr, *sg = nullptr, *pw = nullptr;
+    uint8_t *planes = nullptr;
+    long long n = 0, k = 0, m = 0, ldy = 0;
+    bool have_xq = false, fuse_quantize = false, y_on_host = false;
+
+    TileArgs tile_args() const {
+        return TileArgs{fmt, w, have_xq ? nullptr : (const float *)x, xq, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw, (float *)y, n, k, m, ldy};
+    }
+    size_t plane_bytes() const { return path == TILES ? tile_plane_bytes(tile_args()) : path == PAIR ? prefill_pair_plane_bytes(fmt, m, k) : 0; }
+
+    int prepare(Call &call, int fmt_, const void *W, const float *X, void *Xq, const int8_t *grid, const int8_t *signs, const uint32_t *powers,
+                float *Y, size_t N, size_t K, size_t M, size_t pitch, unsigned flags, bool vec_dot_only, bool gathers) {
+        fmt = fmt_;
+        act = activation_of(fmt);
+        if (check_k(fmt, K) || check_k(act, K)) return 1;
+        if (K == 0 || N == 0 || M == 0) return 0;
+        if (pitch < N) return fail("Y row pitch %zu is smaller than N = %zu", pitch, N);
+        if (fmt == F_Q4_K_I16 && N % 16 != 0) return fail("Q4K_I[16] holds whole cohorts of 16 rows; N = %zu", N);
+        n = (long long)N; k = (long long)K; m = (long long)M; ldy = (long long)pitch;
+        have_xq = vec_dot_only || (flags & 1u);
+        if (call.map(W, N * row_bytes(fmt, K), true, false, &w)) return 1;
+        if ((fmt == F_Q6_K || fmt == F_IQ1_M) && (reinterpret_cast<uintptr_t>(w) & 1u) && call.realign(&w, N * row_bytes(fmt, K))) return 1;
+        if (!have_xq && call.map(X, M * K * sizeof(float), true, false, &x)) return 1;
+        // Decode quantizes X inside the GEMV (its first CTA stores the records, nobody loads them again), so a host Xq can
+        // be written in place; a batch may take a path that reads Xq back.
+        const bool xq_in_place = !have_xq && M < 3 && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+        if (call.map(Xq, M * row_bytes(act, K), have_xq, !have_xq, &xq, xq_in_place)) return 1;
+        if (codebook_bytes(fmt) && (call.map(grid, codebook_bytes(fmt), true, false, &gr) || (has_sign_table(fmt) && call.map(signs, 1024, true, false, &sg)))) return 1;
+        if (fmt == F_TQ1_0 && call.map(powers, 20, true, false, &pw)) return 1;
+        if (fmt == F_IQ1_M && call.map(powers, 65536 * sizeof(float), true, false, &pw)) return 1;   // the caller's float[65536] table of f16 bit patterns
+        // a host Y with a pitch is staged whole (pitch * M floats); device Y is written in place; a small host Y too
+        const size_t y_floats = (M - 1) * pitch + N;
+        if (call.map(Y, y_floats * sizeof(float), pitch != N, true, &y, pitch == N && !gathers)) return 1;
+        y_on_host = call.direct();
+        if ((reinterpret_cast<uintptr_t>(w) & (fmt == F_Q4_K_I16 ? 15u : 1u)) || (reinterpret_cast<uintptr_t>(xq) & (act == F_Q8_K ? 3u : 1u)) ||
+            (reinterpret_cast<uintptr_t>(y) & 3u) || (x && (reinterpret_cast<uintptr_t>(x) & 3u)))
+            return fail("a buffer does not meet its Encoding alignment");
+        path = prefill_pair_supported(fmt, n, k, m, w, xq) ? PAIR : tile_supported(tile_args()) ? TILES : GEMV;
+        // decode: the GEMV's own prologue quantizes X (one launch) when the fp32 rows allow 16-byte loads
+        fuse_quantize = !have_xq && path == GEMV && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+        return 0;
+    }
+
+    void add_to(Key &key) const {
+        key.add(fmt, path, w, x, xq, y, gr, sg, pw, (const void *)planes, n, k, m, ldy, have_xq, fuse_quantize, y_on_host);
+    }
+
+    int enqueue(cudaStream_t stream, const GatherArgs *gather = nullptr) const {
+        const int sms = g.prop.multiProcessorCount;
+        bool gathered = false;
+        if (path == NOTHING) return 0;
+        if (path == TILES) {          // their first kernel quantizes X
+            if (launched(launch_tile(tile_args(), planes, sms, stream), "batched mul_mat", 2)) return 1;
+        } else {
+            if (!have_xq && !fuse_quantize && launched(launch_quantize(act, (const float *)x, xq, m, k, sms, stream), "activation quantize")) return 1;
+            if (path == PAIR) {
+                const PrefillArgs pa{fmt, w, xq, (const uint32_t *)pw, (float *)y, n, k, m, ldy, g.status_dev, planes};
+                if (launched(launch_prefill_pair(pa, sms, stream), "prefill mul_mat", prefill_pair_launches(fmt))) return 1;   // its plane kernel first
+            } else {
+                GemvArgs ga{fmt, w, xq, fuse_quantize ? (const float *)x : nullptr, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw,
+                            (float *)y, n, k, m, ldy, g.status_dev, y_on_host};
+                gathered = gather && gemv_gathers(ga);
+                if (gathered) ga.gather = *gather;
+                if (launched(launch_gemv(ga, sms, stream), "decode mul_mat")) return 1;
+            }
+        }
+        return gather && !gathered ? launched(launch_gather_push(*gather, m, n, ldy, g.status_dev, sms, stream), "peer all-gather") : 0;
+    }
+};
+
 int do_mul_mat(int fmt, const void *W, const float *X, void *Xq, const int8_t *grid, const int8_t *signs,
                const uint32_t *powers, float *Y, size_t N, size_t K, size_t M, size_t ldy, unsigned flags, bool vec_dot_only,
                const GatherArgs *gather = nullptr) {
     std::lock_guard<std::recursive_mutex> guard(g.lock);
     if (ensure_init(-1)) return 1;
-    const int act = activation_of(fmt);
-    if (check_k(fmt, K) || check_k(act, K)) return 1;
-    if (K == 0 || N == 0 || M == 0) return 0;
-    if (ldy < N) return fail("Y row pitch %zu is smaller than N = %zu", ldy, N);
-    if (fmt == F_Q4_K_I16 && N % 16 != 0) return fail("Q4K_I[16] holds whole cohorts of 16 rows; N = %zu", N);
-    const bool have_xq = vec_dot_only || (flags & 1u);
     Call call;
-    void *w, *x = nullptr, *xq, *y, *gr = nullptr, *sg = nullptr, *pw = nullptr;
-    if (call.map(W, N * row_bytes(fmt, K), true, false, &w)) return 1;
-    if ((fmt == F_Q6_K || fmt == F_IQ1_M) && (reinterpret_cast<uintptr_t>(w) & 1u) && call.realign(&w, N * row_bytes(fmt, K))) return 1;
-    if (!have_xq && call.map(X, M * K * sizeof(float), true, false, &x)) return 1;
-    // Decode quantizes X inside the GEMV (its first CTA stores the records, nobody loads them again), so a pinned Xq can
-    // be written in place; a batch may take a path that reads Xq back.
-    const bool xq_in_place = !have_xq && M < 3 && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-    if (call.map(Xq, M * row_bytes(act, K), have_xq, !have_xq, &xq, xq_in_place)) return 1;
-    if (codebook_bytes(fmt) && (call.map(grid, codebook_bytes(fmt), true, false, &gr) || (has_sign_table(fmt) && call.map(signs, 1024, true, false, &sg)))) return 1;
-    if (fmt == F_TQ1_0 && call.map(powers, 20, true, false, &pw)) return 1;
-    if (fmt == F_IQ1_M && call.map(powers, 65536 * sizeof(float), true, false, &pw)) return 1;   // the caller's float[65536] table of f16 bit patterns
-    // a host Y with a pitch is staged whole (pitch * M floats); device Y is written in place; a small pinned Y too
-    const size_t y_floats = (M - 1) * ldy + N;
-    if (call.map(Y, y_floats * sizeof(float), ldy != N, true, &y, ldy == N && gather == nullptr)) return 1;
-    const bool y_on_host = call.direct();
-    if ((reinterpret_cast<uintptr_t>(w) & (fmt == F_Q4_K_I16 ? 15u : 1u)) || (reinterpret_cast<uintptr_t>(xq) & (act == F_Q8_K ? 3u : 1u)) ||
-        (reinterpret_cast<uintptr_t>(y) & 3u) || (x && (reinterpret_cast<uintptr_t>(x) & 3u)))
-        return fail("a buffer does not meet its Encoding alignment");
-    const int sms = g.prop.multiProcessorCount;
-    const bool pair = prefill_pair_supported(fmt, (long long)N, (long long)K, (long long)M, w, xq);
-    const TileArgs ta{fmt, w, have_xq ? nullptr : (const float *)x, xq, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw,
-                      (float *)y, (long long)N, (long long)K, (long long)M, (long long)ldy};
-    bool gathered = false;
-    if (!pair && tile_supported(ta)) {
-        // a batch of tokens: register tiles, the weights read once per tile of tokens; their first kernel quantizes X
-        uint8_t *planes = nullptr;
-        CU(workspace(tile_plane_bytes(ta), g.stream, &planes));
-        if (launched(launch_tile(ta, planes, sms, g.stream), "batched mul_mat", 2)) return 1;
-    } else {
-        // decode: the GEMV's own prologue quantizes X (one launch) when the fp32 rows allow 16-byte loads
-        const bool fuse_quantize = !have_xq && !pair && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-        if (!have_xq && !fuse_quantize &&
-            launched(launch_quantize(act, (const float *)x, xq, (long long)M, (long long)K, sms, g.stream), "activation quantize"))
-            return 1;
-        if (pair) {
-            const PrefillArgs pa{fmt, w, xq, (const uint32_t *)pw, (float *)y, (long long)N, (long long)K, (long long)M, (long long)ldy, g.status_dev};
-            if (launched(launch_prefill_pair(pa, sms, g.stream), "prefill mul_mat", prefill_pair_launches(fmt))) return 1;   // its plane kernel first
-        } else {
-            GemvArgs ga{fmt, w, xq, fuse_quantize ? (const float *)x : nullptr, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw,
-                        (float *)y, (long long)N, (long long)K, (long long)M, (long long)ldy, g.status_dev, y_on_host};
-            gathered = gather && gemv_gathers(ga);
-            if (gathered) ga.gather = *gather;
-            if (launched(launch_gemv(ga, sms, g.stream), "decode mul_mat")) return 1;
-        }
-    }
-    if (gather && !gathered && launched(launch_gather_push(*gather, (long long)M, (long long)N, (long long)ldy, g.status_dev, sms, g.stream), "peer all-gather")) return 1;
-    return call.finish();
+    MulMat op;
+    if (op.prepare(call, fmt, W, X, Xq, grid, signs, powers, Y, N, K, M, ldy, flags, vec_dot_only, gather != nullptr)) return 1;
+    if (op.path == MulMat::NOTHING) return 0;
+    if (const size_t bytes = op.plane_bytes()) CU(workspace(bytes, g.stream, &op.planes));
+    if (gather) call.not_repeatable();       // its kernels meet the other ranks' in a fixed order of launches
+    Key key;
+    key.add(3);
+    op.add_to(key);
+    return call.issue(key, [&](cudaStream_t stream) { return op.enqueue(stream, gather); });
 }
 
 }  // namespace
@@ -539,8 +725,11 @@ static int q4ki_pack(const uint8_t *source, uint8_t *target, size_t rows, size_t
     const size_t bytes = q4ki_packed_size(rows, K);
     if (call.map(source, bytes, true, false, &src) || call.map(target, bytes, false, true, &dst)) return 1;
     if ((reinterpret_cast<uintptr_t>(src) & 1u) || (reinterpret_cast<uintptr_t>(dst) & 15u)) return fail("a buffer does not meet its Encoding alignment");
-    if (launched(launch_interleave_q4k(src, dst, (long long)rows, (long long)K, g.prop.multiProcessorCount, g.stream), "Q4K_I[16] pack")) return 1;
-    return call.finish();
+    Key key;
+    key.add(5, src, dst, rows, K);
+    return call.issue(key, [&](cudaStream_t stream) {
+        return launched(launch_interleave_q4k(src, dst, (long long)rows, (long long)K, g.prop.multiProcessorCount, stream), "Q4K_I[16] pack");
+    });
 }
 size_t q4_k_q8_k_gemv_W_packed_size(size_t M, size_t K) { return q4ki_packed_size(M, K); }
 int q4_k_q8_k_gemv_W_pack(const uint8_t *source, uint8_t *target, size_t M, size_t K) { return q4ki_pack(source, target, M, K); }
@@ -564,60 +753,80 @@ int production_mul_mat_q4_k_persistent(const uint8_t *W, const float *X, uint8_t
     return do_mul_mat(F_Q4_K_I16, W, X, Xq, nullptr, nullptr, nullptr, Y, N, K, M, N, 0, false);
 }
 
-// Steps i .. i + count - 1 of a chain as one grouped launch: same activations, same K, one activation row, Q4_K
-// weights already on the device.  Returns -1 when the steps do not qualify (the caller then issues them one by one).
-static int do_mul_mat_group(const weft_b200_mul_mat_step *steps, int count) {
-    if (ensure_init(-1)) return 1;
-    const weft_b200_mul_mat_step &first = steps[0];
-    Call call;
-    GemvArgs ga{};
-    ga.fmt = F_Q4_K; ga.k = (long long)first.K; ga.m = 1; ga.segments = count; ga.status = g.status_dev;
+// Consecutive Q4_K steps of a chain on the same activations, one token row: one grouped launch when the kernel takes them.
+static bool group_steps(const MulMat *ops, int count, GemvArgs &ga) {
+    const MulMat &first = ops[0];
+    ga = GemvArgs{};
+    ga.fmt = F_Q4_K; ga.k = first.k; ga.m = 1; ga.segments = count; ga.status = g.status_dev;
     for (int i = 0; i < count; ++i) {
-        void *w, *y;
-        if (call.map(steps[i].W, steps[i].N * row_bytes(F_Q4_K, first.K), true, false, &w)) return 1;
-        if (call.map(steps[i].Y, steps[i].N * sizeof(float), false, true, &y)) return 1;
-        ga.seg_w[i] = w; ga.seg_y[i] = static_cast<float *>(y); ga.seg_rows[i] = (long long)steps[i].N;
-        if (reinterpret_cast<uintptr_t>(y) & 3u) return fail("a buffer does not meet its Encoding alignment");
+        ga.seg_w[i] = ops[i].w; ga.seg_y[i] = static_cast<float *>(ops[i].y); ga.seg_rows[i] = ops[i].n;
     }
-    const bool have_xq = (first.flags & 1u) != 0;
-    void *x = nullptr, *xq;
-    if (!have_xq && call.map(first.X, first.K * sizeof(float), true, false, &x)) return 1;
-    if (call.map(first.Xq, row_bytes(F_Q8_K, first.K), have_xq, !have_xq, &xq)) return 1;
-    if ((reinterpret_cast<uintptr_t>(xq) & 3u) || (x && (reinterpret_cast<uintptr_t>(x) & 3u))) return fail("a buffer does not meet its Encoding alignment");
-    const int sms = g.prop.multiProcessorCount;
-    const bool fuse_quantize = !have_xq && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-    ga.xq = xq;
-    ga.x = fuse_quantize ? static_cast<const float *>(x) : nullptr;
-    if (!gemv_q4k_groups(ga)) return -1;
-    if (!have_xq && !fuse_quantize &&
-        launched(launch_quantize(F_Q8_K, (const float *)x, xq, 1, (long long)first.K, sms, g.stream), "activation quantize"))
-        return 1;
-    if (launched(launch_gemv(ga, sms, g.stream), "grouped decode mul_mat")) return 1;
-    return call.finish();
+    ga.xq = first.xq;
+    ga.x = first.fuse_quantize ? static_cast<const float *>(first.x) : nullptr;
+    return gemv_q4k_groups(ga);
+}
+
+static bool chain_format(int f) {    // chains: the formats of the first version
+    return f == F_Q4_0 || f == F_Q8_0 || f == F_Q2_K || f == F_Q3_K || f == F_Q4_K || f == F_Q5_K || f == F_Q6_K || f == F_IQ2_XXS || f == F_TQ1_0;
 }
 
 int weft_b200_mul_mat_chain(const weft_b200_mul_mat_step *steps, size_t count) {
     if (!steps && count) return fail("the step table is NULL");
     std::lock_guard<std::recursive_mutex> guard(g.lock);
+    if (!count) return 0;
+    if (ensure_init(-1)) return 1;
+    // All steps are looked up first and issued together, with one wait at the end.  A chain with host memory in it goes step
+    // by step: a later step may take what an earlier one copied back.
+    bool on_device = true;
+    for (size_t i = 0; i < count && on_device; ++i) {
+        const weft_b200_mul_mat_step &s = steps[i];
+        for (const void *p : {(const void *)s.W, (const void *)s.X, (const void *)s.Xq, (const void *)s.Y, (const void *)s.grid, (const void *)s.signs, (const void *)s.powers})
+            on_device = on_device && (!p || Call::on_device(p));
+    }
     for (size_t i = 0; i < count; ++i) {
         const weft_b200_mul_mat_step &s = steps[i];
-        // consecutive Q4_K steps on the same activations (the later ones marked as reusing Xq) go out as one launch
-        size_t run = 1;
-        if (s.format == F_Q4_K && s.M == 1 && s.N && s.K && s.K % 256 == 0)
-            while (i + run < count && run < (size_t)GEMV_MAX_SEGMENTS && steps[i + run].format == F_Q4_K && steps[i + run].M == 1 &&
-                   steps[i + run].K == s.K && steps[i + run].Xq == s.Xq && (steps[i + run].flags & 1u) && steps[i + run].N)
-                ++run;
-        if (run > 1) {
-            const int grouped = do_mul_mat_group(steps + i, (int)run);
-            if (grouped > 0) return 1;
-            if (grouped == 0) { i += run - 1; continue; }
-        }
-        if (s.format != F_Q4_0 && s.format != F_Q8_0 && s.format != F_Q2_K && s.format != F_Q3_K && s.format != F_Q4_K && s.format != F_Q5_K &&
-            s.format != F_Q6_K && s.format != F_IQ2_XXS && s.format != F_TQ1_0)  /* chains: the formats of the first version */
-            return fail("step %zu: unknown weight format id %d", i, s.format);
-        if (do_mul_mat(s.format, s.W, s.X, s.Xq, s.grid, s.signs, s.powers, s.Y, s.N, s.K, s.M, s.N, s.flags, false)) return 1;
+        if (!chain_format(s.format)) return fail("step %zu: unknown weight format id %d", i, s.format);
+        if (!on_device && do_mul_mat(s.format, s.W, s.X, s.Xq, s.grid, s.signs, s.powers, s.Y, s.N, s.K, s.M, s.N, s.flags, false)) return 1;
     }
-    return 0;
+    if (!on_device) return 0;
+    Call call;
+    std::vector<MulMat> ops(count);
+    for (size_t i = 0; i < count; ++i) {
+        const weft_b200_mul_mat_step &s = steps[i];
+        if (ops[i].prepare(call, s.format, s.W, s.X, s.Xq, s.grid, s.signs, s.powers, s.Y, s.N, s.K, s.M, s.N, s.flags, false, false)) return 1;
+    }
+    size_t plane_bytes = 0;              // the steps follow each other: one workspace serves them all
+    for (const MulMat &op : ops) plane_bytes = op.plane_bytes() > plane_bytes ? op.plane_bytes() : plane_bytes;
+    uint8_t *planes = nullptr;
+    if (plane_bytes) CU(workspace(plane_bytes, g.stream, &planes));
+    Key key;
+    key.add(4, count);
+    for (MulMat &op : ops) {
+        op.planes = planes;
+        op.add_to(key);
+    }
+    return call.issue(key, [&](cudaStream_t stream) {
+        for (size_t i = 0; i < count; ++i) {
+            // consecutive Q4_K steps on the same activations (the later ones marked as reusing Xq) go out as one launch
+            size_t run = 1;
+            if (ops[i].path == MulMat::GEMV && ops[i].fmt == F_Q4_K && ops[i].m == 1 && ops[i].k % 256 == 0)
+                while (i + run < count && run < (size_t)GEMV_MAX_SEGMENTS && ops[i + run].path == MulMat::GEMV && ops[i + run].fmt == F_Q4_K && ops[i + run].m == 1 &&
+                       ops[i + run].k == ops[i].k && ops[i + run].xq == ops[i].xq && ops[i + run].have_xq)
+                    ++run;
+            GemvArgs ga;
+            if (run > 1 && group_steps(&ops[i], (int)run, ga)) {
+                const int sms = g.prop.multiProcessorCount;
+                if (!ops[i].have_xq && !ops[i].fuse_quantize &&
+                    launched(launch_quantize(F_Q8_K, (const float *)ops[i].x, ops[i].xq, 1, ops[i].k, sms, stream), "activation quantize"))
+                    return 1;
+                if (launched(launch_gemv(ga, sms, stream), "grouped decode mul_mat")) return 1;
+                i += run - 1;
+            } else if (ops[i].enqueue(stream)) {
+                return 1;
+            }
+        }
+        return 0;
+    });
 }
 
 // ---- peer memory (CUDA IPC) and the row-sharded mul_mat that gathers through it

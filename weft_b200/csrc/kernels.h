@@ -72,7 +72,9 @@ struct PrefillArgs {
     float *y;                // (m, ldy)
     long long n, k, m, ldy;
     int *status;
+    uint8_t *planes;         // prefill_pair_plane_bytes() of device memory for the activation planes
 };
+size_t prefill_pair_plane_bytes(int fmt, long long m, long long k);
 // tcgen05 int8 contraction on CTA pairs (256 tokens per tile, cta_group::2): Q4_K and TQ1_0 with more than 128 tokens.
 cudaError_t launch_prefill_pair(const PrefillArgs &a, int sm_count, cudaStream_t stream);
 bool prefill_pair_supported(int fmt, long long n, long long k, long long m, const void *w, const void *xq);

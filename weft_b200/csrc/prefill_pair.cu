@@ -1115,9 +1115,7 @@ static cudaError_t launch_prefill_pair_tq1(const PrefillArgs &a, int sm_count, c
     // planes: codes (m, k) int8, then x.d (nb, pitch) float
     p.xd_pitch = (a.m + 63) & ~63LL;
     const size_t code_bytes = ((size_t)a.m * (size_t)a.k + 255) & ~size_t(255);
-    uint8_t *planes = nullptr;
-    e = workspace(code_bytes + (size_t)p.nb * (size_t)p.xd_pitch * sizeof(float), stream, &planes);
-    if (e != cudaSuccess) return e;
+    uint8_t *planes = a.planes;
     p.xd = reinterpret_cast<const float *>(planes + code_bytes);
     {
         const long long records = a.m * p.nb;
@@ -1166,9 +1164,7 @@ static cudaError_t launch_prefill_pair_q4k_planes(const PrefillArgs &a, int sm_c
     p.xd_pitch = (a.m + 63) & ~63LL;
     const size_t code_bytes = ((size_t)a.m * (size_t)a.k + 255) & ~size_t(255);
     const size_t xd_bytes = ((size_t)p.nb * (size_t)p.xd_pitch * sizeof(float) + 255) & ~size_t(255);
-    uint8_t *planes = nullptr;
-    e = workspace(code_bytes + xd_bytes + (size_t)a.m * (size_t)p.nb * 32, stream, &planes);
-    if (e != cudaSuccess) return e;
+    uint8_t *planes = a.planes;
     p.xd = reinterpret_cast<const float *>(planes + code_bytes);
     uint8_t *mins = planes + code_bytes + xd_bytes;
     {
@@ -1194,6 +1190,12 @@ static cudaError_t launch_prefill_pair_q4k_planes(const PrefillArgs &a, int sm_c
     if (e != cudaSuccess) return e;
     prefill_pair_q4k_planes_kernel<<<2 * pairs, PQ_THREADS, PQ_SMEM, stream>>>(p, x_codes, x_mins, w_rows, w_heads);
     return cudaGetLastError();
+}
+
+// codes, x.d (tokens padded to 64), and for Q4_K the min-term operand
+size_t prefill_pair_plane_bytes(int fmt, long long m, long long k) {
+    const size_t nb = (size_t)(k / 256), pitch = ((size_t)m + 63) & ~size_t(63);
+    return (((size_t)m * (size_t)k + 255) & ~size_t(255)) + ((nb * pitch * sizeof(float) + 255) & ~size_t(255)) + (fmt == F_Q4_K ? (size_t)m * nb * 32 : 0);
 }
 
 int prefill_pair_launches(int) { return 2; }   // plane kernel + contraction

@@ -779,4 +779,10 @@ cudaError_t launch_tile_kernel(const TileArgs &a, const uint8_t *planes, int sm_
 #undef TL_CASE
 }
 
+// One translation unit per family instantiates its kernels (tile_*.cu).
+#define TL_EACH_FORMAT(DO) DO(F_Q4_0) DO(F_Q8_0) DO(F_Q2_K) DO(F_Q3_K) DO(F_Q4_K) DO(F_Q5_K) DO(F_Q6_K) DO(F_IQ2_XXS) DO(F_TQ1_0)
+#define TL_ELSEWHERE(FMT) extern template cudaError_t launch_tile_kernel<FMT>(const TileArgs &, const uint8_t *, int, cudaStream_t);
+TL_EACH_FORMAT(TL_ELSEWHERE)
+#undef TL_ELSEWHERE
+
 }  // namespace weft
