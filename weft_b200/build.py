@@ -10,11 +10,14 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
+import time
 from pathlib import Path
 
 PACKAGE = Path(__file__).resolve().parent
 CSRC = PACKAGE / "csrc"
 LIBRARY = PACKAGE / "libweft_b200.so"
+PYCALL = PACKAGE / "_pycall.so"          # extension module: the native call path of CompiledKernel
 SOURCES = ["abi.cu", "abi_noalloc.cu", "dequantize.cu", "quantize.cu", "gemv.cu", "gemv_q4k.cu", "gemv_ring.cu", "gemv_q4ki.cu", "prefill_pair.cu", "mma_peak.cu", "gather.cu", "workspace.cu", "tile.cu", "tile_q45.cu", "tile_q236.cu", "tile_q08.cu", "tile_low.cu"]
 HEADERS = ["common.cuh", "quantize.cuh", "kernels.h", "gemv_units.cuh", "ring.cuh", "tcgen05.cuh", "tensormap.cuh", "prefill_common.cuh", "gather.cuh", "tile.cuh", "../../include/weft_b200.h"]
 
@@ -35,8 +38,22 @@ def nvcc() -> str:
     return found
 
 
+_fresh_until = 0.0
+
+
 def stale() -> bool:
-    if not LIBRARY.exists():
+    """Whether a source is newer than what was built from it; a library found fresh is looked at again after a second."""
+    global _fresh_until
+    if time.monotonic() < _fresh_until:
+        return False
+    if _sources_are_newer():
+        return True
+    _fresh_until = time.monotonic() + 1.0
+    return False
+
+
+def _sources_are_newer() -> bool:
+    if not LIBRARY.exists() or not PYCALL.exists() or (CSRC / "pycall.cpp").stat().st_mtime > PYCALL.stat().st_mtime:
         return True
     built = LIBRARY.stat().st_mtime
     return any((CSRC / name).stat().st_mtime > built for name in SOURCES + HEADERS)
@@ -64,6 +81,12 @@ def build(verbose: bool = False, extra: list[str] | None = None) -> Path:
             sys.stderr.write(f"--- nvcc {name}\n{out}\n")
     if failed:
         raise RuntimeError("nvcc failed; see the compiler output above")
+    fresh = PYCALL.with_suffix(f".so.{os.getpid()}.tmp")
+    try:
+        subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-I{sysconfig.get_paths()['include']}", str(CSRC / "pycall.cpp"), "-o", str(fresh)], check=True)
+        os.replace(fresh, PYCALL)
+    finally:
+        fresh.unlink(missing_ok=True)
     # link under a temporary name and move it into place: a process that loads the library meanwhile sees the old
     # file or the new one, never a half-written one
     fresh = LIBRARY.with_suffix(f".so.{os.getpid()}.tmp")

@@ -33,6 +33,9 @@ def _dense_from_format(fmt: str, itemsize: int) -> str | None:
 class Buffer:
     """A borrowed contiguous storage object with an explicit logical Encoding."""
 
+    # slots: the native call path (csrc/pycall.cpp) reads the fields at their offsets
+    __slots__ = ("address", "nbytes", "readonly", "device", "shape", "encoding", "_owner", "_view", "__dict__", "__weakref__")
+
     def __init__(self, data: object, *, shape: Sequence[int] | None = None, encoding: str | None = None) -> None:
         inferred = None
         if _is_torch_tensor(data):
