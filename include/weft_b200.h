@@ -135,13 +135,13 @@ int production_mul_mat_tq1_0_lane16_decode(const uint8_t *W, const float *X, uin
  * Same arguments.  The reference binds its tile sizes (NC/MC/MR/NR/KC) at compile time
  * (Emitter.h:505-510), so they are not C parameters here either.
  * examples/kernels/mul_mat/q4_0.py:9-30, q8_0.py:9-29, q4_k_staged.py:9-37   mul_mat_runtime.cpp:217-221,277-281,350-357
- * From 32 tokens on these run on the int8 tensor cores (Q4_K: two scaled limbs per 256-block, CTA pairs above 128
- * tokens; Q4_0 / Q8_0: one contraction per 32-element block); smaller batches run the decode GEMV per token row. */
+ * From three tokens on these run on the tensor cores with every weight record read once per tile of tokens; larger batches of
+ * Q4_K, Q5_K and Q6_K with the weights expanded into tensor memory.  One or two tokens run the decode GEMV per token row. */
 int production_mul_mat_q4_0(const uint8_t *W, const float *X, uint8_t *Xq, float *Y, size_t N, size_t K, size_t M);
 int production_mul_mat_q8_0(const uint8_t *W, const float *X, uint8_t *Xq, float *Y, size_t N, size_t K, size_t M);
 int production_mul_mat_q4_k_staged(const uint8_t *W, const float *X, uint8_t *Xq, float *Y, size_t N, size_t K, size_t M);
 /* examples/kernels/mul_mat/tq1_0.py:10-64            mul_mat_runtime.cpp:534-538
- * (tensor cores from 32 tokens on when K is a multiple of 1024; CTA pairs above 128 tokens when K is a multiple of 2048) */
+ * (tensor cores from three tokens on; CTA pairs above 128 tokens when K is a multiple of 2048) */
 int production_mul_mat_tq1_0(const uint8_t *W, const float *X, uint8_t *Xq, const uint32_t *powers,
                              float *Y, size_t N, size_t K, size_t M);
 /* examples/kernels/mul_mat/iq2_xxs_staged.py:9-97    mul_mat_runtime.cpp:458-473

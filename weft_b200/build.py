@@ -18,8 +18,8 @@ PACKAGE = Path(__file__).resolve().parent
 CSRC = PACKAGE / "csrc"
 LIBRARY = PACKAGE / "libweft_b200.so"
 PYCALL = PACKAGE / "_pycall.so"          # extension module: the native call path of CompiledKernel
-SOURCES = ["abi.cu", "abi_noalloc.cu", "dequantize.cu", "quantize.cu", "gemv.cu", "gemv_q4k.cu", "gemv_ring.cu", "gemv_q4ki.cu", "prefill_pair.cu", "mma_peak.cu", "gather.cu", "workspace.cu", "tile.cu", "tile_q45.cu", "tile_q236.cu", "tile_q08.cu", "tile_low.cu"]
-HEADERS = ["common.cuh", "quantize.cuh", "kernels.h", "gemv_units.cuh", "ring.cuh", "tcgen05.cuh", "tensormap.cuh", "prefill_common.cuh", "gather.cuh", "tile.cuh", "../../include/weft_b200.h"]
+SOURCES = ["abi.cu", "abi_noalloc.cu", "dequantize.cu", "quantize.cu", "gemv.cu", "gemv_q4k.cu", "gemv_ring.cu", "gemv_q4ki.cu", "prefill_pair.cu", "mma_peak.cu", "gather.cu", "workspace.cu", "tile.cu", "tile_q45.cu", "tile_q236.cu", "tile_q08.cu", "tile_low.cu", "fold.cu", "fold_q45.cu", "fold_q6.cu"]
+HEADERS = ["common.cuh", "quantize.cuh", "kernels.h", "gemv_units.cuh", "ring.cuh", "tcgen05.cuh", "tensormap.cuh", "prefill_common.cuh", "gather.cuh", "tile.cuh", "fold.cuh", "../../include/weft_b200.h"]
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

@@ -1,0 +1,177 @@
+// Host side of the tensor-memory contraction (fold.cuh) and the kernel that quantizes activations into its planes.
+#include "fold.cuh"
+#include "quantize.cuh"
+
+#include <algorithm>
+
+namespace weft {
+
+#define FD_ELSEWHERE(FMT) extern template int fold_clusters<FMT>(int); extern template cudaError_t launch_fold_kernel<FMT>(const FoldParams &, const CUtensorMap &, const CUtensorMap &, const CUtensorMap &, int, cudaStream_t);
+FD_EACH_FORMAT(FD_ELSEWHERE)
+
+// ------------------------------------------------------------------ activation planes
+// One warp per (token, 256-element block): quantizes the fp32 values (same bodies as the standalone quantizers), stores the
+// caller's records, the codes as f16 (each group of four as elements 0, 2, 1, 3: the order in which the weights unpack), the
+// scales by (block, token) and, where a min term follows, the sums of 32 codes as 64 h + l in two exact f16 limbs.  Without X
+// the caller's records are the source.  HBM/L2-bound: 4 bytes in, 1.14 out to the records and 2.1 to the planes.
+template <bool MINS, bool FROM_X, bool A16>
+__global__ void __launch_bounds__(256) fold_planes_kernel(const float *__restrict__ x, uint8_t *__restrict__ xq, uint4 *__restrict__ codes, float *__restrict__ xd,
+                                                          __half *__restrict__ mins, int m, int nb, long long pitch) {
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int lane = threadIdx.x & 31;
+    const long long unit = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (unit >= (long long)m * nb) return;
+    const int token = (int)(unit / nb), block = (int)(unit - (long long)token * nb);
+    uint32_t q0, q1;
+    float d;
+    {
+        uint8_t *rec = xq + unit * 292;
+        int sum;                                  // of the lane pair's 16 codes (the record's bsum)
+        if constexpr (FROM_X) {
+            float v[8];
+            load8<A16>(x + unit * 256 + 8 * lane, v);
+            q8_k_warp(v, q0, q1, sum, d);
+            store_q8_k(rec, lane, q0, q1, sum, d);
+        } else {
+            q0 = *reinterpret_cast<const uint32_t *>(rec + 4 + 8 * lane);
+            q1 = *reinterpret_cast<const uint32_t *>(rec + 8 + 8 * lane);
+            sum = *reinterpret_cast<const int16_t *>(rec + 260 + (lane & ~1));
+            d = *reinterpret_cast<const float *>(rec);
+        }
+        if (lane == 0) xd[(long long)block * pitch + token] = d;
+        if constexpr (MINS) {
+            const int pair = sum + __shfl_xor_sync(0xffffffffu, sum, 2);       // lanes 4 g .. 4 g + 3: sum of group g
+            if ((lane & 3) == 0) {
+                __half *to = mins + unit * 16 + (lane >> 2);
+                to[0] = __int2half_rn(pair & 63);
+                to[8] = __int2half_rn(pair >> 6);
+            }
+        }
+    }
+    // bytes as f16: set under the exponent of 1024, 128 added to make them unsigned, both taken out again
+    const uint32_t u0 = q0 ^ 0x80808080u, u1 = q1 ^ 0x80808080u;
+    codes[unit * 32 + lane] = make_uint4(hadd2(__byte_perm(u0, 0x64646464u, 0x4240), 0xe480e480u), hadd2(__byte_perm(u0, 0x64646464u, 0x4341), 0xe480e480u),
+                                         hadd2(__byte_perm(u1, 0x64646464u, 0x4240), 0xe480e480u), hadd2(__byte_perm(u1, 0x64646464u, 0x4341), 0xe480e480u));
+}
+
+template <bool MINS>
+static cudaError_t launch_planes(const TileArgs &a, uint4 *codes, float *xd, __half *mins, long long pitch, cudaStream_t stream) {
+    const int nb = (int)(a.k / 256), m = (int)a.m;
+    const unsigned grid = (unsigned)((a.m * nb + 7) / 8);
+    uint8_t *xq = static_cast<uint8_t *>(const_cast<void *>(a.xq));
+    if (!a.x) fold_planes_kernel<MINS, false, false><<<grid, 256, 0, stream>>>(nullptr, xq, codes, xd, mins, m, nb, pitch);
+    else if (reinterpret_cast<uintptr_t>(a.x) & 15u) fold_planes_kernel<MINS, true, false><<<grid, 256, 0, stream>>>(a.x, xq, codes, xd, mins, m, nb, pitch);
+    else fold_planes_kernel<MINS, true, true><<<grid, 256, 0, stream>>>(a.x, xq, codes, xd, mins, m, nb, pitch);
+    return cudaGetLastError();
+}
+
+// ------------------------------------------------------------------ dispatch
+
+struct FoldPlaneSizes { size_t codes, xd, mins; long long pitch; };
+static FoldPlaneSizes plane_sizes(int fmt, long long m, long long k) {
+    const size_t nb = (size_t)(k / 256), rows = nb;
+    FoldPlaneSizes s;
+    s.pitch = (m + 127) / 128 * 128 + 128;       // the last tile of tokens reads whole
+    s.codes = (size_t)m * (size_t)k * 2;
+    s.xd = rows * (size_t)s.pitch * 4;
+    s.mins = (fmt == F_Q4_K || fmt == F_Q5_K) ? (size_t)m * nb * 32 : 0;
+    return s;
+}
+size_t fold_plane_bytes(const TileArgs &a) {
+    const FoldPlaneSizes s = plane_sizes(a.fmt, a.m, a.k);
+    return s.codes + s.xd + s.mins;
+}
+
+// Picks tokens per tile and slices of K by estimated clocks: rounds of the grid times the blocks of a tile.  A block takes about
+// 1800 clocks when A has buffers for two (up to 80 tokens with a min term, 64 without) and 2350 with one, twice that for
+// Q6_K's two limbs, and hardly depends on the tokens (measured from 16 to 128); a tile's start, its stores and the meeting of
+// the slices are small beside it.
+template <int FMT>
+static FoldPlan fold_plan(long long m, long long n, long long nb, int sm_count) {
+    using F = FoldFormat<FMT>;
+    FoldPlan best{0, 0, 0, 0, 0.0};
+    const long long row_tiles = (n + FD_ROWS - 1) / FD_ROWS;
+    for (int nt = 16; nt <= FD_TOKENS; nt += 16) {
+        const int stages = fold_stages<FMT>(nt), abufs = F::COLS * nt + 4 * 64 <= 512 ? 4 : 2;
+        if (stages < 2 || abufs < F::CHUNKS) continue;
+        const long long tiles = row_tiles * ((m + nt - 1) / nt);
+        for (int slices = 1; slices <= 8 && slices <= nb; ++slices) {
+            if (slices > 1 && tiles > fold_clusters<FMT>(slices)) break;
+            const long long rounds = slices > 1 ? 1 : (tiles + sm_count - 1) / sm_count, steps = (nb + slices - 1) / slices;
+            const double step = F::LIMBS * (abufs >= 2 * F::CHUNKS || (F::LIMBS == 2 && nt <= 64) ? 1800.0 : 2350.0);
+            const double cost = rounds * (steps * step + 1200.0 + 4.0 * nt) + (slices > 1 ? 1500.0 : 0.0);
+            if (!best.nt || cost < best.cost) best = FoldPlan{nt, slices, stages, abufs, cost};
+        }
+    }
+    return best;
+}
+
+static int fold_window(int fmt) {
+    switch (fmt) {
+#define FD_WINDOW(FMT) case FMT: return FoldFormat<FMT>::PITCH;
+    FD_EACH_FORMAT(FD_WINDOW)
+    default: return 0;
+    }
+}
+
+static FoldPlan plan_for(int fmt, long long m, long long n, long long nb, int sm_count) {
+    switch (fmt) {
+#define FD_PLAN(FMT) case FMT: return fold_plan<FMT>(m, n, nb, sm_count);
+    FD_EACH_FORMAT(FD_PLAN)
+    default: return FoldPlan{0, 0, 0, 0, 0.0};
+    }
+}
+
+bool fold_supported(const TileArgs &a) {
+    if (a.fmt != F_Q4_K && a.fmt != F_Q5_K && a.fmt != F_Q6_K) return false;
+    // Below these the register tiles are quicker: this kernel starts about 4 us later (cluster, tensor memory, planes) and takes
+    // as long for 16 tokens as for 64; the tiles go by 8 tokens up to 32 and get slow steps at 17, 25 and 33.  Tiles / this, us,
+    // Q4_K: 4096 x 4096 with 32 tokens (0.54e9 products) 13.0 / 14.0, 4099 x 4096 with 33 (0.55e9) 15.4 / 14.3; 1000 x 2560 with
+    // 200 (0.51e9) 13.2 / 13.8, with 256 (0.66e9) 19.7 / 14.2; 14336 x 4096 with 24 tokens 24.8 / 23.2, with 32 27.5 / 24.0,
+    // 28672 x 8192 with 24 72.2 / 68.5.  Q6_K, twice the work here: 14336 x 4096 with 32 39.8 / 41.5, 4099 x 4096 with 33 21.2 / 20.2.
+    if (a.m <= (a.fmt == F_Q6_K ? 32 : 24) || (double)a.m * (double)a.n * (double)a.k < (a.m <= 32 ? 1.2e9 : 5.5e8)) return false;
+    // 16-byte copies of records need a 16-byte aligned matrix (of whole super-rows: fold.cuh); extents are 32-bit in the kernel
+    return a.m < (1 << 20) && a.k % 256 == 0 && a.k < (1LL << 22) && a.n >= 8 && a.n < (1LL << 31) && (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0;
+}
+
+cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream) {
+    const FoldPlaneSizes s = plane_sizes(a.fmt, a.m, a.k);
+    uint4 *codes = reinterpret_cast<uint4 *>(planes);
+    float *xd = reinterpret_cast<float *>(planes + s.codes);
+    __half *mins = reinterpret_cast<__half *>(planes + s.codes + s.xd);
+    cudaError_t e = s.mins ? launch_planes<true>(a, codes, xd, mins, s.pitch, stream) : launch_planes<false>(a, codes, xd, mins, s.pitch, stream);
+    if (e != cudaSuccess) return e;
+    FoldParams p{};
+    p.w = static_cast<const uint8_t *>(a.w);
+    p.xd = xd; p.y = a.y; p.n = a.n; p.ldy = a.ldy; p.pitch = s.pitch; p.status = status;
+    p.m = (int)a.m;
+    p.nb = (int)(a.k / 256);
+    p.row_bytes = (long long)p.nb * unit_bytes(a.fmt);
+    p.w_bytes = p.row_bytes * a.n;
+    const FoldPlan plan = plan_for(a.fmt, a.m, a.n, p.nb, sm_count);
+    if (!plan.nt) return cudaErrorNotSupported;
+    p.nt = plan.nt; p.slices = plan.slices; p.b_stages = plan.stages; p.a_buffers = plan.a_buffers;
+    p.token_tiles = (int)((a.m + p.nt - 1) / p.nt);
+    p.tiles = p.token_tiles * (int)((a.n + FD_ROWS - 1) / FD_ROWS);
+    CUtensorMap x_codes, x_mins;
+    e = encode_tile_map(&x_codes, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, codes, (unsigned long long)a.k, (unsigned long long)a.m, (unsigned long long)a.k * 2, 64, (unsigned)p.nt, true);
+    if (e == cudaSuccess && s.mins)
+        e = encode_tile_map(&x_mins, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, mins, (unsigned long long)p.nb * 16, (unsigned long long)a.m, (unsigned long long)p.nb * 32, 8, (unsigned)p.nt, false);
+    else x_mins = x_codes;
+    // weight records: rows of words, or (fold.cuh) super-rows of eight rows; rows after the last whole super-row are fetched by
+    // the expanders, so fewer than eight rows need no map
+    CUtensorMap w_rows = x_codes;
+    const int unit = unit_bytes(a.fmt);
+    if (e == cudaSuccess && unit % 16 == 0)
+        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT32, a.w, (unsigned long long)p.row_bytes / 4, (unsigned long long)a.n, (unsigned long long)p.row_bytes, (unsigned)unit / 4, FD_ROWS, false);
+    else if (e == cudaSuccess)
+        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT8, a.w, (unsigned long long)p.row_bytes * 8, (unsigned long long)a.n / 8, (unsigned long long)p.row_bytes * 8, (unsigned)fold_window(a.fmt), 16, false);
+    if (e != cudaSuccess) return e;
+    switch (a.fmt) {
+#define FD_LAUNCH(FMT) case FMT: return launch_fold_kernel<FMT>(p, x_codes, x_mins, w_rows, sm_count, stream);
+    FD_EACH_FORMAT(FD_LAUNCH)
+    default: return cudaErrorNotSupported;
+    }
+}
+
+}  // namespace weft

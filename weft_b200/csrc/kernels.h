@@ -13,6 +13,9 @@ namespace weft {
 // to the (function, device) pair, so what was already granted is remembered per device; defined in gemv.cu.
 cudaError_t grant_dynamic_smem(const void *kernel, int bytes);
 
+// Refuses a kernel that was not compiled with the register count its setmaxnreg trade assumes; defined in prefill_pair.cu.
+cudaError_t check_launch_registers(const void *kernel, int expected);
+
 // W: `elements` logical values as contiguous records of `fmt`; Y: `elements` floats.
 cudaError_t launch_dequantize(int fmt, const void *w, const int8_t *grid, const int8_t *signs, const uint32_t *powers,
                               float *y, long long elements, int sm_count, cudaStream_t stream);
@@ -74,11 +77,11 @@ struct PrefillArgs {
     int *status;
     uint8_t *planes;         // prefill_pair_plane_bytes() of device memory for the activation planes
 };
-size_t prefill_pair_plane_bytes(int fmt, long long m, long long k);
-// tcgen05 int8 contraction on CTA pairs (256 tokens per tile, cta_group::2): Q4_K and TQ1_0 with more than 128 tokens.
+size_t prefill_pair_plane_bytes(long long m, long long k);
+// tcgen05 int8 contraction on CTA pairs (256 tokens per tile, cta_group::2): TQ1_0 with more than 128 tokens.
+// Two launches.
 cudaError_t launch_prefill_pair(const PrefillArgs &a, int sm_count, cudaStream_t stream);
 bool prefill_pair_supported(int fmt, long long n, long long k, long long m, const void *w, const void *xq);
-int prefill_pair_launches(int fmt);   // kernels one launch_prefill_pair call puts on the stream (the plane kernel counts)
 
 // More than one token row: the register-tile kernel (tile.cuh) behind the kernel that quantizes X into its planes.
 struct TileArgs {
@@ -95,6 +98,11 @@ bool tile_supported(const TileArgs &a);
 size_t tile_plane_bytes(const TileArgs &a);
 cudaError_t launch_tile(const TileArgs &a, uint8_t *planes, int sm_count, cudaStream_t stream);   // two kernels
 template <int FMT> cudaError_t launch_tile_kernel(const TileArgs &a, const uint8_t *planes, int sm_count, cudaStream_t stream);
+
+// tcgen05 contraction with the weights expanded into tensor memory (fold.cuh), behind the kernel that makes its planes.
+bool fold_supported(const TileArgs &a);
+size_t fold_plane_bytes(const TileArgs &a);
+cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream);   // two kernels
 
 // Device memory for a call's activation planes, valid for the work it puts on `stream` (workspace.cu); the generation
 // changes whenever memory handed out earlier outside a capture is gone.
