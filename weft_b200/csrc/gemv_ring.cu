@@ -1,4 +1,4 @@
-// Decode GEMV for Q4_0, Q8_0, Q2_K, Q3_K, Q5_K, Q6_K, IQ1_S, IQ1_M, IQ2_XXS, IQ2_XS, IQ2_S, IQ3_XXS, IQ3_S and TQ1_0 weights whose rows are whole 16-byte multiples:
+// Decode GEMV for Q4_0, Q8_0, Q2_K, Q3_K, Q5_K, Q6_K, IQ1_S, IQ1_M, IQ2_XXS, IQ2_XS, IQ2_S, IQ3_XXS, IQ3_S and TQ1_0 weights (16-byte aligned matrix):
 // Y[m, n] = quantized_vec_dot(W[n], Xq[m])  (examples/kernels/mul_mat/{q4_0,q8_0,q2_k,q3_k,q5_k,q6_k,iq2_xxs,tq1_0}_decode.py).
 //
 // Same streaming scheme as the Q4_K kernel: one persistent CTA per SM, a producer warp that fills a
@@ -11,6 +11,14 @@
 // two >= units per row, at most 32): lane group g computes rows 2g and 2g + 1 of the iteration, each lane
 // one 256-element unit of both rows per step (two independent instruction streams), and the group
 // reduces with shuffles.  A row is never split across warps, so results do not depend on the grid.
+//
+// Rows whose bytes are no multiple of 16 (records of 210, 110, 84, 66, 54 bytes and K not a multiple of 1024 or 2048): a
+// stage then starts up to 14 bytes past a 16-byte boundary.  Its copy takes the whole 16-byte units around it into a slot
+// with room for them, and the rows lie `head` bytes into the slot; the up to 14 bytes of the matrix's last unit, which must not
+// be read whole, are moved by the producer's own loads.  The record loaders take any even address as it is.  On the kernel
+// without a ring (gemv.cu), which keeps what is not 16-byte aligned as a whole, and here: Q6_K 4096 x 14080 64.0 and 15.4 us,
+// 14336 x 4352 47.6 and 16.7, 1000 x 2560 7.2 and 4.2; 14336 x 4352 Q3_K 26.6 and 17.4, Q2_K 21.7 and 12.1, IQ2_XXS 32.1 and
+// 16.5, TQ1_0 26.1 and 19.3.
 #include "gemv_units.cuh"
 #include "ring.cuh"
 
@@ -57,6 +65,11 @@ struct RingParams {
     GatherArgs gather;
 };
 
+// Bytes of a ring slot: the stage, and the whole 16-byte units that rows of other lengths reach into
+__host__ __device__ constexpr uint32_t ring_slot_bytes(uint32_t row_bytes, int log_rows) {
+    return row_bytes % 16 ? ((row_bytes << log_rows) + 14 + 15) & ~15u : row_bytes << log_rows;
+}
+
 // GATHER: the launch also does the peer all-gather (a separate instantiation: the plain kernel carries none of it)
 template <int FMT, bool QX, int RL, bool GATHER>
 __global__ void __launch_bounds__(ring_max_threads(FMT, RL)) gemv_ring_kernel(const RingParams p) {
@@ -67,7 +80,7 @@ __global__ void __launch_bounds__(ring_max_threads(FMT, RL)) gemv_ring_kernel(co
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int nb = p.nb, LSR = p.log_stage_rows, SR = 1 << LSR, LS = p.log_stages, S = 1 << LS;
     const int LL = p.log_lanes, L = 1 << LL, RPI = RL * (32 >> LL);   // rows per consumer iteration
-    const uint32_t row_bytes = (uint32_t)nb * UB, stage_bytes = row_bytes << LSR;
+    const uint32_t row_bytes = (uint32_t)nb * UB, stage_bytes = row_bytes << LSR, slot_bytes = ring_slot_bytes(row_bytes, LSR);
     const int G = gridDim.x, b = blockIdx.x;
 
     volatile int *s_issued = reinterpret_cast<volatile int *>(smem);
@@ -100,9 +113,24 @@ __global__ void __launch_bounds__(ring_max_threads(FMT, RL)) gemv_ring_kernel(co
         const int slot = s & (S - 1);
         const bool tail = s >= p.full_rounds;
         const long long row0 = tail ? tail_begin : ((long long)s * G + b) << LSR;
-        const uint32_t bytes = tail ? (uint32_t)tail_here * row_bytes : stage_bytes;
+        uint32_t bytes = tail ? (uint32_t)tail_here * row_bytes : stage_bytes;
+        const uint8_t *from = p.w + (size_t)row0 * row_bytes;
+        if (UB % 16 != 0) {
+            const uint32_t head = (uint32_t)reinterpret_cast<uintptr_t>(from) & 15u;
+            from -= head;
+            bytes += head;
+            if (bytes & 15u) {
+                if (row0 + (tail ? tail_here : SR) < p.n) bytes = (bytes + 15u) & ~15u;   // the next row's first bytes come along (a row is longer)
+                else {
+                    const uint32_t whole = bytes & ~15u;
+                    for (uint32_t i = whole; i < bytes; i += 2)
+                        *reinterpret_cast<uint16_t *>(s_ring + (size_t)slot * slot_bytes + i) = __ldg(reinterpret_cast<const uint16_t *>(from + i));
+                    bytes = whole;
+                }
+            }
+        }
         mbar_expect_tx_a(full_addr + 8 * slot, bytes);
-        bulk_g2s_a(ring_addr + (uint32_t)slot * stage_bytes, p.w + (size_t)row0 * row_bytes, bytes, full_addr + 8 * slot);
+        bulk_g2s_a(ring_addr + (uint32_t)slot * slot_bytes, from, bytes, full_addr + 8 * slot);
     };
     if (warp == 0 && lane == 0) {
         const int first = min(min(S, p.inflight), total_stages);
@@ -162,7 +190,8 @@ __global__ void __launch_bounds__(ring_max_threads(FMT, RL)) gemv_ring_kernel(co
             if (!issued) { report(p.status, ST_WAIT_TIMEOUT); return; }
         }
         if (!mbar_wait_a(full_addr + 8 * (s & (S - 1)), (uint32_t)(s >> LS) & 1u)) { report(p.status, ST_WAIT_TIMEOUT); return; }
-        const uint8_t *stage = s_ring + (size_t)(s & (S - 1)) * stage_bytes;
+        const uint8_t *stage = s_ring + (size_t)(s & (S - 1)) * slot_bytes;
+        if (UB % 16 != 0) stage += ((s < p.full_rounds ? (uint32_t)(s * G + b) << LSR : (uint32_t)tail_begin) * row_bytes) & 15u;
         const int in_stage = (t & (SR - 1)) + RL * group;
         const int ta = t + RL * group;
         bool live[RL];
@@ -235,22 +264,24 @@ struct RingPlan { int log_lanes, log_stage_rows, log_stages; size_t smem; bool o
 RingPlan plan_ring(int fmt, long long nb) {
     RingPlan plan{0, 0, 0, 0, false};
     const long long row_bytes = nb * unit_bytes(fmt);
-    if (row_bytes % 16 != 0 || nb <= 0) return plan;
+    if (nb <= 0) return plan;
+    if (row_bytes > (1 << 20)) return plan;   // longer than the ring; the arithmetic below is 32-bit
+    const auto slot = [&](int log_rows) { return (long long)ring_slot_bytes((uint32_t)row_bytes, log_rows); };
     const long long fixed = (512 + codebook_table_bytes(fmt) + nb * (XQ_PITCH + XAUX_BYTES) + 127) & ~127LL;
     int ll = 0;
     while ((1 << ll) < 32 && (1 << ll) < nb) ++ll;
     const int log_rpi = 1 + (5 - ll);
     int lsr = log_rpi;   // at least one consumer iteration per stage
-    while (lsr < 8 && (row_bytes << (lsr + 1)) <= kRingStageBytes) ++lsr;
+    while (lsr < 8 && slot(lsr + 1) <= kRingStageBytes) ++lsr;
     const long long cap = (long long)kRingSmemKB * 1024;
     // A stage that is a single consumer iteration is drained by one warp while the others wait for the next copy:
     // take two iterations per stage when eight such stages still fit (Q5_K 14336 x 4096: 10.7 -> 8.2 us).
-    if (lsr == log_rpi && kRingTwoIterations && fixed + ((row_bytes << (lsr + 1)) << 3) <= cap) ++lsr;
+    if (lsr == log_rpi && kRingTwoIterations && fixed + (slot(lsr + 1) << 3) <= cap) ++lsr;
     int ls = 0;
-    while ((1 << (ls + 1)) <= kRingMaxStages && (1 << (ls + 1)) <= RG_MAX_STAGES && fixed + ((row_bytes << lsr) << (ls + 1)) <= cap) ++ls;
+    while ((1 << (ls + 1)) <= kRingMaxStages && (1 << (ls + 1)) <= RG_MAX_STAGES && fixed + (slot(lsr) << (ls + 1)) <= cap) ++ls;
     if (ls < 1) return plan;
     plan.log_lanes = ll; plan.log_stage_rows = lsr; plan.log_stages = ls;
-    plan.smem = (size_t)(fixed + ((row_bytes << lsr) << ls)) + 16;   // the 2-byte-aligned record loaders read up to 4 bytes past a record
+    plan.smem = (size_t)(fixed + (slot(lsr) << ls)) + 16;   // the 2-byte-aligned record loaders read up to 4 bytes past a record
     plan.ok = true;
     return plan;
 }
