@@ -738,15 +738,28 @@ cudaError_t launch_tile_plan(const TileArgs &a, const uint8_t *planes, const Til
     return cudaLaunchKernelEx(&cfg, tile_kernel<FMT, NT, MT>, p);
 }
 
-// Picks the cut with the least estimated time.  A step of a CTA that has an SM to itself takes about 1.1 + 0.3 nt
-// microseconds (32 rows per warp), a pair of CTAs with 16 rows per warp together 0.9 + 0.29 nt, three with one token group
-// 2.0 (fitted to Q4_K, 8 to 512 tokens; twice the MMAs per group with a scale per 16 elements); the slices' sums cost a
-// little per tile.  What decides is how full the last round of the grid is and how long K is kept in one piece.
+// What a step costs, in units of a step's fixed part with 16 rows per warp (mt = 1): the MMAs of a token group, the same two with
+// 32 rows, a tile's own part, the slices' sums per token group; how much a further CTA on the SM adds to one alone, and how much
+// a ring of only two stages loses.
+struct TileCosts { double group1, fixed2, group2, tile, sums, beside, shallow; };
+template <int FMT> constexpr TileCosts tile_costs() {
+    using F = TileFormat<FMT>;
+    if (F::SUB16) return {0.147, 1.466, 0.206, 0.96, 0.182, 0.583, 0.075};
+    if (F::PAIR32) return {0.116, 1.741, 0.150, 0.0, 0.211, 0.267, 0.033};
+    if (FMT == F_IQ2_XXS) return {0.166, 1.754, 0.171, 0.0, 0.423, 0.729, 0.036};
+    if (FMT == F_TQ1_0) return {0.175, 1.438, 0.220, 0.267, 0.071, 0.224, 0.227};
+    return {0.127, 1.540, 0.153, 0.0, 0.150, 0.492, 0.090};
+}
+
+// Picks the cut with the least estimated time: what decides is how full the last round of the grid is, how long K is kept in one
+// piece and whether CTAs share an SM.  The costs were fitted to the times of every cut at 780 sizes (3 to 512 tokens, 256 to
+// 32768 rows, K 256 to 14336, all formats): the cut picked is 2 % slower than the best one on average (an estimate in
+// microseconds from a few sizes of Q4_K: 5.5 %, some sizes 20 to 30 %).
 template <int FMT>
 TilePlan tile_plan(const TileArgs &a, int sm_count) {
     using F = TileFormat<FMT>;
+    constexpr TileCosts C = tile_costs<FMT>();
     const long long groups = (a.m + 7) / 8, nb = a.k / 256;
-    const double base = F::SUB16 ? 1.6 : 1.0, slope = F::SUB16 ? 1.7 : 1.0;
     TilePlan best{0, 0, 0, 0, 0.0};
     for (int mt = 1; mt <= 2; ++mt)
         for (int nt = 1; nt <= 8 && nt <= groups; ++nt)
@@ -759,9 +772,10 @@ TilePlan tile_plan(const TileArgs &a, int sm_count) {
                 if (stages < 2 || (wk > nb && wk > 1)) continue;
                 const int tile_rows = TL_WARPS / wk * 16 * mt;
                 const long long tiles = ((a.n + tile_rows - 1) / tile_rows) * ((groups + nt - 1) / nt), steps = (nb + wk - 1) / wk;
-                const double step = mt == 2 ? (F::PAIR32 ? 1.4 : 1.1) * base + 0.3 * slope * nt : ctas == 3 ? 2.0 * base : 0.9 * base + 0.29 * slope * nt;
-                const double rounds = std::max(0.7, (double)((tiles + sm_count - 1) / sm_count) / ctas);
-                const double cost = (mt == 2 ? std::max(1.0, rounds) : rounds) * ((double)steps * step + 0.5 + (wk > 1 ? 0.2 * nt : 0.0));
+                const long long on_sm = (tiles + sm_count - 1) / sm_count, rounds = on_sm / ctas, rest = on_sm - rounds * ctas;   // tiles of the busiest SM
+                const double step = (mt == 2 ? C.fixed2 + C.group2 * nt : 1.0 + C.group1 * nt) * (stages == 2 ? 1.0 + C.shallow : 1.0);
+                const double times = rounds * (1.0 + C.beside * (ctas - 1)) + (rest ? 1.0 + C.beside * (rest - 1) : 0.0);
+                const double cost = times * (steps * step + C.tile) + (wk > 1 ? C.sums * nt * on_sm : 0.0);
                 if (!best.nt || cost < best.cost) best = TilePlan{nt, mt, wk, stages, cost};
             }
     return best;
