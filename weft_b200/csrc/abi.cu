@@ -181,11 +181,12 @@ class Call {
             if (a.overflow && a.dev) { cudaStreamSynchronize(g.stream); cudaFree(a.dev); }
     }
     // Returns the device address for `ptr` (bytes long). read: copy in when host; written: copy back.
-    // direct: a written host argument that the kernels only ever store to (never read back) is handed to them in mapped
-    // memory -- their stores go to the caller's pinned buffer (or the bounce buffer), no staging slice and no copy back.
+    // direct: a written host argument that one CTA stores at its start and nobody reads back is handed to it in mapped memory --
+    // its stores go to the caller's pinned buffer (or the bounce buffer), no staging slice and no copy back.  Not for results,
+    // which the whole grid stores a row or two at a time at its end: each of those stores crosses PCIe by itself, and a call with
+    // 14336 of them took 30.7 us, with the results in device memory and a copy kernel behind 26.7 (4096 rows: 24.1 and 22.9).
     int map(const void *ptr, size_t bytes, bool read, bool written, void **out, bool direct = false) {
         *out = nullptr;
-        direct_ = false;
         if (bytes == 0) { *out = const_cast<void *>(ptr); return 0; }
         if (!ptr) return fail("a required buffer is NULL");
         cudaPointerAttributes attr{};
@@ -218,7 +219,6 @@ class Call {
         if (arg.bounce && read) memcpy(arg.bounce, ptr, bytes);
         if (direct && written && !read && arg.mapped) {
             *out = arg.mapped;
-            direct_ = true;
             args_.push_back(arg);
             return 0;
         }
@@ -272,9 +272,6 @@ class Call {
         if (issue_before(g.stream) || enqueue(g.stream) || issue_after(g.stream)) return 1;
         return finish();
     }
-
-    // true when the latest map() handed the kernels mapped host memory
-    bool direct() const { return direct_; }
 
   private:
     struct Copy { void *dst; const void *src; size_t bytes; };
@@ -361,7 +358,7 @@ class Call {
     std::vector<Arg> args_;
     std::vector<Copy> before_, after_;
     size_t used_ = 0, wanted_ = 0, bounced_ = 0;
-    bool any_host_ = false, direct_ = false, repeatable_ = true;
+    bool any_host_ = false, repeatable_ = true;
 };
 
 size_t row_bytes(int fmt, size_t k) { return k / record_elements(fmt) * record_bytes(fmt); }
@@ -424,7 +421,7 @@ struct MulMat {
     void *w = nullptr, *x = nullptr, *xq = nullptr, *y = nullptr, *gr = nullptr, *sg = nullptr, *pw = nullptr;
     uint8_t *planes = nullptr;
     long long n = 0, k = 0, m = 0, ldy = 0;
-    bool have_xq = false, fuse_quantize = false, y_on_host = false;
+    bool have_xq = false, fuse_quantize = false;
 
     TileArgs tile_args() const {
         return TileArgs{fmt, w, have_xq ? nullptr : (const float *)x, xq, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw, (float *)y, n, k, m, ldy};
@@ -432,7 +429,7 @@ struct MulMat {
     size_t plane_bytes() const { return path == FOLD ? fold_plane_bytes(tile_args()) : path == TILES ? tile_plane_bytes(tile_args()) : path == PAIR ? prefill_pair_plane_bytes(m, k) : 0; }
 
     int prepare(Call &call, int fmt_, const void *W, const float *X, void *Xq, const int8_t *grid, const int8_t *signs, const uint32_t *powers,
-                float *Y, size_t N, size_t K, size_t M, size_t pitch, unsigned flags, bool vec_dot_only, bool gathers) {
+                float *Y, size_t N, size_t K, size_t M, size_t pitch, unsigned flags, bool vec_dot_only) {
         fmt = fmt_;
         act = activation_of(fmt);
         if (check_k(fmt, K) || check_k(act, K)) return 1;
@@ -451,10 +448,9 @@ struct MulMat {
         if (codebook_bytes(fmt) && (call.map(grid, codebook_bytes(fmt), true, false, &gr) || (has_sign_table(fmt) && call.map(signs, 1024, true, false, &sg)))) return 1;
         if (fmt == F_TQ1_0 && call.map(powers, 20, true, false, &pw)) return 1;
         if (fmt == F_IQ1_M && call.map(powers, 65536 * sizeof(float), true, false, &pw)) return 1;   // the caller's float[65536] table of f16 bit patterns
-        // a host Y with a pitch is staged whole (pitch * M floats); device Y is written in place; a small host Y too
+        // a host Y with a pitch is staged whole (pitch * M floats); device Y is written in place
         const size_t y_floats = (M - 1) * pitch + N;
-        if (call.map(Y, y_floats * sizeof(float), pitch != N, true, &y, pitch == N && !gathers)) return 1;
-        y_on_host = call.direct();
+        if (call.map(Y, y_floats * sizeof(float), pitch != N, true, &y)) return 1;
         if ((reinterpret_cast<uintptr_t>(w) & (fmt == F_Q4_K_I16 ? 15u : 1u)) || (reinterpret_cast<uintptr_t>(xq) & (act == F_Q8_K ? 3u : 1u)) ||
             (reinterpret_cast<uintptr_t>(y) & 3u) || (x && (reinterpret_cast<uintptr_t>(x) & 3u)))
             return fail("a buffer does not meet its Encoding alignment");
@@ -465,7 +461,7 @@ struct MulMat {
     }
 
     void add_to(Key &key) const {
-        key.add(fmt, path, w, x, xq, y, gr, sg, pw, (const void *)planes, n, k, m, ldy, have_xq, fuse_quantize, y_on_host);
+        key.add(fmt, path, w, x, xq, y, gr, sg, pw, (const void *)planes, n, k, m, ldy, have_xq, fuse_quantize);
     }
 
     int enqueue(cudaStream_t stream, const GatherArgs *gather = nullptr) const {
@@ -483,7 +479,7 @@ struct MulMat {
                 if (launched(launch_prefill_pair(pa, sms, stream), "prefill mul_mat", 2)) return 1;   // its plane kernel first
             } else {
                 GemvArgs ga{fmt, w, xq, fuse_quantize ? (const float *)x : nullptr, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw,
-                            (float *)y, n, k, m, ldy, g.status_dev, y_on_host};
+                            (float *)y, n, k, m, ldy, g.status_dev};
                 gathered = gather && gemv_gathers(ga);
                 if (gathered) ga.gather = *gather;
                 if (launched(launch_gemv(ga, sms, stream), "decode mul_mat")) return 1;
@@ -500,7 +496,7 @@ int do_mul_mat(int fmt, const void *W, const float *X, void *Xq, const int8_t *g
     if (ensure_init(-1)) return 1;
     Call call;
     MulMat op;
-    if (op.prepare(call, fmt, W, X, Xq, grid, signs, powers, Y, N, K, M, ldy, flags, vec_dot_only, gather != nullptr)) return 1;
+    if (op.prepare(call, fmt, W, X, Xq, grid, signs, powers, Y, N, K, M, ldy, flags, vec_dot_only)) return 1;
     if (op.path == MulMat::NOTHING) return 0;
     if (const size_t bytes = op.plane_bytes()) CU(workspace(bytes, g.stream, &op.planes));
     if (gather) call.not_repeatable();       // its kernels meet the other ranks' in a fixed order of launches
@@ -795,7 +791,7 @@ int weft_b200_mul_mat_chain(const weft_b200_mul_mat_step *steps, size_t count) {
     std::vector<MulMat> ops(count);
     for (size_t i = 0; i < count; ++i) {
         const weft_b200_mul_mat_step &s = steps[i];
-        if (ops[i].prepare(call, s.format, s.W, s.X, s.Xq, s.grid, s.signs, s.powers, s.Y, s.N, s.K, s.M, s.N, s.flags, false, false)) return 1;
+        if (ops[i].prepare(call, s.format, s.W, s.X, s.Xq, s.grid, s.signs, s.powers, s.Y, s.N, s.K, s.M, s.N, s.flags, false)) return 1;
     }
     size_t plane_bytes = 0;              // the steps follow each other: one workspace serves them all
     for (const MulMat &op : ops) plane_bytes = op.plane_bytes() > plane_bytes ? op.plane_bytes() : plane_bytes;

@@ -180,12 +180,8 @@ __device__ void q4k_stage_records(const uint8_t *__restrict__ xq, int nb, uint8_
 
 namespace {
 
-// MODE 0: one matrix; 1: grouped launch over several matrices; 2: one matrix with the peer all-gather; 3: one matrix
-// whose results go to pinned host memory: they are collected in shared memory and one warp stores them when the CTA
-// is done, neighbouring rows in one instruction (a store to host memory crosses PCIe by itself; measured 29.3 -> 26.7 us
-// per call with host X, Xq and Y against one store per pair of rows as it completes).  Separate instantiations, so that the
-// single-matrix kernel carries none of the others' code.
-constexpr int QK_HOST_ROWS = 512;   // rows per CTA that MODE 3 can collect
+// MODE 0: one matrix; 1: grouped launch over several matrices; 2: one matrix with the peer all-gather.  Separate instantiations,
+// so that the single-matrix kernel carries none of the others' code.
 template <bool QX, bool XREG, int MODE>
 __global__ void __launch_bounds__(QK_MAX_THREADS) gemv_q4k_kernel(const Q4kParams p) {
     extern __shared__ __align__(128) uint8_t smem[];
@@ -272,7 +268,6 @@ __global__ void __launch_bounds__(QK_MAX_THREADS) gemv_q4k_kernel(const Q4kParam
         return;
     }
 
-    __shared__ float s_out[MODE == 3 ? QK_HOST_ROWS : 1];
     const int tasks = 2 * nb;
     const int consumers = (blockDim.x >> 5) - 1;
     const uint32_t xq_addr = smem_addr(s_xq), aux_addr = smem_addr(s_aux);
@@ -348,8 +343,6 @@ __global__ void __launch_bounds__(QK_MAX_THREADS) gemv_q4k_kernel(const Q4kParam
             if (MODE == 1) {
                 const int sg = segment_of(p, grow);
                 p.seg_y[sg][grow - p.seg_begin[sg]] = v;
-            } else if (MODE == 3) {
-                s_out[tt] = v;
             } else {
                 y[grow] = v;
             }
@@ -361,16 +354,6 @@ __global__ void __launch_bounds__(QK_MAX_THREADS) gemv_q4k_kernel(const Q4kParam
                                                        : tail_begin + (tt - (p.full_rounds << LSR));
             gather_store_spread(p.gather, epoch, blockIdx.y, grow, p.ldy, v, lane & 15);
         }
-    }
-    if (MODE == 3) {
-        __syncthreads();   // the producer warp and any consumer that gave up have exited: they count as arrived
-        if (warp == 1)
-            for (int tt = lane; tt < rows_here; tt += 32) {
-                const int ss = tt >> LSR;
-                const long long grow = ss < p.full_rounds ? ((((long long)ss * G + b) << LSR) + (tt & (SR - 1)))
-                                                           : tail_begin + (tt - (p.full_rounds << LSR));
-                y[grow] = s_out[tt];
-            }
     }
     if (MODE == 2) {
         // a few CTAs receive for the whole grid; the others are done
@@ -484,14 +467,12 @@ cudaError_t launch_gemv_q4k(const GemvArgs &a, int sm_count, cudaStream_t stream
     const int threads = (consumers + 1) * 32;
     dim3 grid((unsigned)ctas, (unsigned)(p.segments ? 1 : a.m));
     const bool xreg = 2 * p.nb <= 32;
-    const bool collect = a.y_on_host && !p.segments && p.gather.world <= 1 && (long long)p.full_rounds * stage_rows + p.tail_rows <= QK_HOST_ROWS;
-    const int mode = p.segments ? 1 : p.gather.world > 1 ? 2 : collect ? 3 : 0;
+    const int mode = p.segments ? 1 : p.gather.world > 1 ? 2 : 0;
 #define WEFT_Q4K_LAUNCH(MODE)                                                                                                                  \
     (a.x ? (xreg ? launch_variant<true, true, MODE>(p, grid, threads, plan.smem, stream) : launch_variant<true, false, MODE>(p, grid, threads, plan.smem, stream)) \
          : (xreg ? launch_variant<false, true, MODE>(p, grid, threads, plan.smem, stream) : launch_variant<false, false, MODE>(p, grid, threads, plan.smem, stream)))
     if (mode == 1) return WEFT_Q4K_LAUNCH(1);
     if (mode == 2) return WEFT_Q4K_LAUNCH(2);
-    if (mode == 3) return WEFT_Q4K_LAUNCH(3);
     return WEFT_Q4K_LAUNCH(0);
 #undef WEFT_Q4K_LAUNCH
 }
