@@ -86,22 +86,54 @@ size_t fold_plane_bytes(const TileArgs &a) {
 // 1800 clocks when A has buffers for two (up to 80 tokens with a min term, 64 without) and 2350 with one, twice that for
 // Q6_K's two limbs, and hardly depends on the tokens (measured from 16 to 128); a tile's start, its stores and the meeting of
 // the slices are small beside it.
+template <int FMT> static int fold_a_buffers(int nt) { return FoldFormat<FMT>::COLS * nt + 4 * 64 <= 512 ? 4 : 2; }
+template <int FMT>
+static double fold_tile_cost(int nt, int abufs, long long steps) {
+    using F = FoldFormat<FMT>;
+    const double step = F::LIMBS * (abufs >= 2 * F::CHUNKS || (F::LIMBS == 2 && nt <= 64) ? 1800.0 : 2350.0);
+    return steps * step + 1200.0 + 4.0 * nt;
+}
+
 template <int FMT>
 static FoldPlan fold_plan(long long m, long long n, long long nb, int sm_count) {
     using F = FoldFormat<FMT>;
     FoldPlan best{0, 0, 0, 0, 0.0};
     const long long row_tiles = (n + FD_ROWS - 1) / FD_ROWS;
     for (int nt = 16; nt <= FD_TOKENS; nt += 16) {
-        const int stages = fold_stages<FMT>(nt), abufs = F::COLS * nt + 4 * 64 <= 512 ? 4 : 2;
+        const int stages = fold_stages<FMT>(nt), abufs = fold_a_buffers<FMT>(nt);
         if (stages < 2 || abufs < F::CHUNKS) continue;
         const long long tiles = row_tiles * ((m + nt - 1) / nt);
         for (int slices = 1; slices <= 8 && slices <= nb; ++slices) {
             if (slices > 1 && tiles > fold_clusters<FMT>(slices)) break;
             const long long rounds = slices > 1 ? 1 : (tiles + sm_count - 1) / sm_count, steps = (nb + slices - 1) / slices;
-            const double step = F::LIMBS * (abufs >= 2 * F::CHUNKS || (F::LIMBS == 2 && nt <= 64) ? 1800.0 : 2350.0);
-            const double cost = rounds * (steps * step + 1200.0 + 4.0 * nt) + (slices > 1 ? 1500.0 : 0.0);
+            const double cost = rounds * fold_tile_cost<FMT>(nt, abufs, steps) + (slices > 1 ? 1500.0 : 0.0);
             if (!best.nt || cost < best.cost) best = FoldPlan{nt, slices, stages, abufs, cost};
         }
+    }
+    return best;
+}
+
+// One launch, or two: where the last round of the grid would be nearly empty, the rows of the full rounds go first and the others
+// follow as a launch of their own, which can share K among the SMs (512 x 14336 x 4096: 448 tiles of 128 tokens are three rounds
+// of 148 and four tiles: 92.7 us as one launch, 86.0 as two; Q6_K 152 and 131; 200 x 28672 x 4096 Q4_K 106 and 82).
+struct FoldSplit { FoldPlan first, second; long long rows; };     // rows of the first launch; all of them: no second
+constexpr double FD_SECOND = 12000.0;     // clocks that a second launch costs beside its tiles
+template <int FMT>
+static FoldSplit fold_split(long long m, long long n, long long nb, int sm_count) {
+    using F = FoldFormat<FMT>;
+    FoldSplit best{fold_plan<FMT>(m, n, nb, sm_count), FoldPlan{0, 0, 0, 0, 0.0}, n};
+    double least = best.first.cost;
+    const long long row_tiles = (n + FD_ROWS - 1) / FD_ROWS;
+    for (int nt = 16; nt <= FD_TOKENS; nt += 16) {
+        const int stages = fold_stages<FMT>(nt), abufs = fold_a_buffers<FMT>(nt);
+        if (stages < 2 || abufs < F::CHUNKS) continue;
+        const long long token_tiles = (m + nt - 1) / nt, rounds = row_tiles * token_tiles / sm_count, rows = rounds * sm_count / token_tiles * FD_ROWS;
+        if (rows <= 0 || rows > n - 8) continue;          // the second launch needs a whole super-row
+        const FoldPlan rest = fold_plan<FMT>(m, n - rows, nb, sm_count);
+        const double cost = rounds * fold_tile_cost<FMT>(nt, abufs, nb);
+        if (!rest.nt || cost + rest.cost + FD_SECOND >= least) continue;
+        least = cost + rest.cost + FD_SECOND;
+        best = FoldSplit{FoldPlan{nt, 1, stages, abufs, cost}, rest, rows};
     }
     return best;
 }
@@ -114,13 +146,15 @@ static int fold_window(int fmt) {
     }
 }
 
-static FoldPlan plan_for(int fmt, long long m, long long n, long long nb, int sm_count) {
+static FoldSplit split_for(int fmt, long long m, long long n, long long nb, int sm_count) {
     switch (fmt) {
-#define FD_PLAN(FMT) case FMT: return fold_plan<FMT>(m, n, nb, sm_count);
-    FD_EACH_FORMAT(FD_PLAN)
-    default: return FoldPlan{0, 0, 0, 0, 0.0};
+#define FD_SPLIT(FMT) case FMT: return fold_split<FMT>(m, n, nb, sm_count);
+    FD_EACH_FORMAT(FD_SPLIT)
+    default: return FoldSplit{};
     }
 }
+
+int fold_launches(const TileArgs &a, int sm_count) { return split_for(a.fmt, a.m, a.n, a.k / 256, sm_count).second.nt ? 3 : 2; }
 
 bool fold_supported(const TileArgs &a) {
     if (a.fmt != F_Q4_K && a.fmt != F_Q5_K && a.fmt != F_Q6_K) return false;
@@ -134,44 +168,53 @@ bool fold_supported(const TileArgs &a) {
     return a.m < (1 << 20) && a.k % 256 == 0 && a.k < (1LL << 22) && a.n >= 8 && a.n < (1LL << 31) && (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0;
 }
 
-cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream) {
-    const FoldPlaneSizes s = plane_sizes(a.fmt, a.m, a.k);
-    uint4 *codes = reinterpret_cast<uint4 *>(planes);
-    float *xd = reinterpret_cast<float *>(planes + s.codes);
-    __half *mins = reinterpret_cast<__half *>(planes + s.codes + s.xd);
-    cudaError_t e = s.mins ? launch_planes<true>(a, codes, xd, mins, s.pitch, stream) : launch_planes<false>(a, codes, xd, mins, s.pitch, stream);
-    if (e != cudaSuccess) return e;
-    FoldParams p{};
-    p.w = static_cast<const uint8_t *>(a.w);
-    p.xd = xd; p.y = a.y; p.n = a.n; p.ldy = a.ldy; p.pitch = s.pitch; p.status = status;
-    p.m = (int)a.m;
-    p.nb = (int)(a.k / 256);
-    p.row_bytes = (long long)p.nb * unit_bytes(a.fmt);
-    p.w_bytes = p.row_bytes * a.n;
-    const FoldPlan plan = plan_for(a.fmt, a.m, a.n, p.nb, sm_count);
-    if (!plan.nt) return cudaErrorNotSupported;
+// The contraction of `n` rows from `w` on into `y`; `planes` holds what does not depend on the cut.
+static cudaError_t launch_rows(const TileArgs &a, const FoldPlan &plan, const FoldParams &planes, const uint4 *codes, const __half *mins,
+                               const uint8_t *w, float *y, long long n, int sm_count, cudaStream_t stream) {
+    FoldParams p = planes;
+    p.w = w; p.y = y; p.n = n;
+    p.w_bytes = p.row_bytes * n;
     p.nt = plan.nt; p.slices = plan.slices; p.b_stages = plan.stages; p.a_buffers = plan.a_buffers;
     p.token_tiles = (int)((a.m + p.nt - 1) / p.nt);
-    p.tiles = p.token_tiles * (int)((a.n + FD_ROWS - 1) / FD_ROWS);
-    CUtensorMap x_codes, x_mins;
-    e = encode_tile_map(&x_codes, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, codes, (unsigned long long)a.k, (unsigned long long)a.m, (unsigned long long)a.k * 2, 64, (unsigned)p.nt, true);
-    if (e == cudaSuccess && s.mins)
+    p.tiles = p.token_tiles * (int)((n + FD_ROWS - 1) / FD_ROWS);
+    CUtensorMap x_codes, x_mins, w_rows;
+    cudaError_t e = encode_tile_map(&x_codes, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, codes, (unsigned long long)a.k, (unsigned long long)a.m, (unsigned long long)a.k * 2, 64, (unsigned)p.nt, true);
+    if (e == cudaSuccess && mins)
         e = encode_tile_map(&x_mins, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, mins, (unsigned long long)p.nb * 16, (unsigned long long)a.m, (unsigned long long)p.nb * 32, 8, (unsigned)p.nt, false);
     else x_mins = x_codes;
     // weight records: rows of words, or (fold.cuh) super-rows of eight rows; rows after the last whole super-row are fetched by
-    // the expanders, so fewer than eight rows need no map
-    CUtensorMap w_rows = x_codes;
+    // the expanders
     const int unit = unit_bytes(a.fmt);
     if (e == cudaSuccess && unit % 16 == 0)
-        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT32, a.w, (unsigned long long)p.row_bytes / 4, (unsigned long long)a.n, (unsigned long long)p.row_bytes, (unsigned)unit / 4, FD_ROWS, false);
+        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT32, w, (unsigned long long)p.row_bytes / 4, (unsigned long long)n, (unsigned long long)p.row_bytes, (unsigned)unit / 4, FD_ROWS, false);
     else if (e == cudaSuccess)
-        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT8, a.w, (unsigned long long)p.row_bytes * 8, (unsigned long long)a.n / 8, (unsigned long long)p.row_bytes * 8, (unsigned)fold_window(a.fmt), 16, false);
+        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT8, w, (unsigned long long)p.row_bytes * 8, (unsigned long long)n / 8, (unsigned long long)p.row_bytes * 8, (unsigned)fold_window(a.fmt), 16, false);
     if (e != cudaSuccess) return e;
     switch (a.fmt) {
 #define FD_LAUNCH(FMT) case FMT: return launch_fold_kernel<FMT>(p, x_codes, x_mins, w_rows, sm_count, stream);
     FD_EACH_FORMAT(FD_LAUNCH)
     default: return cudaErrorNotSupported;
     }
+}
+
+cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream) {
+    const FoldPlaneSizes s = plane_sizes(a.fmt, a.m, a.k);
+    uint4 *codes = reinterpret_cast<uint4 *>(planes);
+    float *xd = reinterpret_cast<float *>(planes + s.codes);
+    __half *mins = s.mins ? reinterpret_cast<__half *>(planes + s.codes + s.xd) : nullptr;
+    FoldParams p{};
+    p.xd = xd; p.ldy = a.ldy; p.pitch = s.pitch; p.status = status;
+    p.m = (int)a.m;
+    p.nb = (int)(a.k / 256);
+    p.row_bytes = (long long)p.nb * unit_bytes(a.fmt);
+    const FoldSplit split = split_for(a.fmt, a.m, a.n, p.nb, sm_count);
+    if (!split.first.nt) return cudaErrorNotSupported;
+    cudaError_t e = mins ? launch_planes<true>(a, codes, xd, mins, s.pitch, stream) : launch_planes<false>(a, codes, xd, mins, s.pitch, stream);
+    const uint8_t *w = static_cast<const uint8_t *>(a.w);
+    if (e == cudaSuccess) e = launch_rows(a, split.first, p, codes, mins, w, a.y, split.rows, sm_count, stream);
+    if (e == cudaSuccess && split.second.nt)
+        e = launch_rows(a, split.second, p, codes, mins, w + split.rows * p.row_bytes, a.y + split.rows, a.n - split.rows, sm_count, stream);
+    return e;
 }
 
 }  // namespace weft
