@@ -25,3 +25,9 @@ def test_rows_at_any_even_address(torch, weft, oracle, golden, name, shape):  # 
 @pytest.mark.parametrize("mnk", [(1, 3, 256), (2, 1193, 2816)])
 def test_quantizing_launch(torch, weft, oracle, golden, name, mnk):  # noqa: F811
     parity.test_mul_mat_decode(torch, weft, oracle, golden, name, mnk)
+
+
+@pytest.mark.parametrize("mnk", [(1, 1, 256), (1, 5, 1024), (1, 301, 2048), (1, 300, 2304), (2, 149, 4352), (1, 3001, 6144), (1, 301, 6400)])
+def test_q4_k_rows_by_half_warps(torch, weft, oracle, golden, mnk):  # noqa: F811
+    """Up to 16 half-records of a row left after whole passes of 32 go to half a warp per row: K at both sides of the line."""
+    parity.test_mul_mat_decode(torch, weft, oracle, golden, "q4_k", mnk)

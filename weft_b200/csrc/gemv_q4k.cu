@@ -35,6 +35,7 @@
 #include "kernels.h"
 #include "ring.cuh"
 
+#include <algorithm>
 #include <climits>
 #include <cstdlib>
 
@@ -115,6 +116,27 @@ __device__ __forceinline__ void half_record2(uint32_t q0, uint32_t q1, const uin
     const int m1 = ps[0] * (int)byte_of(mn1, 0) + ps[1] * (int)byte_of(mn1, 1) + ps[2] * (int)byte_of(mn1, 2) + ps[3] * (int)byte_of(mn1, 3);
     r0 = half_bits_to_float(h0.x) * (float)i0 - half_bits_to_float(h0.x >> 16) * (float)m0;
     r1 = half_bits_to_float(h1.x) * (float)i1 - half_bits_to_float(h1.x >> 16) * (float)m1;
+}
+
+// The same for one row
+__device__ __forceinline__ float half_record1(uint32_t q, const uint4 &head, int h, const uint32_t (&xr)[32], const int (&ps)[4]) {
+    const Q4KScales s = q4k_unpack_scales(head.y, head.z, head.w);
+    const uint32_t sc = h ? s.sc_hi : s.sc_lo, mn = h ? s.mn_hi : s.mn_lo;
+    int isum = 0;
+#pragma unroll
+    for (int jj = 0; jj < 2; ++jj) {
+        const uint4 a = lds128(q + 32 * jj), b = lds128(q + 32 * jj + 16);
+        const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+        int lo[2] = {0, 0}, hi[2] = {0, 0};                       // two chains each
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            lo[i & 1] = dp4a_us(w[i] & 0x0f0f0f0fu, xr[16 * jj + i], lo[i & 1]);
+            hi[i & 1] = dp4a_us(w[i] & 0xf0f0f0f0u, xr[16 * jj + 8 + i], hi[i & 1]);
+        }
+        isum += (lo[0] + lo[1]) * (int)byte_of(sc, 2 * jj) + ((hi[0] + hi[1]) >> 4) * (int)byte_of(sc, 2 * jj + 1);
+    }
+    const int m = ps[0] * (int)byte_of(mn, 0) + ps[1] * (int)byte_of(mn, 1) + ps[2] * (int)byte_of(mn, 2) + ps[3] * (int)byte_of(mn, 3);
+    return half_bits_to_float(head.x) * (float)isum - half_bits_to_float(head.x >> 16) * (float)m;
 }
 
 // fp32 row -> staged Q8_K records (codes at u*QK_XQ_PITCH, aux {d, pair sums}); optionally also to global.
@@ -313,8 +335,7 @@ __global__ void __launch_bounds__(QK_MAX_THREADS) gemv_q4k_kernel(const Q4kParam
                 acc1 = xd * r1;
             }
         } else {
-            for (int task = lane; task < tasks; task += 32) {
-                const int r = task >> 1, h = task & 1;
+            auto load_x = [&](int r, int h) {
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const uint4 v = lds128(xq_addr + r * QK_XQ_PITCH + 128 * h + 16 * i);
@@ -323,12 +344,26 @@ __global__ void __launch_bounds__(QK_MAX_THREADS) gemv_q4k_kernel(const Q4kParam
                 const uint4 pv = lds128(aux_addr + r * QK_XAUX + 16 + 16 * h);
                 ps[0] = (int)pv.x; ps[1] = (int)pv.y; ps[2] = (int)pv.z; ps[3] = (int)pv.w;
                 xd = __uint_as_float(lds32(aux_addr + r * QK_XAUX));
+            };
+            // Up to sixteen tasks left over: half the warp takes each row's, in place of a pass that leaves the other half idle
+            int base = 0;
+            for (; tasks - base > 16; base += 32) {
+                const int task = base + lane, r = task >> 1, h = task & 1;
+                if (task >= tasks) continue;
+                load_x(r, h);
                 const uint32_t rec0 = row0 + r * 144, rec1 = row1 + r * 144;
                 const uint4 h0 = lds128(rec0), h1 = lds128(rec1);
                 float r0, r1;
                 half_record2(rec0 + 16 + 64 * h, rec1 + 16 + 64 * h, h0, h1, h, xr, ps, r0, r1);
                 acc0 += xd * r0;
                 acc1 += xd * r1;
+            }
+            const int task = base + (lane & 15), r = task >> 1, h = task & 1;
+            if (task < tasks) {
+                load_x(r, h);
+                const uint32_t rec = (lane < 16 ? row0 : row1) + r * 144;
+                const float v = xd * half_record1(rec + 16 + 64 * h, lds128(rec), h, xr, ps);
+                if (lane < 16) acc0 += v; else acc1 += v;
             }
         }
         // two sums, five shuffles: the halves of the warp swap, then each half reduces one row
@@ -367,10 +402,13 @@ __global__ void __launch_bounds__(QK_MAX_THREADS) gemv_q4k_kernel(const Q4kParam
 // Measured on B200 for 14336 x 4096: 18 KB stages, 8-deep ring (147 KB in flight per SM), 15 consumer warps.
 constexpr int kQ4kConsumers = 15;
 constexpr int kQ4kStageBytes = 18432;
-constexpr int kQ4kMaxStages = 8;
+// rows of 2448 bytes come four to a stage: sixteen such stages hold what fifteen warps of two rows need (14336 x 4352: 11.5 us with
+// eight, 9.6 with sixteen; 4096 x 8448 7.8 and 6.6)
+constexpr int kQ4kMaxStages = 16;
 constexpr int kQ4kOverlap = 1;
 constexpr int kQ4kSmemCap = 200;   // per-CTA shared-memory budget tried first
-constexpr int kQ4kInflight = 3;   // measured: 2 -> 7.8 us, 3 -> 7.05, 4 -> 7.14, 6 -> 7.6, 8 -> 8.1
+// copies outstanding, in full stages (more of smaller ones, for the same bytes on the way)
+constexpr int kQ4kInflightBytes = 3 * kQ4kStageBytes;   // measured: 2 -> 7.8 us, 3 -> 7.05, 4 -> 7.14, 6 -> 7.6, 8 -> 8.1
 
 template <bool QX, bool XREG, int MODE>
 cudaError_t launch_variant(const Q4kParams &p, dim3 grid, int threads, size_t smem, cudaStream_t stream) {
@@ -434,9 +472,11 @@ bool gemv_q4k_groups(const GemvArgs &a) {
 cudaError_t launch_gemv_q4k(const GemvArgs &a, int sm_count, cudaStream_t stream) {
     Q4kParams p;
     p.w = static_cast<const uint8_t *>(a.w); p.xq = static_cast<const uint8_t *>(a.xq); p.x = a.x; p.y = a.y; p.gather = a.gather;
-    p.n = a.n; p.ldy = a.ldy; p.nb = (int)(a.k / 256); p.status = a.status; p.inflight = kQ4kInflight < 1 ? 1 : kQ4kInflight;
+    p.n = a.n; p.ldy = a.ldy; p.nb = (int)(a.k / 256); p.status = a.status;
     const Q4kPlan plan = plan_q4k(p.nb);
     if (!plan.ok) return cudaErrorInvalidConfiguration;
+    const int stage_bytes = (p.nb * 144) << plan.log_stage_rows;
+    p.inflight = std::max(3, (kQ4kInflightBytes + stage_bytes / 2) / stage_bytes);
     p.log_stage_rows = plan.log_stage_rows; p.log_stages = plan.log_stages;
     const long long stage_rows = 1LL << plan.log_stage_rows;
     p.segments = a.segments > 1 ? a.segments : 0;
