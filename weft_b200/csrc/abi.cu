@@ -185,7 +185,8 @@ class Call {
     // its stores go to the caller's pinned buffer (or the bounce buffer), no staging slice and no copy back.  Not for results,
     // which the whole grid stores a row or two at a time at its end: each of those stores crosses PCIe by itself, and a call with
     // 14336 of them took 30.7 us, with the results in device memory and a copy kernel behind 26.7 (4096 rows: 24.1 and 22.9).
-    int map(const void *ptr, size_t bytes, bool read, bool written, void **out, bool direct = false) {
+    // weights: the kernels fetch them ahead of their wait for the kernel before them.
+    int map(const void *ptr, size_t bytes, bool read, bool written, void **out, bool direct = false, bool weights = false) {
         *out = nullptr;
         if (bytes == 0) { *out = const_cast<void *>(ptr); return 0; }
         if (!ptr) return fail("a required buffer is NULL");
@@ -224,10 +225,10 @@ class Call {
         }
         if (slice(arg)) return 1;
         if (read) {
-            if (arg.mapped) before_.push_back(Copy{arg.dev, arg.mapped, bytes});
+            if (arg.mapped) before_.push_back(Copy{arg.dev, arg.mapped, bytes, !weights});
             else { repeatable_ = false; CU(cudaMemcpyAsync(arg.dev, ptr, bytes, cudaMemcpyHostToDevice, g.stream)); }
         }
-        if (written && arg.mapped) after_.push_back(Copy{arg.mapped, arg.dev, bytes});
+        if (written && arg.mapped) after_.push_back(Copy{arg.mapped, arg.dev, bytes, false});
         *out = arg.dev;
         return 0;
     }
@@ -274,17 +275,17 @@ class Call {
     }
 
   private:
-    struct Copy { void *dst; const void *src; size_t bytes; };
+    struct Copy { void *dst; const void *src; size_t bytes; bool dependents_wait; };
 
     int issue_before(cudaStream_t stream) {
         for (const Copy &c : before_)
-            if (launched(launch_copy_bytes(c.dst, c.src, c.bytes, stream), "argument copy", 0)) return 1;
+            if (launched(launch_copy_bytes(c.dst, c.src, c.bytes, c.dependents_wait, stream), "argument copy", 0)) return 1;
         before_.clear();
         return 0;
     }
     int issue_after(cudaStream_t stream) {
         for (const Copy &c : after_)
-            if (launched(launch_copy_bytes(c.dst, c.src, c.bytes, stream), "result copy", 0)) return 1;
+            if (launched(launch_copy_bytes(c.dst, c.src, c.bytes, c.dependents_wait, stream), "result copy", 0)) return 1;
         return 0;
     }
     template <typename F> void capture(GraphEntry &entry, F &&enqueue) {
@@ -438,7 +439,7 @@ struct MulMat {
         if (fmt == F_Q4_K_I16 && N % 16 != 0) return fail("Q4K_I[16] holds whole cohorts of 16 rows; N = %zu", N);
         n = (long long)N; k = (long long)K; m = (long long)M; ldy = (long long)pitch;
         have_xq = vec_dot_only || (flags & 1u);
-        if (call.map(W, N * row_bytes(fmt, K), true, false, &w)) return 1;
+        if (call.map(W, N * row_bytes(fmt, K), true, false, &w, false, true)) return 1;
         if ((fmt == F_Q6_K || fmt == F_IQ1_M) && (reinterpret_cast<uintptr_t>(w) & 1u) && call.realign(&w, N * row_bytes(fmt, K))) return 1;
         if (!have_xq && call.map(X, M * K * sizeof(float), true, false, &x)) return 1;
         // Decode quantizes X inside the GEMV (its first CTA stores the records, nobody loads them again), so a host Xq can
