@@ -96,3 +96,28 @@ def test_batch_workspace_is_per_stream_and_per_capture(torch, lib, oracle, golde
     small.check()
     large.check()
     del graph
+
+
+def test_batch_workspace_of_a_capture_that_forks(torch, lib, oracle, golden):
+    """Two streams of one capture are branches that may run side by side in the graph: different batches on each, replayed."""
+    left, right = Problem(torch, oracle, golden, "Q4_K", 40, 900, 4096), Problem(torch, oracle, golden, "Q4_K", 37, 900, 4096)
+    side, fork, graph = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    lib.weft_b200_set_async(1)
+    try:
+        with torch.cuda.graph(graph, stream=side):
+            fork.wait_stream(side)
+            for problem, stream in [(left, side), (right, fork)] * 2:
+                lib.weft_b200_set_stream(ctypes.c_void_p(stream.cuda_stream))
+                problem.run(lib)
+            side.wait_stream(fork)
+        for _ in range(5):
+            for problem in (left, right):
+                problem.y.fill_(float("nan"))
+            torch.cuda.synchronize()
+            graph.replay()
+            torch.cuda.synchronize()
+            left.check()
+            right.check()
+    finally:
+        lib.weft_b200_set_stream(None)
+        lib.weft_b200_set_async(0)

@@ -4,8 +4,9 @@
 // first kernel starts after the previous call's last one has read it.  A handful of streams is remembered; a further one
 // takes the place of the longest unused, whose work is waited for first.
 //
-// A captured call may be replayed at any time and on any stream, so a capture gets memory of its own: one buffer per
-// captured graph and size, tied to the graph by a user object.  When the graph and everything instantiated from it are
+// A captured call may be replayed at any time and on any stream, so a capture gets memory of its own: one buffer per stream
+// that takes part in it and size (calls captured on one stream follow each other in the graph, those on streams that the capture
+// forked to may run beside them), tied to the graph by a user object.  When the graph and everything instantiated from it are
 // gone the buffer goes to a free list that the next capture or the next growing stream takes from.
 //
 // Callers hold the library's lock.
@@ -20,7 +21,7 @@ namespace {
 
 struct Buffer { uint8_t *base; size_t bytes; int device; };
 struct StreamBuffer { cudaStream_t stream; int device; Buffer buffer; unsigned long long used; };
-struct CaptureBuffer { unsigned long long id; Buffer buffer; };
+struct CaptureBuffer { unsigned long long id; cudaStream_t stream; Buffer buffer; };
 
 constexpr size_t kStreams = 8, kFree = 8;
 std::vector<StreamBuffer> g_streams;
@@ -84,7 +85,7 @@ cudaError_t workspace(size_t bytes, cudaStream_t stream, uint8_t **out) {
     if (e != cudaSuccess) return e;
     if (status == cudaStreamCaptureStatusActive) {
         for (const CaptureBuffer &c : g_captures)
-            if (c.id == id && c.buffer.bytes >= bytes) { *out = c.buffer.base; return cudaSuccess; }
+            if (c.id == id && c.stream == stream && c.buffer.bytes >= bytes) { *out = c.buffer.base; return cudaSuccess; }
         Buffer b;
         e = obtain(bytes, device, &b);
         if (e != cudaSuccess) return e;
@@ -95,7 +96,7 @@ cudaError_t workspace(size_t bytes, cudaStream_t stream, uint8_t **out) {
         e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
         if (e != cudaSuccess) { cudaUserObjectRelease(object, 1); return e; }
         if (g_captures.size() >= kStreams) g_captures.erase(g_captures.begin());
-        g_captures.push_back(CaptureBuffer{id, b});
+        g_captures.push_back(CaptureBuffer{id, stream, b});
         *out = b.base;
         return cudaSuccess;
     }
