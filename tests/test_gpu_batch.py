@@ -121,3 +121,32 @@ def test_batch_workspace_of_a_capture_that_forks(torch, lib, oracle, golden):
     finally:
         lib.weft_b200_set_stream(None)
         lib.weft_b200_set_async(0)
+
+
+def test_batch_workspace_of_the_per_thread_stream(torch, lib, oracle, golden):
+    """The per-thread default stream is another stream in every thread behind one handle: each thread's calls have their own planes."""
+    import threading
+
+    problems = [Problem(torch, oracle, golden, "Q4_K", m, 900, 4096) for m in (40, 37, 21)]
+    failures = []
+
+    def work(problem):
+        try:
+            for _ in range(20):
+                problem.run(lib)
+            assert lib.weft_b200_synchronize() == 0
+        except BaseException as error:
+            failures.append(error)
+
+    lib.weft_b200_set_async(1)
+    lib.weft_b200_set_stream(ctypes.c_void_p(2))         # cudaStreamPerThread
+    try:
+        threads = [threading.Thread(target=work, args=(problem,)) for problem in problems]
+        for thread in threads: thread.start()
+        for thread in threads: thread.join()
+    finally:
+        lib.weft_b200_set_stream(None)
+        lib.weft_b200_set_async(0)
+    assert not failures
+    for problem in problems:
+        problem.check()

@@ -9,6 +9,10 @@
 // forked to may run beside them), tied to the graph by a user object.  When the graph and everything instantiated from it are
 // gone the buffer goes to a free list that the next capture or the next growing stream takes from.
 //
+// Streams are told apart by their ids, which are never given out twice: a handle is reused once its stream is destroyed (while
+// that stream's last work may still be running), and the per-thread default stream has one handle for every thread.  (A stream
+// that is being captured must not be asked for its id and cannot be destroyed: there the handle, and the thread.)
+//
 // Callers hold the library's lock.
 #include "kernels.h"
 
@@ -20,8 +24,9 @@ namespace weft {
 namespace {
 
 struct Buffer { uint8_t *base; size_t bytes; int device; };
-struct StreamBuffer { cudaStream_t stream; int device; Buffer buffer; unsigned long long used; };
-struct CaptureBuffer { unsigned long long id; cudaStream_t stream; Buffer buffer; };
+struct StreamBuffer { unsigned long long stream; int device; Buffer buffer; unsigned long long used; };
+struct CaptureBuffer { unsigned long long id; const void *stream; Buffer buffer; };
+thread_local char t_thread;                 // its address tells threads apart
 
 constexpr size_t kStreams = 8, kFree = 8;
 std::vector<StreamBuffer> g_streams;
@@ -38,6 +43,16 @@ void give_back(void *p) {                   // no CUDA calls are allowed here
     delete b;
 }
 
+// In this mode a thread may allocate, free and wait while it or another thread captures.
+class Relaxed {
+  public:
+    Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+    ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode_); }
+
+  private:
+    mutable cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+};
+
 // A buffer of at least `bytes`: a returned one that fits without being four times too large, or a new allocation.
 cudaError_t obtain(size_t bytes, int device, Buffer *out) {
     {
@@ -50,12 +65,8 @@ cudaError_t obtain(size_t bytes, int device, Buffer *out) {
             }
     }
     const size_t want = (bytes + bytes / 4 + 65535) & ~size_t(65535);
-    // an allocation is legal while this thread captures, in the relaxed mode
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaThreadExchangeStreamCaptureMode(&mode);
     uint8_t *base = nullptr;
     const cudaError_t e = cudaMalloc(reinterpret_cast<void **>(&base), want);
-    cudaThreadExchangeStreamCaptureMode(&mode);
     if (e != cudaSuccess) return e;
     *out = Buffer{base, want, device};
     return cudaSuccess;
@@ -79,13 +90,15 @@ cudaError_t workspace(size_t bytes, cudaStream_t stream, uint8_t **out) {
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    unsigned long long id = 0;
+    unsigned long long id = 0, stream_id = 0;
     cudaGraph_t graph = nullptr;
+    const Relaxed relaxed;
     e = cudaStreamGetCaptureInfo(stream, &status, &id, &graph);
     if (e != cudaSuccess) return e;
     if (status == cudaStreamCaptureStatusActive) {
+        const void *who = stream == cudaStreamPerThread ? static_cast<const void *>(&t_thread) : stream;
         for (const CaptureBuffer &c : g_captures)
-            if (c.id == id && c.stream == stream && c.buffer.bytes >= bytes) { *out = c.buffer.base; return cudaSuccess; }
+            if (c.id == id && c.stream == who && c.buffer.bytes >= bytes) { *out = c.buffer.base; return cudaSuccess; }
         Buffer b;
         e = obtain(bytes, device, &b);
         if (e != cudaSuccess) return e;
@@ -96,14 +109,16 @@ cudaError_t workspace(size_t bytes, cudaStream_t stream, uint8_t **out) {
         e = cudaGraphRetainUserObject(graph, object, 1, cudaGraphUserObjectMove);
         if (e != cudaSuccess) { cudaUserObjectRelease(object, 1); return e; }
         if (g_captures.size() >= kStreams) g_captures.erase(g_captures.begin());
-        g_captures.push_back(CaptureBuffer{id, stream, b});
+        g_captures.push_back(CaptureBuffer{id, who, b});
         *out = b.base;
         return cudaSuccess;
     }
+    e = cudaStreamGetId(stream, &stream_id);
+    if (e != cudaSuccess) return e;
     drop_surplus();
     StreamBuffer *mine = nullptr;
     for (StreamBuffer &s : g_streams)
-        if (s.stream == stream && s.device == device) mine = &s;
+        if (s.stream == stream_id && s.device == device) mine = &s;
     if (!mine) {
         if (g_streams.size() >= kStreams) {
             size_t oldest = 0;
@@ -115,7 +130,7 @@ cudaError_t workspace(size_t bytes, cudaStream_t stream, uint8_t **out) {
             g_streams.erase(g_streams.begin() + oldest);
             ++g_generation;
         }
-        g_streams.push_back(StreamBuffer{stream, device, Buffer{nullptr, 0, device}, 0});
+        g_streams.push_back(StreamBuffer{stream_id, device, Buffer{nullptr, 0, device}, 0});
         mine = &g_streams.back();
     }
     mine->used = ++g_clock;
