@@ -100,6 +100,11 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) {
     asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmul.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
     return d;
 }
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    float2 d;
+    asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tadd.rn.f32x2 z, x, y;\n\tmov.b64 {%0, %1}, z;\n\t}" : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return d;
+}
 __device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
     float2 d;
     asm("{\n\t.reg .b64 x, y, z;\n\tmov.b64 x, {%2, %3};\n\tmov.b64 y, {%4, %5};\n\tmov.b64 z, {%6, %7};\n\tfma.rn.f32x2 z, x, y, z;\n\tmov.b64 {%0, %1}, z;\n\t}"
@@ -369,8 +374,8 @@ __device__ __forceinline__ void tile_half(const uint8_t *stage, int lane, const 
         const uint4 q0 = *reinterpret_cast<const uint4 *>(group + 1024 * H + 16 * lane), q1 = *reinterpret_cast<const uint4 *>(group + 1024 * H + 512 + 16 * lane);
         const uint32_t b[4][2] = {{q0.x, q0.y}, {q0.z, q0.w}, {q1.x, q1.y}, {q1.z, q1.w}};
         if constexpr (F::PAIR32) {
-            // acc += (isum * d_w) * d_x per group.  isum * d_w is one fused multiply-add on the biased accumulator: the product
-            // bias * d_w has 13 significant bits, so the sum is isum * d_w rounded once
+            // acc += (isum * d_w) * d_x per group.  The bias comes off first, exactly: inside a multiply-add, as -bias * d_w, it
+            // would make NaN of every sum under an infinite d_w
 #pragma unroll
             for (int g = 0; g < 4; ++g) {
                 const float2 dx = *reinterpret_cast<const float2 *>(group + 2048 + 32 * (4 * H + g) + 8 * t);
@@ -380,8 +385,8 @@ __device__ __forceinline__ void tile_half(const uint8_t *stage, int lane, const 
                     mma_k32(d, wt.a[mt][g], b[g][0], b[g][1], MAGIC, MAGIC);
 #pragma unroll
                     for (int e = 0; e < 2; ++e) {
-                        const float dw = wt.dw[mt][e][g], back = -12582912.0f * dw;
-                        const float2 v = fma2(make_float2(__int_as_float(d[2 * e]), __int_as_float(d[2 * e + 1])), make_float2(dw, dw), make_float2(back, back));
+                        const float dw = wt.dw[mt][e][g];
+                        const float2 v = mul2(add2(make_float2(__int_as_float(d[2 * e]), __int_as_float(d[2 * e + 1])), make_float2(-12582912.0f, -12582912.0f)), make_float2(dw, dw));
                         fma2_into(acc[nt][mt][2 * e], acc[nt][mt][2 * e + 1], v, dx);
                     }
                 }
