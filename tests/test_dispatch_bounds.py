@@ -1,0 +1,36 @@
+"""Bounds of the batch kernels' dispatch rules, called in the built library without a device."""
+from __future__ import annotations
+
+import ctypes
+
+import pytest
+
+UNIT_BYTES = {1: 144, 5: 272, 6: 84, 7: 110, 8: 144, 9: 176, 10: 210, 15: 66, 20: 54}      # Q4_0 Q8_0 Q2_K Q3_K Q4_K Q5_K Q6_K IQ2_XXS TQ1_0
+
+
+class TileArgs(ctypes.Structure):               # weft::TileArgs of csrc/kernels.h
+    _fields_ = [("fmt", ctypes.c_int)] + [(name, ctypes.c_void_p) for name in ("w", "x", "xq", "grid", "signs", "powers", "y")] + \
+               [(name, ctypes.c_longlong) for name in ("n", "k", "m", "ldy")]
+
+
+@pytest.fixture(scope="module")
+def tile_supported():
+    from weft_b200.build import ensure_built
+
+    rule = ctypes.CDLL(str(ensure_built()))["_ZN4weft14tile_supportedERKNS_8TileArgsE"]
+    rule.restype, rule.argtypes = ctypes.c_bool, [ctypes.POINTER(TileArgs)]
+    return lambda fmt, m, n, k, w=1 << 20: rule(TileArgs(fmt, w, 1, 1, 1, 1, 1, 1, n, k, m, n))
+
+
+@pytest.mark.parametrize("fmt", UNIT_BYTES)
+def test_tile_rows_keep_to_32_bit_offsets(tile_supported, fmt):
+    """A warp reaches its 32 rows and the 16-byte window around the last record of each by 32-bit offsets."""
+    assert tile_supported(fmt, 3, 64, 256 * 1024)
+    for blocks in sorted({1 << shift for shift in range(24)} | {(1 << 32) // 32 // UNIT_BYTES[fmt] + step for step in (-2, -1, 0, 1)}):
+        fits = 32 * blocks * UNIT_BYTES[fmt] + 32 <= 1 << 32
+        assert fits or not tile_supported(fmt, 3, 64, 256 * blocks), blocks
+    assert tile_supported(fmt, 3, 64, 256 * ((1 << 32) // 32 // UNIT_BYTES[fmt] - 1))
+
+
+def test_tile_sizes_that_are_left_to_others(tile_supported):
+    assert not tile_supported(8, 2, 64, 4096) and not tile_supported(8, 3, 64, 4096 + 32) and not tile_supported(8, 3, 64, 4096, w=(1 << 20) + 8)
