@@ -29,7 +29,8 @@ def test_tile_rows_keep_to_32_bit_offsets(tile_supported, fmt):
     for blocks in sorted({1 << shift for shift in range(24)} | {(1 << 32) // 32 // UNIT_BYTES[fmt] + step for step in (-2, -1, 0, 1)}):
         fits = 32 * blocks * UNIT_BYTES[fmt] + 32 <= 1 << 32
         assert fits or not tile_supported(fmt, 3, 64, 256 * blocks), blocks
-    assert tile_supported(fmt, 3, 64, 256 * ((1 << 32) // 32 // UNIT_BYTES[fmt] - 1))
+    assert tile_supported(fmt, 3, 64, 256 * min(1 << 20, (1 << 32) // 32 // UNIT_BYTES[fmt] - 1))
+    assert not tile_supported(fmt, 3, 64, 256 * ((1 << 20) + 1))
 
 
 def test_tile_sizes_that_are_left_to_others(tile_supported):

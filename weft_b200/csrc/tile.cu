@@ -129,7 +129,7 @@ bool tile_supported(const TileArgs &a) {
     // From three tokens on: up to there a GEMV per token row, which reads the matrix each time, is as quick (two tokens,
     // 14336 x 4096: Q4_K 13.6 us against 16 us, Q6_K 20 against 24; three: 19.6 and 28.9 against the same).
     // 16-byte copies of weight rows need a 16-byte aligned matrix; offsets within a warp's 32 rows are 32-bit in the kernel
-    return tile_format(a.fmt) && a.m >= 3 && a.m <= (1 << 20) && a.k % 256 == 0 && a.k / 256 <= 0xffffff00LL / 32 / unit_bytes(a.fmt) &&
+    return tile_format(a.fmt) && a.m >= 3 && a.m <= (1 << 20) && a.k % 256 == 0 && a.k / 256 <= std::min(1LL << 20, 0xffffff00LL / 32 / unit_bytes(a.fmt)) &&
            (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0;
 }
 
