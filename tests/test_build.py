@@ -1,0 +1,54 @@
+"""The CUDA library builds and resolves without the native call path: that one needs a C++ compiler and Python's headers."""
+from __future__ import annotations
+
+import os
+import shutil
+import sysconfig
+
+import pytest
+
+from weft_b200 import build
+
+
+@pytest.fixture
+def tree(monkeypatch, tmp_path):
+    """A package folder of its own whose nvcc only makes its output file."""
+    sources = tmp_path / "csrc"
+    sources.mkdir()
+    for name in ("one.cu", "pycall.cpp"):
+        (sources / name).write_text("#error\n")
+    fake = tmp_path / "nvcc"
+    fake.write_text('#!/bin/sh\nwhile [ "$1" != "-o" ]; do shift; done\n: > "$2"\n')
+    fake.chmod(0o755)
+    for name, value in {"PACKAGE": tmp_path, "CSRC": sources, "LIBRARY": tmp_path / "lib.so", "PYCALL": tmp_path / build.PYCALL.name,
+                        "SOURCES": ["one.cu"], "HEADERS": [], "_fresh_until": 0.0}.items():
+        monkeypatch.setattr(build, name, value)
+    monkeypatch.setattr(build, "nvcc", lambda: str(fake))
+    monkeypatch.delenv("WEFT_B200_NO_BUILD", raising=False)
+    return tmp_path
+
+
+@pytest.mark.parametrize("missing", ["compiler", "headers", "nothing"])
+def test_library_without_the_call_path(tree, monkeypatch, missing):
+    """Without g++, without Python.h, and with a pycall.cpp that does not compile."""
+    if missing == "compiler":
+        monkeypatch.setattr(shutil, "which", lambda name: None)
+    if missing == "headers":
+        monkeypatch.setattr(sysconfig, "get_paths", lambda: {"include": str(tree)})
+    assert build.stale()
+    assert build.build() == tree / "lib.so" and (tree / "lib.so").exists()
+    assert not build.PYCALL.exists() and list(tree.glob("*.tmp")) == []
+    monkeypatch.setattr(build, "_fresh_until", 0.0)
+    assert not build.stale()                     # a built library is used as it is, whatever became of the call path
+    assert build.refresh_call_path() is False
+
+
+def test_call_path_is_named_for_its_interpreter():
+    assert build.PYCALL.name == "_pycall" + sysconfig.get_config_var("EXT_SUFFIX")
+
+
+def test_call_path_alone_is_not_a_reason_to_run_nvcc(tree, monkeypatch):
+    (tree / "lib.so").touch()
+    os.utime(tree / "lib.so", (2e9, 2e9))
+    (tree / "csrc" / "pycall.cpp").write_text("int weft_pycall_placeholder;\n")
+    assert not build.stale() and build.refresh_call_path() and build.PYCALL.exists()

@@ -6,6 +6,7 @@ call (it only compiles when a source is newer than the library).
 """
 from __future__ import annotations
 
+import importlib
 import os
 import shutil
 import subprocess
@@ -17,7 +18,8 @@ from pathlib import Path
 PACKAGE = Path(__file__).resolve().parent
 CSRC = PACKAGE / "csrc"
 LIBRARY = PACKAGE / "libweft_b200.so"
-PYCALL = PACKAGE / "_pycall.so"          # extension module: the native call path of CompiledKernel
+# extension module: the native call path of CompiledKernel, for the interpreter that builds it
+PYCALL = PACKAGE / ("_pycall" + sysconfig.get_config_var("EXT_SUFFIX"))
 SOURCES = ["abi.cu", "abi_noalloc.cu", "dequantize.cu", "quantize.cu", "gemv.cu", "gemv_q4k.cu", "gemv_ring.cu", "gemv_q4ki.cu", "prefill_pair.cu", "mma_peak.cu", "gather.cu", "workspace.cu", "tile.cu", "tile_q45.cu", "tile_q236.cu", "tile_q08.cu", "tile_low.cu", "fold.cu", "fold_q45.cu", "fold_q6.cu"]
 HEADERS = ["common.cuh", "quantize.cuh", "kernels.h", "gemv_units.cuh", "ring.cuh", "tcgen05.cuh", "tensormap.cuh", "prefill_common.cuh", "gather.cuh", "tile.cuh", "fold.cuh", "../../include/weft_b200.h"]
 
@@ -53,10 +55,34 @@ def stale() -> bool:
 
 
 def _sources_are_newer() -> bool:
-    if not LIBRARY.exists() or not PYCALL.exists() or (CSRC / "pycall.cpp").stat().st_mtime > PYCALL.stat().st_mtime:
+    if not LIBRARY.exists():
         return True
     built = LIBRARY.stat().st_mtime
     return any((CSRC / name).stat().st_mtime > built for name in SOURCES + HEADERS)
+
+
+def refresh_call_path() -> bool:
+    """Compile the native call path when its source is newer than it.  The library is complete without it (calls then go through
+    ctypes), so a missing C++ compiler, missing Python headers or a failed compilation are no error."""
+    source = CSRC / "pycall.cpp"
+    if PYCALL.exists() and PYCALL.stat().st_mtime >= source.stat().st_mtime:
+        return True
+    include, compiler = Path(sysconfig.get_paths()["include"]), shutil.which("g++")
+    if compiler is None or not (include / "Python.h").exists() or os.environ.get("WEFT_B200_NO_BUILD"):
+        return False
+    fresh = PYCALL.with_name(f"{PYCALL.name}.{os.getpid()}.tmp")
+    try:
+        done = subprocess.run([compiler, "-O2", "-std=c++17", "-shared", "-fPIC", f"-I{include}", str(source), "-o", str(fresh)], capture_output=True, text=True)
+        if done.returncode == 0:
+            os.replace(fresh, PYCALL)
+            importlib.invalidate_caches()
+        else:
+            sys.stderr.write(f"--- {source.name}: not compiled, calls go through ctypes\n{done.stderr}\n")
+        return done.returncode == 0
+    except OSError:              # a package directory that cannot be written
+        return False
+    finally:
+        fresh.unlink(missing_ok=True)
 
 
 def build(verbose: bool = False, extra: list[str] | None = None) -> Path:
@@ -81,12 +107,7 @@ def build(verbose: bool = False, extra: list[str] | None = None) -> Path:
             sys.stderr.write(f"--- nvcc {name}\n{out}\n")
     if failed:
         raise RuntimeError("nvcc failed; see the compiler output above")
-    fresh = PYCALL.with_suffix(f".so.{os.getpid()}.tmp")
-    try:
-        subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", f"-I{sysconfig.get_paths()['include']}", str(CSRC / "pycall.cpp"), "-o", str(fresh)], check=True)
-        os.replace(fresh, PYCALL)
-    finally:
-        fresh.unlink(missing_ok=True)
+    refresh_call_path()
     # link under a temporary name and move it into place: a process that loads the library meanwhile sees the old
     # file or the new one, never a half-written one
     fresh = LIBRARY.with_suffix(f".so.{os.getpid()}.tmp")
@@ -103,6 +124,7 @@ def ensure_built(extra: list[str] | None = None) -> Path:
     """Build when a source is newer than the library.  Several ranks of one job may call this at once: they
     take a file lock in turn, and all but the first find the library fresh."""
     if not stale():
+        refresh_call_path()
         return LIBRARY
     if os.environ.get("WEFT_B200_NO_BUILD"):
         raise RuntimeError(f"{LIBRARY} is missing or stale and WEFT_B200_NO_BUILD is set")

@@ -52,6 +52,8 @@ class Toolchain:
                     build.ensure_built(extra=list(self.cflags))   # file-locked: ranks of one job build once
                 except Exception as error:  # nvcc diagnostics are in the message
                     raise CompilationError(str(error)) from error
+            else:
+                build.refresh_call_path()
         if not library.exists():
             raise CompilationError(f"native toolchain is unavailable: kernel library {library} does not exist")
         return Toolchain(str(library.resolve()), self.cc, self.cflags)
