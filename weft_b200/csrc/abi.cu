@@ -225,10 +225,10 @@ class Call {
         }
         if (slice(arg)) return 1;
         if (read) {
-            if (arg.mapped) before_.push_back(Copy{arg.dev, arg.mapped, bytes, !weights});
+            if (arg.mapped) before_.push_back(Copy{arg.dev, arg.mapped, bytes, weights ? StagedCopy::WEIGHTS : StagedCopy::ACTIVATIONS});
             else { repeatable_ = false; CU(cudaMemcpyAsync(arg.dev, ptr, bytes, cudaMemcpyHostToDevice, g.stream)); }
         }
-        if (written && arg.mapped) after_.push_back(Copy{arg.mapped, arg.dev, bytes, false});
+        if (written && arg.mapped) after_.push_back(Copy{arg.mapped, arg.dev, bytes, StagedCopy::RESULTS});
         *out = arg.dev;
         return 0;
     }
@@ -275,17 +275,17 @@ class Call {
     }
 
   private:
-    struct Copy { void *dst; const void *src; size_t bytes; bool dependents_wait; };
+    struct Copy { void *dst; const void *src; size_t bytes; StagedCopy what; };
 
     int issue_before(cudaStream_t stream) {
         for (const Copy &c : before_)
-            if (launched(launch_copy_bytes(c.dst, c.src, c.bytes, c.dependents_wait, stream), "argument copy", 0)) return 1;
+            if (launched(launch_copy_bytes(c.dst, c.src, c.bytes, c.what, stream), "argument copy", 0)) return 1;
         before_.clear();
         return 0;
     }
     int issue_after(cudaStream_t stream) {
         for (const Copy &c : after_)
-            if (launched(launch_copy_bytes(c.dst, c.src, c.bytes, c.dependents_wait, stream), "result copy", 0)) return 1;
+            if (launched(launch_copy_bytes(c.dst, c.src, c.bytes, c.what, stream), "result copy", 0)) return 1;
         return 0;
     }
     template <typename F> void capture(GraphEntry &entry, F &&enqueue) {

@@ -22,9 +22,9 @@ cudaError_t launch_dequantize(int fmt, const void *w, const int8_t *grid, const 
 
 // dst[0..bytes) = src[0..bytes) by a kernel (either side may be mapped pinned host memory): for the small host
 // arguments of a call this is a few microseconds quicker than a copy-engine transfer between two kernels.
-// dependents_wait: whatever kernel comes next reads dst after its griddepcontrol.wait only and may start early; weights are
-// read before it.
-cudaError_t launch_copy_bytes(void *dst, const void *src, size_t bytes, bool dependents_wait, cudaStream_t stream);
+// What is copied decides how the launch meets its neighbours on the stream.
+enum class StagedCopy { WEIGHTS, ACTIVATIONS, RESULTS };
+cudaError_t launch_copy_bytes(void *dst, const void *src, size_t bytes, StagedCopy what, cudaStream_t stream);
 
 // X (rows, k) fp32 -> Q8_0 / Q8_K records, Weft rounding and tie rules.
 cudaError_t launch_quantize(int act_fmt, const float *x, void *y, long long rows, long long k, int sm_count, cudaStream_t stream);

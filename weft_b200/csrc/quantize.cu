@@ -45,11 +45,13 @@ __global__ void __launch_bounds__(QZ_WARPS * 32) quantize_q8_0_kernel(const floa
 }
 
 // Byte copy for small staged arguments; 16-byte words when both sides allow, whole bytes otherwise.
-// EARLY: the kernel behind this one may start its prologue now (programmatic dependent launch).  Only for what that kernel
-// touches after its wait: the GEMVs fetch their first weights before it, so weights are copied by the other form.
-template <bool EARLY>
+// ACTIVATIONS: the kernel behind this one may start its prologue now (programmatic dependent launch); it waits for this grid
+// before it touches what is copied.  Not for weights: the GEMVs fetch their first ones before that wait.
+// RESULTS: this grid is launched the same way behind the kernel whose results it copies.
+template <StagedCopy WHAT>
 __global__ void __launch_bounds__(256) copy_bytes_kernel(uint8_t *__restrict__ dst, const uint8_t *__restrict__ src, size_t bytes, int vec) {
-    if (EARLY) asm volatile("griddepcontrol.launch_dependents;");
+    if (WHAT == StagedCopy::ACTIVATIONS) asm volatile("griddepcontrol.launch_dependents;");
+    if (WHAT == StagedCopy::RESULTS) asm volatile("griddepcontrol.wait;" ::: "memory");
     const size_t stride = (size_t)gridDim.x * 256, first = (size_t)blockIdx.x * 256 + threadIdx.x;
     if (vec) {
         for (size_t i = first; i < bytes / 16; i += stride) reinterpret_cast<uint4 *>(dst)[i] = reinterpret_cast<const uint4 *>(src)[i];
@@ -59,14 +61,28 @@ __global__ void __launch_bounds__(256) copy_bytes_kernel(uint8_t *__restrict__ d
     }
 }
 
-cudaError_t launch_copy_bytes(void *dst, const void *src, size_t bytes, bool dependents_wait, cudaStream_t stream) {
+cudaError_t launch_copy_bytes(void *dst, const void *src, size_t bytes, StagedCopy what, cudaStream_t stream) {
     if (!bytes) return cudaSuccess;
+    uint8_t *to = static_cast<uint8_t *>(dst);
+    const uint8_t *from = static_cast<const uint8_t *>(src);
     const int vec = ((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15u) == 0;
     size_t ctas = ((vec ? bytes / 16 : bytes) + 255) / 256;
     if (ctas > 64) ctas = 64;
     if (ctas < 1) ctas = 1;
-    if (dependents_wait) copy_bytes_kernel<true><<<(unsigned)ctas, 256, 0, stream>>>(static_cast<uint8_t *>(dst), static_cast<const uint8_t *>(src), bytes, vec);
-    else copy_bytes_kernel<false><<<(unsigned)ctas, 256, 0, stream>>>(static_cast<uint8_t *>(dst), static_cast<const uint8_t *>(src), bytes, vec);
+    if (what == StagedCopy::RESULTS) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)ctas);
+        cfg.blockDim = dim3(256);
+        cfg.stream = stream;
+        cudaLaunchAttribute attribute;
+        attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attribute.val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = &attribute;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, copy_bytes_kernel<StagedCopy::RESULTS>, to, from, bytes, vec);
+    }
+    if (what == StagedCopy::ACTIVATIONS) copy_bytes_kernel<StagedCopy::ACTIVATIONS><<<(unsigned)ctas, 256, 0, stream>>>(to, from, bytes, vec);
+    else copy_bytes_kernel<StagedCopy::WEIGHTS><<<(unsigned)ctas, 256, 0, stream>>>(to, from, bytes, vec);
     return cudaGetLastError();
 }
 
