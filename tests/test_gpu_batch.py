@@ -170,3 +170,28 @@ def test_batch_workspace_of_the_per_thread_stream(torch, lib, oracle, golden):
     assert not failures
     for problem in problems:
         problem.check()
+
+
+def test_batch_calls_beside_a_capture(torch, lib, oracle, golden):
+    """Another stream is being captured, in the mode that forbids unsafe calls everywhere: batches on this one, the second with a
+    larger workspace, neither fail nor spoil the capture."""
+    problems = [Problem(torch, oracle, golden, "Q4_K", m, 200, 1024) for m in (5, 600)]
+    inside = Problem(torch, oracle, golden, "Q6_K", 9, 200, 1024)
+    side, other, graph = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    lib.weft_b200_set_async(1)
+    try:
+        lib.weft_b200_set_stream(ctypes.c_void_p(other.cuda_stream))
+        problems[0].run(lib)
+        other.synchronize()
+        with torch.cuda.graph(graph, stream=side, capture_error_mode="global"):
+            for problem in problems[:1] * 2 + problems[1:]:
+                problem.run(lib)
+            lib.weft_b200_set_stream(ctypes.c_void_p(side.cuda_stream))
+            inside.run(lib)
+        graph.replay()
+    finally:
+        lib.weft_b200_set_stream(None)
+        lib.weft_b200_set_async(0)
+    torch.cuda.synchronize()
+    for problem in problems + [inside]:
+        problem.check()

@@ -50,7 +50,7 @@ class Relaxed {
     ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode_); }
 
   private:
-    mutable cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
+    cudaStreamCaptureMode mode_ = cudaStreamCaptureModeRelaxed;
 };
 
 // A buffer of at least `bytes`: a returned one that fits without being four times too large, or a new allocation.
@@ -78,6 +78,8 @@ void drop_surplus() {                       // outside a capture: keep a few ret
         std::lock_guard<std::mutex> guard(g_returned_lock);
         while (g_returned.size() > kFree) { surplus.push_back(g_returned.front()); g_returned.erase(g_returned.begin()); }
     }
+    if (surplus.empty()) return;
+    Relaxed relaxed;
     for (const Buffer &b : surplus) cudaFree(b.base);
 }
 
@@ -92,13 +94,13 @@ cudaError_t workspace(size_t bytes, cudaStream_t stream, uint8_t **out) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     unsigned long long id = 0, stream_id = 0;
     cudaGraph_t graph = nullptr;
-    const Relaxed relaxed;
     e = cudaStreamGetCaptureInfo(stream, &status, &id, &graph);
     if (e != cudaSuccess) return e;
     if (status == cudaStreamCaptureStatusActive) {
         const void *who = stream == cudaStreamPerThread ? static_cast<const void *>(&t_thread) : stream;
         for (const CaptureBuffer &c : g_captures)
             if (c.id == id && c.stream == who && c.buffer.bytes >= bytes) { *out = c.buffer.base; return cudaSuccess; }
+        Relaxed relaxed;
         Buffer b;
         e = obtain(bytes, device, &b);
         if (e != cudaSuccess) return e;
@@ -119,6 +121,12 @@ cudaError_t workspace(size_t bytes, cudaStream_t stream, uint8_t **out) {
     StreamBuffer *mine = nullptr;
     for (StreamBuffer &s : g_streams)
         if (s.stream == stream_id && s.device == device) mine = &s;
+    if (mine && mine->buffer.bytes >= bytes) {
+        mine->used = ++g_clock;
+        *out = mine->buffer.base;
+        return cudaSuccess;
+    }
+    Relaxed relaxed;
     if (!mine) {
         if (g_streams.size() >= kStreams) {
             size_t oldest = 0;
