@@ -1,6 +1,6 @@
 """Weights in ordinary host memory, other ones at each call: the kernels fetch their first weights ahead of their wait for the
-kernel before them, so the copy that brings host weights must be complete by then.  Eight calls on the same buffers: the later
-ones are replayed from a graph.  Bound: 1e-5 relative L2 (exact integer sums, another order of the fp32 additions)."""
+kernel before them, so the copy that brings host weights must be complete by then.  24 calls on the same buffers: the last
+seven are replayed from a graph.  Bound: 1e-5 relative L2 (exact integer sums, another order of the fp32 additions)."""
 from __future__ import annotations
 
 import numpy as np
@@ -37,7 +37,7 @@ def test_weights_of_this_call(torch, oracle, name, pinned):
     xq = torch.zeros((1, oracle.row_bytes(act_fmt, k)), dtype=torch.uint8, device="cuda")
     y = torch.zeros((1, n), device="cuda")
     args = (Buffer(held, shape=(n, k), encoding=name), Buffer(torch.from_numpy(x).cuda()), Buffer(xq, shape=(1, k), encoding=act), Buffer(y))
-    for call in range(8):
+    for call in range(24):
         held[:] = weights(fmt, rng, n, k)
         kernel(*args)
         want, _ = oracle.mul_mat(fmt, held.copy(), x, n, k, 1, rule=1)
@@ -55,7 +55,7 @@ def test_interleaved_weights_behind_a_large_copy(torch, oracle):
     kernel = weft.compile(mul_mat.production_mul_mat_q4_k_persistent)
     x, held = activations(rng, m, k), np.zeros((n, k // 256 * 144), np.uint8)
     xq, y = np.zeros((m, oracle.row_bytes(oracle.Q8_K, k)), np.uint8), np.zeros((m, n), np.float32)
-    for call in range(8):
+    for call in range(24):
         w = weights(oracle.Q4_K, rng, n, k)
         held[:] = oracle.interleave(oracle.Q4_K, w, k).reshape(held.shape)
         kernel(Buffer(held, shape=(n, k), encoding="Q4K_I[16]"), Buffer(x), Buffer(xq, shape=(m, k), encoding="Q8_K"), Buffer(y))

@@ -6,6 +6,8 @@ import pytest
 
 from helpers import activations, rel_l2, weights
 
+from test_gpu_batch import lib  # noqa: F401  (fixture)
+
 pytestmark = pytest.mark.gpu
 
 
@@ -37,8 +39,8 @@ def test_repeated_call_follows_its_inputs(torch, oracle, m, where):
         x, xq, y = (torch.from_numpy(a).cuda() for a in (x, xq, y))
     args = (w, Buffer(x), Buffer(xq, shape=(m, k), encoding="Q8_K"), Buffer(y))
     host = (lambda a: a.cpu().numpy()) if where == "device" else (lambda a: a)
-    for call in range(8):
-        fresh = activations(rng, m, k) * (1 + call)
+    for call in range(24):
+        fresh = activations(rng, m, k) * (1 + call % 8)
         if where == "device":
             x.copy_(torch.from_numpy(fresh))
             torch.cuda.synchronize()
@@ -48,7 +50,93 @@ def test_repeated_call_follows_its_inputs(torch, oracle, m, where):
         want, want_xq = oracle.mul_mat(oracle.Q4_K, packed, fresh, n, k, m, rule=1)
         assert np.array_equal(host(xq), want_xq), call
         assert rel_l2(host(y), want) <= 1e-5, call
-        if call == 5:
+        if call in (5, 20):
             big = 700 * m
             kernel(w, torch.zeros((big, k), device="cuda"), Buffer(torch.zeros((big, xq.shape[1]), dtype=torch.uint8, device="cuda"), shape=(big, k), encoding="Q8_K"),
                    np.zeros((big, n), np.float32))
+
+
+def grow_and_leave(torch, lib, problem):
+    """A batch on the same stream that makes its workspace grow, and one on another stream."""
+    import ctypes
+
+    side = torch.cuda.Stream()
+    for stream in (None, side.cuda_stream):
+        lib.weft_b200_set_stream(ctypes.c_void_p(stream))
+        try:
+            problem.run(lib)
+        finally:
+            lib.weft_b200_set_stream(None)
+
+
+# a contraction in tensor memory with K in slices, one with a launch for its last rows, the CTA-pair kernel, Q6_K in tensor memory
+@pytest.mark.parametrize("name, mnk", [("Q4_K", (64, 2200, 4096)), ("Q5_K", (58, 18949, 512)), ("TQ1_0", (200, 520, 2048)), ("Q6_K", (129, 1027, 4352))])
+def test_repeated_batch_follows_its_inputs(torch, lib, oracle, golden, name, mnk):  # noqa: F811
+    from test_gpu_batch import Problem
+
+    problem, other = Problem(torch, oracle, golden, name, *mnk), None
+    k = mnk[2]
+    first, codes = problem.x.clone(), problem.want_xq.copy()
+    for call in range(24):
+        sign = 1.0 if call % 2 else -1.0                       # -x gives -codes and the same scale: Y changes its sign exactly
+        problem.x.copy_(first * sign)
+        problem.y.fill_(float("nan"))
+        torch.cuda.synchronize()
+        problem.run(lib)
+        got = problem.y.cpu().numpy()
+        assert rel_l2(got * sign, problem.want) <= 1e-5, call
+        if call in (3, 19):
+            other = other or Problem(torch, oracle, golden, "Q4_K", 700, 64, k)
+            grow_and_leave(torch, lib, other)
+    problem.x.copy_(first)
+    torch.cuda.synchronize()
+    problem.run(lib)
+    assert np.array_equal(problem.xq.cpu().numpy(), codes)
+    problem.check()
+
+
+def test_repeated_dequantize_follows_its_weights(torch, oracle):
+    import weft_b200 as weft
+    from weft_b200.kernels import rows
+    from weft_b200.runtime import Buffer
+
+    n, k = 40, 1024
+    rng = np.random.default_rng(5)
+    kernel = weft.compile(rows.row_dequantize_q4_k_rows)
+    held, y = torch.zeros((n, k // 256 * 144), dtype=torch.uint8, device="cuda"), torch.zeros((n, k), device="cuda")
+    args = Buffer(held, shape=(n, k), encoding="Q4_K"), Buffer(y)
+    for call in range(24):
+        packed = weights(oracle.Q4_K, rng, n, k)
+        held.copy_(torch.from_numpy(packed))
+        torch.cuda.synchronize()
+        kernel(*args)
+        assert np.array_equal(y.cpu().numpy().view(np.uint32), oracle.dequantize(oracle.Q4_K, packed, k).view(np.uint32)), call
+
+
+@pytest.mark.parametrize("steps", [3, 13])          # a graph, and a chain too long for one
+def test_repeated_chain_follows_its_inputs(torch, oracle, steps):
+    from weft_b200.layers import Projection, ProjectionChain
+    from weft_b200.runtime.driver import Toolchain, load_library
+
+    k, rng = 1024, np.random.default_rng(steps)
+    lib = load_library(Toolchain().resolve().compiler)
+    names = ["Q4_K", "Q4_K", "Q6_K", "Q5_K"]
+    parts = []
+    for step in range(steps):
+        name, n, m = names[step % 4], 96 + 8 * step, 1 if step % 4 < 2 else 5
+        packed, x = weights(getattr(oracle, name), rng, n, k), torch.zeros((m, k), device="cuda")
+        reuse = step % 4 == 1                                  # the second Q4_K step takes the first one's records
+        xq = parts[-1][3] if reuse else torch.zeros((m, oracle.row_bytes(oracle.Q8_K, k)), dtype=torch.uint8, device="cuda")
+        parts.append((name, packed, parts[-1][2] if reuse else x, xq, torch.zeros((m, n), device="cuda"), torch.from_numpy(packed).cuda(), n, m, reuse))
+    chain = ProjectionChain(lib, [Projection(name, w.data_ptr(), x.data_ptr(), xq.data_ptr(), y.data_ptr(), n, k, m, reuse)
+                                  for name, _, x, xq, y, w, n, m, reuse in parts])
+    for call in range(20):
+        for _, _, x, _, y, _, _, m, reuse in parts:
+            if not reuse:
+                x.copy_(torch.from_numpy(activations(rng, m, k)))
+            y.fill_(float("nan"))
+        torch.cuda.synchronize()
+        chain.run()
+        for name, packed, x, _, y, _, n, m, _ in parts:
+            want, _ = oracle.mul_mat(getattr(oracle, name), packed, x.cpu().numpy(), n, k, m, rule=1)
+            assert rel_l2(y.cpu().numpy(), want) <= 1e-5, (call, name)
