@@ -140,3 +140,42 @@ def test_repeated_chain_follows_its_inputs(torch, oracle, steps):
         for name, packed, x, _, y, _, n, m, _ in parts:
             want, _ = oracle.mul_mat(getattr(oracle, name), packed, x.cpu().numpy(), n, k, m, rule=1)
             assert rel_l2(y.cpu().numpy(), want) <= 1e-5, (call, name)
+
+
+@pytest.mark.parametrize("where", ["host", "resident"])
+def test_chain_with_host_memory_groups_its_steps(torch, lib, oracle, where):  # noqa: F811
+    """q / k / v on the same activations are one launch with the activations in host memory or the weights registered too, and a
+    later step sees what an earlier one copied back.  Calls enough for replays."""
+    import ctypes
+
+    from weft_b200.layers import Projection, ProjectionChain
+
+    k, rng = 1024, np.random.default_rng(3)
+    rows = {"q": 1024, "k": 160, "v": 160, "o": 96}
+    packed = {part: weights(oracle.Q4_K, rng, n, k) for part, n in rows.items()}
+    held = {part: torch.from_numpy(w) if where == "resident" else torch.from_numpy(w).cuda() for part, w in packed.items()}
+    if where == "resident":
+        for w in held.values():
+            assert lib.weft_b200_weights_resident(ctypes.c_void_p(w.data_ptr()), w.numel()) == 0
+    device = "cpu" if where == "host" else "cuda"
+    record_bytes = oracle.row_bytes(oracle.Q8_K, k)
+    x, xq, oq = torch.zeros((1, k), device=device), torch.zeros(record_bytes, dtype=torch.uint8, device=device), torch.zeros(record_bytes, dtype=torch.uint8, device=device)
+    y = {part: torch.zeros((1, n), device=device) for part, n in rows.items()}
+    source = {"o": (y["q"], oq)}                               # the last step multiplies what the first one gave
+    chain = ProjectionChain(lib, [Projection("Q4_K", held[part].data_ptr(), source.get(part, (x, xq))[0].data_ptr(), source.get(part, (x, xq))[1].data_ptr(),
+                                             y[part].data_ptr(), n, k, reuse_xq=part in "kv") for part, n in rows.items()])
+    try:
+        for call in range(20):
+            x.copy_(torch.from_numpy(activations(rng, 1, k)))
+            torch.cuda.synchronize()
+            before = lib.weft_b200_launch_count()
+            chain.run()
+            assert lib.weft_b200_launch_count() - before == 2, "one launch for q, k and v, one for o"
+            for part, n in rows.items():
+                want, want_xq = oracle.mul_mat(oracle.Q4_K, packed[part], source.get(part, (x, xq))[0].cpu().numpy(), n, k, 1, rule=1)
+                assert rel_l2(y[part].cpu().numpy(), want) <= 1e-5, (call, part)
+                assert np.array_equal(source.get(part, (x, xq))[1].cpu().numpy(), want_xq.reshape(-1))
+    finally:
+        if where == "resident":
+            for w in held.values():
+                lib.weft_b200_weights_release(ctypes.c_void_p(w.data_ptr()))

@@ -434,8 +434,10 @@ struct MulMat {
     }
     size_t plane_bytes() const { return path == FOLD ? fold_plane_bytes(tile_args()) : path == TILES ? tile_plane_bytes(tile_args()) : path == PAIR ? prefill_pair_plane_bytes(m, k) : 0; }
 
+    // records: the activation records of an earlier step of the same call, where the kernels find them (have_xq then); that step
+    // is not alone
     int prepare(Call &call, int fmt_, const void *W, const float *X, void *Xq, const int8_t *grid, const int8_t *signs, const uint32_t *powers,
-                float *Y, size_t N, size_t K, size_t M, size_t pitch, unsigned flags, bool vec_dot_only) {
+                float *Y, size_t N, size_t K, size_t M, size_t pitch, unsigned flags, bool vec_dot_only, void *records = nullptr, bool alone = true) {
         fmt = fmt_;
         act = activation_of(fmt);
         if (check_k(fmt, K) || check_k(act, K)) return 1;
@@ -449,8 +451,9 @@ struct MulMat {
         if (!have_xq && call.map(X, M * K * sizeof(float), true, false, &x)) return 1;
         // Decode quantizes X inside the GEMV (its first CTA stores the records, nobody loads them again), so a host Xq can
         // be written in place; a batch may take a path that reads Xq back.
-        const bool xq_in_place = !have_xq && M < 3 && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
-        if (call.map(Xq, M * row_bytes(act, K), have_xq, !have_xq, &xq, xq_in_place)) return 1;
+        const bool xq_in_place = alone && !have_xq && M < 3 && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+        if (records) xq = records;
+        else if (call.map(Xq, M * row_bytes(act, K), have_xq, !have_xq, &xq, xq_in_place)) return 1;
         if (codebook_bytes(fmt) && (call.map(grid, codebook_bytes(fmt), true, false, &gr) || (has_sign_table(fmt) && call.map(signs, 1024, true, false, &sg)))) return 1;
         if (fmt == F_TQ1_0 && call.map(powers, 20, true, false, &pw)) return 1;
         if (fmt == F_IQ1_M && call.map(powers, 65536 * sizeof(float), true, false, &pw)) return 1;   // the caller's float[65536] table of f16 bit patterns
@@ -774,47 +777,39 @@ static bool chain_format(int f) {    // chains: the formats of the first version
     return f == F_Q4_0 || f == F_Q8_0 || f == F_Q2_K || f == F_Q3_K || f == F_Q4_K || f == F_Q5_K || f == F_Q6_K || f == F_IQ2_XXS || f == F_TQ1_0;
 }
 
-int weft_b200_mul_mat_chain(const weft_b200_mul_mat_step *steps, size_t count) {
-    if (!steps && count) return fail("the step table is NULL");
-    std::lock_guard<std::recursive_mutex> guard(g.lock);
-    if (!count) return 0;
-    if (ensure_init(-1)) return 1;
-    // All steps are looked up first and issued together, with one wait at the end.  A chain with host memory in it goes step
-    // by step: a later step may take what an earlier one copied back.
-    bool on_device = true;
-    for (size_t i = 0; i < count && on_device; ++i) {
-        const weft_b200_mul_mat_step &s = steps[i];
-        for (const void *p : {(const void *)s.W, (const void *)s.X, (const void *)s.Xq, (const void *)s.Y, (const void *)s.grid, (const void *)s.signs, (const void *)s.powers})
-            on_device = on_device && (!p || Call::on_device(p));
-    }
-    for (size_t i = 0; i < count; ++i) {
-        const weft_b200_mul_mat_step &s = steps[i];
-        if (!chain_format(s.format)) return fail("step %zu: unknown weight format id %d", i, s.format);
-        if (!on_device && do_mul_mat(s.format, s.W, s.X, s.Xq, s.grid, s.signs, s.powers, s.Y, s.N, s.K, s.M, s.N, s.flags, false)) return 1;
-    }
-    if (!on_device) return 0;
-    Call call;
-    std::vector<MulMat> ops(count);
-    for (size_t i = 0; i < count; ++i) {
-        const weft_b200_mul_mat_step &s = steps[i];
-        if (ops[i].prepare(call, s.format, s.W, s.X, s.Xq, s.grid, s.signs, s.powers, s.Y, s.N, s.K, s.M, s.N, s.flags, false)) return 1;
-    }
+static int prepare_step(Call &call, MulMat &op, const weft_b200_mul_mat_step &s, void *records, bool alone) {
+    return op.prepare(call, s.format, s.W, s.X, s.Xq, s.grid, s.signs, s.powers, s.Y, s.N, s.K, s.M, s.N, s.flags, false, records, alone);
+}
+
+// How many steps from `at` on take the activation records of the first (the later ones marked as reusing Xq).
+static size_t steps_on_same_records(const weft_b200_mul_mat_step *steps, size_t at, size_t count) {
+    const weft_b200_mul_mat_step &s = steps[at];
+    size_t run = 1;
+    if (s.format == F_Q4_K && s.M == 1 && s.N && s.K && s.K % 256 == 0)
+        while (at + run < count && run < (size_t)GEMV_MAX_SEGMENTS && steps[at + run].format == F_Q4_K && steps[at + run].M == 1 && steps[at + run].K == s.K &&
+               steps[at + run].Xq == s.Xq && (steps[at + run].flags & 1u) && steps[at + run].N)
+            ++run;
+    return run;
+}
+
+// Prepared steps, issued as one call.
+static int issue_steps(Call &call, std::vector<MulMat> &ops) {
     size_t plane_bytes = 0;              // the steps follow each other: one workspace serves them all
     for (const MulMat &op : ops) plane_bytes = op.plane_bytes() > plane_bytes ? op.plane_bytes() : plane_bytes;
     uint8_t *planes = nullptr;
     if (plane_bytes) CU(workspace(plane_bytes, g.stream, &planes));
     Key key;
-    key.add(4, count);
+    key.add(4, ops.size());
     for (MulMat &op : ops) {
         op.planes = planes;
         op.add_to(key);
     }
     return call.issue(key, [&](cudaStream_t stream) {
-        for (size_t i = 0; i < count; ++i) {
+        for (size_t i = 0; i < ops.size(); ++i) {
             // consecutive Q4_K steps on the same activations (the later ones marked as reusing Xq) go out as one launch
             size_t run = 1;
             if (ops[i].path == MulMat::GEMV && ops[i].fmt == F_Q4_K && ops[i].m == 1 && ops[i].k % 256 == 0)
-                while (i + run < count && run < (size_t)GEMV_MAX_SEGMENTS && ops[i + run].path == MulMat::GEMV && ops[i + run].fmt == F_Q4_K && ops[i + run].m == 1 &&
+                while (i + run < ops.size() && run < (size_t)GEMV_MAX_SEGMENTS && ops[i + run].path == MulMat::GEMV && ops[i + run].fmt == F_Q4_K && ops[i + run].m == 1 &&
                        ops[i + run].k == ops[i].k && ops[i + run].xq == ops[i].xq && ops[i + run].have_xq)
                     ++run;
             GemvArgs ga;
@@ -831,6 +826,34 @@ int weft_b200_mul_mat_chain(const weft_b200_mul_mat_step *steps, size_t count) {
         }
         return 0;
     });
+}
+
+int weft_b200_mul_mat_chain(const weft_b200_mul_mat_step *steps, size_t count) {
+    if (!steps && count) return fail("the step table is NULL");
+    std::lock_guard<std::recursive_mutex> guard(g.lock);
+    if (!count) return 0;
+    if (ensure_init(-1)) return 1;
+    // All steps are looked up first and issued together, with one wait at the end.  A chain with host memory in it goes
+    // piece by piece, a wait behind each: a later step may take what an earlier one copied back.  A piece is one step, or
+    // the steps that one launch serves (they share records that nothing copies back in between).
+    bool on_device = true;
+    for (size_t i = 0; i < count && on_device; ++i) {
+        const weft_b200_mul_mat_step &s = steps[i];
+        for (const void *p : {(const void *)s.W, (const void *)s.X, (const void *)s.Xq, (const void *)s.Y, (const void *)s.grid, (const void *)s.signs, (const void *)s.powers})
+            on_device = on_device && (!p || Call::on_device(p));
+    }
+    for (size_t i = 0; i < count;) {
+        const size_t piece = on_device ? count : steps_on_same_records(steps, i, count), end = i + piece;
+        Call call;
+        std::vector<MulMat> ops(piece);
+        for (size_t j = 0; i < end; ++i, ++j) {
+            const weft_b200_mul_mat_step &s = steps[i];
+            if (!chain_format(s.format)) return fail("step %zu: unknown weight format id %d", i, s.format);
+            if (prepare_step(call, ops[j], s, !on_device && j ? ops[0].xq : nullptr, piece == 1)) return 1;
+        }
+        if (issue_steps(call, ops)) return 1;
+    }
+    return 0;
 }
 
 // ---- peer memory (CUDA IPC) and the row-sharded mul_mat that gathers through it
