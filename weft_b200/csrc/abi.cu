@@ -480,7 +480,9 @@ struct MulMat {
         if (path == TILES) {          // their first kernel quantizes X
             if (launched(launch_tile(tile_args(), planes, sms, stream), "batched mul_mat", 2)) return 1;
         } else if (path == FOLD) {
-            if (launched(launch_fold(tile_args(), planes, g.status_dev, sms, stream), "batched mul_mat", fold_launches(tile_args(), sms))) return 1;
+            unsigned kernels = 0;
+            const cudaError_t e = launch_fold(tile_args(), planes, g.status_dev, sms, stream, &kernels);
+            if (launched(e, "batched mul_mat", kernels)) return 1;
         } else {
             if (!have_xq && !fuse_quantize && launched(launch_quantize(act, (const float *)x, xq, m, k, sms, stream), "activation quantize")) return 1;
             if (path == PAIR) {

@@ -154,8 +154,6 @@ static FoldSplit split_for(int fmt, long long m, long long n, long long nb, int 
     }
 }
 
-int fold_launches(const TileArgs &a, int sm_count) { return split_for(a.fmt, a.m, a.n, a.k / 256, sm_count).second.nt ? 3 : 2; }
-
 bool fold_supported(const TileArgs &a) {
     if (a.fmt != F_Q4_K && a.fmt != F_Q5_K && a.fmt != F_Q6_K) return false;
     // Below these the register tiles are quicker: this kernel starts about 4 us later (cluster, tensor memory, planes) and takes
@@ -197,7 +195,7 @@ static cudaError_t launch_rows(const TileArgs &a, const FoldPlan &plan, const Fo
     }
 }
 
-cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream) {
+cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches) {
     const FoldPlaneSizes s = plane_sizes(a.fmt, a.m, a.k);
     uint4 *codes = reinterpret_cast<uint4 *>(planes);
     float *xd = reinterpret_cast<float *>(planes + s.codes);
@@ -209,6 +207,7 @@ cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_
     p.row_bytes = (long long)p.nb * unit_bytes(a.fmt);
     const FoldSplit split = split_for(a.fmt, a.m, a.n, p.nb, sm_count);
     if (!split.first.nt) return cudaErrorNotSupported;
+    *launches = split.second.nt ? 3 : 2;
     cudaError_t e = mins ? launch_planes<true>(a, codes, xd, mins, s.pitch, stream) : launch_planes<false>(a, codes, xd, mins, s.pitch, stream);
     const uint8_t *w = static_cast<const uint8_t *>(a.w);
     if (e == cudaSuccess) e = launch_rows(a, split.first, p, codes, mins, w, a.y, split.rows, sm_count, stream);

@@ -103,8 +103,7 @@ template <int FMT> cudaError_t launch_tile_kernel(const TileArgs &a, const uint8
 // tcgen05 contraction with the weights expanded into tensor memory (fold.cuh), behind the kernel that makes its planes.
 bool fold_supported(const TileArgs &a);
 size_t fold_plane_bytes(const TileArgs &a);
-cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream);
-int fold_launches(const TileArgs &a, int sm_count);   // kernels one launch_fold call puts on the stream
+cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches);   // two or three kernels
 
 // Device memory for a call's activation planes, valid for the work it puts on `stream` (workspace.cu); the generation
 // changes whenever memory handed out earlier outside a capture is gone.
