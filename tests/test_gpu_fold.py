@@ -5,15 +5,15 @@ the edges of its tiles: rows that do not fill the last 128 (nor, for Q6_K, the l
 tokens just above a tile, one block of K, blocks that do not divide among the slices of K, more tiles than SMs, a last round of
 13 rows that is a launch of its own.
 
-Bound: 1e-5 relative L2 and the reference harnesses' |a - e| <= 1e-4 + 2e-3 |e|.  The sums of a block are integers in fp32
-accumulators, exact below 2^24; above, the 16 accumulation steps of a block (Q6_K: 32, two operands) each lose at most
-2^-23 of the running sum, so terms of one sign lose at most 32 * 2^-23 = 3.9e-6.
+Bound: 1e-5 relative L2 and the reference harnesses' |a - e| <= 1e-4 + 2e-3 |e|.  The sums of a block are integers, held
+exactly by the accumulators; the block's sum is rounded once (Q4_K: in its last accumulation step, by at most 2^-23).
 """
 from __future__ import annotations
 
 import numpy as np
 import pytest
 
+from helpers import rel_l2
 from test_gpu_batch import Problem, lib, torch  # noqa: F401  (fixtures)
 
 pytestmark = pytest.mark.gpu
@@ -62,3 +62,67 @@ def test_largest_codes_and_scales(torch, lib, oracle, golden, name, monkeypatch)
     problem = Problem(torch, oracle, golden, name, 64, 2200, 4096)
     problem.run(lib)
     problem.check()
+
+
+class Records(Problem):
+    """A problem whose weights and activation records are given: codes (m, k), every scale of the activations 1."""
+
+    def __init__(self, torch, oracle, name, w, codes, n):  # noqa: F811
+        self.fmt, (self.m, self.k), self.n = oracle.FORMAT_IDS[name], codes.shape, n
+        blocks = codes.reshape(self.m, -1, 256)
+        records = np.zeros((self.m, blocks.shape[1], 292), np.uint8)
+        records[:, :, :4] = np.float32(1).reshape(1).view(np.uint8)
+        records[:, :, 4:260] = blocks.view(np.uint8)
+        records[:, :, 260:] = blocks.reshape(self.m, -1, 16, 16).sum(-1, dtype=np.int16).view(np.uint8).reshape(self.m, -1, 32)
+        self.want_xq = records.reshape(self.m, -1)
+        self.want, _ = oracle.mul_mat(self.fmt, w, None, n, self.k, self.m, xq=self.want_xq)
+        self.w, self.xq = torch.from_numpy(w).cuda(), torch.from_numpy(self.want_xq).cuda()
+        self.grid = self.signs = self.powers = self.x = self.xq
+        self.y = torch.full((self.m, n), float("nan"), device="cuda")
+
+
+RECORD_BYTES, ONE = {"Q4_K": 144, "Q5_K": 176, "Q6_K": 210}, np.float16(1).reshape(1).view(np.uint8)
+
+
+@pytest.mark.parametrize("name", FORMATS)
+@pytest.mark.parametrize("m", [48, 64, 128])
+def test_large_partial_sums_that_cancel(torch, lib, oracle, name, m):  # noqa: F811
+    """Largest weights against activations of one sign, then of the other: the sum of a block passes 2^24 and comes back to a few
+    thousand.  The integer sums are exact, so the bound is the one of the additions over 16 blocks."""
+    rng = np.random.default_rng(m)
+    n, k = 2900, 4096
+    w = np.full((n, k // 256, RECORD_BYTES[name]), 0xFF, np.uint8)
+    if name == "Q6_K":
+        w[:, :, 192:208], w[:, :, 208:] = 0x7F, ONE
+    else:
+        w[:, :, :2], w[:, :, 2:4] = ONE, 0
+    codes = np.full((m, k // 256, 256), 127, np.int8)
+    codes[:, :, 128:] = -127
+    codes[:, :, 128:136] += rng.integers(0, 3, size=(m, k // 256, 8), dtype=np.int8)
+    problem = Records(torch, oracle, name, w.reshape(n, -1), codes.reshape(m, k), n)
+    problem.run(lib, flags=1)
+    problem.check()
+    if name != "Q6_K":                               # the first 160 of a block against its last 96
+        first = np.arange(k) % 256 < 160
+        codes = np.where(first, 127 - rng.integers(0, 2, size=(m, k)), -127).astype(np.int8)
+        problem = Records(torch, oracle, name, w.reshape(n, -1), codes, n)
+        problem.run(lib, flags=1)
+        problem.check()
+
+
+@pytest.mark.parametrize("name", FORMATS)
+@pytest.mark.parametrize("m", [40, 64, 90, 700])
+def test_integer_sums_are_exact(torch, lib, oracle, name, m):  # noqa: F811
+    """One block, every bit of codes, scales and mins random, all super-scales 1: the results are integers."""
+    rng = np.random.default_rng(m)
+    n, k = int(5.5e8 / m / 256) // 128 * 128 + 131, 256
+    w = rng.integers(0, 256, size=(n, RECORD_BYTES[name]), dtype=np.uint8)
+    if name == "Q6_K": w[:, 208:] = ONE
+    else: w[:, :2], w[:, 2:4] = ONE, ONE
+    codes = rng.integers(-127, 128, size=(m, k), dtype=np.int8)
+    codes[m // 2:] = np.abs(codes[m // 2:])          # large sums of one sign
+    problem = Records(torch, oracle, name, w, codes, n)
+    problem.run(lib, flags=1)
+    got, whole = problem.y.cpu().numpy(), np.abs(problem.want) < 2.0 ** 24
+    assert np.array_equal(got[whole], problem.want[whole])
+    assert rel_l2(got, problem.want) <= 2.0 ** -23

@@ -86,7 +86,10 @@ size_t fold_plane_bytes(const TileArgs &a) {
 // 1800 clocks when A has buffers for two (up to 80 tokens with a min term, 64 without) and 2350 with one, twice that for
 // Q6_K's two limbs, and hardly depends on the tokens (measured from 16 to 128); a tile's start, its stores and the meeting of
 // the slices are small beside it.
-template <int FMT> static int fold_a_buffers(int nt) { return FoldFormat<FMT>::COLS * nt + 4 * 64 <= 512 ? 4 : 2; }
+// Tensor memory (512 columns) goes to A buffers for a whole block, then to a second set of accumulators, then to a second block
+// of A; one limb has two sets always, and half a block of two limbs will do where three accumulators of 128 leave no more.
+template <int FMT> static int fold_sets(int nt) { return FoldFormat<FMT>::LIMBS == 1 || FoldFormat<FMT>::columns(nt, 2) + 256 <= 512 ? 2 : 1; }
+template <int FMT> static int fold_a_buffers(int nt) { return FoldFormat<FMT>::columns(nt, fold_sets<FMT>(nt)) + 256 <= 512 ? 4 : 2; }
 template <int FMT>
 static double fold_tile_cost(int nt, int abufs, long long steps) {
     using F = FoldFormat<FMT>;
@@ -97,17 +100,17 @@ static double fold_tile_cost(int nt, int abufs, long long steps) {
 template <int FMT>
 static FoldPlan fold_plan(long long m, long long n, long long nb, int sm_count) {
     using F = FoldFormat<FMT>;
-    FoldPlan best{0, 0, 0, 0, 0.0};
+    FoldPlan best{0, 0, 0, 0, 0, 0.0};
     const long long row_tiles = (n + FD_ROWS - 1) / FD_ROWS;
     for (int nt = 16; nt <= FD_TOKENS; nt += 16) {
         const int stages = fold_stages<FMT>(nt), abufs = fold_a_buffers<FMT>(nt);
-        if (stages < 2 || abufs < F::CHUNKS) continue;
+        if (stages < 2) continue;
         const long long tiles = row_tiles * ((m + nt - 1) / nt);
         for (int slices = 1; slices <= 8 && slices <= nb; ++slices) {
             if (slices > 1 && tiles > fold_clusters<FMT>(slices)) break;
             const long long rounds = slices > 1 ? 1 : (tiles + sm_count - 1) / sm_count, steps = (nb + slices - 1) / slices;
             const double cost = rounds * fold_tile_cost<FMT>(nt, abufs, steps) + (slices > 1 ? 1500.0 : 0.0);
-            if (!best.nt || cost < best.cost) best = FoldPlan{nt, slices, stages, abufs, cost};
+            if (!best.nt || cost < best.cost) best = FoldPlan{nt, slices, stages, abufs, fold_sets<FMT>(nt), cost};
         }
     }
     return best;
@@ -121,19 +124,19 @@ constexpr double FD_SECOND = 12000.0;     // clocks that a second launch costs b
 template <int FMT>
 static FoldSplit fold_split(long long m, long long n, long long nb, int sm_count) {
     using F = FoldFormat<FMT>;
-    FoldSplit best{fold_plan<FMT>(m, n, nb, sm_count), FoldPlan{0, 0, 0, 0, 0.0}, n};
+    FoldSplit best{fold_plan<FMT>(m, n, nb, sm_count), FoldPlan{0, 0, 0, 0, 0, 0.0}, n};
     double least = best.first.cost;
     const long long row_tiles = (n + FD_ROWS - 1) / FD_ROWS;
     for (int nt = 16; nt <= FD_TOKENS; nt += 16) {
         const int stages = fold_stages<FMT>(nt), abufs = fold_a_buffers<FMT>(nt);
-        if (stages < 2 || abufs < F::CHUNKS) continue;
+        if (stages < 2) continue;
         const long long token_tiles = (m + nt - 1) / nt, rounds = row_tiles * token_tiles / sm_count, rows = rounds * sm_count / token_tiles * FD_ROWS;
         if (rows <= 0 || rows > n - 8) continue;          // the second launch needs a whole super-row
         const FoldPlan rest = fold_plan<FMT>(m, n - rows, nb, sm_count);
         const double cost = rounds * fold_tile_cost<FMT>(nt, abufs, nb);
         if (!rest.nt || cost + rest.cost + FD_SECOND >= least) continue;
         least = cost + rest.cost + FD_SECOND;
-        best = FoldSplit{FoldPlan{nt, 1, stages, abufs, cost}, rest, rows};
+        best = FoldSplit{FoldPlan{nt, 1, stages, abufs, fold_sets<FMT>(nt), cost}, rest, rows};
     }
     return best;
 }
@@ -172,7 +175,7 @@ static cudaError_t launch_rows(const TileArgs &a, const FoldPlan &plan, const Fo
     FoldParams p = planes;
     p.w = w; p.y = y; p.n = n;
     p.w_bytes = p.row_bytes * n;
-    p.nt = plan.nt; p.slices = plan.slices; p.b_stages = plan.stages; p.a_buffers = plan.a_buffers;
+    p.nt = plan.nt; p.slices = plan.slices; p.b_stages = plan.stages; p.a_buffers = plan.a_buffers; p.sets = plan.sets;
     p.token_tiles = (int)((a.m + p.nt - 1) / p.nt);
     p.tiles = p.token_tiles * (int)((n + FD_ROWS - 1) / FD_ROWS);
     CUtensorMap x_codes, x_mins, w_rows;

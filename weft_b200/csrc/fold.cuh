@@ -1,10 +1,17 @@
 // mul_mat for batches of tokens on tcgen05 with the weights as the operand in TENSOR MEMORY.
 //
 // D[128 weight rows, Nt tokens] += A[128, 256] * B[256, Nt] per 256-element block, kind::f16 with fp32 accumulators.  The A
-// operand is the block's integers with the sub-block scales multiplied in (Q4_K: scale * nibble <= 945, exact in f16, so are
-// the 8-bit activation codes; every product and every sum below 2^24 is exact, above that an fp32 cannot hold the integer
-// either), B the activation codes as f16.  One scale pair per (row, block) and one per (token, block) is left for the
-// epilogue: acc += x.d * (d * S - dmin * M).
+// operand is the block's integers with the sub-block scales multiplied in, B the activation codes as f16.  One scale pair per
+// (row, block) and one per (token, block) is left for the epilogue: acc += x.d * (d * S - dmin * M).
+//
+// S is an integer, and every accumulator holds its part of it exactly, whatever the order of its terms: operands are cut so that
+// no partial sum passes 2^24 (times the power of two that all terms share), with codes up to 128 and every bit of a record set.
+//   Q4_K  scale * (q - 8), at most 504 * 128 * 256 in all.  8 * sum(scale * sum of the group's codes), what the centre left
+//         out, follows as one K = 16 step, the only one that may round (sums beyond 2^24, by at most 2^-23)
+//   Q5_K  scale * (low nibble - 8) in one accumulator; 16 * scale * (fifth bit), multiples of 16, and the centre's step in another
+//   Q6_K  16 * (scale / 16) * (q - 32), multiples of 16, in one accumulator, (scale % 16) * (q - 32) in another
+// S of two accumulators is their sum, rounded once, as the conversion of an exact integer would be.  (Scales times whole codes
+// in one accumulator reach 3.1e7, 6.4e7 and 1.3e8: a block whose terms cancel lost its low bits on the way.)
 //
 // Why this split.  A weight row is a TMEM lane and a thread: it reads its record, unpacks it in registers and writes it to
 // tensor memory with tcgen05.st -- no transposition, no swizzle, no shared-memory round trip, and shared memory (128 bytes a
@@ -12,14 +19,14 @@
 // need no integer conversion and are overwritten by the next block's first MMA, so the epilogue is one load and three packed
 // operations per pair of values.
 //
-// Q6_K: scale * (q - 32) needs 13 bits.  The scale is taken as its even part and its last bit, two operands into the same
-// accumulator, both exact.
-//
 // A CTA takes up to 128 tokens: an MMA with A in tensor memory runs at N / 2 clocks (measured from N = 32 to 128, both operands
 // in shared memory: 32 + N / 4) but takes 15 to 25 clocks to issue, so the tokens go into one wide MMA per K step, and one
-// expansion of the weights, the largest part of the instructions, serves them all.  S is double-buffered; M is small work at a
-// block's end and has one buffer: 3 x 128 columns and A buffers for one block fill the 512.  Fewer tokens leave room for two
-// blocks.  A passes from the expanders to the MMAs in half blocks (Q4_K, Q5_K) or quarter blocks of two operands (Q6_K), the
+// expansion of the weights, the largest part of the instructions, serves them all.  Tensor memory (512 columns of 32 bits) bounds
+// the rest.  Q4_K: S twice (a block's is read while the next one is summed), M once, A for one block up to 128 tokens, for two up
+// to 80.  Two limbs: one set of accumulators above 64 (Q5_K: 48) tokens; its first 64 tokens are completed, and read, before the
+// others, so that the reading runs beside the MMAs of the last and of the first A buffer of a block (Q6_K 512 x 4096 x 14336 with
+// the set as a whole 160 us, in halves 153, with two sets, which the accumulators no longer leave room for, 137).
+// A passes from the expanders to the MMAs in half blocks (Q4_K) or quarter blocks of two operands, the
 // quarters being unpacked in registers before the buffer is waited for: 180 to 136 us for Q6_K, 512 x 4096 x 14336; Q4_K, with
 // half the MMAs between two hand-overs, lost more to the MMA warp's waits (about 150 clocks each) than it gained.
 //
@@ -36,11 +43,12 @@
 // rank order.
 //
 // What bounds it: the hand-overs of A (expanders, MMAs, expanders) and the instructions of the unpacking, 1750 clocks a Q4_K
-// block up to 64 tokens and 2500 with 128 against 1088 of tensor work, 4500 against 2048 for Q6_K.  Measured on B200 (us, device
-// time with the kernel that makes the planes; before: register tiles, for Q4_K above 128 tokens CTA pairs on int8 limbs):
-//   Q4_K  128 x 4096 x 4096 27.5 -> 16.9   512 x 4096 x 4096 46.8 -> 31.8   512 x 14336 x 4096 110 -> 91   512 x 4096 x 14336 127 -> 86
-//   Q5_K  512 x 14336 x 4096 218 -> 107
-//   Q6_K  512 x 14336 x 4096 329 -> 151    512 x 4096 x 14336 338 -> 137
+// block up to 64 tokens and 2500 with 128 against 1088 of tensor work, 5000 against 2048 (Q5_K 2176) for two limbs.  Measured on
+// B200 (us, device time with the kernel that makes the planes; before: register tiles, for Q4_K above 128 tokens CTA pairs on int8
+// limbs):
+//   Q4_K  128 x 4096 x 4096 27.5 -> 18.5   512 x 4096 x 4096 46.8 -> 32.8   512 x 14336 x 4096 110 -> 86   512 x 4096 x 14336 127 -> 86
+//   Q5_K  512 x 14336 x 4096 218 -> 149    512 x 4096 x 14336 228 -> 161
+//   Q6_K  512 x 14336 x 4096 329 -> 144    512 x 4096 x 14336 338 -> 153
 #pragma once
 
 #include "prefill_common.cuh"
@@ -55,6 +63,7 @@ namespace weft {
 constexpr int FD_WARPS = 28, FD_THREADS = FD_WARPS * 32, FD_ROWS = 128;
 constexpr int FD_GROUPS = 4, FD_E_WARP0 = 4 * FD_GROUPS, FD_TMA_WARP = 24, FD_W_WARP = 25, FD_MMA_WARP = 26;
 constexpr int FD_TOKENS = 128, FD_AMIN = 4;      // most tokens of a tile; slots of the min term's A operand
+constexpr int FD_HALF = 64;                     // tokens of the first half where one set of accumulators is filled and drained in halves
 constexpr int FD_W_SLOTS = 4;                   // most blocks of weight records
 constexpr int FD_SMEM = 227 * 1024;
 constexpr int FD_B_MAX = 6, FD_SLOTS = 8;      // most half-block stages of tokens; slots of the x.d ring
@@ -66,12 +75,13 @@ static_assert(FD_GROUPS * 128 * FD_X_REGS + 256 * FD_E_REGS + 128 * FD_IO_REGS <
 template <int FMT> struct FoldFormat {
     static constexpr int UNIT = unit_bytes(FMT);
     static constexpr bool MINS = FMT == F_Q4_K || FMT == F_Q5_K;
-    static constexpr int LIMBS = FMT == F_Q6_K ? 2 : 1;
+    static constexpr int LIMBS = FMT == F_Q4_K ? 1 : 2;             // operands of a weight, each with an accumulator of its own
     static constexpr bool SHIFTED = UNIT % 16 != 0;                 // records at any even address: a window of whole 16-byte pieces
     static constexpr int PITCH = SHIFTED ? ((UNIT + 14 + 15) / 16 | 1) * 16 : UNIT;   // an odd number of pieces: 128-bit loads of a warp's rows do not conflict
-    static constexpr int COLS = MINS ? 3 : 2;                       // accumulators of nt columns
     static constexpr int PER = LIMBS == 2 ? 1 : 2;                  // quarters of a block in an A buffer of 64 columns
     static constexpr int CHUNKS = 4 / PER;                          // A buffers of a block
+    // accumulators of nt columns: the limbs, once or twice (sets: a block's are drained while the next one's are filled), and M
+    static constexpr int columns(int nt, int sets) { return (sets * LIMBS + (MINS ? 1 : 0)) * nt; }
 };
 static_assert(FoldFormat<F_Q4_K>::PITCH / 16 % 2 == 1 && FoldFormat<F_Q5_K>::PITCH / 16 % 2 == 1 && FoldFormat<F_Q6_K>::PITCH / 16 % 2 == 1, "rows in different banks");
 
@@ -84,7 +94,7 @@ struct FoldParams {
     float *y;
     long long n, ldy, row_bytes, w_bytes, pitch;
     int m, nb, nt;               // tokens, blocks per row, tokens per tile (a multiple of 16)
-    int token_tiles, tiles, slices, b_stages, a_buffers;
+    int token_tiles, tiles, slices, b_stages, a_buffers, sets;
     int *status;
 };
 
@@ -108,7 +118,8 @@ template <int FMT> struct FoldLayout {
     static __host__ __device__ constexpr int xd_at(int tt, int stages) { return dd_at(tt, stages) + FD_DD_SLOTS * 2 * FD_ROWS * 4; }
     static __host__ __device__ constexpr int xmin_at(int tt, int stages) { return xd_at(tt, stages) + FD_SLOTS * tt * 4; }
     static __host__ __device__ constexpr int amin_at(int tt, int stages) { return xmin_at(tt, stages) + (F::MINS ? 4 * tt * 32 : 0); }
-    static __host__ __device__ constexpr int bytes(int tt, int stages) { return amin_at(tt, stages) + (F::MINS ? FD_AMIN * 4096 : 0); }
+    // A operands over the sums of 32 codes: FD_AMIN slots for the mins, as many for the scales
+    static __host__ __device__ constexpr int bytes(int tt, int stages) { return amin_at(tt, stages) + (F::MINS ? 2 * FD_AMIN * 4096 : 0); }
 };
 
 // ------------------------------------------------------------------ instructions
@@ -177,8 +188,9 @@ __device__ __forceinline__ bool fd_wait(uint64_t *bar, uint32_t parity, FoldCont
 
 // ------------------------------------------------------------------ unpacking: a quarter of a block (64 elements) of one row
 // Word i of the result holds elements {0, 2} (even i) or {1, 3} (odd i) of the i / 2 -th group of four: the order of the
-// activation plane.  An f16 pair is built by setting the exponent of 1024 above the bits; the multiply-add that applies the
-// scale takes the 1024 (or what it became) back out, with one rounding of an exact result.
+// activation plane.  Q4_K and Q5_K: a code's bits where they lie are an f16 below the normal range, q * 2^-24 (high nibbles
+// q * 2^-20); one multiply-add applies the scale and the centre: q * 2^-24 * (scale * 2^10) - 8 * scale * 2^-14, exactly.
+// Q6_K: set under the exponent of 1024, the 1024 and the 32 taken out again.
 
 template <int FMT>
 struct FoldRow {
@@ -203,11 +215,23 @@ struct FoldRow {
 // the 6-bit scales of a Q4_K / Q5_K record, four to a word: [0] scales 0..3, [1] 4..7; mins alike
 template <int FMT> struct FoldScales { uint32_t sc[FMT == F_Q6_K ? 4 : 2], mn[2]; };   // Q6_K: sixteen int8 scales
 
+// The scales of quarter q's two groups and what centres their codes, as f16 pairs
 template <int FMT>
-__device__ __forceinline__ void fold_quarter(int q, const FoldRow<FMT> &row, const FoldScales<FMT> &s, uint32_t (&out)[32]) {
-    const uint32_t scales = (q & 2 ? s.sc[1] : s.sc[0]) >> (16 * (q & 1));
-    const uint32_t slo = small_half2(scales & 255u), shi = hmul2(small_half2((scales >> 8) & 255u), 0x2c002c00u);   // / 16: the nibble stays where it is
-    const uint32_t clo = hmul2(slo, 0xe400e400u), chi = hmul2(shi, 0xe400e400u);                                    // -1024 * scale
+struct FoldQuarterScales {
+    uint32_t slo, shi, clo, chi;
+    __device__ __forceinline__ FoldQuarterScales(int q, const FoldScales<FMT> &s) {
+        const uint32_t scales = (q & 2 ? s.sc[1] : s.sc[0]) >> (16 * (q & 1));
+        const uint32_t lo = small_half2(scales & 255u), hi = small_half2((scales >> 8) & 255u);
+        slo = hmul2(lo, 0x64006400u);                  // * 2^10
+        shi = hmul2(hi, 0x54005400u);                  // * 2^6: high nibbles stay where they are
+        clo = hmul2(lo, 0x90009000u);                  // * -2^-11
+        chi = hmul2(hi, 0x90009000u);
+    }
+};
+
+// Q4_K: (q - 8) * scale * 2^-14.  Q5_K: the five bits of a code in place, for both limbs.
+template <int FMT>
+__device__ __forceinline__ void fold_quarter(int q, const FoldRow<FMT> &row, const FoldQuarterScales<FMT> &s, uint32_t (&out)[32]) {
     const uint8_t *codes = row.p + (FMT == F_Q4_K ? 16 : 48) + 32 * q;
 #pragma unroll
     for (int v = 0; v < 2; ++v) {
@@ -223,13 +247,16 @@ __device__ __forceinline__ void fold_quarter(int q, const FoldRow<FMT> &row, con
 #pragma unroll
             for (int o = 0; o < 2; ++o) {
                 const uint32_t w = o ? w4[i] >> 8 : w4[i];
-                uint32_t l = and_or(w, 0x000f000fu, row.exponent), h = and_or(w, 0x00f000f0u, row.exponent);
+                uint32_t &l = out[8 * v + 2 * i + o], &h = out[16 + 8 * v + 2 * i + o];
+                l = w & 0x000f000fu;
+                h = w & 0x00f000f0u;
                 if constexpr (FMT == F_Q5_K) {
                     l = and_or(o ? f[i] >> 4 : f[i] << 4, 0x00100010u, l);
                     h = and_or(o ? f[i] >> 1 : f[i] << 7, 0x01000100u, h);
+                } else {
+                    l = hfma2(l, s.slo, s.clo);
+                    h = hfma2(h, s.shi, s.chi);
                 }
-                out[8 * v + 2 * i + o] = hfma2(l, slo, clo);
-                out[16 + 8 * v + 2 * i + o] = hfma2(h, shi, chi);
             }
     }
 }
@@ -271,7 +298,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
     extern __shared__ __align__(1024) uint8_t smem[];
     FoldControl *ctl = reinterpret_cast<FoldControl *>(smem);
     const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int nt = p.nt, stages = p.b_stages, abufs = p.a_buffers, w_slots = L::w_slots(nt), w_shift = w_slots == 4 ? 2 : 1;
+    const int nt = p.nt, stages = p.b_stages, abufs = p.a_buffers, sets = p.sets, halves = sets == 1 && nt > FD_HALF ? 2 : 1, w_slots = L::w_slots(nt), w_shift = w_slots == 4 ? 2 : 1;
     const int slice = (int)blockIdx.x % p.slices, first_tile = (int)blockIdx.x / p.slices, stride = (int)gridDim.x / p.slices;
     const int begin = (int)((long long)p.nb * slice / p.slices), end = (int)((long long)p.nb * (slice + 1) / p.slices);
     const int my_tiles = first_tile < p.tiles ? (p.tiles - first_tile + stride - 1) / stride : 0;
@@ -301,7 +328,13 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
     // The expander groups take the blocks in turn and the A buffers hold one or two blocks, so a buffer passes from group to
     // group.  A parity wait cannot tell a phase from the one two before: every (buffer, group) has a release barrier of its own,
     // signalled for the group that fills the buffer next, and every group one for its records.
-    const int a_blocks = abufs / F::CHUNKS;
+    const int a_blocks = abufs / F::CHUNKS;             // 0: two buffers, each filled twice in a block of four
+    // Parity of the release that chunk c of a block waits for, by the number of releases of its (buffer, group) that came before;
+    // the first fill of a buffer needs none.
+    auto a_parity = [&](int block, int c) {
+        const int group = block % FD_GROUPS;
+        return a_blocks ? ((uint32_t)(block / FD_GROUPS) & 1u) ^ (group >= a_blocks ? 0u : 1u) : ((uint32_t)(c >> 1) & 1u) ^ (group == 0 ? 1u : 0u);
+    };
     const bool tmem_ok = *reinterpret_cast<volatile uint32_t *>(&ctl->tmem_base) == tmem;
     asm volatile("griddepcontrol.launch_dependents;");
 
@@ -341,7 +374,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
             float d[2];
             if constexpr (F::MINS) {
                 const uint4 head = *reinterpret_cast<const uint4 *>(row.p);
-                d[0] = half_bits_to_float(head.x);
+                d[0] = half_bits_to_float(head.x) * 16384.0f;           // the operands carry 2^-14
                 d[1] = -half_bits_to_float(head.x >> 16);
                 const Q4KScales u = q4k_unpack_scales(head.y, head.z, head.w);
                 s.sc[0] = u.sc_lo; s.sc[1] = u.sc_hi; s.mn[0] = u.mn_lo; s.mn[1] = u.mn_hi;
@@ -350,7 +383,6 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
                 d[1] = 0.0f;
                 row.words4(12, s.sc);
             }
-            const uint32_t parity = ((uint32_t)(it / FD_GROUPS) & 1u) ^ (group >= a_blocks ? 0u : 1u);
             // One loop body for all quarters: the roles' code has to stay in the instruction caches.  Unrolled by quarters, every
             // instruction took 7 to 19 clocks (Q4_K 1.8 to 2.4 thousand clocks a block, Q6_K 4.7 thousand).
 #pragma unroll 1
@@ -359,39 +391,58 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
                 const uint32_t to = lane_base + (uint32_t)(64 * buf + 32 * (c % F::PER));
                 uint32_t v[32];
                 if constexpr (FMT == F_Q6_K) fold_quarter_q6_k(c >> 1, c & 1, row, v);
-                else fold_quarter<FMT>(c, row, s, v);
+                else fold_quarter<FMT>(c, row, FoldQuarterScales<FMT>(c, s), v);
                 if (c % F::PER == 0) {
-                    if (!fd_wait(&ctl->a_empty[buf][group], parity, ctl, p.status)) { ok = false; break; }
+                    if (!fd_wait(&ctl->a_empty[buf][group], a_parity(it, c / F::PER), ctl, p.status)) { ok = false; break; }
                     tc::fence_after_sync();
                 }
                 if (c == 0) { dd[0] = d[0]; dd[FD_ROWS] = d[1]; }
-                if constexpr (FMT == F_Q6_K) {                  // the scale's even part into the first columns, its last bit into the others
+                if constexpr (FMT == F_Q6_K) {                  // 16 * (scale / 16) into the first columns, scale % 16 into the others
 #pragma unroll
                     for (int g = 0; g < 4; ++g) {
-                        const uint32_t sc = ((c & 2 ? s.sc[2 + (g >> 1)] : s.sc[g >> 1]) >> (8 * ((c & 1) + 2 * (g & 1)))) & 255u, e = (sc ^ 0x80u) & ~1u, bit = 0u - (sc & 1u);
-                        const uint32_t even = hadd2(0x64006400u | e | (e << 16), 0xe480e480u);
+                        const uint32_t sc = ((c & 2 ? s.sc[2 + (g >> 1)] : s.sc[g >> 1]) >> (8 * ((c & 1) + 2 * (g & 1)))) & 255u, e = (sc ^ 0x80u) & 0xf0u;
+                        const uint32_t high = hadd2(0x64006400u | e | (e << 16), 0xe480e480u), low = small_half2(sc & 15u);
                         uint32_t part[8];
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) part[i] = hmul2(v[8 * g + i], even);
+                        for (int i = 0; i < 8; ++i) part[i] = hmul2(v[8 * g + i], high);
                         tmem_st8(to + 8 * g, part);
 #pragma unroll
-                        for (int i = 0; i < 8; ++i) part[i] = v[8 * g + i] & bit;
+                        for (int i = 0; i < 8; ++i) part[i] = hmul2(v[8 * g + i], low);
+                        tmem_st8(to + 32 + 8 * g, part);
+                    }
+                } else if constexpr (FMT == F_Q5_K) {           // the nibble, centred, into the first columns, the fifth bit into the others
+                    const FoldQuarterScales<FMT> w(c, s);
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        uint32_t part[8];
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) part[i] = hfma2(v[8 * g + i] & (g < 2 ? 0x000f000fu : 0x00f000f0u), g < 2 ? w.slo : w.shi, g < 2 ? w.clo : w.chi);
+                        tmem_st8(to + 8 * g, part);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) part[i] = hmul2(v[8 * g + i] & (g < 2 ? 0x00100010u : 0x01000100u), g < 2 ? w.slo : w.shi);
                         tmem_st8(to + 32 + 8 * g, part);
                     }
                 } else {
                     tmem_st32(to, v);
-                    if (F::MINS && c == 3) {         // {m_0 .. m_7 | 64 m_0 .. 64 m_7}, two 16-byte chunks of a K = 16 operand
-                        uint32_t m[4];
+                }
+                if (F::MINS && c == 3) {             // two 16-byte chunks of a K = 16 operand: {m_0 .. m_7 | 64 m_0 .. 64 m_7}, and 8 * 2^-14 times the scales
+                    const uint32_t am = smem_addr(s_amin + (it & (FD_AMIN - 1)) * 4096 + (quarter * 32 + lane) * 16), as = am + FD_AMIN * 4096;
+                    uint32_t m[4];
 #pragma unroll
-                        for (int i = 0; i < 4; ++i) {
-                            const uint32_t v = s.mn[i >> 1] >> (16 * (i & 1));
-                            m[i] = hadd2(0x64006400u | (v & 63u) | ((v & 0x3f00u) << 8), 0xe400e400u);
-                        }
-                        const uint32_t am = smem_addr(s_amin + (it & (FD_AMIN - 1)) * 4096 + (quarter * 32 + lane) * 16);
-                        sts_u128(am, m[0], m[1], m[2], m[3]);
-                        sts_u128(am + 2048, hmul2(m[0], 0x54005400u), hmul2(m[1], 0x54005400u), hmul2(m[2], 0x54005400u), hmul2(m[3], 0x54005400u));
-                        fence_proxy_async();
+                    for (int i = 0; i < 4; ++i) {
+                        const uint32_t w = s.mn[i >> 1] >> (16 * (i & 1));
+                        m[i] = hadd2(0x64006400u | (w & 63u) | ((w & 0x3f00u) << 8), 0xe400e400u);
                     }
+                    sts_u128(am, m[0], m[1], m[2], m[3]);
+                    sts_u128(am + 2048, hmul2(m[0], 0x54005400u), hmul2(m[1], 0x54005400u), hmul2(m[2], 0x54005400u), hmul2(m[3], 0x54005400u));
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const uint32_t w = s.sc[i >> 1] >> (16 * (i & 1));
+                        m[i] = hmul2(hadd2(0x64006400u | (w & 63u) | ((w & 0x3f00u) << 8), 0xe400e400u), 0x10001000u);
+                    }
+                    sts_u128(as, m[0], m[1], m[2], m[3]);
+                    sts_u128(as + 2048, hmul2(m[0], 0x54005400u), hmul2(m[1], 0x54005400u), hmul2(m[2], 0x54005400u), hmul2(m[3], 0x54005400u));
+                    fence_proxy_async();
                 }
                 if (c % F::PER == F::PER - 1) {
                     tc::tmem_st_wait();
@@ -422,25 +473,50 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
             for (int i = 0; i < OWN; ++i) acc[i] = 0.0f;
             const int tile = at.tile;
             for (int b = begin; b < end; ++b, ++it, at.advance(begin, end, stride)) {
-                const int slot = it % FD_SLOTS, buf = it & 1;
+                const int slot = it % FD_SLOTS, buf = sets == 2 ? it & 1 : 0;
+                const uint32_t d_phase = (uint32_t)(sets == 2 ? it >> 1 : it) & 1u;
                 const float *xd = s_xd + slot * nt + 8 * group, *dd = s_dd + (it % FD_DD_SLOTS) * (2 * FD_ROWS) + row;
-                if (!fd_wait(&ctl->xd_full[slot], (uint32_t)(it / FD_SLOTS) & 1u, ctl, p.status) || !fd_wait(&ctl->d_full[buf], (uint32_t)(it >> 1) & 1u, ctl, p.status)) { ok = false; break; }
+                if (!fd_wait(&ctl->xd_full[slot], (uint32_t)(it / FD_SLOTS) & 1u, ctl, p.status) || !fd_wait(&ctl->d_full[buf], d_phase, ctl, p.status)) { ok = false; break; }
                 tc::fence_after_sync();
                 const float d0 = dd[0], d1 = dd[FD_ROWS];
                 const uint64_t s0 = pack2(d0, d0), s1 = pack2(d1, d1);
-                const uint32_t from = lane_base + (uint32_t)(buf * nt), from_min = lane_base + (uint32_t)(2 * nt);
-                // eight columns at a time, the next ones on their way while these are added
-                uint32_t v0[2][8], v1[2][8];
+                const uint32_t from = lane_base + (uint32_t)(buf * F::LIMBS * nt), from_min = lane_base + (uint32_t)(sets * F::LIMBS * nt);
+                // eight columns at a time, the next ones on their way while these are added (two limbs: asked for once
+                // d * S - dmin * M of these is formed)
+                constexpr int AHEAD = F::LIMBS == 2 ? 1 : 2;
+                uint32_t v0[AHEAD][8], v1[AHEAD][8], vm[AHEAD][8];
                 auto load = [&](int k) {
-                    tc::tmem_ld8(from + (uint32_t)(16 * k), v0[k & 1]);
-                    if (F::MINS) tc::tmem_ld8(from_min + (uint32_t)(16 * k), v1[k & 1]);
+                    tc::tmem_ld8(from + (uint32_t)(16 * k), v0[k % AHEAD]);
+                    if (F::LIMBS == 2) tc::tmem_ld8(from + (uint32_t)(nt + 16 * k), v1[k % AHEAD]);
+                    if (F::MINS) tc::tmem_ld8(from_min + (uint32_t)(16 * k), vm[k % AHEAD]);
+                };
+                auto pair = [&](const uint32_t (&v)[8], int e) { return pack2(__uint_as_float(v[2 * e]), __uint_as_float(v[2 * e + 1])); };
+                auto scaled = [&](int k, int e) {                       // d * S - dmin * M
+                    uint64_t sum = pair(v0[k % AHEAD], e);
+                    // the limbs' sums are exact; S is their sum, rounded once as the integer would be
+                    if constexpr (F::LIMBS == 2) sum = add2(sum, pair(v1[k % AHEAD], e));
+                    sum = mul2(s0, sum);
+                    if constexpr (F::MINS) sum = fma2(s1, pair(vm[k % AHEAD], e), sum);
+                    return sum;
                 };
                 load(0);
                 tc::tmem_ld_wait();
 #pragma unroll
                 for (int k = 0; k < OWN / 8; ++k) {
+                    if (F::LIMBS == 2 && k == FD_HALF / 16 && halves == 2) {
+                        if (!fd_wait(&ctl->d_full[1], d_phase, ctl, p.status)) { ok = false; break; }
+                        tc::fence_after_sync();
+                        load(k);
+                        tc::tmem_ld_wait();
+                    }
+                    const int whole = F::LIMBS == 2 && halves == 2 && k < FD_HALF / 16 ? FD_HALF / 16 : pieces;   // pieces whose accumulators are complete
                     if (k < pieces) {
-                        if (k + 1 < pieces) load(k + 1);
+                        uint64_t v[4];
+                        if constexpr (AHEAD == 1) {
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) v[e] = scaled(k, e);
+                        }
+                        if (k + 1 < whole) load(k + 1);
 #pragma unroll
                         for (int i = 0; i < 8; i += 4) {
                             const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(xd + 16 * k + i);
@@ -448,20 +524,20 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
                             for (int e = 0; e < 2; ++e) {
                                 const int j = i + 2 * e;
                                 uint64_t a = pack2(acc[8 * k + j], acc[8 * k + j + 1]);
-                                uint64_t v = mul2(s0, pack2(__uint_as_float(v0[k & 1][j]), __uint_as_float(v0[k & 1][j + 1])));
-                                if constexpr (F::MINS) v = fma2(s1, pack2(__uint_as_float(v1[k & 1][j]), __uint_as_float(v1[k & 1][j + 1])), v);
-                                a = fma2(e ? x.y : x.x, v, a);
+                                a = fma2(e ? x.y : x.x, AHEAD == 1 ? v[j / 2] : scaled(k, j / 2), a);
                                 unpack2(a, acc[8 * k + j], acc[8 * k + j + 1]);
                             }
                         }
-                        if (k + 1 < pieces) tc::tmem_ld_wait();
+                        if (k + 1 < whole) tc::tmem_ld_wait();
                     }
-                    if (k == 0 ? pieces <= 2 : k + 2 == pieces) {       // all read: the buffers are free
+                    // all read: the buffers are free
+                    if (k == 0 ? whole <= 2 : k + 2 == whole || (F::LIMBS == 2 && k == FD_HALF / 16 && halves == 2 && whole == k + 1)) {
                         tc::fence_before_sync();
                         __syncwarp();
-                        if (lane == 0) mbar_arrive(&ctl->d_empty[buf]);
+                        if (lane == 0) mbar_arrive(&ctl->d_empty[F::LIMBS == 2 && halves == 2 && k >= FD_HALF / 16 ? 1 : buf]);
                     }
                 }
+                if (!ok) break;
             }
             if (!ok) break;
             if (p.slices == 1) {
@@ -530,38 +606,80 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
             bool ok = true;
             int s = 0, buf = 0;
             uint32_t b_phase = 0, a_phase = 0;
+            // tokens [n0, n0 + n) of the tile: chunk j of the block's products, and what the block's end adds
+            auto products = [&](int j, uint32_t a, uint64_t b, uint32_t d, int n0, uint32_t shape) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    // K steps of the half-block in order; two limbs: the four of a quarter for the one and then the other, a
+                    // quarter of Q6_K holding every other step of the half
+                    const uint32_t at = F::LIMBS == 1 ? (uint32_t)(k >> 2) * slab + 32u * (k & 3)
+                                      : FMT == F_Q6_K ? ((uint32_t)(k & 3) >> 1) * slab + 64u * (k & 1) + 32u * (j & 1)
+                                                      : (uint32_t)(j & 1) * slab + 32u * (k & 3);
+                    mma_f16_ts(d + (uint32_t)(n0 + (F::LIMBS == 2 && k >= 4 ? nt : 0)), a + (uint32_t)(8 * k), b + (uint64_t)((at + 128u * (uint32_t)n0) >> 4), shape, j | (F::LIMBS == 2 ? k & 3 : k));
+                }
+            };
+            // 8 * scales * sums of the codes, what the centred codes left out: into the last limb
+            auto centre = [&](int it, uint32_t d, int n0, uint32_t shape) {
+                tc::mma_f16(d + (uint32_t)((F::LIMBS - 1) * nt + n0), am0 + (uint64_t)((FD_AMIN + (it & (FD_AMIN - 1))) * (4096 >> 4)),
+                            xm0 + (uint64_t)((uint32_t)((it & 3) * nt * 32 + 16 * n0) >> 4), shape, 1);
+            };
+            auto minimums = [&](int it, uint32_t dm, int n0, uint32_t shape) {
+                tc::mma_f16(dm + (uint32_t)n0, am0 + (uint64_t)((it & (FD_AMIN - 1)) * (4096 >> 4)), xm0 + (uint64_t)((uint32_t)((it & 3) * nt * 32 + 16 * n0) >> 4), shape, 0);
+            };
+            const uint32_t shape0 = tc::idesc_f16_f32acc(FD_ROWS, FD_HALF), shape1 = tc::idesc_f16_f32acc(FD_ROWS, nt - FD_HALF);
             for (int it = 0; it < total && ok; ++it) {
-                const uint32_t d = tmem + (uint32_t)((it & 1) * nt), dm = tmem + (uint32_t)(2 * nt);
-                // S of two blocks ago has been read (with a min term: waited for at the end of the block before)
-                if (!F::MINS && !fd_wait(&ctl->d_empty[it & 1], ((uint32_t)(it >> 1) & 1u) ^ 1u, ctl, p.status)) { ok = false; break; }
+                const int set = sets == 2 ? it & 1 : 0;
+                const uint32_t d = tmem + (uint32_t)(set * F::LIMBS * nt), dm = tmem + (uint32_t)(sets * F::LIMBS * nt), d_phase = ((uint32_t)(sets == 2 ? it >> 1 : it) & 1u) ^ 1u;
+                // the accumulators have been read: those of this set (two sets with a min term: at the end of the block before)
+                const bool at_end = F::MINS && sets == 2;
+                if (!at_end && !fd_wait(&ctl->d_empty[set], d_phase, ctl, p.status)) { ok = false; break; }
 #pragma unroll 1
                 for (int j = 0; j < F::CHUNKS; ++j) {
                     const bool enters = F::CHUNKS == 2 || (j & 1) == 0, leaves = F::CHUNKS == 2 || (j & 1) == 1;   // a half-block of tokens
                     if ((enters && !fd_wait(&ctl->b_full[s], b_phase, ctl, p.status)) || !fd_wait(&ctl->a_full[buf], a_phase, ctl, p.status)) { ok = false; break; }
                     const uint64_t b = b0 + (uint64_t)((uint32_t)(s * L::stage(nt)) >> 4);
                     const uint32_t a = a_base + 64u * (uint32_t)buf;
+                    const bool last = j == F::CHUNKS - 1, split = F::LIMBS == 2 && halves == 2 && (j == 0 || last);
                     tc::fence_after_sync();
-                    if (elect_one()) {
-#pragma unroll
-                        for (int k = 0; k < 8; ++k) {
-                            // K steps of the half-block in order; a quarter of Q6_K holds every other one, for the one limb and then the other
-                            if (F::LIMBS == 2) mma_f16_ts(d, a + (uint32_t)(8 * k), b + (uint64_t)((((uint32_t)(k & 3) >> 1) * slab + 64u * (k & 1) + 32u * (j & 1)) >> 4), idesc, j | k);
-                            else mma_f16_ts(d, a + (uint32_t)(8 * k), b + (uint64_t)(((uint32_t)(k >> 2) * slab + 32u * (k & 3)) >> 4), idesc, j | k);
+                    if (split) {
+                        // one set of accumulators: the first half of the tokens is complete, and drained, before the second
+                        if (elect_one()) {
+                            products(j, a, b, d, 0, shape0);
+                            if (last) {
+                                if (F::MINS) { centre(it, d, 0, shape0); minimums(it, dm, 0, shape0); }
+                                tc::commit(&ctl->d_full[0]);
+                            }
                         }
-                        tc::commit(&ctl->a_empty[buf][(it + a_blocks) % FD_GROUPS]);
+                        __syncwarp();
+                        if (j == 0) {
+                            if (!fd_wait(&ctl->d_empty[1], d_phase, ctl, p.status)) { ok = false; break; }
+                            tc::fence_after_sync();
+                        }
+                    }
+                    if (elect_one()) {
+                        if (split) products(j, a, b, d, FD_HALF, shape1);
+                        else products(j, a, b, d, 0, idesc);
+                        tc::commit(&ctl->a_empty[buf][(it * F::CHUNKS + j + abufs) / F::CHUNKS % FD_GROUPS]);
                         if (leaves) tc::commit(&ctl->b_empty[s]);
-                        if (!F::MINS && j == F::CHUNKS - 1) tc::commit(&ctl->d_full[it & 1]);
+                        if (last) {
+                            if (F::MINS) {
+                                centre(it, d, split ? FD_HALF : 0, split ? shape1 : idesc);
+                                if (!at_end) minimums(it, dm, split ? FD_HALF : 0, split ? shape1 : idesc);
+                            }
+                            if (!at_end) tc::commit(&ctl->d_full[split ? 1 : set]);
+                        }
                     }
                     __syncwarp();
                     if (++buf == abufs) { buf = 0; a_phase ^= 1u; }
                     if (leaves && ++s == stages) { s = 0; b_phase ^= 1u; }
                 }
-                if (F::MINS && ok) {                                    // M of the block before has been read, and so has its S
+                if (at_end && ok) {
+                    // M of the block before has been read, and so has its S
                     if (it > 0 && !fd_wait(&ctl->d_empty[(it - 1) & 1], (uint32_t)((it - 1) >> 1) & 1u, ctl, p.status)) { ok = false; break; }
                     tc::fence_after_sync();
                     if (elect_one()) {
-                        tc::mma_f16(dm, am0 + (uint64_t)((it & (FD_AMIN - 1)) * (4096 >> 4)), xm0 + (uint64_t)((uint32_t)((it & 3) * nt * 32) >> 4), idesc, 0);
-                        tc::commit(&ctl->d_full[it & 1]);
+                        minimums(it, dm, 0, idesc);
+                        tc::commit(&ctl->d_full[set]);
                     }
                     __syncwarp();
                 }
@@ -569,8 +687,8 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
             // the last commits have to arrive before the CTA leaves
             if (ok && !*reinterpret_cast<volatile int *>(&ctl->abort)) {
                 for (int k = max(0, F::CHUNKS * total - abufs); k < F::CHUNKS * total; ++k) {
-                    const int next = k / F::CHUNKS + a_blocks, group = next % FD_GROUPS;
-                    mbar_wait(&ctl->a_empty[k & (abufs - 1)][group], ((uint32_t)(next / FD_GROUPS) & 1u) ^ (group >= a_blocks ? 0u : 1u), 1u << 20);
+                    const int next = k + abufs, block = next / F::CHUNKS;
+                    mbar_wait(&ctl->a_empty[k & (abufs - 1)][block % FD_GROUPS], a_parity(block, next % F::CHUNKS), 1u << 20);
                 }
                 for (int k = max(0, 2 * total - stages); k < 2 * total; ++k) mbar_wait(&ctl->b_empty[k % stages], (uint32_t)(k / stages) & 1u, 1u << 20);
             }
@@ -631,7 +749,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
 
 // ------------------------------------------------------------------ launch (fold_*.cu instantiate one family each)
 
-struct FoldPlan { int nt, slices, stages, a_buffers; double cost; };
+struct FoldPlan { int nt, slices, stages, a_buffers, sets; double cost; };
 
 template <int FMT>
 int fold_stages(int tt) {
