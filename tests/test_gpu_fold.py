@@ -1,6 +1,7 @@
 """GPU parity of the contraction with the weights in tensor memory (larger batches of Q4_K, Q5_K, Q6_K) against the CPU oracle.
 
-Sizes are the smallest that reach it (above 32 tokens and 5.5e8 products; Q4_K and Q5_K from 25 tokens and 1.2e9) and sit at
+Sizes are the smallest that reach it (above 32 tokens and 5.5e8 products, Q4_K also from 25 tokens and 1.2e9, Q5_K from 65 tokens
+and 1.5e9) and sit at
 the edges of its tiles: rows that do not fill the last 128 (nor, for Q6_K, the last super-row of 8), a matrix of eight rows,
 tokens just above a tile, one block of K, blocks that do not divide among the slices of K, more tiles than SMs, a last round of
 13 rows that is a launch of its own.
@@ -37,6 +38,11 @@ def test_tile_edges(torch, lib, oracle, golden, name, mnk):  # noqa: F811
     check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
 
 
+@pytest.mark.parametrize("mnk", [(65, 5643, 4096), (129, 2707, 4352), (300, 24, 229632), (700, 8377, 256), (90, 32571, 512), (97, 3779, 4096), (66, 18957, 4096)])
+def test_tile_edges_q5_k(torch, lib, oracle, golden, mnk):  # noqa: F811
+    check_both_sources(torch, lib, Problem(torch, oracle, golden, "Q5_K", *mnk))
+
+
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K"])
 def test_fewest_tokens(torch, lib, oracle, golden, name):  # noqa: F811
     check_both_sources(torch, lib, Problem(torch, oracle, golden, name, 25, 3190, 15360))
@@ -59,7 +65,7 @@ def test_largest_codes_and_scales(torch, lib, oracle, golden, name, monkeypatch)
     draw_weights = batch.weights
     monkeypatch.setattr(batch, "weights", largest)
     monkeypatch.setattr(batch, "activations", lambda rng, m, k: np.full((m, k), 0.75, dtype=np.float32))
-    problem = Problem(torch, oracle, golden, name, 64, 2200, 4096)
+    problem = Problem(torch, oracle, golden, name, 66, 5700, 4096)
     problem.run(lib)
     problem.check()
 
@@ -85,12 +91,12 @@ RECORD_BYTES, ONE = {"Q4_K": 144, "Q5_K": 176, "Q6_K": 210}, np.float16(1).resha
 
 
 @pytest.mark.parametrize("name", FORMATS)
-@pytest.mark.parametrize("m", [48, 64, 128])
+@pytest.mark.parametrize("m", [66, 90, 128])
 def test_large_partial_sums_that_cancel(torch, lib, oracle, name, m):  # noqa: F811
     """Largest weights against activations of one sign, then of the other: the sum of a block passes 2^24 and comes back to a few
     thousand.  The integer sums are exact, so the bound is the one of the additions over 16 blocks."""
     rng = np.random.default_rng(m)
-    n, k = 2900, 4096
+    n, k = 5700, 4096
     w = np.full((n, k // 256, RECORD_BYTES[name]), 0xFF, np.uint8)
     if name == "Q6_K":
         w[:, :, 192:208], w[:, :, 208:] = 0x7F, ONE
@@ -111,11 +117,11 @@ def test_large_partial_sums_that_cancel(torch, lib, oracle, name, m):  # noqa: F
 
 
 @pytest.mark.parametrize("name", FORMATS)
-@pytest.mark.parametrize("m", [40, 64, 90, 700])
+@pytest.mark.parametrize("m", [66, 90, 128, 700])
 def test_integer_sums_are_exact(torch, lib, oracle, name, m):  # noqa: F811
     """One block, every bit of codes, scales and mins random, all super-scales 1: the results are integers."""
     rng = np.random.default_rng(m)
-    n, k = int(5.5e8 / m / 256) // 128 * 128 + 131, 256
+    n, k = int(1.5e9 / m / 256) // 128 * 128 + 131, 256
     w = rng.integers(0, 256, size=(n, RECORD_BYTES[name]), dtype=np.uint8)
     if name == "Q6_K": w[:, 208:] = ONE
     else: w[:, :2], w[:, 2:4] = ONE, ONE

@@ -82,18 +82,18 @@ size_t fold_plane_bytes(const TileArgs &a) {
     return s.codes + s.xd + s.mins;
 }
 
-// Picks tokens per tile and slices of K by estimated clocks: rounds of the grid times the blocks of a tile.  A block takes about
-// 1800 clocks when A has buffers for two (up to 80 tokens with a min term, 64 without) and 2350 with one, twice that for
-// Q6_K's two limbs, and hardly depends on the tokens (measured from 16 to 128); a tile's start, its stores and the meeting of
-// the slices are small beside it.
 // Tensor memory (512 columns) goes to A buffers for a whole block, then to a second set of accumulators, then to a second block
 // of A; one limb has two sets always, and half a block of two limbs will do where three accumulators of 128 leave no more.
 template <int FMT> static int fold_sets(int nt) { return FoldFormat<FMT>::LIMBS == 1 || FoldFormat<FMT>::columns(nt, 2) + 256 <= 512 ? 2 : 1; }
 template <int FMT> static int fold_a_buffers(int nt) { return FoldFormat<FMT>::columns(nt, fold_sets<FMT>(nt)) + 256 <= 512 ? 4 : 2; }
+// Picks tokens per tile and slices of K by estimated clocks: rounds of the grid times the blocks of a tile.  A Q4_K block takes
+// about 1800 clocks when A has buffers for two (up to 80 tokens) and 2350 with one, whatever the tokens (measured from 16 to
+// 128); a block of two limbs 4100 with two sets of accumulators and 4600 (64 tokens) to 5300 (128) with one, Q5_K and Q6_K
+// alike.  A tile's start, its stores and the meeting of the slices are small beside it.
 template <int FMT>
 static double fold_tile_cost(int nt, int abufs, long long steps) {
     using F = FoldFormat<FMT>;
-    const double step = F::LIMBS * (abufs >= 2 * F::CHUNKS || (F::LIMBS == 2 && nt <= 64) ? 1800.0 : 2350.0);
+    const double step = F::LIMBS == 2 ? (fold_sets<FMT>(nt) == 2 ? 4100.0 : 3900.0 + 11.0 * nt) : abufs >= 2 * F::CHUNKS ? 1800.0 : 2350.0;
     return steps * step + 1200.0 + 4.0 * nt;
 }
 
@@ -164,7 +164,11 @@ bool fold_supported(const TileArgs &a) {
     // Q4_K: 4096 x 4096 with 32 tokens (0.54e9 products) 13.0 / 14.0, 4099 x 4096 with 33 (0.55e9) 15.4 / 14.3; 1000 x 2560 with
     // 200 (0.51e9) 13.2 / 13.8, with 256 (0.66e9) 19.7 / 14.2; 14336 x 4096 with 24 tokens 24.8 / 23.2, with 32 27.5 / 24.0,
     // 28672 x 8192 with 24 72.2 / 68.5.  Q6_K, twice the work here: 14336 x 4096 with 32 39.8 / 41.5, 4099 x 4096 with 33 21.2 / 20.2.
-    if (a.m <= (a.fmt == F_Q6_K ? 32 : 24) || (double)a.m * (double)a.n * (double)a.k < (a.m <= 32 ? 1.2e9 : 5.5e8)) return false;
+    // Q5_K, twice the work here too and only a tenth more there, from 65 tokens and 1.5e9 products on: 4096 x 4096 with 80 (1.3e9)
+    // 18.3 / 20.0, with 96 (1.6e9) 21.2 / 20.6; 1024 x 4096 with 256 (1.1e9) 17.0 / 19.2; 14336 x 4096 with 56 40.1 / 43.3, with 64 43.7 /
+    // 43.5, with 80 48.2 / 46.3; 28672 x 4096 with 64 66.2 / 79.7, with 80 93.0 / 85.7.
+    const double products = (double)a.m * (double)a.n * (double)a.k;
+    if (a.fmt == F_Q5_K ? a.m <= 64 || products < 1.5e9 : a.m <= (a.fmt == F_Q6_K ? 32 : 24) || products < (a.m <= 32 ? 1.2e9 : 5.5e8)) return false;
     // 16-byte copies of records need a 16-byte aligned matrix (of whole super-rows: fold.cuh); extents are 32-bit in the kernel
     return a.m < (1 << 20) && a.k % 256 == 0 && a.k < (1LL << 22) && a.n >= 8 && a.n < (1LL << 31) && (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0;
 }
