@@ -41,6 +41,7 @@ struct State {
     cudaDeviceProp prop{};
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
+    unsigned long long stream_id = 0;         // of `stream`, once a workspace has been asked for (workspace.cu)
     bool async = false;
     int *status_host = nullptr;   // mapped, pinned: the kernels write here only on failure
     int *status_dev = nullptr;
@@ -509,7 +510,7 @@ int do_mul_mat(int fmt, const void *W, const float *X, void *Xq, const int8_t *g
     MulMat op;
     if (op.prepare(call, fmt, W, X, Xq, grid, signs, powers, Y, N, K, M, ldy, flags, vec_dot_only)) return 1;
     if (op.path == MulMat::NOTHING) return 0;
-    if (const size_t bytes = op.plane_bytes()) CU(workspace(bytes, g.stream, &op.planes));
+    if (const size_t bytes = op.plane_bytes()) CU(workspace(bytes, g.stream, &g.stream_id, &op.planes));
     if (gather) call.not_repeatable();       // its kernels meet the other ranks' in a fixed order of launches
     Key key;
     key.add(3);
@@ -543,6 +544,7 @@ int weft_b200_set_stream(void *cuda_stream) {
     std::lock_guard<std::recursive_mutex> guard(g.lock);
     if (ensure_init(-1)) return 1;
     g.stream = cuda_stream ? static_cast<cudaStream_t>(cuda_stream) : g.own_stream;
+    g.stream_id = 0;
     return 0;
 }
 
@@ -799,7 +801,7 @@ static int issue_steps(Call &call, std::vector<MulMat> &ops) {
     size_t plane_bytes = 0;              // the steps follow each other: one workspace serves them all
     for (const MulMat &op : ops) plane_bytes = op.plane_bytes() > plane_bytes ? op.plane_bytes() : plane_bytes;
     uint8_t *planes = nullptr;
-    if (plane_bytes) CU(workspace(plane_bytes, g.stream, &planes));
+    if (plane_bytes) CU(workspace(plane_bytes, g.stream, &g.stream_id, &planes));
     Key key;
     key.add(4, ops.size());
     for (MulMat &op : ops) {

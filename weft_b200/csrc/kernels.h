@@ -107,7 +107,8 @@ cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_
 
 // Device memory for a call's activation planes, valid for the work it puts on `stream` (workspace.cu); the generation
 // changes whenever memory handed out earlier outside a capture is gone.
-cudaError_t workspace(size_t bytes, cudaStream_t stream, uint8_t **out);
+// *stream_id: 0 when the caller binds a stream; the id is kept there.
+cudaError_t workspace(size_t bytes, cudaStream_t stream, unsigned long long *stream_id, uint8_t **out);
 unsigned long long workspace_generation();
 
 // Bare tcgen05.mma issue loop on every SM (mode 0: kind::i8, one CTA per SM; 1: kind::i8 on CTA pairs; 2: kind::f16):
