@@ -76,20 +76,21 @@ def test_batch_shapes(torch, lib, oracle, golden, name, mnk):
 
 
 @pytest.mark.parametrize("name", ["Q4_0", "Q8_0"])
-@pytest.mark.parametrize("m", [3, 20, 70])
-def test_infinite_scales(torch, lib, oracle, golden, name, m, monkeypatch):
+@pytest.mark.parametrize("m, n, k", [(3, 40, 2048), (20, 40, 2048), (70, 40, 2048), (5, 3000, 256), (90, 1300, 256), (512, 1000, 512)])
+def test_infinite_scales(torch, lib, oracle, golden, name, m, n, k, monkeypatch):
     """Records whose f16 scale is infinite or NaN (a quantizer's overflow): what the oracle gives, infinities with their signs."""
     def overflown(fmt, rng, n, k):
         w = draw_weights(fmt, rng, n, k)
         d = w.reshape(n, k // 32, -1)[:, :, :2]
-        d[0, 0], d[1, 9], d[2, k // 32 - 1], d[17, 3] = [0, 0x7c], [0, 0xfc], [0, 0x7c], [0, 0x7e]
+        for row in range(0, n - 17, 37):
+            d[row, 0], d[row + 1, k // 64], d[row + 2, k // 32 - 1], d[row + 17, 3] = [0, 0x7c], [0, 0xfc], [0, 0x7c], [0, 0x7e]
         return w
 
     draw_weights = weights
     monkeypatch.setitem(globals(), "weights", overflown)
-    problem = Problem(torch, oracle, golden, name, m, 40, 2048)
+    problem = Problem(torch, oracle, golden, name, m, n, k)
     problem.run(lib)
-    got, rows = problem.y.cpu().numpy(), [0, 1, 2, 17]
+    got, rows = problem.y.cpu().numpy(), sorted(row + i for row in range(0, n - 17, 37) for i in (0, 1, 2, 17))
     assert np.isinf(problem.want[:, rows[:3]]).any() and np.isnan(problem.want[:, 17]).all()
     assert np.array_equal(got[:, rows], problem.want[:, rows], equal_nan=True)
     assert rel_l2(np.delete(got, rows, axis=1), np.delete(problem.want, rows, axis=1)) <= 1e-5
