@@ -90,7 +90,7 @@ template <int FMT> __device__ __forceinline__ int fold_row_of(int l) { return Fo
 
 struct FoldParams {
     const uint8_t *w;
-    const float *xd;             // (nb * XROWS, pitch)
+    const float *xd;             // (nb, pitch)
     float *y;
     long long n, ldy, row_bytes, w_bytes, pitch;
     int m, nb, nt;               // tokens, blocks per row, tokens per tile (a multiple of 16)
