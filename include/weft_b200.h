@@ -15,8 +15,16 @@
  *     found again by address, so only activations and outputs move per call.
  *
  * Records are the GGML block formats, never repacked: Q4_0 18 B/32, Q8_0 34 B/32, Q4_K 144 B/256,
- * Q2_K 84 B/256, Q3_K 110 B/256, Q5_K 176 B/256, Q6_K 210 B/256, Q8_K 292 B/256, IQ2_XXS 66 B/256, IQ1_S 50 B/256, IQ1_M 56 B/256, IQ2_XS 74 B/256, IQ2_S 82 B/256, IQ3_XXS 98 B/256, IQ3_S 110 B/256, TQ1_0 54 B/256.  No entry point allocates a hidden workspace for
- * device-pointer arguments: Xq is the caller's written workspace, as in the reference.
+ * Q2_K 84 B/256, Q3_K 110 B/256, Q5_K 176 B/256, Q6_K 210 B/256, Q8_K 292 B/256, IQ2_XXS 66 B/256, IQ1_S 50 B/256, IQ1_M 56 B/256, IQ2_XS 74 B/256, IQ2_S 82 B/256, IQ3_XXS 98 B/256, IQ3_S 110 B/256, TQ1_0 54 B/256. 
+ * Weights, activations, Xq (the caller's written workspace, as in the reference) and Y are used where they are.  What the library
+ * keeps of its own beside them: a batch of three tokens and more (production_mul_mat_* over Q4_0, Q8_0, Q2_K to Q6_K, IQ2_XXS and
+ * TQ1_0, at any entry point) writes its activations into planes, 1 to 2.4 bytes per activation, in device memory that the
+ * library allocates: one buffer per stream that grows to the largest call (eight streams at most, then the longest unused one's is
+ * freed), one per stream of a captured graph for the life of the graph, and up to eight returned ones for reuse.  The first such call
+ * of a stream, and every larger one, allocates (and a larger one waits for that stream, a ninth stream for the device), also in
+ * the asynchronous mode.  production_mul_mat_q4_k_decode_noalloc allocates nothing.  A synchronous call that is repeated on the same
+ * arguments (17 times and more) is replayed from a CUDA graph of the library's, at most 1024 of them; a chain of more than eleven
+ * steps is not.
  * Codebook tables arrive as arguments: grid int8[256][8] (IQ2_XXS), int8[512][8] (IQ2_XS), int8[256][4] (IQ3_XXS, values
  * 4..62), int8[1024][8] (IQ2_S), int8[512][4] (IQ3_S), int8[2048][8] with values -1 / 0 / +1 (IQ1_S, IQ1_M); signs int8[128][8] with entries +1 / -1 (IQ2_S and IQ3_S carry
  * their sign bits in the record and take no sign table).
@@ -145,8 +153,7 @@ int production_mul_mat_q4_k_staged(const uint8_t *W, const float *X, uint8_t *Xq
 int production_mul_mat_tq1_0(const uint8_t *W, const float *X, uint8_t *Xq, const uint32_t *powers,
                              float *Y, size_t N, size_t K, size_t M);
 /* examples/kernels/mul_mat/iq2_xxs_staged.py:9-97    mul_mat_runtime.cpp:458-473
- * (from 32 tokens on, K a multiple of 1024: one tensor-core contraction per 32-element group, integer group scales
- * combined in the epilogue) */
+ * (tensor cores from three tokens on, integer group scales combined in the epilogue) */
 int production_mul_mat_iq2_xxs_staged(const uint8_t *W, const float *X, uint8_t *Xq, const int8_t *grid, const int8_t *signs,
                                       float *Y, size_t N, size_t K, size_t M);
 /* examples/kernels/mul_mat/iq2_xxs.py:10-17: the function of the staged form under the reference's other name */

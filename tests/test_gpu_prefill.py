@@ -54,8 +54,7 @@ def test_prefill_q4_k_one_tile(torch, oracle):
 @pytest.mark.parametrize("mnk", [(128, 128, 1024), (130, 200, 512), (512, 384, 1024), (32, 128, 4096), (200, 1000, 2048), (512, 4736, 1024),
                                  (300, 77, 768), (257, 1001, 1280), (129, 16, 256)])
 def test_prefill_q4_k_shapes(torch, oracle, mnk):
-    """Up to 128 tokens the single-CTA kernel (K a multiple of 1024; the GEMV per token row otherwise); above, the CTA-pair kernel
-    on activation planes with tiles of 256 tokens x 16..80 weights, for every K that is a multiple of 256; ragged N and M."""
+    """Register tiles, and the contraction in tensor memory for the larger products; ragged N and M."""
     m, n, k = mnk
     _run(torch, oracle, m, n, k, seed=sum(mnk))
 
@@ -89,8 +88,7 @@ def test_prefill_matches_decode_path(torch, oracle):
 @pytest.mark.parametrize("m", [64, 300])
 def test_prefill_q4_k_saturated_records(torch, oracle, m):
     """Every weight nibble 15, every 6-bit scale and min 63, every activation code +-127: the largest sums a block can
-    produce (limb sums of 3.4 million, min-term sums of 2 million), through the single-CTA (64 tokens) and the
-    CTA-pair (300 tokens) kernels.  The integer part must still be exact."""
+    produce (31 million, min-term sums of 2 million).  The integer part must still be exact."""
     import weft_b200 as weft
     from weft_b200.kernels import mul_mat
     from weft_b200.runtime import Buffer
