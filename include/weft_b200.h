@@ -17,7 +17,7 @@
  * Records are the GGML block formats, never repacked: Q4_0 18 B/32, Q8_0 34 B/32, Q4_K 144 B/256,
  * Q2_K 84 B/256, Q3_K 110 B/256, Q5_K 176 B/256, Q6_K 210 B/256, Q8_K 292 B/256, IQ2_XXS 66 B/256, IQ1_S 50 B/256, IQ1_M 56 B/256, IQ2_XS 74 B/256, IQ2_S 82 B/256, IQ3_XXS 98 B/256, IQ3_S 110 B/256, TQ1_0 54 B/256. 
  * Weights, activations, Xq (the caller's written workspace, as in the reference) and Y are used where they are.  What the library
- * keeps of its own beside them: a batch of three tokens and more (production_mul_mat_* over Q4_0, Q8_0, Q2_K to Q6_K, IQ2_XXS and
+ * keeps of its own beside them: a batch of three tokens and more (of small matrices: of more; production_mul_mat_* over Q4_0, Q8_0, Q2_K to Q6_K, IQ2_XXS and
  * TQ1_0, at any entry point) writes its activations into planes, 1 to 2.4 bytes per activation, in device memory that the
  * library allocates: one buffer per stream that grows to the largest call (eight streams at most, then the longest unused one's is
  * freed), one per stream of a captured graph for the life of the graph, and up to eight returned ones for reuse.  The first such call
@@ -143,7 +143,7 @@ int production_mul_mat_tq1_0_lane16_decode(const uint8_t *W, const float *X, uin
  * Same arguments.  The reference binds its tile sizes (NC/MC/MR/NR/KC) at compile time
  * (Emitter.h:505-510), so they are not C parameters here either.
  * examples/kernels/mul_mat/q4_0.py:9-30, q8_0.py:9-29, q4_k_staged.py:9-37   mul_mat_runtime.cpp:217-221,277-281,350-357
- * From three tokens on these run on the tensor cores with every weight record read once per tile of tokens; larger batches of
+ * From three tokens on (small matrices: more) these run on the tensor cores with every weight record read once per tile of tokens; larger batches of
  * Q4_K, Q5_K and Q6_K with the weights expanded into tensor memory.  One or two tokens run the decode GEMV per token row. */
 int production_mul_mat_q4_0(const uint8_t *W, const float *X, uint8_t *Xq, float *Y, size_t N, size_t K, size_t M);
 int production_mul_mat_q8_0(const uint8_t *W, const float *X, uint8_t *Xq, float *Y, size_t N, size_t K, size_t M);

@@ -33,5 +33,14 @@ def test_tile_rows_keep_to_32_bit_offsets(tile_supported, fmt):
     assert not tile_supported(fmt, 3, 64, 256 * ((1 << 20) + 1))
 
 
+@pytest.mark.parametrize("fmt", UNIT_BYTES)
+def test_small_batches_go_by_token_rows(tile_supported, fmt):
+    """Up to a number of products, except rows too long for some GEMV, and Q4_K up to 2048 results."""
+    line = {6: 1e7, 15: 1e7, 20: 1e7, 5: 2.5e6}.get(fmt, 5e6)
+    for m, n, k in [(3, 1, 256), (3, 1, 16384), (8, 256, 1024), (8, 257, 1024), (4, 512, 2048), (16, 128, 2048), (32, 64, 2048), (3, 3000, 512)]:
+        assert tile_supported(fmt, m, n, k) == (m * n * k > line or (fmt == 8 and m * n > 2048)), (m, n, k)
+    assert tile_supported(fmt, 3, 1, 16640)
+
+
 def test_tile_sizes_that_are_left_to_others(tile_supported):
     assert not tile_supported(8, 2, 64, 4096) and not tile_supported(8, 3, 64, 4096 + 32) and not tile_supported(8, 3, 64, 4096, w=(1 << 20) + 8)

@@ -1,7 +1,7 @@
 """GPU parity of the register-tile kernel (three tokens and more, every format it takes) against the CPU oracle.
 
 Sizes sit at the edges of its tiles: eight tokens per MMA column group, 16 or 32 rows per warp, 1 to 8 slices of K per
-CTA, one to eight token groups per tile, rows that start at any even address.  Bound: 1e-5 relative L2 and the reference
+CTA, one to eight token groups per tile, rows that start at any even address; the smallest are at both sides of the line to the GEMVs.  Bound: 1e-5 relative L2 and the reference
 harnesses' |a - e| <= 1e-4 + 2e-3 |e|: integer sums are exact, only the order of the fp32 additions differs.
 """
 from __future__ import annotations
@@ -63,7 +63,9 @@ class Problem:
 
 
 @pytest.mark.parametrize("name", FORMATS)
-@pytest.mark.parametrize("mnk", [(3, 1, 256), (3, 17, 512), (8, 300, 1792), (9, 129, 4096), (17, 515, 2304), (40, 64, 2560), (65, 1000, 768), (77, 33, 4352), (136, 700, 512)])
+@pytest.mark.parametrize("mnk", [(3, 1, 256), (3, 17, 512), (8, 300, 1792), (9, 129, 4096), (17, 515, 2304), (40, 64, 2560), (65, 1000, 768), (77, 33, 4352), (136, 700, 512),
+                                 # the edges that the smallest of these stand for, past the line below which a GEMV per row takes them
+                                 (3, 1, 16640), (3, 17, 16640), (8, 300, 4352), (9, 129, 16896), (40, 64, 4352), (90, 500, 256)])
 def test_batch_shapes(torch, lib, oracle, golden, name, mnk):
     problem = Problem(torch, oracle, golden, name, *mnk)
     problem.run(lib)
@@ -76,7 +78,7 @@ def test_batch_shapes(torch, lib, oracle, golden, name, mnk):
 
 
 @pytest.mark.parametrize("name", ["Q4_0", "Q8_0"])
-@pytest.mark.parametrize("m, n, k", [(3, 40, 2048), (20, 40, 2048), (70, 40, 2048), (5, 3000, 256), (90, 1300, 256), (512, 1000, 512)])
+@pytest.mark.parametrize("m, n, k", [(3, 40, 16640), (20, 40, 16640), (70, 40, 4096), (5, 9000, 256), (90, 1300, 256), (512, 1000, 512), (3, 40, 2048)])
 def test_infinite_scales(torch, lib, oracle, golden, name, m, n, k, monkeypatch):
     """Records whose f16 scale is infinite or NaN (a quantizer's overflow): what the oracle gives, infinities with their signs."""
     def overflown(fmt, rng, n, k):
@@ -98,7 +100,7 @@ def test_infinite_scales(torch, lib, oracle, golden, name, m, n, k, monkeypatch)
 
 def test_batch_workspace_is_per_stream_and_per_capture(torch, lib, oracle, golden):
     """A captured call keeps working while calls of another size run on another stream in between."""
-    small, large = Problem(torch, oracle, golden, "Q4_K", 5, 200, 1024), Problem(torch, oracle, golden, "Q6_K", 60, 300, 2048)
+    small, large = Problem(torch, oracle, golden, "Q4_K", 5, 700, 4096), Problem(torch, oracle, golden, "Q6_K", 60, 300, 2048)
     side, other, graph = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
     lib.weft_b200_set_async(1)
     try:
@@ -176,8 +178,8 @@ def test_batch_workspace_of_the_per_thread_stream(torch, lib, oracle, golden):
 def test_batch_calls_beside_a_capture(torch, lib, oracle, golden):
     """Another stream is being captured, in the mode that forbids unsafe calls everywhere: batches on this one, the second with a
     larger workspace, neither fail nor spoil the capture."""
-    problems = [Problem(torch, oracle, golden, "Q4_K", m, 200, 1024) for m in (5, 600)]
-    inside = Problem(torch, oracle, golden, "Q6_K", 9, 200, 1024)
+    problems = [Problem(torch, oracle, golden, "Q4_K", m, 500, 1024) for m in (5, 600)]
+    inside = Problem(torch, oracle, golden, "Q6_K", 9, 1100, 1024)
     side, other, graph = torch.cuda.Stream(), torch.cuda.Stream(), torch.cuda.CUDAGraph()
     lib.weft_b200_set_async(1)
     try:

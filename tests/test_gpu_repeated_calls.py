@@ -29,7 +29,7 @@ def test_repeated_call_follows_its_inputs(torch, oracle, m, where):
     from weft_b200.kernels import mul_mat
     from weft_b200.runtime import Buffer
 
-    n, k = 96, 1024
+    n, k = 420, 1280
     rng = np.random.default_rng(m)
     packed = weights(oracle.Q4_K, rng, n, k)
     kernel = weft.compile(mul_mat.production_mul_mat_q4_k_staged)
@@ -123,7 +123,7 @@ def test_repeated_chain_follows_its_inputs(torch, oracle, steps):
     names = ["Q4_K", "Q4_K", "Q6_K", "Q5_K"]
     parts = []
     for step in range(steps):
-        name, n, m = names[step % 4], 96 + 8 * step, 1 if step % 4 < 2 else 5
+        name, n, m = names[step % 4], 96 + 8 * step + (0 if step % 4 < 2 else 1000), 1 if step % 4 < 2 else 5
         packed, x = weights(getattr(oracle, name), rng, n, k), torch.zeros((m, k), device="cuda")
         reuse = step % 4 == 1                                  # the second Q4_K step takes the first one's records
         xq = parts[-1][3] if reuse else torch.zeros((m, oracle.row_bytes(oracle.Q8_K, k)), dtype=torch.uint8, device="cuda")
