@@ -61,9 +61,16 @@ def _sources_are_newer() -> bool:
     return any((CSRC / name).stat().st_mtime > built for name in SOURCES + HEADERS)
 
 
-def refresh_call_path() -> bool:
+_looked_at: set[Path] = set()
+
+
+def refresh_call_path(once: bool = False) -> bool:
     """Compile the native call path when its source is newer than it.  The library is complete without it (calls then go through
-    ctypes), so a missing C++ compiler, missing Python headers or a failed compilation are no error."""
+    ctypes), so a missing C++ compiler, missing Python headers or a failed compilation are no error.  ``once``: nothing is looked at again in
+    this process (a module that was imported stays the one it is)."""
+    if once and PYCALL in _looked_at:
+        return True
+    _looked_at.add(PYCALL)
     source = CSRC / "pycall.cpp"
     if PYCALL.exists() and PYCALL.stat().st_mtime >= source.stat().st_mtime:
         return True

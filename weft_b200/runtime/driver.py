@@ -53,7 +53,7 @@ class Toolchain:
                 except Exception as error:  # nvcc diagnostics are in the message
                     raise CompilationError(str(error)) from error
             else:
-                build.refresh_call_path()
+                build.refresh_call_path(once=True)
         if not library.exists():
             raise CompilationError(f"native toolchain is unavailable: kernel library {library} does not exist")
         return Toolchain(str(library.resolve()), self.cc, self.cflags)
