@@ -1,6 +1,6 @@
 """GPU parity of the contraction with the weights in tensor memory (larger batches of Q4_K, Q5_K, Q6_K) against the CPU oracle.
 
-Sizes are the smallest that reach it (above 32 tokens and 5.5e8 products, Q4_K also from 25 tokens and 1.2e9, Q5_K from 65 tokens
+Sizes are the smallest that reach it (above 32 tokens and 9e8 products, Q4_K also from 25 tokens and 1.2e9, Q5_K from 65 tokens
 and 1.5e9) and sit at
 the edges of its tiles: rows that do not fill the last 128 (nor, for Q6_K, the last super-row of 8), a matrix of eight rows,
 tokens just above a tile, one block of K, blocks that do not divide among the slices of K, more tiles than SMs, a last round of
@@ -38,9 +38,16 @@ def test_tile_edges(torch, lib, oracle, golden, name, mnk):  # noqa: F811
     check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
 
 
+@pytest.mark.parametrize("name", FORMATS)
 @pytest.mark.parametrize("mnk", [(65, 5643, 4096), (129, 2707, 4352), (300, 24, 229632), (700, 8377, 256), (90, 32571, 512), (97, 3779, 4096), (66, 18957, 4096)])
-def test_tile_edges_q5_k(torch, lib, oracle, golden, mnk):  # noqa: F811
-    check_both_sources(torch, lib, Problem(torch, oracle, golden, "Q5_K", *mnk))
+def test_tile_edges_further_on(torch, lib, oracle, golden, name, mnk):  # noqa: F811
+    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
+
+
+@pytest.mark.parametrize("name", ["Q4_K", "Q6_K"])
+@pytest.mark.parametrize("mnk", [(33, 6689, 4096), (48, 4587, 4096), (300, 16, 229632)])
+def test_narrow_tiles(torch, lib, oracle, golden, name, mnk):  # noqa: F811
+    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
 
 
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K"])

@@ -70,7 +70,7 @@ def grow_and_leave(torch, lib, problem):
 
 
 # a contraction in tensor memory with K in slices, one with a launch for its last rows, the CTA-pair kernel, two limbs
-@pytest.mark.parametrize("name, mnk", [("Q4_K", (64, 2200, 4096)), ("Q4_K", (58, 18949, 512)), ("TQ1_0", (200, 520, 2048)), ("Q6_K", (129, 1027, 4352)), ("Q5_K", (97, 3779, 4096))])
+@pytest.mark.parametrize("name, mnk", [("Q4_K", (64, 3450, 4096)), ("Q4_K", (33, 18957, 4096)), ("TQ1_0", (200, 520, 2048)), ("Q6_K", (129, 1611, 4352)), ("Q5_K", (97, 3779, 4096))])
 def test_repeated_batch_follows_its_inputs(torch, lib, oracle, golden, name, mnk):  # noqa: F811
     from test_gpu_batch import Problem
 

@@ -160,15 +160,16 @@ static FoldSplit split_for(int fmt, long long m, long long n, long long nb, int 
 bool fold_supported(const TileArgs &a) {
     if (a.fmt != F_Q4_K && a.fmt != F_Q5_K && a.fmt != F_Q6_K) return false;
     // Below these the register tiles are quicker: this kernel starts about 4 us later (cluster, tensor memory, planes) and takes
-    // as long for 16 tokens as for 64; the tiles go by 8 tokens up to 32 and get slow steps at 17, 25 and 33.  Tiles / this, us,
-    // Q4_K: 4096 x 4096 with 32 tokens (0.54e9 products) 13.0 / 14.0, 4099 x 4096 with 33 (0.55e9) 15.4 / 14.3; 1000 x 2560 with
-    // 200 (0.51e9) 13.2 / 13.8, with 256 (0.66e9) 19.7 / 14.2; 14336 x 4096 with 24 tokens 24.8 / 23.2, with 32 27.5 / 24.0,
-    // 28672 x 8192 with 24 72.2 / 68.5.  Q6_K, twice the work here: 14336 x 4096 with 32 39.8 / 41.5, 4099 x 4096 with 33 21.2 / 20.2.
+    // as long for 16 tokens as for 64; the tiles go by 8 tokens up to 32 and get slow steps at 17, 25 and 33.  Tiles / this, us on
+    // the device, Q4_K: 4096 x 4096 with 48 tokens (0.81e9 products) 13.4 / 13.7, with 56 (0.94e9) 15.4 / 14.0; 1024 x 4096 with 160
+    // (0.67e9) 13.0 / 13.9, with 256 (1.07e9) 15.6 / 15.0; 14336 x 4096 with 24 tokens 22.5 / 24.3, with 33 29.0 / 25.0.  Q6_K: 4096 x
+    // 4096 with 48 18.2 / 19.1, with 56 19.6 / 19.2; 1024 x 4096 with 160 16.4 / 18.1, with 256 22.0 / 19.4; 14336 x 4096 with 24 32.7 /
+    // 40.4, with 33 42.8 / 41.1.
     // Q5_K, twice the work here too and only a tenth more there, from 65 tokens and 1.5e9 products on: 4096 x 4096 with 80 (1.3e9)
     // 18.3 / 20.0, with 96 (1.6e9) 21.2 / 20.6; 1024 x 4096 with 256 (1.1e9) 17.0 / 19.2; 14336 x 4096 with 56 40.1 / 43.3, with 64 43.7 /
     // 43.5, with 80 48.2 / 46.3; 28672 x 4096 with 64 66.2 / 79.7, with 80 93.0 / 85.7.
     const double products = (double)a.m * (double)a.n * (double)a.k;
-    if (a.fmt == F_Q5_K ? a.m <= 64 || products < 1.5e9 : a.m <= (a.fmt == F_Q6_K ? 32 : 24) || products < (a.m <= 32 ? 1.2e9 : 5.5e8)) return false;
+    if (a.fmt == F_Q5_K ? a.m <= 64 || products < 1.5e9 : a.m <= (a.fmt == F_Q6_K ? 32 : 24) || products < (a.m <= 32 ? 1.2e9 : 9e8)) return false;
     // 16-byte copies of records need a 16-byte aligned matrix (of whole super-rows: fold.cuh); extents are 32-bit in the kernel
     return a.m < (1 << 20) && a.k % 256 == 0 && a.k < (1LL << 22) && a.n >= 8 && a.n < (1LL << 31) && (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0;
 }
