@@ -128,12 +128,12 @@ static int tile_group_bytes(int fmt) {
 // Batches so small that a GEMV per token row is quicker: it is one launch, all rows of tokens side by side on the chip, where the
 // tiles are two kernels, 1.3 to 2 us more.  By products, the line lies where the GEMVs' CTAs no longer run in one round; those of
 // Q4_K fill an SM each from fewer rows on.  Measured at 480 sizes for each format (64 to 3072 rows, K 256 to 8192, 3 to 32 tokens):
-// the choice is 0.3 % slower than the better of the two on average, tiles everywhere 20 %.  Tiles / GEMV, us: 3 x 1024 x 1024 Q3_K
+// the choice is nowhere slower than the tiles, 0.8 % slower than the better of the two on average (tiles everywhere: 20 %).  Tiles / GEMV, us: 3 x 1024 x 1024 Q3_K
 // 4.7 / 2.9, 8 x 1024 x 1024 4.8 / 5.7; Q2_K 4.3 / 2.7 and 4.3 / 3.1; 3 x 300 x 768 Q4_K 4.6 / 2.5, 8 x 300 x 768 4.7 / 4.7.
 static bool by_token_rows(const TileArgs &a) {
     const double products = (double)a.m * (double)a.n * (double)a.k;
     if (a.k > 16384 || (a.fmt == F_Q4_K && a.m * a.n > 2048)) return false;       // longer rows: not every GEMV takes them
-    return products <= (a.fmt == F_Q2_K || a.fmt == F_IQ2_XXS || a.fmt == F_TQ1_0 ? 1e7 : a.fmt == F_Q8_0 ? 2.5e6 : 5e6);
+    return products <= (a.fmt == F_Q2_K || a.fmt == F_IQ2_XXS || a.fmt == F_TQ1_0 ? 8.4e6 : a.fmt == F_Q8_0 ? 2.5e6 : 4.2e6);
 }
 
 bool tile_supported(const TileArgs &a) {
