@@ -1,0 +1,54 @@
+"""GPU parity of the contraction on CTA pairs (larger batches of Q4_K, Q5_K, Q6_K and TQ1_0) against the CPU oracle.
+
+Sizes are the smallest that reach it (1.2e9 products; Q4_K up to 128 tokens from 8192 rows on) and sit at the edges of its tiles: rows
+that do not fill the last 256, nor the last super-row of 8, a matrix of eight rows, tokens just above a chunk and a tile, one block of K,
+fewer tiles than pairs (each shared by several), more tiles than pairs with the rest whole or shared.
+
+Bound: 1e-5 relative L2 and the reference harnesses' |a - e| <= 1e-4 + 2e-3 |e|: the sums of a block are integers and exact, only the
+order of the fp32 additions over the blocks differs.
+"""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+from helpers import rel_l2
+from test_gpu_batch import Problem, lib, torch  # noqa: F401  (fixtures)
+from test_gpu_fold import check_both_sources
+
+pytestmark = pytest.mark.gpu
+
+FORMATS = ["Q4_K", "Q5_K", "Q6_K", "TQ1_0"]
+
+
+@pytest.mark.parametrize("name", FORMATS)
+@pytest.mark.parametrize("mnk", [(129, 2311, 4096),          # few tiles, each shared by several pairs
+                                 (300, 8, 512000),           # one row tile of eight rows, two thousand blocks
+                                 (257, 9371, 512),           # a second tile of one token
+                                 (700, 6703, 256),           # one block: nothing to share
+                                 (40, 14341, 2304),          # one chunk; fewer tiles than pairs, blocks that do not divide
+                                 (65, 19331, 1024),          # more tiles than pairs
+                                 (512, 5003, 768)])
+def test_tile_edges(torch, lib, oracle, golden, name, mnk):  # noqa: F811
+    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
+
+
+@pytest.mark.parametrize("m, n, k", [(130, 2311, 4096), (300, 8203, 512)])
+def test_infinite_scales_of_ternary_records(torch, lib, oracle, golden, m, n, k, monkeypatch):  # noqa: F811
+    """Records whose f16 scale is infinite or NaN: what the oracle gives, infinities with their signs."""
+    import test_gpu_batch as batch
+
+    def overflown(fmt, rng, n, k):
+        w = draw_weights(fmt, rng, n, k)
+        d = w.reshape(n, k // 256, 54)[:, :, 52:]
+        d[5, 0], d[70, -1], d[n - 1, 0], d[n - 9, 1] = [0, 0x7c], [0, 0xfc], [0, 0x7c], [0, 0x7e]
+        return w
+
+    draw_weights = batch.weights
+    monkeypatch.setattr(batch, "weights", overflown)
+    problem = Problem(torch, oracle, golden, "TQ1_0", m, n, k)
+    problem.run(lib)
+    got, rows = problem.y.cpu().numpy(), [5, 70, n - 9, n - 1]
+    assert np.isinf(problem.want[:, rows[:2]]).any() and np.isnan(problem.want[:, n - 9]).all()
+    assert np.array_equal(got[:, rows], problem.want[:, rows], equal_nan=True)
+    assert rel_l2(np.delete(got, rows, axis=1), np.delete(problem.want, rows, axis=1)) <= 1e-5

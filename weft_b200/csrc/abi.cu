@@ -422,7 +422,7 @@ int do_quantize(int act, const float *X, uint8_t *Y, size_t M, size_t K) {
 // One mul_mat with its arguments where the kernels find them, and which kernels run.  One path for the decode and the tiled
 // symbols: what runs is chosen by the number of token rows, the format and the shape.
 struct MulMat {
-    enum Path { NOTHING, GEMV, PAIR, TILES, FOLD };
+    enum Path { NOTHING, GEMV, TILES, FOLD, PAIRS };
     int fmt = 0, act = 0;
     Path path = NOTHING;
     void *w = nullptr, *x = nullptr, *xq = nullptr, *y = nullptr, *gr = nullptr, *sg = nullptr, *pw = nullptr;
@@ -433,7 +433,7 @@ struct MulMat {
     TileArgs tile_args() const {
         return TileArgs{fmt, w, have_xq ? nullptr : (const float *)x, xq, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw, (float *)y, n, k, m, ldy};
     }
-    size_t plane_bytes() const { return path == FOLD ? fold_plane_bytes(tile_args()) : path == TILES ? tile_plane_bytes(tile_args()) : path == PAIR ? prefill_pair_plane_bytes(m, k) : 0; }
+    size_t plane_bytes() const { return path == PAIRS ? pair_plane_bytes(tile_args(), g.prop.multiProcessorCount) : path == FOLD ? fold_plane_bytes(tile_args()) : path == TILES ? tile_plane_bytes(tile_args()) : 0; }
 
     // records: the activation records of an earlier step of the same call, where the kernels find them (have_xq then); that step
     // is not alone
@@ -464,7 +464,7 @@ struct MulMat {
         if ((reinterpret_cast<uintptr_t>(w) & (fmt == F_Q4_K_I16 ? 15u : 1u)) || (reinterpret_cast<uintptr_t>(xq) & (act == F_Q8_K ? 3u : 1u)) ||
             (reinterpret_cast<uintptr_t>(y) & 3u) || (x && (reinterpret_cast<uintptr_t>(x) & 3u)))
             return fail("a buffer does not meet its Encoding alignment");
-        path = prefill_pair_supported(fmt, n, k, m, w, xq) ? PAIR : fold_supported(tile_args()) ? FOLD : tile_supported(tile_args()) ? TILES : GEMV;
+        path = pair_supported(tile_args()) ? PAIRS : fold_supported(tile_args()) ? FOLD : tile_supported(tile_args()) ? TILES : GEMV;
         // decode: the GEMV's own prologue quantizes X (one launch) when the fp32 rows allow 16-byte loads
         fuse_quantize = !have_xq && path == GEMV && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
         return 0;
@@ -480,22 +480,21 @@ struct MulMat {
         if (path == NOTHING) return 0;
         if (path == TILES) {          // their first kernel quantizes X
             if (launched(launch_tile(tile_args(), planes, sms, stream), "batched mul_mat", 2)) return 1;
+        } else if (path == PAIRS) {
+            unsigned kernels = 0;
+            const cudaError_t e = launch_pair(tile_args(), planes, g.status_dev, sms, stream, &kernels);
+            if (launched(e, "batched mul_mat", kernels)) return 1;
         } else if (path == FOLD) {
             unsigned kernels = 0;
             const cudaError_t e = launch_fold(tile_args(), planes, g.status_dev, sms, stream, &kernels);
             if (launched(e, "batched mul_mat", kernels)) return 1;
         } else {
             if (!have_xq && !fuse_quantize && launched(launch_quantize(act, (const float *)x, xq, m, k, sms, stream), "activation quantize")) return 1;
-            if (path == PAIR) {
-                const PrefillArgs pa{fmt, w, xq, (const uint32_t *)pw, (float *)y, n, k, m, ldy, g.status_dev, planes};
-                if (launched(launch_prefill_pair(pa, sms, stream), "prefill mul_mat", 2)) return 1;   // its plane kernel first
-            } else {
-                GemvArgs ga{fmt, w, xq, fuse_quantize ? (const float *)x : nullptr, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw,
-                            (float *)y, n, k, m, ldy, g.status_dev};
-                gathered = gather && gemv_gathers(ga);
-                if (gathered) ga.gather = *gather;
-                if (launched(launch_gemv(ga, sms, stream), "decode mul_mat")) return 1;
-            }
+            GemvArgs ga{fmt, w, xq, fuse_quantize ? (const float *)x : nullptr, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw,
+                        (float *)y, n, k, m, ldy, g.status_dev};
+            gathered = gather && gemv_gathers(ga);
+            if (gathered) ga.gather = *gather;
+            if (launched(launch_gemv(ga, sms, stream), "decode mul_mat")) return 1;
         }
         return gather && !gathered ? launched(launch_gather_push(*gather, m, n, ldy, g.status_dev, sms, stream), "peer all-gather") : 0;
     }

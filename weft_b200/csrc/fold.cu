@@ -6,15 +6,12 @@
 
 namespace weft {
 
-#define FD_ELSEWHERE(FMT) extern template int fold_clusters<FMT>(int); extern template cudaError_t launch_fold_kernel<FMT>(const FoldParams &, const CUtensorMap &, const CUtensorMap &, const CUtensorMap &, int, cudaStream_t);
-FD_EACH_FORMAT(FD_ELSEWHERE)
-
 // ------------------------------------------------------------------ activation planes
 // One warp per (token, 256-element block): quantizes the fp32 values (same bodies as the standalone quantizers), stores the
 // caller's records, the codes as f16 (each group of four as elements 0, 2, 1, 3: the order in which the weights unpack), the
-// scales by (block, token) and, where a min term follows, the sums of 32 codes as 64 h + l in two exact f16 limbs.  Without X
+// scales by (block, token) and the sums of 32 codes as 64 h + l in two exact f16 limbs.  Without X
 // the caller's records are the source.  HBM/L2-bound: 4 bytes in, 1.14 out to the records and 2.1 to the planes.
-template <bool MINS, bool FROM_X, bool A16>
+template <bool FROM_X, bool A16>
 __global__ void __launch_bounds__(256) fold_planes_kernel(const float *__restrict__ x, uint8_t *__restrict__ xq, uint4 *__restrict__ codes, float *__restrict__ xd,
                                                           __half *__restrict__ mins, int m, int nb, long long pitch) {
     asm volatile("griddepcontrol.launch_dependents;");
@@ -39,7 +36,7 @@ __global__ void __launch_bounds__(256) fold_planes_kernel(const float *__restric
             d = *reinterpret_cast<const float *>(rec);
         }
         if (lane == 0) xd[(long long)block * pitch + token] = d;
-        if constexpr (MINS) {
+        {
             const int pair = sum + __shfl_xor_sync(0xffffffffu, sum, 2);       // lanes 4 g .. 4 g + 3: sum of group g
             if ((lane & 3) == 0) {
                 __half *to = mins + unit * 16 + (lane >> 2);
@@ -54,63 +51,52 @@ __global__ void __launch_bounds__(256) fold_planes_kernel(const float *__restric
                                          hadd2(__byte_perm(u1, 0x64646464u, 0x4240), 0xe480e480u), hadd2(__byte_perm(u1, 0x64646464u, 0x4341), 0xe480e480u));
 }
 
-template <bool MINS>
 static cudaError_t launch_planes(const TileArgs &a, uint4 *codes, float *xd, __half *mins, long long pitch, cudaStream_t stream) {
     const int nb = (int)(a.k / 256), m = (int)a.m;
     const unsigned grid = (unsigned)((a.m * nb + 7) / 8);
     uint8_t *xq = static_cast<uint8_t *>(const_cast<void *>(a.xq));
-    if (!a.x) fold_planes_kernel<MINS, false, false><<<grid, 256, 0, stream>>>(nullptr, xq, codes, xd, mins, m, nb, pitch);
-    else if (reinterpret_cast<uintptr_t>(a.x) & 15u) fold_planes_kernel<MINS, true, false><<<grid, 256, 0, stream>>>(a.x, xq, codes, xd, mins, m, nb, pitch);
-    else fold_planes_kernel<MINS, true, true><<<grid, 256, 0, stream>>>(a.x, xq, codes, xd, mins, m, nb, pitch);
+    if (!a.x) fold_planes_kernel<false, false><<<grid, 256, 0, stream>>>(nullptr, xq, codes, xd, mins, m, nb, pitch);
+    else if (reinterpret_cast<uintptr_t>(a.x) & 15u) fold_planes_kernel<true, false><<<grid, 256, 0, stream>>>(a.x, xq, codes, xd, mins, m, nb, pitch);
+    else fold_planes_kernel<true, true><<<grid, 256, 0, stream>>>(a.x, xq, codes, xd, mins, m, nb, pitch);
     return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------ dispatch
 
 struct FoldPlaneSizes { size_t codes, xd, mins; long long pitch; };
-static FoldPlaneSizes plane_sizes(int fmt, long long m, long long k) {
+static FoldPlaneSizes plane_sizes(long long m, long long k) {
     const size_t nb = (size_t)(k / 256), rows = nb;
     FoldPlaneSizes s;
     s.pitch = (m + 127) / 128 * 128 + 128;       // the last tile of tokens reads whole
     s.codes = (size_t)m * (size_t)k * 2;
     s.xd = rows * (size_t)s.pitch * 4;
-    s.mins = (fmt == F_Q4_K || fmt == F_Q5_K) ? (size_t)m * nb * 32 : 0;
+    s.mins = (size_t)m * nb * 32;
     return s;
 }
 size_t fold_plane_bytes(const TileArgs &a) {
-    const FoldPlaneSizes s = plane_sizes(a.fmt, a.m, a.k);
+    const FoldPlaneSizes s = plane_sizes(a.m, a.k);
     return s.codes + s.xd + s.mins;
 }
 
-// Tensor memory (512 columns) goes to A buffers for a whole block, then to a second set of accumulators, then to a second block
-// of A; one limb has two sets always, and half a block of two limbs will do where three accumulators of 128 leave no more.
-template <int FMT> static int fold_sets(int nt) { return FoldFormat<FMT>::LIMBS == 1 || FoldFormat<FMT>::columns(nt, 2) + 256 <= 512 ? 2 : 1; }
-template <int FMT> static int fold_a_buffers(int nt) { return FoldFormat<FMT>::columns(nt, fold_sets<FMT>(nt)) + 256 <= 512 ? 4 : 2; }
-// Picks tokens per tile and slices of K by estimated clocks: rounds of the grid times the blocks of a tile.  A Q4_K block takes
+// Tensor memory (512 columns): the accumulators, and A for two blocks where there is room, else for one.
+static int fold_a_buffers(int nt) { return fold_columns(nt) + 256 <= 512 ? 4 : 2; }
+// Picks tokens per tile and slices of K by estimated clocks: rounds of the grid times the blocks of a tile.  A block takes
 // about 1800 clocks when A has buffers for two (up to 80 tokens) and 2350 with one, whatever the tokens (measured from 16 to
-// 128); a block of two limbs 4100 with two sets of accumulators and 4600 (64 tokens) to 5300 (128) with one, Q5_K and Q6_K
-// alike.  A tile's start, its stores and the meeting of the slices are small beside it.
-template <int FMT>
-static double fold_tile_cost(int nt, int abufs, long long steps) {
-    using F = FoldFormat<FMT>;
-    const double step = F::LIMBS == 2 ? (fold_sets<FMT>(nt) == 2 ? 4100.0 : 3900.0 + 11.0 * nt) : abufs >= 2 * F::CHUNKS ? 1800.0 : 2350.0;
-    return steps * step + 1200.0 + 4.0 * nt;
-}
+// 128).  A tile's start, its stores and the meeting of the slices are small beside it.
+static double fold_tile_cost(int nt, int abufs, long long steps) { return steps * (abufs >= 2 * FD_CHUNKS ? 1800.0 : 2350.0) + 1200.0 + 4.0 * nt; }
 
-template <int FMT>
 static FoldPlan fold_plan(long long m, long long n, long long nb, int sm_count) {
-    using F = FoldFormat<FMT>;
-    FoldPlan best{0, 0, 0, 0, 0, 0.0};
+    FoldPlan best{0, 0, 0, 0, 0.0};
     const long long row_tiles = (n + FD_ROWS - 1) / FD_ROWS;
     for (int nt = 16; nt <= FD_TOKENS; nt += 16) {
-        const int stages = fold_stages<FMT>(nt), abufs = fold_a_buffers<FMT>(nt);
+        const int stages = fold_stages(nt), abufs = fold_a_buffers(nt);
         if (stages < 2) continue;
         const long long tiles = row_tiles * ((m + nt - 1) / nt);
         for (int slices = 1; slices <= 8 && slices <= nb; ++slices) {
-            if (slices > 1 && tiles > fold_clusters<FMT>(slices)) break;
+            if (slices > 1 && tiles > fold_clusters(slices)) break;
             const long long rounds = slices > 1 ? 1 : (tiles + sm_count - 1) / sm_count, steps = (nb + slices - 1) / slices;
-            const double cost = rounds * fold_tile_cost<FMT>(nt, abufs, steps) + (slices > 1 ? 1500.0 : 0.0);
-            if (!best.nt || cost < best.cost) best = FoldPlan{nt, slices, stages, abufs, fold_sets<FMT>(nt), cost};
+            const double cost = rounds * fold_tile_cost(nt, abufs, steps) + (slices > 1 ? 1500.0 : 0.0);
+            if (!best.nt || cost < best.cost) best = FoldPlan{nt, slices, stages, abufs, cost};
         }
     }
     return best;
@@ -118,109 +104,74 @@ static FoldPlan fold_plan(long long m, long long n, long long nb, int sm_count) 
 
 // One launch, or two: where the last round of the grid would be nearly empty, the rows of the full rounds go first and the others
 // follow as a launch of their own, which can share K among the SMs (512 x 14336 x 4096: 448 tiles of 128 tokens are three rounds
-// of 148 and four tiles: 92.7 us as one launch, 86.0 as two; Q6_K 152 and 131; 200 x 28672 x 4096 Q4_K 106 and 82).
+// of 148 and four tiles: 92.7 us as one launch, 86.0 as two; 200 x 28672 x 4096 106 and 82).
 struct FoldSplit { FoldPlan first, second; long long rows; };     // rows of the first launch; all of them: no second
 constexpr double FD_SECOND = 12000.0;     // clocks that a second launch costs beside its tiles
-template <int FMT>
 static FoldSplit fold_split(long long m, long long n, long long nb, int sm_count) {
-    using F = FoldFormat<FMT>;
-    FoldSplit best{fold_plan<FMT>(m, n, nb, sm_count), FoldPlan{0, 0, 0, 0, 0, 0.0}, n};
+    FoldSplit best{fold_plan(m, n, nb, sm_count), FoldPlan{0, 0, 0, 0, 0.0}, n};
     double least = best.first.cost;
     const long long row_tiles = (n + FD_ROWS - 1) / FD_ROWS;
     for (int nt = 16; nt <= FD_TOKENS; nt += 16) {
-        const int stages = fold_stages<FMT>(nt), abufs = fold_a_buffers<FMT>(nt);
+        const int stages = fold_stages(nt), abufs = fold_a_buffers(nt);
         if (stages < 2) continue;
         const long long token_tiles = (m + nt - 1) / nt, rounds = row_tiles * token_tiles / sm_count, rows = rounds * sm_count / token_tiles * FD_ROWS;
-        if (rows <= 0 || rows > n - 8) continue;          // the second launch needs a whole super-row
-        const FoldPlan rest = fold_plan<FMT>(m, n - rows, nb, sm_count);
-        const double cost = rounds * fold_tile_cost<FMT>(nt, abufs, nb);
+        if (rows <= 0 || rows >= n) continue;
+        const FoldPlan rest = fold_plan(m, n - rows, nb, sm_count);
+        const double cost = rounds * fold_tile_cost(nt, abufs, nb);
         if (!rest.nt || cost + rest.cost + FD_SECOND >= least) continue;
         least = cost + rest.cost + FD_SECOND;
-        best = FoldSplit{FoldPlan{nt, 1, stages, abufs, fold_sets<FMT>(nt), cost}, rest, rows};
+        best = FoldSplit{FoldPlan{nt, 1, stages, abufs, cost}, rest, rows};
     }
     return best;
 }
 
-static int fold_window(int fmt) {
-    switch (fmt) {
-#define FD_WINDOW(FMT) case FMT: return FoldFormat<FMT>::PITCH;
-    FD_EACH_FORMAT(FD_WINDOW)
-    default: return 0;
-    }
-}
-
-static FoldSplit split_for(int fmt, long long m, long long n, long long nb, int sm_count) {
-    switch (fmt) {
-#define FD_SPLIT(FMT) case FMT: return fold_split<FMT>(m, n, nb, sm_count);
-    FD_EACH_FORMAT(FD_SPLIT)
-    default: return FoldSplit{};
-    }
-}
-
 bool fold_supported(const TileArgs &a) {
-    if (a.fmt != F_Q4_K && a.fmt != F_Q5_K && a.fmt != F_Q6_K) return false;
+    if (a.fmt != F_Q4_K) return false;
     // Below these the register tiles are quicker: this kernel starts about 4 us later (cluster, tensor memory, planes) and takes
     // as long for 16 tokens as for 64; the tiles go by 8 tokens up to 32 and get slow steps at 17, 25 and 33.  Tiles / this, us on
-    // the device, Q4_K: 4096 x 4096 with 48 tokens (0.81e9 products) 13.4 / 13.7, with 56 (0.94e9) 15.4 / 14.0; 1024 x 4096 with 160
-    // (0.67e9) 13.0 / 13.9, with 256 (1.07e9) 15.6 / 15.0; 14336 x 4096 with 24 tokens 22.5 / 24.3, with 33 29.0 / 25.0.  Q6_K: 4096 x
-    // 4096 with 48 18.2 / 19.1, with 56 19.6 / 19.2; 1024 x 4096 with 160 16.4 / 18.1, with 256 22.0 / 19.4; 14336 x 4096 with 24 32.7 /
-    // 40.4, with 33 42.8 / 41.1.
-    // Q5_K, twice the work here too and only a tenth more there, from 65 tokens and 1.5e9 products on: 4096 x 4096 with 80 (1.3e9)
-    // 18.3 / 20.0, with 96 (1.6e9) 21.2 / 20.6; 1024 x 4096 with 256 (1.1e9) 17.0 / 19.2; 14336 x 4096 with 56 40.1 / 43.3, with 64 43.7 /
-    // 43.5, with 80 48.2 / 46.3; 28672 x 4096 with 64 66.2 / 79.7, with 80 93.0 / 85.7.
+    // the device: 4096 x 4096 with 48 tokens (0.81e9 products) 13.4 / 13.7, with 56 (0.94e9) 15.4 / 14.0; 1024 x 4096 with 160
+    // (0.67e9) 13.0 / 13.9, with 256 (1.07e9) 15.6 / 15.0; 14336 x 4096 with 24 tokens 22.5 / 24.3, with 33 29.0 / 25.0.
     const double products = (double)a.m * (double)a.n * (double)a.k;
-    if (a.fmt == F_Q5_K ? a.m <= 64 || products < 1.5e9 : a.m <= (a.fmt == F_Q6_K ? 32 : 24) || products < (a.m <= 32 ? 1.2e9 : 9e8)) return false;
-    // 16-byte copies of records need a 16-byte aligned matrix (of whole super-rows: fold.cuh); extents are 32-bit in the kernel
+    if (a.m <= 24 || products < (a.m <= 32 ? 1.2e9 : 9e8)) return false;
+    // 16-byte copies of records need a 16-byte aligned matrix; extents are 32-bit in the kernel
     return a.m < (1 << 20) && a.k % 256 == 0 && a.k < (1LL << 22) && a.n >= 8 && a.n < (1LL << 31) && (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0;
 }
 
 // The contraction of `n` rows from `w` on into `y`; `planes` holds what does not depend on the cut.
 static cudaError_t launch_rows(const TileArgs &a, const FoldPlan &plan, const FoldParams &planes, const uint4 *codes, const __half *mins,
-                               const uint8_t *w, float *y, long long n, int sm_count, cudaStream_t stream) {
+                               const uint8_t *w, long long row_bytes, float *y, long long n, int sm_count, cudaStream_t stream) {
     FoldParams p = planes;
-    p.w = w; p.y = y; p.n = n;
-    p.w_bytes = p.row_bytes * n;
-    p.nt = plan.nt; p.slices = plan.slices; p.b_stages = plan.stages; p.a_buffers = plan.a_buffers; p.sets = plan.sets;
+    p.y = y; p.n = n;
+    p.nt = plan.nt; p.slices = plan.slices; p.b_stages = plan.stages; p.a_buffers = plan.a_buffers;
     p.token_tiles = (int)((a.m + p.nt - 1) / p.nt);
     p.tiles = p.token_tiles * (int)((n + FD_ROWS - 1) / FD_ROWS);
     CUtensorMap x_codes, x_mins, w_rows;
     cudaError_t e = encode_tile_map(&x_codes, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, codes, (unsigned long long)a.k, (unsigned long long)a.m, (unsigned long long)a.k * 2, 64, (unsigned)p.nt, true);
-    if (e == cudaSuccess && mins)
+    if (e == cudaSuccess)
         e = encode_tile_map(&x_mins, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, mins, (unsigned long long)p.nb * 16, (unsigned long long)a.m, (unsigned long long)p.nb * 32, 8, (unsigned)p.nt, false);
-    else x_mins = x_codes;
-    // weight records: rows of words, or (fold.cuh) super-rows of eight rows; rows after the last whole super-row are fetched by
-    // the expanders
-    const int unit = unit_bytes(a.fmt);
-    if (e == cudaSuccess && unit % 16 == 0)
-        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT32, w, (unsigned long long)p.row_bytes / 4, (unsigned long long)n, (unsigned long long)p.row_bytes, (unsigned)unit / 4, FD_ROWS, false);
-    else if (e == cudaSuccess)
-        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT8, w, (unsigned long long)p.row_bytes * 8, (unsigned long long)n / 8, (unsigned long long)p.row_bytes * 8, (unsigned)fold_window(a.fmt), 16, false);
-    if (e != cudaSuccess) return e;
-    switch (a.fmt) {
-#define FD_LAUNCH(FMT) case FMT: return launch_fold_kernel<FMT>(p, x_codes, x_mins, w_rows, sm_count, stream);
-    FD_EACH_FORMAT(FD_LAUNCH)
-    default: return cudaErrorNotSupported;
-    }
+    if (e == cudaSuccess)
+        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT32, w, (unsigned long long)row_bytes / 4, (unsigned long long)n, (unsigned long long)row_bytes, FD_UNIT / 4, FD_ROWS, false);
+    return e == cudaSuccess ? launch_fold_kernel(p, x_codes, x_mins, w_rows, sm_count, stream) : e;
 }
 
 cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches) {
-    const FoldPlaneSizes s = plane_sizes(a.fmt, a.m, a.k);
+    const FoldPlaneSizes s = plane_sizes(a.m, a.k);
     uint4 *codes = reinterpret_cast<uint4 *>(planes);
     float *xd = reinterpret_cast<float *>(planes + s.codes);
-    __half *mins = s.mins ? reinterpret_cast<__half *>(planes + s.codes + s.xd) : nullptr;
+    __half *mins = reinterpret_cast<__half *>(planes + s.codes + s.xd);
     FoldParams p{};
     p.xd = xd; p.ldy = a.ldy; p.pitch = s.pitch; p.status = status;
     p.m = (int)a.m;
     p.nb = (int)(a.k / 256);
-    p.row_bytes = (long long)p.nb * unit_bytes(a.fmt);
-    const FoldSplit split = split_for(a.fmt, a.m, a.n, p.nb, sm_count);
+    const long long row_bytes = (long long)p.nb * FD_UNIT;
+    const FoldSplit split = fold_split(a.m, a.n, p.nb, sm_count);
     if (!split.first.nt) return cudaErrorNotSupported;
     *launches = split.second.nt ? 3 : 2;
-    cudaError_t e = mins ? launch_planes<true>(a, codes, xd, mins, s.pitch, stream) : launch_planes<false>(a, codes, xd, mins, s.pitch, stream);
+    cudaError_t e = launch_planes(a, codes, xd, mins, s.pitch, stream);
     const uint8_t *w = static_cast<const uint8_t *>(a.w);
-    if (e == cudaSuccess) e = launch_rows(a, split.first, p, codes, mins, w, a.y, split.rows, sm_count, stream);
+    if (e == cudaSuccess) e = launch_rows(a, split.first, p, codes, mins, w, row_bytes, a.y, split.rows, sm_count, stream);
     if (e == cudaSuccess && split.second.nt)
-        e = launch_rows(a, split.second, p, codes, mins, w + split.rows * p.row_bytes, a.y + split.rows, a.n - split.rows, sm_count, stream);
+        e = launch_rows(a, split.second, p, codes, mins, w + split.rows * row_bytes, row_bytes, a.y + split.rows, a.n - split.rows, sm_count, stream);
     return e;
 }
 

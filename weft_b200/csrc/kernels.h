@@ -13,7 +13,7 @@ namespace weft {
 // to the (function, device) pair, so what was already granted is remembered per device; defined in gemv.cu.
 cudaError_t grant_dynamic_smem(const void *kernel, int bytes);
 
-// Refuses a kernel that was not compiled with the register count its setmaxnreg trade assumes; defined in prefill_pair.cu.
+// Refuses a kernel that was not compiled with the register count its setmaxnreg trade assumes; defined in pairs.cu.
 cudaError_t check_launch_registers(const void *kernel, int expected);
 
 // W: `elements` logical values as contiguous records of `fmt`; Y: `elements` floats.
@@ -68,22 +68,6 @@ bool gemv_q4ki_supported(const GemvArgs &a);
 cudaError_t launch_gemv_q4ki(const GemvArgs &a, int sm_count, cudaStream_t stream);
 cudaError_t launch_interleave_q4k(const void *source, void *target, long long rows, long long k, int sm_count, cudaStream_t stream);
 
-struct PrefillArgs {
-    int fmt;
-    const void *w;           // (n, k) records
-    const void *xq;          // (m, k) Q8_K records (already quantized)
-    const uint32_t *powers;  // TQ1_0 only
-    float *y;                // (m, ldy)
-    long long n, k, m, ldy;
-    int *status;
-    uint8_t *planes;         // prefill_pair_plane_bytes() of device memory for the activation planes
-};
-size_t prefill_pair_plane_bytes(long long m, long long k);
-// tcgen05 int8 contraction on CTA pairs (256 tokens per tile, cta_group::2): TQ1_0 with more than 128 tokens.
-// Two launches.
-cudaError_t launch_prefill_pair(const PrefillArgs &a, int sm_count, cudaStream_t stream);
-bool prefill_pair_supported(int fmt, long long n, long long k, long long m, const void *w, const void *xq);
-
 // More than one token row: the register-tile kernel (tile.cuh) behind the kernel that quantizes X into its planes.
 struct TileArgs {
     int fmt;
@@ -104,6 +88,11 @@ template <int FMT> cudaError_t launch_tile_kernel(const TileArgs &a, const uint8
 bool fold_supported(const TileArgs &a);
 size_t fold_plane_bytes(const TileArgs &a);
 cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches);   // two or three kernels
+
+// tcgen05 contraction on CTA pairs (pairs.cuh), behind the kernel that makes its planes.
+bool pair_supported(const TileArgs &a);
+size_t pair_plane_bytes(const TileArgs &a, int sm_count);
+cudaError_t launch_pair(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches);   // two or three kernels
 
 // Device memory for a call's activation planes, valid for the work it puts on `stream` (workspace.cu); the generation
 // changes whenever memory handed out earlier outside a capture is gone.

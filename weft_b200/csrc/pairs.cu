@@ -1,0 +1,210 @@
+// Host side of the contraction on CTA pairs (pairs.cuh) and the kernel that quantizes activations into its planes.
+#include "pairs.cuh"
+#include "quantize.cuh"
+
+#include <algorithm>
+
+namespace weft {
+
+#define PR_ELSEWHERE(FMT) extern template cudaError_t launch_pair_kernel<FMT>(const PairParams &, const CUtensorMap &, const CUtensorMap &, const CUtensorMap &, int, cudaStream_t);
+PR_EACH_FORMAT(PR_ELSEWHERE)
+
+// ------------------------------------------------------------------ activation planes
+// One warp per (token, 256-element block): quantizes the fp32 values (same bodies as the standalone quantizers), stores the
+// caller's records, the codes in the contraction's operand order and type, the scales by (block, token) and, where a min term
+// follows, the sums of 32 codes as 64 h + l in two exact f16 limbs.  Without X the caller's records are the source.  HBM/L2-bound:
+// 4 bytes in, 1.14 out to the records and 1 or 2.1 to the planes.
+template <int FMT, bool FROM_X, bool A16>
+__global__ void __launch_bounds__(256) pair_planes_kernel(const float *__restrict__ x, uint8_t *__restrict__ xq, uint8_t *__restrict__ codes, float *__restrict__ xd,
+                                                          __half *__restrict__ mins, int m, int nb, long long pitch) {
+    using F = PairFormat<FMT>;
+    __shared__ uint8_t s_codes[F::TABLE ? 8 : 1][256];
+    asm volatile("griddepcontrol.launch_dependents;");
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const long long unit = (long long)blockIdx.x * 8 + warp;
+    if (unit >= (long long)m * nb) return;
+    const int token = (int)(unit / nb), block = (int)(unit - (long long)token * nb);
+    uint32_t q0, q1;
+    float d;
+    uint8_t *rec = xq + unit * 292;
+    int sum;                                  // of the lane pair's 16 codes (the record's bsum)
+    if constexpr (FROM_X) {
+        float v[8];
+        load8<A16>(x + unit * 256 + 8 * lane, v);
+        q8_k_warp(v, q0, q1, sum, d);
+        store_q8_k(rec, lane, q0, q1, sum, d);
+    } else {
+        q0 = *reinterpret_cast<const uint32_t *>(rec + 4 + 8 * lane);
+        q1 = *reinterpret_cast<const uint32_t *>(rec + 8 + 8 * lane);
+        sum = *reinterpret_cast<const int16_t *>(rec + 260 + (lane & ~1));
+        d = *reinterpret_cast<const float *>(rec);
+    }
+    if (lane == 0) xd[(long long)block * pitch + token] = d;
+    if constexpr (F::MINS) {
+        const int pair = sum + __shfl_xor_sync(0xffffffffu, sum, 2);       // lanes 4 g .. 4 g + 3: sum of group g
+        if ((lane & 3) == 0) {
+            __half *to = mins + unit * 16 + (lane >> 2);
+            to[0] = __int2half_rn(pair & 63);
+            to[8] = __int2half_rn(pair >> 6);
+        }
+    }
+    if constexpr (!F::I8) {
+        // bytes as f16: set under the exponent of 1024, 128 added to make them unsigned, both taken out again
+        const uint32_t u0 = q0 ^ 0x80808080u, u1 = q1 ^ 0x80808080u;
+        reinterpret_cast<uint4 *>(codes)[unit * 32 + lane] =
+            make_uint4(hadd2(__byte_perm(u0, 0x64646464u, 0x4240), 0xe480e480u), hadd2(__byte_perm(u0, 0x64646464u, 0x4341), 0xe480e480u),
+                       hadd2(__byte_perm(u1, 0x64646464u, 0x4240), 0xe480e480u), hadd2(__byte_perm(u1, 0x64646464u, 0x4341), 0xe480e480u));
+    } else if constexpr (F::TABLE != 0) {
+        *reinterpret_cast<uint2 *>(&s_codes[warp][8 * lane]) = make_uint2(q0, q1);
+        __syncwarp();
+        uint32_t out[2] = {0, 0};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) out[i >> 2] |= (uint32_t)s_codes[warp][tq1_operand_element(8 * lane + i)] << (8 * (i & 3));
+        reinterpret_cast<uint2 *>(codes)[unit * 32 + lane] = make_uint2(out[0], out[1]);
+    } else {
+        reinterpret_cast<uint2 *>(codes)[unit * 32 + lane] = make_uint2(q0, q1);
+    }
+}
+
+// ------------------------------------------------------------------ dispatch
+
+// Chunks of a tile, pairs, and whether tiles are shared: by estimated time (us).  A block takes a pair this long, measured on 14336 x 4096
+// with 64 to 256 tokens; sharing costs a kernel that adds the parts (512 x 4096 x 768 Q6_K: 13.6 us whole, 18 to 20 with shared tiles of
+// any size).
+struct PairPlan { int chunks, pairs; bool share; };
+template <int FMT>
+static PairPlan pair_plan(const TileArgs &a, int sm_count) {
+    using F = PairFormat<FMT>;
+    constexpr double BLOCK = FMT == F_Q4_K ? 0.62 : FMT == F_Q5_K ? 0.75 : FMT == F_Q6_K ? 1.3 : 0.85;
+    constexpr double TOKEN = FMT == F_Q4_K ? 0.0046 : FMT == F_Q5_K ? 0.0088 : FMT == F_Q6_K ? 0.0039 : 0.0023;
+    constexpr double SHARING = 5.0;
+    const long long row_tiles = (a.n + PR_ROWS - 1) / PR_ROWS, nb = a.k / 256, most = sm_count / 2;
+    PairPlan best{0, 0, false};
+    double least = 0.0;
+    auto consider = [&](int chunks, long long pairs, bool share, long long blocks) {
+        const double cost = (double)blocks * (BLOCK + TOKEN * chunks * F::CHUNK) + (share ? SHARING : 0.0);
+        if (!best.chunks || cost < least) { best = PairPlan{chunks, (int)pairs, share}; least = cost; }
+    };
+    for (int chunks = 1; chunks <= F::TOKENS / F::CHUNK; ++chunks) {
+        const long long tiles = row_tiles * ((a.m + chunks * F::CHUNK - 1) / (chunks * F::CHUNK)), pairs = std::min(tiles, most);
+        consider(chunks, pairs, false, (tiles + pairs - 1) / pairs * nb);
+        if (tiles >= most) consider(chunks, most, true, (tiles * nb + most - 1) / most);
+        else for (long long parts = 2; parts <= std::min(most / tiles, nb); ++parts) consider(chunks, tiles * parts, true, (nb + parts - 1) / parts);
+    }
+    return best;
+}
+
+struct PairPlanes { size_t codes, xd, mins, parts; long long pitch; };      // bytes of each, one after the other
+template <int FMT>
+static PairPlanes pair_planes(const TileArgs &a, const PairPlan &plan) {
+    using F = PairFormat<FMT>;
+    const size_t nb = (size_t)(a.k / 256), m = (size_t)a.m;
+    auto whole = [](size_t bytes) { return (bytes + 255) & ~size_t(255); };
+    PairPlanes s;
+    s.pitch = (a.m + F::TOKENS - 1) / F::TOKENS * F::TOKENS + F::TOKENS;       // the last tile of tokens reads whole
+    s.codes = whole(m * nb * (F::I8 ? 256 : 512));
+    s.xd = whole(nb * (size_t)s.pitch * 4);
+    s.mins = F::MINS ? whole(m * nb * 32) : 0;
+    s.parts = plan.share ? (size_t)plan.pairs * 2 * PR_ROWS * F::TOKENS * sizeof(float) : 0;
+    return s;
+}
+template <int FMT> static size_t plane_bytes(const TileArgs &a, int sm_count) {
+    const PairPlanes s = pair_planes<FMT>(a, pair_plan<FMT>(a, sm_count));
+    return s.codes + s.xd + s.mins + s.parts;
+}
+size_t pair_plane_bytes(const TileArgs &a, int sm_count) {
+    switch (a.fmt) {
+#define PR_BYTES(FMT) case FMT: return plane_bytes<FMT>(a, sm_count);
+    PR_EACH_FORMAT(PR_BYTES)
+    default: return 0;
+    }
+}
+
+bool pair_supported(const TileArgs &a) {
+    // Where this kernel is the quickest, us on the device of what runs otherwise (register tiles, for Q4_K fold.cuh) / this:
+    // Q6_K  from 33 tokens and 8.2e8 products on: 48 x 4096 x 4096 (8.1e8) 18.4 / 18.9, 200 x 1024 x 4096 (8.4e8) 19.0 / 17.9, 256 x 2048 x
+    //       2048 (1.1e9) 22.3 / 16.8, 64 x 4096 x 4096 21.7 / 19.2
+    // Q5_K  1.2e9: 64 x 4096 x 4096 (1.1e9) 16.5 / 17.8, 384 x 4096 x 768 (1.2e9) 14.0 / 12.5, 96 x 4096 x 4096 21.5 / 19.0; short rows from 65
+    //       tokens: 40 x 32000 x 2048 27.3 / 30.4, 64 35.8 / 31
+    // TQ1_0 1.2e9: 256 x 2048 x 2048 (1.1e9) 15.3 / 16.9, 384 x 4096 x 768 13.3 / 12.9, 384 x 1024 x 4096 20.4 / 19.5; up to 40 tokens the tiles
+    //       of 8 are quicker unless there are many long rows: 40 x 4096 x 14336 27.4 / 29.3, 40 x 14336 x 4096 29.1 / 27.0
+    // Q4_K  1.2e9 and more than 128 tokens: 160 x 4096 x 2048 (1.3e9) 15.4 / 14.6, 160 x 4096 x 4096 20.9 / 19.0, 128 x 4096 x 4096 16.4 / 17.1; but few
+    //       short rows leave too little for every pair: 512 x 1024 x 4096 17.7 / 18.9, 256 x 1024 x 14336 27.4 / 25.2.  Fewer tokens where
+    //       there are many rows: 40 x 14336 x 4096 25.1 / 23.1, 128 x 4096 x 14336 31.0 / 31.5
+    const double products = (double)a.m * (double)a.n * (double)a.k;
+    if (a.m <= 32) return false;
+    switch (a.fmt) {
+    case F_Q6_K: if (products < 8.2e8) return false; break;
+    case F_Q5_K: if (products < 1.2e9 || (a.m <= 64 && a.k < 4096)) return false; break;
+    case F_TQ1_0: if (products < 1.2e9 || (a.m <= 40 && (a.n < 8192 || a.k < 4096))) return false; break;
+    case F_Q4_K: if (products < 1.2e9 || (a.m <= 128 ? a.n < 8192 : a.n < 2048 && a.k < 8192)) return false; break;
+    default: return false;
+    }
+    // 16-byte copies of records need a 16-byte aligned matrix (of whole super-rows); extents are 32-bit in the kernel
+    const long long blocks = (a.n + PR_ROWS - 1) / PR_ROWS * ((a.m + 31) / 32) * (a.k / 256);
+    return a.m < (1 << 20) && a.k % 256 == 0 && a.k < (1LL << 22) && a.n >= 8 && a.n < (1LL << 31) && blocks < (1LL << 30) && (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0;
+}
+
+template <int FMT>
+static cudaError_t launch_pair_format(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches) {
+    using F = PairFormat<FMT>;
+    const PairPlan plan = pair_plan<FMT>(a, sm_count);
+    const PairPlanes s = pair_planes<FMT>(a, plan);
+    uint8_t *codes = planes;
+    float *xd = reinterpret_cast<float *>(codes + s.codes);
+    __half *mins = reinterpret_cast<__half *>(codes + s.codes + s.xd);
+    PairParams p{};
+    p.parts = reinterpret_cast<ulonglong2 *>(codes + s.codes + s.xd + s.mins);
+    p.w = static_cast<const uint8_t *>(a.w); p.powers = a.powers; p.xd = xd; p.y = a.y; p.n = a.n; p.ldy = a.ldy; p.pitch = s.pitch; p.status = status;
+    p.m = (int)a.m; p.nb = (int)(a.k / 256); p.chunks = plan.chunks;
+    p.row_bytes = (long long)p.nb * F::UNIT;
+    p.token_tiles = (int)((a.m + plan.chunks * F::CHUNK - 1) / (plan.chunks * F::CHUNK));
+    const int tiles = (int)((a.n + PR_ROWS - 1) / PR_ROWS) * p.token_tiles;
+    p.pairs = plan.pairs;
+    p.rounds = tiles / p.pairs;
+    p.rest = tiles % p.pairs;
+    p.unit = plan.share ? 1 : p.nb;
+    p.per = plan.share ? p.rest * p.nb / p.pairs : 0;
+    p.extra = plan.share ? p.rest * p.nb % p.pairs : p.rest;
+    *launches = p.rest && plan.share ? 3 : 2;
+    const unsigned grid = (unsigned)((a.m * p.nb + 7) / 8);
+    uint8_t *xq = static_cast<uint8_t *>(const_cast<void *>(a.xq));
+    if (!a.x) pair_planes_kernel<FMT, false, false><<<grid, 256, 0, stream>>>(nullptr, xq, codes, xd, mins, p.m, p.nb, s.pitch);
+    else if (reinterpret_cast<uintptr_t>(a.x) & 15u) pair_planes_kernel<FMT, true, false><<<grid, 256, 0, stream>>>(a.x, xq, codes, xd, mins, p.m, p.nb, s.pitch);
+    else pair_planes_kernel<FMT, true, true><<<grid, 256, 0, stream>>>(a.x, xq, codes, xd, mins, p.m, p.nb, s.pitch);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+
+    CUtensorMap x_codes, x_mins, w_rows;
+    const unsigned long long m = (unsigned long long)a.m, nb = (unsigned long long)p.nb;
+    e = F::I8 ? encode_piece_map(&x_codes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, codes, 128, m, 2 * nb, F::CHUNK / 2, 2, true)
+              : encode_piece_map(&x_codes, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, codes, 64, m, 4 * nb, F::CHUNK / 2, 4, true);
+    if (e == cudaSuccess && F::MINS) e = encode_piece_map(&x_mins, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, mins, 8, m, 2 * nb, F::CHUNK / 2, 2, false);
+    else x_mins = x_codes;
+    // weight records: rows of words, or super-rows of eight rows; rows after the last whole super-row are fetched by the expanders
+    if (e == cudaSuccess && !F::SHIFTED)
+        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT32, p.w, (unsigned long long)p.row_bytes / 4, (unsigned long long)a.n, (unsigned long long)p.row_bytes, F::UNIT / 4, 128, false);
+    else if (e == cudaSuccess)
+        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.w, (unsigned long long)p.row_bytes * 8, (unsigned long long)a.n / 8, (unsigned long long)p.row_bytes * 8, F::PITCH, 16, false);
+    if (e != cudaSuccess) return e;
+    return launch_pair_kernel<FMT>(p, x_codes, x_mins, w_rows, plan.pairs, stream);
+}
+
+// The register trade assumes the allocation the kernel was compiled with: a build with another one must not run
+cudaError_t check_launch_registers(const void *kernel, int expected) {
+    cudaFuncAttributes attr;
+    const cudaError_t e = cudaFuncGetAttributes(&attr, kernel);
+    if (e != cudaSuccess) return e;
+    return attr.numRegs == expected ? cudaSuccess : cudaErrorInvalidConfiguration;
+}
+
+cudaError_t launch_pair(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches) {
+    if (a.fmt == F_TQ1_0 && !a.powers) return cudaErrorInvalidValue;
+    switch (a.fmt) {
+#define PR_LAUNCH(FMT) case FMT: return launch_pair_format<FMT>(a, planes, status, sm_count, stream, launches);
+    PR_EACH_FORMAT(PR_LAUNCH)
+    default: return cudaErrorNotSupported;
+    }
+}
+
+}  // namespace weft

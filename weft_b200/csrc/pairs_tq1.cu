@@ -1,0 +1,6 @@
+// Instantiations of the contraction on CTA pairs (pairs.cuh), a file per family so that they compile side by side.
+#include "pairs.cuh"
+
+namespace weft {
+template cudaError_t launch_pair_kernel<F_TQ1_0>(const PairParams &, const CUtensorMap &, const CUtensorMap &, const CUtensorMap &, int, cudaStream_t);
+}  // namespace weft

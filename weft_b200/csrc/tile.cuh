@@ -2,7 +2,7 @@
 // registers (mma.sync m16n8k32 / m16n8k16), for every format of the path that a batch of tokens is multiplied with.
 // (Same functions as the decode GEMVs; examples/kernels/mul_mat/*.py of the reference.)
 //
-// What it is for: from 3 tokens up to the sizes that fold.cuh and prefill_pair.cu take.  A weight record carries
+// What it is for: from 3 tokens up to the sizes that fold.cuh and pairs.cuh take.  A weight record carries
 // an integer scale per 16 or 32 elements, so a product can be accumulated on the tensor core over 16 or 32 elements only
 // before the scale has to be applied.  With tensor-memory accumulators that is a round trip per group or two int8 limbs
 // per weight; a register accumulator costs one integer multiply-add per value, which runs beside the next MMA (measured on
