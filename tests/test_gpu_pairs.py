@@ -1,4 +1,4 @@
-"""GPU parity of the contraction on CTA pairs (larger batches of Q4_K, Q5_K, Q6_K and TQ1_0) against the CPU oracle.
+"""GPU parity of the contraction on CTA pairs (larger batches of Q4_K, Q5_K, Q6_K, TQ1_0, Q4_0 and Q8_0) against the CPU oracle.
 
 Sizes are the smallest that reach it (1.2e9 products; Q4_K up to 128 tokens from 8192 rows on) and sit at the edges of its tiles: rows
 that do not fill the last 256, nor the last super-row of 8, a matrix of eight rows, tokens just above a chunk and a tile, one block of K,
@@ -18,7 +18,7 @@ from test_gpu_fold import check_both_sources
 
 pytestmark = pytest.mark.gpu
 
-FORMATS = ["Q4_K", "Q5_K", "Q6_K", "TQ1_0"]
+FORMATS = ["Q4_K", "Q5_K", "Q6_K", "TQ1_0", "Q4_0", "Q8_0"]
 
 
 @pytest.mark.parametrize("name", FORMATS)
@@ -28,7 +28,8 @@ FORMATS = ["Q4_K", "Q5_K", "Q6_K", "TQ1_0"]
                                  (700, 6703, 256),           # one block: nothing to share
                                  (40, 14341, 2304),          # one chunk; fewer tiles than pairs, blocks that do not divide
                                  (65, 19331, 1024),          # more tiles than pairs
-                                 (512, 5003, 768)])
+                                 (512, 5003, 768),
+                                 (384, 3000, 1280)])          # fewer tiles than pairs, all pairs sharing them
 def test_tile_edges(torch, lib, oracle, golden, name, mnk):  # noqa: F811
     check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
 
@@ -50,5 +51,26 @@ def test_infinite_scales_of_ternary_records(torch, lib, oracle, golden, m, n, k,
     problem.run(lib)
     got, rows = problem.y.cpu().numpy(), [5, 70, n - 9, n - 1]
     assert np.isinf(problem.want[:, rows[:2]]).any() and np.isnan(problem.want[:, n - 9]).all()
+    assert np.array_equal(got[:, rows], problem.want[:, rows], equal_nan=True)
+    assert rel_l2(np.delete(got, rows, axis=1), np.delete(problem.want, rows, axis=1)) <= 1e-5
+
+
+@pytest.mark.parametrize("name", ["Q4_0", "Q8_0"])
+def test_infinite_scales_of_groups(torch, lib, oracle, golden, name, monkeypatch):  # noqa: F811
+    """Records of 32 elements whose f16 scale is infinite or NaN: the rows are what the oracle gives, NaN where its sums are."""
+    import test_gpu_batch as batch
+
+    def overflown(fmt, rng, n, k):
+        w = draw_weights(fmt, rng, n, k)
+        d = w.reshape(n, k // 32, -1)[:, :, :2]
+        d[5, 0], d[70, -1], d[n - 1, 3], d[n - 9, 1] = [0, 0x7c], [0, 0xfc], [0, 0x7c], [0, 0x7e]
+        return w
+
+    draw_weights = batch.weights
+    monkeypatch.setattr(batch, "weights", overflown)
+    problem = Problem(torch, oracle, golden, name, 250, 2311, 4096)
+    problem.run(lib)
+    got, rows = problem.y.cpu().numpy(), [5, 70, 2311 - 9, 2311 - 1]
+    assert np.isinf(problem.want[:, rows[:2]]).any() and np.isnan(problem.want[:, 2311 - 9]).all()
     assert np.array_equal(got[:, rows], problem.want[:, rows], equal_nan=True)
     assert rel_l2(np.delete(got, rows, axis=1), np.delete(problem.want, rows, axis=1)) <= 1e-5

@@ -26,9 +26,23 @@ __global__ void __launch_bounds__(256) pair_planes_kernel(const float *__restric
     const int token = (int)(unit / nb), block = (int)(unit - (long long)token * nb);
     uint32_t q0, q1;
     float d;
-    uint8_t *rec = xq + unit * 292;
+    uint8_t *rec = xq + unit * (F::GROUPED ? 272 : 292);
     int sum;                                  // of the lane pair's 16 codes (the record's bsum)
-    if constexpr (FROM_X) {
+    if constexpr (F::GROUPED) {
+        rec += 34 * (lane >> 2);
+        if constexpr (FROM_X) {
+            float v[8];
+            load8<A16>(x + unit * 256 + 8 * lane, v);
+            q8_0_warp(v, q0, q1, sum, d);
+            store_q8_0(rec, lane & 3, q0, q1, d);
+            d = __half2float(__float2half_rn(d));
+        } else {
+            q0 = ld_u32_a2(rec + 2 + 8 * (lane & 3));
+            q1 = ld_u32_a2(rec + 6 + 8 * (lane & 3));
+            d = half_bits_to_float(ld_u16(rec));
+        }
+        if ((lane & 3) == 0) xd[(long long)(8 * block + (lane >> 2)) * pitch + token] = d;
+    } else if constexpr (FROM_X) {
         float v[8];
         load8<A16>(x + unit * 256 + 8 * lane, v);
         q8_k_warp(v, q0, q1, sum, d);
@@ -39,7 +53,7 @@ __global__ void __launch_bounds__(256) pair_planes_kernel(const float *__restric
         sum = *reinterpret_cast<const int16_t *>(rec + 260 + (lane & ~1));
         d = *reinterpret_cast<const float *>(rec);
     }
-    if (lane == 0) xd[(long long)block * pitch + token] = d;
+    if (!F::GROUPED && lane == 0) xd[(long long)block * pitch + token] = d;
     if constexpr (F::MINS) {
         const int pair = sum + __shfl_xor_sync(0xffffffffu, sum, 2);       // lanes 4 g .. 4 g + 3: sum of group g
         if ((lane & 3) == 0) {
@@ -70,26 +84,27 @@ __global__ void __launch_bounds__(256) pair_planes_kernel(const float *__restric
 
 // Chunks of a tile, pairs, and whether tiles are shared: by estimated time (us).  A block takes a pair this long, measured on 14336 x 4096
 // with 64 to 256 tokens; sharing costs a kernel that adds the parts (512 x 4096 x 768 Q6_K: 13.6 us whole, 18 to 20 with shared tiles of
-// any size).
-struct PairPlan { int chunks, pairs; bool share; };
+// any size).  Fewer tiles than pairs: a whole number of pairs to a tile; where a block takes long (GROUPED), all pairs (384 x 4096 x 4096 Q8_0
+// 54.7 -> 46.2 us, 512 x 4096 x 14336 174 -> 161).
+struct PairPlan { int chunks, pairs; bool share; double cost; };
 template <int FMT>
 static PairPlan pair_plan(const TileArgs &a, int sm_count) {
     using F = PairFormat<FMT>;
-    constexpr double BLOCK = FMT == F_Q4_K ? 0.62 : FMT == F_Q5_K ? 0.75 : FMT == F_Q6_K ? 1.3 : 0.85;
-    constexpr double TOKEN = FMT == F_Q4_K ? 0.0046 : FMT == F_Q5_K ? 0.0088 : FMT == F_Q6_K ? 0.0039 : 0.0023;
+    constexpr double BLOCK = FMT == F_Q4_K ? 0.62 : FMT == F_Q5_K ? 0.75 : FMT == F_Q6_K ? 1.3 : FMT == F_TQ1_0 ? 0.85 : 3.3;
+    constexpr double TOKEN = FMT == F_Q4_K ? 0.0046 : FMT == F_Q5_K ? 0.0088 : FMT == F_Q6_K ? 0.0039 : FMT == F_TQ1_0 ? 0.0023 : 0.0;
     constexpr double SHARING = 5.0;
     const long long row_tiles = (a.n + PR_ROWS - 1) / PR_ROWS, nb = a.k / 256, most = sm_count / 2;
-    PairPlan best{0, 0, false};
-    double least = 0.0;
+    PairPlan best{0, 0, false, 0.0};
     auto consider = [&](int chunks, long long pairs, bool share, long long blocks) {
         const double cost = (double)blocks * (BLOCK + TOKEN * chunks * F::CHUNK) + (share ? SHARING : 0.0);
-        if (!best.chunks || cost < least) { best = PairPlan{chunks, (int)pairs, share}; least = cost; }
+        if (!best.chunks || cost < best.cost) best = PairPlan{chunks, (int)pairs, share, cost};
     };
     for (int chunks = 1; chunks <= F::TOKENS / F::CHUNK; ++chunks) {
         const long long tiles = row_tiles * ((a.m + chunks * F::CHUNK - 1) / (chunks * F::CHUNK)), pairs = std::min(tiles, most);
         consider(chunks, pairs, false, (tiles + pairs - 1) / pairs * nb);
-        if (tiles >= most) consider(chunks, most, true, (tiles * nb + most - 1) / most);
-        else for (long long parts = 2; parts <= std::min(most / tiles, nb); ++parts) consider(chunks, tiles * parts, true, (nb + parts - 1) / parts);
+        if (tiles >= most || (F::GROUPED && tiles * nb >= most)) consider(chunks, most, true, (tiles * nb + most - 1) / most);
+        if (tiles < most)
+            for (long long parts = 2; parts <= std::min(most / tiles, nb); ++parts) consider(chunks, tiles * parts, true, (nb + parts - 1) / parts);
     }
     return best;
 }
@@ -103,7 +118,7 @@ static PairPlanes pair_planes(const TileArgs &a, const PairPlan &plan) {
     PairPlanes s;
     s.pitch = (a.m + F::TOKENS - 1) / F::TOKENS * F::TOKENS + F::TOKENS;       // the last tile of tokens reads whole
     s.codes = whole(m * nb * (F::I8 ? 256 : 512));
-    s.xd = whole(nb * (size_t)s.pitch * 4);
+    s.xd = whole(nb * F::HALVES * F::GROUPS * (size_t)s.pitch * 4);
     s.mins = F::MINS ? whole(m * nb * 32) : 0;
     s.parts = plan.share ? (size_t)plan.pairs * 2 * PR_ROWS * F::TOKENS * sizeof(float) : 0;
     return s;
@@ -131,12 +146,18 @@ bool pair_supported(const TileArgs &a) {
     // Q4_K  1.2e9 and more than 128 tokens: 160 x 4096 x 2048 (1.3e9) 15.4 / 14.6, 160 x 4096 x 4096 20.9 / 19.0, 128 x 4096 x 4096 16.4 / 17.1; but few
     //       short rows leave too little for every pair: 512 x 1024 x 4096 17.7 / 18.9, 256 x 1024 x 14336 27.4 / 25.2.  Fewer tokens where
     //       there are many rows: 40 x 14336 x 4096 25.1 / 23.1, 128 x 4096 x 14336 31.0 / 31.5
+    // Q4_0, Q8_0: tiles of 128 tokens, so by the plan's own estimate against that of the register tiles, which is linear in the products (within
+    //       5 % from 2e9 on): Q8_0 128 x 4096 x 4096 29.4 / 23.1, 160 x 4096 x 4096 32.7 / 34.3, 64 x 28672 x 4096 72.1 / 83.1, 300 x 14336 x 4096 138 / 119;
+    //       Q4_0 128 x 4096 x 4096 25.8 / 22.2, 260 x 4096 x 4096 41.6 / 52.7, 512 x 1024 x 4096 27.3 / 23.6.  Below 1.5e9 they are even: 256 x 1024 x
+    //       4096 Q8_0 17.8 / 18.2, 256 x 4096 x 1024 14.9 / 16.4
     const double products = (double)a.m * (double)a.n * (double)a.k;
     if (a.m <= 32) return false;
     switch (a.fmt) {
     case F_Q6_K: if (products < 8.2e8) return false; break;
     case F_Q5_K: if (products < 1.2e9 || (a.m <= 64 && a.k < 4096)) return false; break;
     case F_TQ1_0: if (products < 1.2e9 || (a.m <= 40 && (a.n < 8192 || a.k < 4096))) return false; break;
+    case F_Q4_0: if (products < 1.5e9 || pair_plan<F_Q4_0>(a, 148).cost + 5.0 > 10.0 + 7.0e-9 * products) return false; break;
+    case F_Q8_0: if (products < 1.5e9 || pair_plan<F_Q8_0>(a, 148).cost + 5.0 > 12.0 + 7.8e-9 * products) return false; break;
     case F_Q4_K: if (products < 1.2e9 || (a.m <= 128 ? a.n < 8192 : a.n < 2048 && a.k < 8192)) return false; break;
     default: return false;
     }
@@ -178,7 +199,7 @@ static cudaError_t launch_pair_format(const TileArgs &a, uint8_t *planes, int *s
     CUtensorMap x_codes, x_mins, w_rows;
     const unsigned long long m = (unsigned long long)a.m, nb = (unsigned long long)p.nb;
     e = F::I8 ? encode_piece_map(&x_codes, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, codes, 128, m, 2 * nb, F::CHUNK / 2, 2, true)
-              : encode_piece_map(&x_codes, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, codes, 64, m, 4 * nb, F::CHUNK / 2, 4, true);
+              : encode_piece_map(&x_codes, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, codes, 64, m, 4 * nb, F::CHUNK / 2, 4 / F::HALVES, true);
     if (e == cudaSuccess && F::MINS) e = encode_piece_map(&x_mins, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, mins, 8, m, 2 * nb, F::CHUNK / 2, 2, false);
     else x_mins = x_codes;
     // weight records: rows of words, or super-rows of eight rows; rows after the last whole super-row are fetched by the expanders

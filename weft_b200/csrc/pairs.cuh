@@ -32,12 +32,20 @@
 // multiple of 16 bytes start at any even address; eight rows together are a multiple of 16, so the matrix is taken as super-rows of
 // eight, and row j of each by a box whose columns start at the 16-byte boundary before the record.
 //
+// Q4_0 and Q8_0 have a scale pair per 32 elements: every group of 32 is an accumulator of its own (f16 codes, 2 MMAs, at most 127 * 127 * 32
+// < 2^24 and exact), acc += x.d * (d * S) eight times a block, and A goes by half blocks.  The epilogue bounds it: a hand-over and 32
+// multiply-adds of two per warp for 128 clocks of MMAs, 700 clocks in all.  Tiles of 256 tokens: 173 us where 128 take 158 (the sums do not fit
+// the registers); scales of tokens as f16 in shared memory 201; chunks of 32 to 128 tokens chosen at run time 178; the scales read ahead of the
+// waits 162.
+//
 // What bounds it: instructions and their latency.  A block of 256 tokens takes 3400 (Q4_K), 4500 (Q6_K), 2500 (TQ1_0) clocks against 2304,
 // 2048 and 1024 of tensor work; issue slots are 50 to 65 % busy and every barrier operation takes 100 to 250 clocks.
 // Measured on B200 (us, device time with the kernels before and behind it; before: fold.cuh, TQ1_0 CTA pairs with the tokens as rows):
 //   Q4_K   512 x 14336 x 4096  84.2 -> 64.9    512 x 4096 x 14336  83.4 -> 70.5    512 x 28672 x 8192 274 -> 215
 //   Q5_K   512 x 14336 x 4096   146 -> 94.7    512 x 4096 x 14336   159 -> 105     128 x 14336 x 4096 50.8 -> 37.5
 //   Q6_K   512 x 14336 x 4096   141 -> 76.8    512 x 4096 x 14336   150 -> 83.5    512 x 28672 x 8192 495 -> 248
+//   Q8_0   512 x 14336 x 4096   247 -> 160     512 x 4096 x 14336   239 -> 161     128 x 14336 x 4096 71.3 -> 50.4   (before: register tiles)
+//   Q4_0   512 x 14336 x 4096   221 -> 156     512 x 4096 x 14336   214 -> 157     128 x 14336 x 4096 63.3 -> 48.5
 //   TQ1_0  512 x 14336 x 4096  83.2 -> 57.3    512 x 4096 x 14336  80.8 -> 66.0    512 x 28672 x 8192 217 -> 165
 // Every wait is bounded; one that runs out raises a flag in both CTAs, every role leaves its loop, copies in flight are waited for, tensor
 // memory is freed, and the host sees a status code.  Only this GPU's memory is read or written.
@@ -59,19 +67,21 @@ constexpr float PR_MAGIC = 12582912.0f;         // 1.5 * 2^23
 template <int FMT> struct PairFormat {
     static constexpr int UNIT = unit_bytes(FMT);
     static constexpr bool MINS = FMT == F_Q4_K || FMT == F_Q5_K;
-    static constexpr bool I8 = FMT != F_Q4_K;                       // int8 operands and int32 accumulators; else f16 and fp32
+    static constexpr bool GROUPED = FMT == F_Q4_0 || FMT == F_Q8_0;     // a scale pair per 32 elements: an accumulator for each, half blocks in turn
+    static constexpr bool I8 = FMT != F_Q4_K && !GROUPED;           // int8 operands and int32 accumulators; else f16 and fp32
+    static constexpr int HALVES = GROUPED ? 2 : 1, GROUPS = GROUPED ? 4 : 1;     // rounds through A of a block; accumulations of a round
     static constexpr int LIMBS = FMT == F_Q5_K || FMT == F_Q6_K ? 2 : 1;
     static constexpr bool SHIFTED = UNIT % 16 != 0;                 // records at any even address: a window of whole 16-byte pieces
     static constexpr int PITCH = SHIFTED ? ((UNIT + 14 + 15) / 16 | 1) * 16 : UNIT;   // an odd number of pieces: 128-bit loads of a warp's rows do not conflict
     static constexpr int SUMS = LIMBS + (MINS ? 1 : 0);             // accumulators of a token
     static constexpr int CHUNK = SUMS == 3 ? 32 : 128 / SUMS;       // tokens of a chunk
-    static constexpr int TOKENS = 256;                              // tokens of a tile at most
+    static constexpr int TOKENS = GROUPED ? 128 : 256;              // tokens of a tile at most; GROUPED: unpacking is the lesser part, half the sums leave registers free
     static constexpr int OWN = CHUNK / 4;                           // columns of a chunk that an epilogue warp takes
-    static constexpr int STEPS = I8 ? 8 : 16;                       // MMAs of a block and limb
-    static constexpr int A_COLUMNS = LIMBS * STEPS * 8, A_BUFFERS = 2, SLOTS = (512 - A_BUFFERS * A_COLUMNS) / (SUMS * CHUNK);   // tensor memory: accumulators, then A
-    static constexpr int STAGE = CHUNK / 2 * (I8 ? 256 : 512);      // this CTA's tokens of a chunk, a block
-    static constexpr int STAGES = FMT == F_Q4_K ? 8 : FMT == F_Q5_K ? 24 : FMT == F_Q6_K ? 12 : 6;
-    static constexpr int W_SLOTS = FMT == F_TQ1_0 ? 6 : 3;
+    static constexpr int STEPS = (I8 ? 8 : 16) / (HALVES * GROUPS); // MMAs of an accumulation and limb
+    static constexpr int A_COLUMNS = LIMBS * STEPS * GROUPS * 8, A_BUFFERS = 2, SLOTS = (512 - A_BUFFERS * A_COLUMNS) / (SUMS * CHUNK);   // tensor memory: accumulators, then A
+    static constexpr int STAGE = CHUNK / 2 * (I8 ? 256 : 512 / HALVES);      // this CTA's tokens of a chunk, a block
+    static constexpr int STAGES = GROUPED ? 6 : FMT == F_Q4_K ? 8 : FMT == F_Q5_K ? 24 : FMT == F_Q6_K ? 12 : 6;
+    static constexpr int W_SLOTS = FMT == F_TQ1_0 ? 6 : FMT == F_Q8_0 ? 2 : 3;
     // expanders, a thread for half a record or a whole one; epilogue; tokens, records and MMAs
     static constexpr int X_WARPS = LIMBS == 2 ? 8 : 4, WARPS = X_WARPS + PR_E_WARPS + 4, THREADS = 32 * WARPS;
     static constexpr int E_WARP0 = X_WARPS, TOKEN_WARP = E_WARP0 + PR_E_WARPS, W_WARP = TOKEN_WARP + 1, MMA_WARP = TOKEN_WARP + 2;
@@ -82,15 +92,15 @@ template <int FMT> struct PairFormat {
     static constexpr int TABLE = FMT == F_TQ1_0 ? 256 * 8 * 16 : 0;
     // shared memory
     static constexpr int TOKENS_AT = 1024, XMIN_AT = TOKENS_AT + STAGES * STAGE, RAW_AT = XMIN_AT + (MINS ? STAGES * CHUNK * 16 : 0);
-    static constexpr int DD_AT = RAW_AT + W_SLOTS * 128 * PITCH, XD_AT = DD_AT + PR_RING * (MINS ? 2 : 1) * 128 * 4;
-    static constexpr int AMIN_AT = XD_AT + PR_RING * TOKENS * 4, TABLE_AT = AMIN_AT + (MINS ? A_BUFFERS * AMIN : 0), BYTES = TABLE_AT + TABLE;
+    static constexpr int DD_AT = RAW_AT + W_SLOTS * 128 * PITCH, XD_AT = DD_AT + PR_RING * (MINS ? 2 : GROUPS) * 128 * 4;
+    static constexpr int AMIN_AT = XD_AT + PR_RING * GROUPS * TOKENS * 4, TABLE_AT = AMIN_AT + (MINS ? A_BUFFERS * AMIN : 0), BYTES = TABLE_AT + TABLE;
     static_assert(BYTES <= PR_SMEM && STAGE % 1024 == 0 && RAW_AT % 128 == 0 && TABLE_AT % 128 == 0, "shared memory");
 };
 
 struct PairParams {
     const uint8_t *w;
     const uint32_t *powers;      // TQ1_0
-    const float *xd;             // (nb, pitch)
+    const float *xd;             // (nb, or eight times that, pitch)
     float *y;
     ulonglong2 *parts;           // sums of the parts of tiles that pairs share: two slots a pair
     long long n, ldy, row_bytes, pitch;
@@ -399,6 +409,60 @@ __device__ __forceinline__ void pair_expand_tq1_0(const uint32_t (&w)[6], uint32
     tmem_st8(to + 24, fifth);
 }
 
+// Codes as f16, in the order of the activation plane: under the exponent of 1024, where their offset comes out again
+__device__ __forceinline__ void pair_bytes_f16(uint32_t codes, uint32_t &even, uint32_t &odd) {
+    const uint32_t u = codes ^ 0x80808080u;
+    even = hadd2(__byte_perm(u, 0x64646464u, 0x4240), 0xe480e480u);
+    odd = hadd2(__byte_perm(u, 0x64646464u, 0x4341), 0xe480e480u);
+}
+// Two groups of 32 lie in `words` words: a scale, the first's codes a half word off, the other's scale, its codes on a word
+template <int FMT> struct PairGroups {
+    static constexpr int WORDS = 2 * record_bytes(FMT) / 4, CODES = WORDS / 2;     // words of two groups, of a group's codes
+    // the scales of groups 4 half .. 4 half + 3
+    static __device__ __forceinline__ void scales(int half, const uint8_t *row, float (&d)[4]) {
+        const uint8_t *p = row + 8 * WORDS * half;
+#pragma unroll
+        for (int g = 0; g < 4; ++g) d[g] = half_bits_to_float(ld_u16(p + g * (2 * WORDS)));
+    }
+    template <int HALF> static __device__ __forceinline__ void expand(const uint8_t *row, uint32_t to) {
+        constexpr int FIRST = 2 * WORDS * HALF & ~3, PIECES = (2 * WORDS * (HALF + 1) - FIRST + 3) / 4, SKIP = 2 * WORDS * HALF - FIRST;
+        uint32_t w[4 * PIECES];
+#pragma unroll
+        for (int i = 0; i < PIECES; ++i) {
+            const uint4 v = *reinterpret_cast<const uint4 *>(row + 4 * FIRST + 16 * i);
+            w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+        }
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            const uint32_t *from = w + SKIP + (g >> 1) * WORDS + (g & 1 ? CODES + 1 : 0);
+            uint32_t c[CODES];
+#pragma unroll
+            for (int i = 0; i < CODES; ++i) c[i] = g & 1 ? from[i] : __byte_perm(from[i], from[i + 1], 0x5432);
+            if constexpr (FMT == F_Q8_0) {
+#pragma unroll
+                for (int v = 0; v < 2; ++v) {
+                    uint32_t out[8];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) pair_bytes_f16(c[4 * v + i], out[2 * i], out[2 * i + 1]);
+                    tmem_st8(to + 16 * g + 8 * v, out);
+                }
+            } else {
+                uint32_t lo[8], hi[8];
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int o = 0; o < 2; ++o) {
+                        const uint32_t q = o ? c[i] >> 8 : c[i];
+                        lo[2 * i + o] = hadd2(and_or(q, 0x000f000fu, 0x64006400u), 0xe408e408u);
+                        hi[2 * i + o] = hfma2(and_or(q, 0x00f000f0u, 0x64006400u), 0x2c002c00u, 0xd480d480u);      // (1024 + 16 v) / 16 - 72
+                    }
+                tmem_st8(to + 16 * g, lo);
+                tmem_st8(to + 16 * g + 8, hi);
+            }
+        }
+    }
+};
+
 // What a thread holds of its record between reading and unpacking it
 template <int FMT> struct PairRecord;
 template <> struct PairRecord<F_Q4_K> {
@@ -455,6 +519,17 @@ template <> struct PairRecord<F_TQ1_0> {
     __device__ __forceinline__ void expand(int, const Window &, uint32_t table, uint32_t to, uint32_t) const { pair_expand_tq1_0(w, qh, table, to); }
 };
 
+template <int FMT> struct PairGroupedRecord {
+    static constexpr float d0 = 0.0f, d1 = 0.0f;
+    const uint8_t *row;
+    __device__ __forceinline__ void read(int, const Window &w, uint32_t) { row = w.p; }
+    __device__ __forceinline__ void expand(int half, const Window &, uint32_t, uint32_t to, uint32_t) const {
+        if (half) PairGroups<FMT>::template expand<1>(row, to); else PairGroups<FMT>::template expand<0>(row, to);
+    }
+};
+template <> struct PairRecord<F_Q4_0> : PairGroupedRecord<F_Q4_0> {};
+template <> struct PairRecord<F_Q8_0> : PairGroupedRecord<F_Q8_0> {};
+
 // where lane `lane` of an epilogue warp leaves its sums of a part, 16 bytes every 512
 template <int FMT> __device__ __forceinline__ size_t pair_part(int pair, bool began_before, int rank, int e, int lane) {
     return ((size_t)((2 * pair + (began_before ? 0 : 1)) * 2 + rank) * PR_E_WARPS + e) * (PairFormat<FMT>::TOKENS / 16 * 32) + lane;
@@ -480,9 +555,9 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
     };
     uint8_t *s_raw = smem + F::RAW_AT;
     float *s_dd = reinterpret_cast<float *>(smem + F::DD_AT), *s_xd = reinterpret_cast<float *>(smem + F::XD_AT);
-    constexpr int DD = (F::MINS ? 2 : 1) * 128;
+    constexpr int DD = (F::MINS ? 2 : F::GROUPS) * 128, XD = F::GROUPS * F::TOKENS;     // floats of a round in the rings
     if (threadIdx.x == 0) {
-        for (int s = 0; s < F::STAGES; ++s) { mbar_init(&ctl->b_full[s], 1); mbar_init(&ctl->b_empty[s], 1); }
+        for (int s = 0; s < F::STAGES; ++s) { mbar_init(&ctl->b_full[s], 1); mbar_init(&ctl->b_empty[s], F::GROUPED ? PR_MMA_WARPS : 1); }
         for (int s = 0; s < F::A_BUFFERS; ++s) { mbar_init(&ctl->a_full[s], 2 * F::X_WARPS); mbar_init(&ctl->a_empty[s], PR_MMA_WARPS); }
         for (int s = 0; s < F::SLOTS; ++s) { mbar_init(&ctl->d_full[s], 1); mbar_init(&ctl->d_empty[s], 2 * PR_E_WARPS); }
         for (int s = 0; s < PR_RING; ++s) { mbar_init(&ctl->scales_full[s], 1 + 4); mbar_init(&ctl->scales_empty[s], PR_E_WARPS); }
@@ -548,6 +623,34 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
             return true;
         };
         bool ok = tmem_ok && read();
+        if constexpr (F::GROUPED) {                             // a block is two rounds through A
+            for (int it = 0; ok && it < total; ++it) {
+#pragma unroll 1
+                for (int h = 0; h < 2; ++h) {
+                    const int ring = (2 * it + h) & (PR_RING - 1);      // free without asking, as below
+                    float d[4];
+                    PairGroups<FMT>::scales(h, win.p, d);
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) s_dd[ring * DD + g * 128 + l] = d[g];
+                    __syncwarp();
+                    if (lane == 0) pr_arrive(PR_BAR(scales_full, ring));
+                    ok = pr_wait(PR_BAR(a_empty, buf), a_phase, bars, p.status);
+                    if (!ok) break;
+                    tc::fence_after_sync();
+                    rec.expand(h, win, 0u, lane_base + (uint32_t)(buf * F::A_COLUMNS), 0u);
+                    tc::tmem_st_wait();
+                    tc::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) tc::mbar_arrive_cluster(full_base + 8u * (uint32_t)buf);
+                    if (++buf == F::A_BUFFERS) { buf = 0; a_phase ^= 1u; }
+                }
+                if (!ok) break;
+                if (lane == 0) pr_arrive(PR_BAR(w_empty, slot));
+                if (++slot == F::W_SLOTS) { slot = 0; w_phase ^= 1u; }
+                advance(it, tile, b);
+                if (it + 1 < total) ok = read();
+            }
+        } else
         for (int it = 0; ok && it < total; ++it) {
             if (half == 0) {
                 // The ring's slot is free without asking: the A buffer of the block before was free, so the block A_BUFFERS before that is
@@ -597,6 +700,49 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
 #pragma unroll
             for (int i = 0; i < SUMS; ++i) acc[i] = 0;
             const int from_b = b, tile_end = min(it + p.nb - b, total);
+            if constexpr (F::GROUPED) {
+#pragma unroll 1
+                for (int at = 2 * it; at < 2 * tile_end; ++at) {        // half blocks
+                    const int ring = at & (PR_RING - 1);
+                    if (!pr_wait(PR_BAR(scales_full, ring), (uint32_t)(at / PR_RING) & 1u, bars, p.status)) { ok = false; break; }
+#pragma unroll
+                    for (int c = 0; c < MOST; ++c) {
+                        if (c >= chunks) break;
+                        const float *xd = xd_base + ring * XD + c * F::CHUNK;
+#pragma unroll
+                        for (int g = 0; g < F::GROUPS; ++g, xd += F::TOKENS) {
+                            ok = pr_wait(PR_BAR(d_full, slot), d_phase, bars, p.status);
+                            if (!ok) break;
+                            tc::fence_after_sync();
+                            const uint32_t from = lane_base + (uint32_t)(F::CHUNK * slot);
+                            const float d = dd[ring * DD + g * 128];
+                            const uint64_t scale = pack2(d, d);
+#pragma unroll
+                            for (int k = 0; k < OWN / 16; ++k) {
+                                uint64_t v[8];
+                                tmem_pairs(from + 16 * k, v);
+                                if (k == OWN / 16 - 1) {                // all read: the slot is free
+                                    tc::fence_before_sync();
+                                    __syncwarp();
+                                    if (lane == 0) tc::mbar_arrive_cluster(empty_base + 8u * (uint32_t)slot);
+                                    if (++slot == F::SLOTS) { slot = 0; d_phase ^= 1u; }
+                                }
+#pragma unroll
+                                for (int j = 0; j < 8; j += 2) {
+                                    const ulonglong2 x = *reinterpret_cast<const ulonglong2 *>(xd + 16 * k + 2 * j);
+                                    uint64_t &to = acc[(c * OWN + 16 * k) / 2 + j], &next = acc[(c * OWN + 16 * k) / 2 + j + 1];
+                                    to = fma2(x.x, mul2(scale, v[j]), to);
+                                    next = fma2(x.y, mul2(scale, v[j + 1]), next);
+                                }
+                            }
+                        }
+                        if (!ok) break;
+                    }
+                    if (!ok) break;
+                    __syncwarp();
+                    if (lane == 0) pr_arrive(PR_BAR(scales_empty, ring));
+                }
+            } else
 #pragma unroll 1
             for (int at = it; at < tile_end; ++at) {
                 const int ring = at & (PR_RING - 1);
@@ -683,25 +829,30 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
             uint32_t phase = 1;
             bool ok = tmem_ok;
             for (int it = 0; ok && it < total; ++it) {
-                const int t0 = (tile % p.token_tiles) * chunks * F::CHUNK, ring = it & (PR_RING - 1);
-                if (!pr_wait(PR_BAR(scales_empty, ring), ((uint32_t)(it / PR_RING) & 1u) ^ 1u, bars, p.status)) break;
-                if (elect_one()) {
-                    const uint32_t bytes = (uint32_t)(chunks * F::CHUNK * 4);
-                    pr_expect(PR_BAR(scales_full, ring), bytes);
-                    bulk_g2s(s_xd + ring * F::TOKENS, p.xd + (long long)b * p.pitch + t0, bytes, &ctl->scales_full[ring]);
-                }
-                __syncwarp();
-                for (int c = 0; c < chunks; ++c) {
-                    if (!pr_wait(PR_BAR(b_empty, s), phase, bars, p.status)) { ok = false; break; }
+                const int t0 = (tile % p.token_tiles) * chunks * F::CHUNK;
+                for (int h = 0; ok && h < F::HALVES; ++h) {
+                    const int at = F::HALVES * it + h, ring = at & (PR_RING - 1);
+                    ok = pr_wait(PR_BAR(scales_empty, ring), ((uint32_t)(at / PR_RING) & 1u) ^ 1u, bars, p.status);
+                    if (!ok) break;
                     if (elect_one()) {
-                        const int token = t0 + c * F::CHUNK + rank * (F::CHUNK / 2);
-                        const uint32_t full = full_base + 8u * (uint32_t)s;
-                        if (rank == 0) pr_expect(PR_BAR(b_full, s), 2u * (F::STAGE + (F::MINS ? F::CHUNK * 16 : 0)));
-                        pair_load_3d(base + F::TOKENS_AT + (uint32_t)(s * F::STAGE), &x_codes, 0, token, (F::I8 ? 2 : 4) * b, full);
-                        if (F::MINS) pair_load_3d(base + F::XMIN_AT + (uint32_t)(s * (F::CHUNK * 16)), &x_mins, 0, token, 2 * b, full);
+                        const uint32_t bytes = (uint32_t)(chunks * F::CHUNK * 4);
+                        pr_expect(PR_BAR(scales_full, ring), F::GROUPS * bytes);
+                        for (int g = 0; g < F::GROUPS; ++g)
+                            bulk_g2s(s_xd + ring * XD + g * F::TOKENS, p.xd + (long long)((F::HALVES * b + h) * F::GROUPS + g) * p.pitch + t0, bytes, &ctl->scales_full[ring]);
                     }
                     __syncwarp();
-                    if (++s == F::STAGES) { s = 0; phase ^= 1u; }
+                    for (int c = 0; c < chunks; ++c) {
+                        if (!pr_wait(PR_BAR(b_empty, s), phase, bars, p.status)) { ok = false; break; }
+                        if (elect_one()) {
+                            const int token = t0 + c * F::CHUNK + rank * (F::CHUNK / 2);
+                            const uint32_t full = full_base + 8u * (uint32_t)s;
+                            if (rank == 0) pr_expect(PR_BAR(b_full, s), 2u * (F::STAGE + (F::MINS ? F::CHUNK * 16 : 0)));
+                            pair_load_3d(base + F::TOKENS_AT + (uint32_t)(s * F::STAGE), &x_codes, 0, token, F::I8 ? 2 * b : 4 * b + 2 * h, full);
+                            if (F::MINS) pair_load_3d(base + F::XMIN_AT + (uint32_t)(s * (F::CHUNK * 16)), &x_mins, 0, token, 2 * b, full);
+                        }
+                        __syncwarp();
+                        if (++s == F::STAGES) { s = 0; phase ^= 1u; }
+                    }
                 }
                 advance(it, tile, b);
             }
@@ -737,6 +888,41 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
             int s = 0, buf = 0, slot = 0;
             uint32_t b_phase = 0, a_phase = 0, d_phase = 1, turn = issuer ^ 1;
             bool ok = tmem_ok, mine = issuer == 0;
+            if constexpr (F::GROUPED) {
+                const uint32_t floats = tc::idesc_f16_f32acc(PR_ROWS, F::CHUNK);
+                for (int at = 0; ok && at < 2 * total; ++at) {          // half blocks; a group of 32 elements a turn
+                    if (!pr_wait(PR_BAR(a_full, buf), a_phase, bars, p.status)) break;
+                    const uint32_t a = a_base + (uint32_t)(buf * F::A_COLUMNS);
+                    for (int c = 0; ok && c < chunks; ++c) {
+                        const uint64_t bs = b0 + (uint64_t)((uint32_t)(s * F::STAGE) >> 4);
+                        if (!pr_wait(PR_BAR(b_full, s), b_phase, bars, p.status)) { ok = false; break; }
+#pragma unroll 1
+                        for (int g = 0; g < F::GROUPS; ++g) {
+                            if ((g & 1) == issuer) {
+                                if (!pr_wait(PR_BAR(d_empty, slot), d_phase, bars, p.status)) { ok = false; break; }
+                                if (!pr_wait(PR_BAR(turn, issuer), turn, bars, p.status)) { ok = false; break; }
+                                turn ^= 1u;
+                                tc::fence_after_sync();
+                                if (elect_one()) {
+                                    const uint32_t d = tmem + (uint32_t)(F::CHUNK * slot);
+                                    const uint64_t bg = bs + (uint64_t)((g >> 1) * (F::CHUNK / 2 * 128 >> 4)) + (uint64_t)((g & 1) * 4);
+                                    pair_mma<false>(d, a + 16u * (uint32_t)g, bg, floats, 0);
+                                    pair_mma<false>(d, a + 16u * (uint32_t)g + 8u, bg + 2, floats, 1);
+                                    pr_arrive(PR_BAR(turn, issuer ^ 1));
+                                    commit_both(PR_BAR(d_full, slot));
+                                    if (g >= F::GROUPS - 2) commit_both(PR_BAR(b_empty, s));
+                                }
+                                __syncwarp();
+                            }
+                            if (++slot == F::SLOTS) { slot = 0; d_phase ^= 1u; }
+                        }
+                        if (++s == F::STAGES) { s = 0; b_phase ^= 1u; }
+                    }
+                    if (ok && elect_one()) commit_both(PR_BAR(a_empty, buf));
+                    __syncwarp();
+                    if (++buf == F::A_BUFFERS) { buf = 0; a_phase ^= 1u; }
+                }
+            } else
             for (int it = 0; ok && it < total; ++it) {
                 if (!pr_wait(PR_BAR(a_full, buf), a_phase, bars, p.status)) break;
                 const uint32_t a = a_base + (uint32_t)(buf * F::A_COLUMNS);
@@ -786,10 +972,10 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
         if (warp == F::W_WARP)
             for (int s = 0; s < F::W_SLOTS; ++s) { mbar_wait(&ctl->w_full[s], 0u, 1u << 10); mbar_wait(&ctl->w_full[s], 1u, 1u << 10); }
     } else if (warp == F::TOKEN_WARP) {
-        const long long loads = (long long)total * chunks;
+        const long long loads = (long long)total * F::HALVES * chunks;
         for (long long k = max(0LL, loads - F::STAGES); k < loads; ++k) mbar_wait(&ctl->b_empty[k % F::STAGES], (uint32_t)(k / F::STAGES) & 1u, 1u << 20);
     } else if (warp == F::MMA_WARP) {
-        for (int k = max(0, total - F::A_BUFFERS); k < total; ++k) mbar_wait(&ctl->a_empty[k % F::A_BUFFERS], (uint32_t)(k / F::A_BUFFERS) & 1u, 1u << 20);
+        for (int k = max(0, total * F::HALVES - F::A_BUFFERS); k < total * F::HALVES; ++k) mbar_wait(&ctl->a_empty[k % F::A_BUFFERS], (uint32_t)(k / F::A_BUFFERS) & 1u, 1u << 20);
     }
     tc::fence_before_sync();
     __syncthreads();
@@ -844,6 +1030,6 @@ template <int FMT> cudaError_t launch_pair_kernel(const PairParams &params, cons
     return cudaLaunchKernelEx(&cfg, pair_parts_kernel<FMT>, params);
 }
 
-#define PR_EACH_FORMAT(DO) DO(F_Q4_K) DO(F_Q5_K) DO(F_Q6_K) DO(F_TQ1_0)
+#define PR_EACH_FORMAT(DO) DO(F_Q4_K) DO(F_Q5_K) DO(F_Q6_K) DO(F_TQ1_0) DO(F_Q4_0) DO(F_Q8_0)
 
 }  // namespace weft
