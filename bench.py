@@ -72,7 +72,6 @@ DEFAULT_WORKLOAD = "q4_k_decode_14336x4096"
 NCU_DRAM_TRAFFIC = {
     "q4_k_decode_14336x4096": 33_078_272,
     "iq2_xxs_decode_28672x8192": 60_635_904,
-    "tq1_0_prefill_28672x8192": 69_316_352,
     "q4_k_dequantize_14336x4096": 33_041_920 + 177_308_928,
 }
 
