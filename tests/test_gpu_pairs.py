@@ -1,6 +1,6 @@
 """GPU parity of the contraction on CTA pairs (larger batches of Q4_K, Q5_K, Q6_K, TQ1_0, Q4_0 and Q8_0) against the CPU oracle.
 
-Sizes are the smallest that reach it (1.2e9 products; Q4_K up to 128 tokens from 8192 rows on) and sit at the edges of its tiles: rows
+Sizes are the smallest that reach it (1.2e9 products, Q4_0 and Q8_0 1.5e9; Q4_K up to 128 tokens from 8192 rows on) and sit at the edges of its tiles: rows
 that do not fill the last 256, nor the last super-row of 8, a matrix of eight rows, tokens just above a chunk and a tile, one block of K,
 fewer tiles than pairs (each shared by several), more tiles than pairs with the rest whole or shared.
 
@@ -18,7 +18,7 @@ from test_gpu_fold import check_both_sources
 
 pytestmark = pytest.mark.gpu
 
-FORMATS = ["Q4_K", "Q5_K", "Q6_K", "TQ1_0", "Q4_0", "Q8_0"]
+FORMATS, GROUPED = ["Q4_K", "Q5_K", "Q6_K", "TQ1_0"], ["Q4_0", "Q8_0"]
 
 
 @pytest.mark.parametrize("name", FORMATS)
@@ -28,9 +28,19 @@ FORMATS = ["Q4_K", "Q5_K", "Q6_K", "TQ1_0", "Q4_0", "Q8_0"]
                                  (700, 6703, 256),           # one block: nothing to share
                                  (40, 14341, 2304),          # one chunk; fewer tiles than pairs, blocks that do not divide
                                  (65, 19331, 1024),          # more tiles than pairs
-                                 (512, 5003, 768),
-                                 (384, 3000, 1280)])          # fewer tiles than pairs, all pairs sharing them
+                                 (512, 5003, 768)])
 def test_tile_edges(torch, lib, oracle, golden, name, mnk):  # noqa: F811
+    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
+
+
+@pytest.mark.parametrize("name", GROUPED)                      # tiles of 128 tokens, a scale pair per 32 elements
+@pytest.mark.parametrize("mnk", [(128, 3001, 4352),          # few tiles, each shared by several pairs
+                                 (500, 2311, 2304),          # fewer tiles than pairs, blocks that do not divide
+                                 (250, 6703, 1280),          # a tile each, some pairs idle
+                                 (255, 9371, 768),           # a tile for each of 74 pairs
+                                 (384, 19331, 256),          # one block: nothing to share
+                                 (640, 9001, 1024)])         # more tiles than pairs, the rest shared
+def test_group_tile_edges(torch, lib, oracle, golden, name, mnk):  # noqa: F811
     check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
 
 
@@ -55,7 +65,7 @@ def test_infinite_scales_of_ternary_records(torch, lib, oracle, golden, m, n, k,
     assert rel_l2(np.delete(got, rows, axis=1), np.delete(problem.want, rows, axis=1)) <= 1e-5
 
 
-@pytest.mark.parametrize("name", ["Q4_0", "Q8_0"])
+@pytest.mark.parametrize("name", GROUPED)
 def test_infinite_scales_of_groups(torch, lib, oracle, golden, name, monkeypatch):  # noqa: F811
     """Records of 32 elements whose f16 scale is infinite or NaN: the rows are what the oracle gives, NaN where its sums are."""
     import test_gpu_batch as batch
