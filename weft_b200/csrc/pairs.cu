@@ -84,27 +84,28 @@ __global__ void __launch_bounds__(256) pair_planes_kernel(const float *__restric
 
 // Chunks of a tile, pairs, and whether tiles are shared: by estimated time (us).  A block takes a pair this long, measured on 14336 x 4096
 // with 64 to 256 tokens; sharing costs a kernel that adds the parts (512 x 4096 x 768 Q6_K: 13.6 us whole, 18 to 20 with shared tiles of
-// any size).  Fewer tiles than pairs: a whole number of pairs to a tile; where a block takes long (GROUPED), all pairs (384 x 4096 x 4096 Q8_0
-// 54.7 -> 46.2 us, 512 x 4096 x 14336 174 -> 161).
+// any size).  Fewer tiles than pairs: a whole number of pairs to a tile, or all pairs,
+// whose runs may then span two tiles, where that saves more than the second tile's parts cost: 512 x 4096 x 14336 Q6_K 84.4 -> 80.0, Q8_0
+// 174 -> 161, 384 x 4096 x 4096 Q8_0 54.7 -> 46.2; but 512 x 4096 x 4096 Q4_K 29.8 -> 32.5, 128 x 14336 x 4096 Q6_K 37.9 -> 41.1.
 struct PairPlan { int chunks, pairs; bool share; double cost; };
 template <int FMT>
 static PairPlan pair_plan(const TileArgs &a, int sm_count) {
     using F = PairFormat<FMT>;
     constexpr double BLOCK = FMT == F_Q4_K ? 0.62 : FMT == F_Q5_K ? 0.75 : FMT == F_Q6_K ? 1.3 : FMT == F_TQ1_0 ? 0.85 : 3.3;
     constexpr double TOKEN = FMT == F_Q4_K ? 0.0046 : FMT == F_Q5_K ? 0.0088 : FMT == F_Q6_K ? 0.0039 : FMT == F_TQ1_0 ? 0.0023 : 0.0;
-    constexpr double SHARING = 5.0;
+    constexpr double SHARING = 5.0, SPANNING = 3.2;
     const long long row_tiles = (a.n + PR_ROWS - 1) / PR_ROWS, nb = a.k / 256, most = sm_count / 2;
     PairPlan best{0, 0, false, 0.0};
-    auto consider = [&](int chunks, long long pairs, bool share, long long blocks) {
-        const double cost = (double)blocks * (BLOCK + TOKEN * chunks * F::CHUNK) + (share ? SHARING : 0.0);
+    auto consider = [&](int chunks, long long pairs, bool share, long long blocks, double more) {
+        const double cost = (double)blocks * (BLOCK + TOKEN * chunks * F::CHUNK) + (share ? SHARING : 0.0) + more;
         if (!best.chunks || cost < best.cost) best = PairPlan{chunks, (int)pairs, share, cost};
     };
     for (int chunks = 1; chunks <= F::TOKENS / F::CHUNK; ++chunks) {
         const long long tiles = row_tiles * ((a.m + chunks * F::CHUNK - 1) / (chunks * F::CHUNK)), pairs = std::min(tiles, most);
-        consider(chunks, pairs, false, (tiles + pairs - 1) / pairs * nb);
-        if (tiles >= most || (F::GROUPED && tiles * nb >= most)) consider(chunks, most, true, (tiles * nb + most - 1) / most);
+        consider(chunks, pairs, false, (tiles + pairs - 1) / pairs * nb, 0.0);
+        if (tiles * nb >= most) consider(chunks, most, true, (tiles * nb + most - 1) / most, tiles < most ? SPANNING : 0.0);
         if (tiles < most)
-            for (long long parts = 2; parts <= std::min(most / tiles, nb); ++parts) consider(chunks, tiles * parts, true, (nb + parts - 1) / parts);
+            for (long long parts = 2; parts <= std::min(most / tiles, nb); ++parts) consider(chunks, tiles * parts, true, (nb + parts - 1) / parts, 0.0);
     }
     return best;
 }
