@@ -9,6 +9,8 @@ order of the fp32 additions over the blocks differs.
 """
 from __future__ import annotations
 
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -84,3 +86,25 @@ def test_infinite_scales_of_groups(torch, lib, oracle, golden, name, monkeypatch
     assert np.isinf(problem.want[:, rows[:2]]).any() and np.isnan(problem.want[:, 2311 - 9]).all()
     assert np.array_equal(got[:, rows], problem.want[:, rows], equal_nan=True)
     assert rel_l2(np.delete(got, rows, axis=1), np.delete(problem.want, rows, axis=1)) <= 1e-5
+
+
+@pytest.mark.parametrize("name, mnk, kernels", [("Q6_K", (700, 6703, 256), 2),      # one block of K: more tiles than pairs, nothing to share
+                                                ("Q8_0", (384, 19331, 256), 2),
+                                                ("Q5_K", (512, 5003, 768), 2),
+                                                ("TQ1_0", (129, 2311, 4096), 3)])
+def test_launches_are_counted_as_they_are_made(torch, lib, oracle, golden, name, mnk, kernels):  # noqa: F811
+    """Planes, contraction and, where tiles are shared, the kernel that adds their parts: as many as a capture of the call holds."""
+    problem, graph, side = Problem(torch, oracle, golden, name, *mnk), torch.cuda.CUDAGraph(keep_graph=True), torch.cuda.Stream()
+    nodes = ctypes.c_size_t()
+    lib.weft_b200_set_async(1)
+    lib.weft_b200_set_stream(ctypes.c_void_p(side.cuda_stream))
+    try:
+        before = lib.weft_b200_launch_count()
+        with torch.cuda.graph(graph, stream=side):
+            problem.run(lib)
+        counted = lib.weft_b200_launch_count() - before
+        assert ctypes.CDLL("libcuda.so.1").cuGraphGetNodes(ctypes.c_void_p(graph.raw_cuda_graph()), None, ctypes.byref(nodes)) == 0
+    finally:
+        lib.weft_b200_set_stream(None)
+        lib.weft_b200_set_async(0)
+    assert (nodes.value, counted) == (kernels, kernels)

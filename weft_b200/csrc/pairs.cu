@@ -185,6 +185,7 @@ static cudaError_t launch_pair_format(const TileArgs &a, uint8_t *planes, int *s
     p.pairs = plan.pairs;
     p.rounds = tiles / p.pairs;
     p.rest = tiles % p.pairs;
+    p.share = plan.share;
     p.unit = plan.share ? 1 : p.nb;
     p.per = plan.share ? p.rest * p.nb / p.pairs : 0;
     p.extra = plan.share ? p.rest * p.nb % p.pairs : p.rest;

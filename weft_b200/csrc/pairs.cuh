@@ -107,9 +107,10 @@ struct PairParams {
     int m, nb, chunks, token_tiles;
     int pairs, rounds, rest;     // every pair has `rounds` whole tiles; the blocks of the `rest` last tiles are shared out in units
     int unit, per, extra;        // (a block, or a tile's): `per` to a pair, one more to the first `extra` pairs
+    bool share;                  // units are blocks: tiles may be shared, and their parts are added behind
     int *status;
     __device__ __forceinline__ int start_of(int pair) const { return (pair * per + min(pair, extra)) * unit; }
-    __device__ __forceinline__ int pair_of(int block) const {   // unit 1
+    __device__ __forceinline__ int pair_of(int block) const {   // where tiles are shared
         const int longer = extra * (per + 1);
         return block < longer ? block / (per + 1) : extra + (block - longer) / per;
     }
@@ -1023,7 +1024,7 @@ template <int FMT> cudaError_t launch_pair_kernel(const PairParams &params, cons
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     e = cudaLaunchKernelEx(&cfg, pair_kernel<FMT>, params, codes, mins, rows);
-    if (e != cudaSuccess || !params.rest || params.unit > 1) return e;
+    if (e != cudaSuccess || !params.rest || !params.share) return e;
     cfg.gridDim = dim3((unsigned)params.rest, 2 * PR_E_WARPS);
     cfg.blockDim = dim3(F::TOKENS / 16 * 32);
     cfg.dynamicSmemBytes = 0;
