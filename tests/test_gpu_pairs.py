@@ -35,6 +35,13 @@ def test_tile_edges(torch, lib, oracle, golden, name, mnk):  # noqa: F811
     check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
 
 
+@pytest.mark.parametrize("name", ["Q6_K", "TQ1_0"])            # records at any even address
+@pytest.mark.parametrize("n", [3081, 3210, 3083, 3212, 3085, 3214, 3087])
+def test_rows_after_the_last_super_row(torch, lib, oracle, golden, name, n):  # noqa: F811
+    """One to seven rows, in the even and in the odd CTA of a pair; the last record ends at every offset from a 16-byte boundary that there is."""
+    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, 310, n, 1280))
+
+
 @pytest.mark.parametrize("name", GROUPED)                      # tiles of 128 tokens, a scale pair per 32 elements
 @pytest.mark.parametrize("mnk", [(128, 3001, 4352),          # few tiles, each shared by several pairs
                                  (500, 2311, 2304),          # fewer tiles than pairs, blocks that do not divide

@@ -30,7 +30,9 @@
 // Roles: expanders (four warps, a thread per row; eight for two limbs, half a record each), 16 epilogue warps (lane quarter x quarter of
 // the chunk), a warp each for token copies and weight records, two for MMAs.  Records come by TMA.  Rows of formats whose records are no
 // multiple of 16 bytes start at any even address; eight rows together are a multiple of 16, so the matrix is taken as super-rows of
-// eight, and row j of each by a box whose columns start at the 16-byte boundary before the record.
+// eight, and row j of each by a box whose columns start at the 16-byte boundary before the record.  Up to seven rows after the last whole
+// super-row come by a copy each into a place of their own; fetched by the expanders two bytes at a time, every block of their tile waited
+// for 3 us and more (Q6_K 45 x 9086 x 12288 104.7 -> 57.5 us, 56 x 14735 x 6144 92.3 -> 51.2, 91 x 15300 x 6400 86.6 -> 58.4).
 //
 // Q4_0 and Q8_0 have a scale pair per 32 elements: every group of 32 is an accumulator of its own (f16 codes, 2 MMAs, at most 127 * 127 * 32
 // < 2^24 and exact), acc += x.d * (d * S) eight times a block, and A goes by half blocks.  The epilogue bounds it: a hand-over and 32
@@ -93,7 +95,8 @@ template <int FMT> struct PairFormat {
     // shared memory
     static constexpr int TOKENS_AT = 1024, XMIN_AT = TOKENS_AT + STAGES * STAGE, RAW_AT = XMIN_AT + (MINS ? STAGES * CHUNK * 16 : 0);
     static constexpr int DD_AT = RAW_AT + W_SLOTS * 128 * PITCH, XD_AT = DD_AT + PR_RING * (MINS ? 2 : GROUPS) * 128 * 4;
-    static constexpr int AMIN_AT = XD_AT + PR_RING * GROUPS * TOKENS * 4, TABLE_AT = AMIN_AT + (MINS ? A_BUFFERS * AMIN : 0), BYTES = TABLE_AT + TABLE;
+    static constexpr int AMIN_AT = XD_AT + PR_RING * GROUPS * TOKENS * 4, TABLE_AT = AMIN_AT + (MINS ? A_BUFFERS * AMIN : 0), TAIL_AT = TABLE_AT + TABLE;
+    static constexpr int TAIL = SHIFTED ? 7 * PITCH : 0, BYTES = TAIL_AT + W_SLOTS * TAIL;       // rows after the last whole super-row, a slot
     static_assert(BYTES <= PR_SMEM && STAGE % 1024 == 0 && RAW_AT % 128 == 0 && TABLE_AT % 128 == 0, "shared memory");
 };
 
@@ -610,16 +613,19 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
             if (!pr_wait(PR_BAR(w_full, slot), w_phase, bars, p.status)) return false;
             const uint8_t *raw = s_raw + slot * (128 * F::PITCH) + record * F::PITCH;
             const uint32_t skew = F::SHIFTED ? (skew0 + (uint32_t)(b * F::UNIT)) & 15u : 0u;
-            win = Window{raw, skew >> 2, skew & 2u ? 0x5432u : 0x3210u};
-            if (F::SHIFTED && tail) {                           // rows after the last whole super-row: both threads of the row fetch its record
+            if (F::SHIFTED && tail) {                           // rows after the last whole super-row lie apart
                 const long long r = (long long)(tile / p.token_tiles) * PR_ROWS + 128 * rank + row;
                 if (r >= (p.n & ~7LL) && r < p.n) {
-                    const uint16_t *src = reinterpret_cast<const uint16_t *>(p.w + r * p.row_bytes + (long long)b * F::UNIT);
-                    uint16_t *dst = reinterpret_cast<uint16_t *>(const_cast<uint8_t *>(raw) + skew);
-                    for (int i = 0; i < F::UNIT / 2; ++i) dst[i] = __ldg(src + i);
-                    fence_proxy_async();                        // the next box lands on these bytes
+                    raw = smem + F::TAIL_AT + slot * F::TAIL + (row & 7) * F::PITCH;
+                    if (r == p.n - 1 && b == p.nb - 1) {        // what follows the matrix's last whole 16 bytes: both threads of the row fetch it
+                        const uint8_t *src = p.w + r * p.row_bytes + (long long)b * F::UNIT - skew;
+                        for (uint32_t i = (skew + F::UNIT) & ~15u; i < skew + F::UNIT; i += 2)
+                            *reinterpret_cast<uint16_t *>(const_cast<uint8_t *>(raw) + i) = __ldg(reinterpret_cast<const uint16_t *>(src + i));
+                        fence_proxy_async();                    // the next copy lands on these bytes
+                    }
                 }
             }
+            win = Window{raw, skew >> 2, skew & 2u ? 0x5432u : 0x3210u};
             rec.read(half, win, skew);
             return true;
         };
@@ -866,13 +872,22 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
                 if (elect_one()) {
                     uint8_t *to = s_raw + slot * (128 * F::PITCH);
                     const int row0 = (tile / p.token_tiles) * PR_ROWS + 128 * rank;
-                    pr_expect(PR_BAR(w_full, slot), 128 * F::PITCH);
                     if constexpr (F::SHIFTED) {
-                        int x = b * F::UNIT;                            // byte of the record in the super-row, row by row
+                        // The rows after the last whole super-row, where this CTA has them: copies of their windows up to the matrix's last whole 16 bytes
+                        const long long whole = p.n & ~7LL;
+                        const int rows = whole >= row0 && whole < row0 + 128 ? (int)(p.n - whole) : 0;
+                        const int end = (int)p.row_bytes * rows & ~15;
+                        int x = b * F::UNIT, bytes = 128 * F::PITCH;    // byte of the record in the super-row, row by row
+                        for (int j = 0, at = x; j < rows; ++j, at += (int)p.row_bytes) bytes += min(F::PITCH, end - (at & ~15));
+                        pr_expect(PR_BAR(w_full, slot), (uint32_t)bytes);
 #pragma unroll 1
-                        for (int j = 0; j < 8; ++j, x += (int)p.row_bytes)
+                        for (int j = 0; j < 8; ++j, x += (int)p.row_bytes) {
                             tma_load_2d(to + j * (16 * F::PITCH), &w_rows, x & ~15, row0 / 8, &ctl->w_full[slot]);
+                            if (j < rows)
+                                bulk_g2s(smem + F::TAIL_AT + slot * F::TAIL + j * F::PITCH, p.w + whole * p.row_bytes + (x & ~15), (uint32_t)min(F::PITCH, end - (x & ~15)), &ctl->w_full[slot]);
+                        }
                     } else {
+                        pr_expect(PR_BAR(w_full, slot), 128 * F::PITCH);
                         tma_load_2d(to, &w_rows, b * (F::UNIT / 4), row0, &ctl->w_full[slot]);
                     }
                 }
