@@ -13,11 +13,15 @@ class TileArgs(ctypes.Structure):               # weft::TileArgs of csrc/kernels
                [(name, ctypes.c_longlong) for name in ("n", "k", "m", "ldy")]
 
 
-@pytest.fixture(scope="module")
-def tile_supported():
+def library():
     from weft_b200.build import ensure_built
 
-    rule = ctypes.CDLL(str(ensure_built()))["_ZN4weft14tile_supportedERKNS_8TileArgsE"]
+    return ctypes.CDLL(str(ensure_built()))
+
+
+@pytest.fixture(scope="module")
+def tile_supported():
+    rule = library()["_ZN4weft14tile_supportedERKNS_8TileArgsE"]
     rule.restype, rule.argtypes = ctypes.c_bool, [ctypes.POINTER(TileArgs)]
     return lambda fmt, m, n, k, w=1 << 20: rule(TileArgs(fmt, w, 1, 1, 1, 1, 1, 1, n, k, m, n))
 
@@ -44,3 +48,28 @@ def test_small_batches_go_by_token_rows(tile_supported, fmt):
 
 def test_tile_sizes_that_are_left_to_others(tile_supported):
     assert not tile_supported(8, 2, 64, 4096) and not tile_supported(8, 3, 64, 4096 + 32) and not tile_supported(8, 3, 64, 4096, w=(1 << 20) + 8)
+
+
+@pytest.fixture(scope="module")
+def pair_supported():
+    rule = library()["_ZN4weft14pair_supportedERKNS_8TileArgsEi"]
+    rule.restype, rule.argtypes = ctypes.c_bool, [ctypes.POINTER(TileArgs), ctypes.c_int]
+    return lambda fmt, m, n, k, w=1 << 20, sms=148: rule(TileArgs(fmt, w, 1, 1, 1, 1, 1, 1, n, k, m, n), sms)
+
+
+PAIR_FORMATS = [1, 5, 8, 9, 10, 20]
+
+
+@pytest.mark.parametrize("fmt", PAIR_FORMATS)
+def test_pairs_take_whole_aligned_matrices(pair_supported, fmt):
+    """Larger batches of whole 256-element blocks in a 16-byte aligned matrix; sums of a block's index stay in 32 bits."""
+    assert pair_supported(fmt, 512, 14336, 4096)
+    assert not pair_supported(fmt, 512, 14336, 4096 + 32) and not pair_supported(fmt, 512, 14336, 4096, w=(1 << 20) + 8)
+    assert not pair_supported(fmt, 32, 14336, 4096) and not pair_supported(fmt, 512, 1024, 1024)
+    assert not pair_supported(fmt, 1 << 19, 1 << 20, 4096)
+
+
+@pytest.mark.parametrize("fmt", [1, 5])
+def test_pair_plans_are_made_for_the_devices_sms(pair_supported, fmt):
+    """With half a tile a pair and more, a third of the SMs takes three times as long, where the register tiles' estimate stays."""
+    assert pair_supported(fmt, 128, 4096, 4096) and not pair_supported(fmt, 128, 4096, 4096, sms=48)

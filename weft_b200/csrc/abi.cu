@@ -419,12 +419,38 @@ int do_quantize(int act, const float *X, uint8_t *Y, size_t M, size_t K) {
     });
 }
 
-// One mul_mat with its arguments where the kernels find them, and which kernels run.  One path for the decode and the tiled
-// symbols: what runs is chosen by the number of token rows, the format and the shape.
+// Which kernels a mul_mat takes, and the device memory they need between them: by the number of token rows, the format and the
+// shape, one path for the decode and the tiled symbols.
+enum Path { NOTHING, GEMV, TILES, FOLD, PAIRS };
+struct Route { Path path; size_t plane_bytes; };
+
+Route find_route(const TileArgs &a) {
+    const int sms = g.prop.multiProcessorCount;
+    if (pair_supported(a, sms)) return Route{PAIRS, pair_plane_bytes(a, sms)};
+    if (fold_supported(a)) return Route{FOLD, fold_plane_bytes(a)};
+    if (tile_supported(a)) return Route{TILES, tile_plane_bytes(a)};
+    return Route{GEMV, 0};
+}
+
+// A route follows from the sizes and from whether the matrix is 16-byte aligned, and takes 1 to 4 us to find where plans are
+// compared, of calls that take 15 us and more: the sizes in use are kept, each in the one place its hash gives.  Called under g.lock.
+Route route(const TileArgs &a) {
+    struct Known { long long n, k, m; int fmt; bool aligned; Route route; };
+    static Known known[256];
+    const bool aligned = (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0;
+    uint64_t hash = (uint64_t)a.fmt * 2 + aligned;
+    for (long long v : {a.n, a.k, a.m}) hash = (hash ^ (uint64_t)v) * 0x9e3779b97f4a7c15ull;
+    Known &place = known[hash >> 56];
+    if (place.m != a.m || place.n != a.n || place.k != a.k || place.fmt != a.fmt || place.aligned != aligned)
+        place = Known{a.n, a.k, a.m, a.fmt, aligned, find_route(a)};
+    return place.route;
+}
+
+// One mul_mat with its arguments where the kernels find them, and which kernels run.
 struct MulMat {
-    enum Path { NOTHING, GEMV, TILES, FOLD, PAIRS };
     int fmt = 0, act = 0;
     Path path = NOTHING;
+    size_t plane_bytes = 0;
     void *w = nullptr, *x = nullptr, *xq = nullptr, *y = nullptr, *gr = nullptr, *sg = nullptr, *pw = nullptr;
     uint8_t *planes = nullptr;
     long long n = 0, k = 0, m = 0, ldy = 0;
@@ -433,7 +459,6 @@ struct MulMat {
     TileArgs tile_args() const {
         return TileArgs{fmt, w, have_xq ? nullptr : (const float *)x, xq, (const int8_t *)gr, (const int8_t *)sg, (const uint32_t *)pw, (float *)y, n, k, m, ldy};
     }
-    size_t plane_bytes() const { return path == PAIRS ? pair_plane_bytes(tile_args(), g.prop.multiProcessorCount) : path == FOLD ? fold_plane_bytes(tile_args()) : path == TILES ? tile_plane_bytes(tile_args()) : 0; }
 
     // records: the activation records of an earlier step of the same call, where the kernels find them (have_xq then); that step
     // is not alone
@@ -464,7 +489,9 @@ struct MulMat {
         if ((reinterpret_cast<uintptr_t>(w) & (fmt == F_Q4_K_I16 ? 15u : 1u)) || (reinterpret_cast<uintptr_t>(xq) & (act == F_Q8_K ? 3u : 1u)) ||
             (reinterpret_cast<uintptr_t>(y) & 3u) || (x && (reinterpret_cast<uintptr_t>(x) & 3u)))
             return fail("a buffer does not meet its Encoding alignment");
-        path = pair_supported(tile_args()) ? PAIRS : fold_supported(tile_args()) ? FOLD : tile_supported(tile_args()) ? TILES : GEMV;
+        const Route r = route(tile_args());
+        path = r.path;
+        plane_bytes = r.plane_bytes;
         // decode: the GEMV's own prologue quantizes X (one launch) when the fp32 rows allow 16-byte loads
         fuse_quantize = !have_xq && path == GEMV && K % 256 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
         return 0;
@@ -508,8 +535,8 @@ int do_mul_mat(int fmt, const void *W, const float *X, void *Xq, const int8_t *g
     Call call;
     MulMat op;
     if (op.prepare(call, fmt, W, X, Xq, grid, signs, powers, Y, N, K, M, ldy, flags, vec_dot_only)) return 1;
-    if (op.path == MulMat::NOTHING) return 0;
-    if (const size_t bytes = op.plane_bytes()) CU(workspace(bytes, g.stream, &g.stream_id, &op.planes));
+    if (op.path == NOTHING) return 0;
+    if (op.plane_bytes) CU(workspace(op.plane_bytes, g.stream, &g.stream_id, &op.planes));
     if (gather) call.not_repeatable();       // its kernels meet the other ranks' in a fixed order of launches
     Key key;
     key.add(3);
@@ -798,7 +825,7 @@ static size_t steps_on_same_records(const weft_b200_mul_mat_step *steps, size_t 
 // Prepared steps, issued as one call.
 static int issue_steps(Call &call, std::vector<MulMat> &ops) {
     size_t plane_bytes = 0;              // the steps follow each other: one workspace serves them all
-    for (const MulMat &op : ops) plane_bytes = op.plane_bytes() > plane_bytes ? op.plane_bytes() : plane_bytes;
+    for (const MulMat &op : ops) plane_bytes = op.plane_bytes > plane_bytes ? op.plane_bytes : plane_bytes;
     uint8_t *planes = nullptr;
     if (plane_bytes) CU(workspace(plane_bytes, g.stream, &g.stream_id, &planes));
     Key key;
@@ -811,8 +838,8 @@ static int issue_steps(Call &call, std::vector<MulMat> &ops) {
         for (size_t i = 0; i < ops.size(); ++i) {
             // consecutive Q4_K steps on the same activations (the later ones marked as reusing Xq) go out as one launch
             size_t run = 1;
-            if (ops[i].path == MulMat::GEMV && ops[i].fmt == F_Q4_K && ops[i].m == 1 && ops[i].k % 256 == 0)
-                while (i + run < ops.size() && run < (size_t)GEMV_MAX_SEGMENTS && ops[i + run].path == MulMat::GEMV && ops[i + run].fmt == F_Q4_K && ops[i + run].m == 1 &&
+            if (ops[i].path == GEMV && ops[i].fmt == F_Q4_K && ops[i].m == 1 && ops[i].k % 256 == 0)
+                while (i + run < ops.size() && run < (size_t)GEMV_MAX_SEGMENTS && ops[i + run].path == GEMV && ops[i + run].fmt == F_Q4_K && ops[i + run].m == 1 &&
                        ops[i + run].k == ops[i].k && ops[i + run].xq == ops[i].xq && ops[i + run].have_xq)
                     ++run;
             GemvArgs ga;

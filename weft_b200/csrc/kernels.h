@@ -90,7 +90,9 @@ size_t fold_plane_bytes(const TileArgs &a);
 cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches);   // two or three kernels
 
 // tcgen05 contraction on CTA pairs (pairs.cuh), behind the kernel that makes its planes.
-bool pair_supported(const TileArgs &a);
+struct PairPlan { int chunks, pairs; bool share; double cost; };      // chunks of tokens of a tile, pairs, whether they share tiles, and the estimated time (us) of that
+PairPlan pair_plan(const TileArgs &a, int sm_count);
+bool pair_supported(const TileArgs &a, int sm_count);
 size_t pair_plane_bytes(const TileArgs &a, int sm_count);
 cudaError_t launch_pair(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches);   // two or three kernels
 

@@ -87,9 +87,8 @@ __global__ void __launch_bounds__(256) pair_planes_kernel(const float *__restric
 // any size).  Fewer tiles than pairs: a whole number of pairs to a tile, or all pairs,
 // whose runs may then span two tiles, where that saves more than the second tile's parts cost: 512 x 4096 x 14336 Q6_K 84.4 -> 80.0, Q8_0
 // 174 -> 161, 384 x 4096 x 4096 Q8_0 54.7 -> 46.2; but 512 x 4096 x 4096 Q4_K 29.8 -> 32.5, 128 x 14336 x 4096 Q6_K 37.9 -> 41.1.
-struct PairPlan { int chunks, pairs; bool share; double cost; };
 template <int FMT>
-static PairPlan pair_plan(const TileArgs &a, int sm_count) {
+static PairPlan plan_format(const TileArgs &a, int sm_count) {
     using F = PairFormat<FMT>;
     constexpr double BLOCK = FMT == F_Q4_K ? 0.62 : FMT == F_Q5_K ? 0.75 : FMT == F_Q6_K ? 1.3 : FMT == F_TQ1_0 ? 0.85 : 3.3;
     constexpr double TOKEN = FMT == F_Q4_K ? 0.0046 : FMT == F_Q5_K ? 0.0088 : FMT == F_Q6_K ? 0.0039 : FMT == F_TQ1_0 ? 0.0023 : 0.0;
@@ -110,6 +109,14 @@ static PairPlan pair_plan(const TileArgs &a, int sm_count) {
     return best;
 }
 
+PairPlan pair_plan(const TileArgs &a, int sm_count) {
+    switch (a.fmt) {
+#define PR_PLAN(FMT) case FMT: return plan_format<FMT>(a, sm_count);
+    PR_EACH_FORMAT(PR_PLAN)
+    default: return PairPlan{0, 0, false, 0.0};
+    }
+}
+
 struct PairPlanes { size_t codes, xd, mins, parts; long long pitch; };      // bytes of each, one after the other
 template <int FMT>
 static PairPlanes pair_planes(const TileArgs &a, const PairPlan &plan) {
@@ -125,7 +132,7 @@ static PairPlanes pair_planes(const TileArgs &a, const PairPlan &plan) {
     return s;
 }
 template <int FMT> static size_t plane_bytes(const TileArgs &a, int sm_count) {
-    const PairPlanes s = pair_planes<FMT>(a, pair_plan<FMT>(a, sm_count));
+    const PairPlanes s = pair_planes<FMT>(a, plan_format<FMT>(a, sm_count));
     return s.codes + s.xd + s.mins + s.parts;
 }
 size_t pair_plane_bytes(const TileArgs &a, int sm_count) {
@@ -136,7 +143,7 @@ size_t pair_plane_bytes(const TileArgs &a, int sm_count) {
     }
 }
 
-bool pair_supported(const TileArgs &a) {
+bool pair_supported(const TileArgs &a, int sm_count) {
     // Where this kernel is the quickest, us on the device of what runs otherwise (register tiles, for Q4_K fold.cuh) / this:
     // Q6_K  from 33 tokens and 8.2e8 products on: 48 x 4096 x 4096 (8.1e8) 18.4 / 18.9, 200 x 1024 x 4096 (8.4e8) 19.0 / 17.9, 256 x 2048 x
     //       2048 (1.1e9) 22.3 / 16.8, 64 x 4096 x 4096 21.7 / 19.2
@@ -157,8 +164,8 @@ bool pair_supported(const TileArgs &a) {
     case F_Q6_K: if (products < 8.2e8) return false; break;
     case F_Q5_K: if (products < 1.2e9 || (a.m <= 64 && a.k < 4096)) return false; break;
     case F_TQ1_0: if (products < 1.2e9 || (a.m <= 40 && (a.n < 8192 || a.k < 4096))) return false; break;
-    case F_Q4_0: if (products < 1.5e9 || pair_plan<F_Q4_0>(a, 148).cost + 5.0 > 10.0 + 7.0e-9 * products) return false; break;
-    case F_Q8_0: if (products < 1.5e9 || pair_plan<F_Q8_0>(a, 148).cost + 5.0 > 12.0 + 7.8e-9 * products) return false; break;
+    case F_Q4_0: if (products < 1.5e9 || pair_plan(a, sm_count).cost + 5.0 > 10.0 + 7.0e-9 * products) return false; break;
+    case F_Q8_0: if (products < 1.5e9 || pair_plan(a, sm_count).cost + 5.0 > 12.0 + 7.8e-9 * products) return false; break;
     case F_Q4_K: if (products < 1.2e9 || (a.m <= 128 ? a.n < 8192 : a.n < 2048 && a.k < 8192)) return false; break;
     default: return false;
     }
@@ -170,7 +177,7 @@ bool pair_supported(const TileArgs &a) {
 template <int FMT>
 static cudaError_t launch_pair_format(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches) {
     using F = PairFormat<FMT>;
-    const PairPlan plan = pair_plan<FMT>(a, sm_count);
+    const PairPlan plan = plan_format<FMT>(a, sm_count);
     const PairPlanes s = pair_planes<FMT>(a, plan);
     uint8_t *codes = planes;
     float *xd = reinterpret_cast<float *>(codes + s.codes);
