@@ -73,3 +73,13 @@ def test_pairs_take_whole_aligned_matrices(pair_supported, fmt):
 def test_pair_plans_are_made_for_the_devices_sms(pair_supported, fmt):
     """With half a tile a pair and more, a third of the SMs takes three times as long, where the register tiles' estimate stays."""
     assert pair_supported(fmt, 128, 4096, 4096) and not pair_supported(fmt, 128, 4096, 4096, sms=48)
+
+
+@pytest.mark.parametrize("fmt, m, n, k, pairs", [(5, 128, 4096, 4096, True), (5, 160, 4096, 4096, False), (5, 455, 4689, 768, False), (5, 181, 11200, 768, False),
+                                                 (5, 512, 14336, 4096, True), (1, 128, 4096, 4096, True), (1, 177, 7387, 1280, False), (1, 317, 14656, 512, False),
+                                                 (1, 570, 8000, 512, False), (1, 512, 4096, 14336, True), (20, 50, 4722, 5888, False), (20, 40, 8192, 8192, False),
+                                                 (20, 38, 8512, 5376, False), (20, 40, 14336, 4096, True), (20, 384, 1024, 4096, True), (20, 512, 28672, 8192, True),
+                                                 (9, 40, 8192, 8192, False), (9, 40, 14336, 4096, True)])
+def test_pairs_and_register_tiles_by_what_was_measured(pair_supported, fmt, m, n, k, pairs):
+    """Sizes at which one of the two is quicker by 5 % and more."""
+    assert pair_supported(fmt, m, n, k) == pairs

@@ -17,6 +17,7 @@ import pytest
 from helpers import rel_l2
 from test_gpu_batch import Problem, lib, torch  # noqa: F401  (fixtures)
 from test_gpu_fold import check_both_sources
+from test_dispatch_bounds import pair_supported  # noqa: F401  (fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -115,3 +116,10 @@ def test_launches_are_counted_as_they_are_made(torch, lib, oracle, golden, name,
         lib.weft_b200_set_stream(None)
         lib.weft_b200_set_async(0)
     assert (nodes.value, counted) == (kernels, kernels)
+
+
+@pytest.mark.parametrize("m, n, k, pairs", [(68, 8416, 6912, False), (380, 6158, 4864, False), (122, 8841, 6912, False), (512, 14336, 4096, True), (512, 4096, 14336, True),
+                                            (160, 4096, 4096, True), (77, 28672, 8192, True)])
+def test_pairs_and_single_ctas_by_what_was_measured(torch, lib, pair_supported, m, n, k, pairs):  # noqa: F811
+    """Q4_K at sizes where one of the two is quicker by 5 % and more.  How many clusters the device holds decides with."""
+    assert pair_supported(8, m, n, k, sms=torch.cuda.get_device_properties(0).multi_processor_count) == pairs

@@ -81,16 +81,18 @@ struct TileArgs {
 };
 bool tile_supported(const TileArgs &a);
 size_t tile_plane_bytes(const TileArgs &a);
+double tile_estimate(const TileArgs &a, int sm_count);      // us on the device, with the kernel that makes the planes: Q4_0, Q8_0, Q5_K and TQ1_0
 cudaError_t launch_tile(const TileArgs &a, uint8_t *planes, int sm_count, cudaStream_t stream);   // two kernels
 template <int FMT> cudaError_t launch_tile_kernel(const TileArgs &a, const uint8_t *planes, int sm_count, cudaStream_t stream);
 
 // tcgen05 contraction with the weights expanded into tensor memory (fold.cuh), behind the kernel that makes its planes.
 bool fold_supported(const TileArgs &a);
 size_t fold_plane_bytes(const TileArgs &a);
+double fold_estimate(const TileArgs &a, int sm_count);      // us on the device, with the kernel that makes the planes
 cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches);   // two or three kernels
 
 // tcgen05 contraction on CTA pairs (pairs.cuh), behind the kernel that makes its planes.
-struct PairPlan { int chunks, pairs; bool share; double cost; };      // chunks of tokens of a tile, pairs, whether they share tiles, and the estimated time (us) of that
+struct PairPlan { int chunks, pairs; bool share; long long tiles; double cost; };      // chunks of tokens of a tile, pairs, whether they share the tiles, and the estimated time (us) of that
 PairPlan pair_plan(const TileArgs &a, int sm_count);
 bool pair_supported(const TileArgs &a, int sm_count);
 size_t pair_plane_bytes(const TileArgs &a, int sm_count);

@@ -94,17 +94,17 @@ static PairPlan plan_format(const TileArgs &a, int sm_count) {
     constexpr double TOKEN = FMT == F_Q4_K ? 0.0046 : FMT == F_Q5_K ? 0.0088 : FMT == F_Q6_K ? 0.0039 : FMT == F_TQ1_0 ? 0.0023 : 0.0;
     constexpr double SHARING = 5.0, SPANNING = 3.2;
     const long long row_tiles = (a.n + PR_ROWS - 1) / PR_ROWS, nb = a.k / 256, most = sm_count / 2;
-    PairPlan best{0, 0, false, 0.0};
-    auto consider = [&](int chunks, long long pairs, bool share, long long blocks, double more) {
+    PairPlan best{0, 0, false, 0, 0.0};
+    auto consider = [&](int chunks, long long tiles, long long pairs, bool share, long long blocks, double more) {
         const double cost = (double)blocks * (BLOCK + TOKEN * chunks * F::CHUNK) + (share ? SHARING : 0.0) + more;
-        if (!best.chunks || cost < best.cost) best = PairPlan{chunks, (int)pairs, share, cost};
+        if (!best.chunks || cost < best.cost) best = PairPlan{chunks, (int)pairs, share, tiles, cost};
     };
     for (int chunks = 1; chunks <= F::TOKENS / F::CHUNK; ++chunks) {
         const long long tiles = row_tiles * ((a.m + chunks * F::CHUNK - 1) / (chunks * F::CHUNK)), pairs = std::min(tiles, most);
-        consider(chunks, pairs, false, (tiles + pairs - 1) / pairs * nb, 0.0);
-        if (tiles * nb >= most) consider(chunks, most, true, (tiles * nb + most - 1) / most, tiles < most ? SPANNING : 0.0);
+        consider(chunks, tiles, pairs, false, (tiles + pairs - 1) / pairs * nb, 0.0);
+        if (tiles * nb >= most) consider(chunks, tiles, most, true, (tiles * nb + most - 1) / most, tiles < most ? SPANNING : 0.0);
         if (tiles < most)
-            for (long long parts = 2; parts <= std::min(most / tiles, nb); ++parts) consider(chunks, tiles * parts, true, (nb + parts - 1) / parts, 0.0);
+            for (long long parts = 2; parts <= std::min(most / tiles, nb); ++parts) consider(chunks, tiles, tiles * parts, true, (nb + parts - 1) / parts, 0.0);
     }
     return best;
 }
@@ -113,7 +113,7 @@ PairPlan pair_plan(const TileArgs &a, int sm_count) {
     switch (a.fmt) {
 #define PR_PLAN(FMT) case FMT: return plan_format<FMT>(a, sm_count);
     PR_EACH_FORMAT(PR_PLAN)
-    default: return PairPlan{0, 0, false, 0.0};
+    default: return PairPlan{0, 0, false, 0, 0.0};
     }
 }
 
@@ -143,6 +143,20 @@ size_t pair_plane_bytes(const TileArgs &a, int sm_count) {
     }
 }
 
+// The plan's cost beside a start, the planes and the results: within 3 (Q4_0, Q8_0) to 6 % (TQ1_0) rms of the times of 600 to 930 sizes of a
+// format.  A tile of many parts takes 0.16 us longer for each.
+static double pair_estimate(const TileArgs &a, int sm_count) {
+    const PairPlan plan = pair_plan(a, sm_count);
+    const double planes = (double)a.m * (double)a.k * 1e-6, results = (double)a.m * (double)a.n * 1e-6, parts = plan.share ? std::max(0.0, (double)plan.pairs / (double)plan.tiles - 1.0) : 0.0;
+    switch (a.fmt) {
+    case F_Q4_K: return 6.4 + 1.05 * plan.cost + 1.15 * planes + 0.69 * results + 0.16 * parts;
+    case F_Q4_0: return 6.7 + 0.82 * plan.cost + 1.25 * planes + 0.65 * results;
+    case F_Q8_0: return 6.8 + 0.84 * plan.cost + 1.15 * planes + 0.70 * results;
+    case F_Q5_K: return 7.7 + 1.00 * plan.cost + 1.07 * planes + 0.38 * results;
+    default: return 8.4 + 0.98 * plan.cost + 2.35 * planes + 0.66 * results;
+    }
+}
+
 bool pair_supported(const TileArgs &a, int sm_count) {
     // Where this kernel is the quickest, us on the device of what runs otherwise (register tiles, for Q4_K fold.cuh) / this:
     // Q6_K  from 33 tokens and 8.2e8 products on: 48 x 4096 x 4096 (8.1e8) 18.4 / 18.9, 200 x 1024 x 4096 (8.4e8) 19.0 / 17.9, 256 x 2048 x
@@ -158,20 +172,29 @@ bool pair_supported(const TileArgs &a, int sm_count) {
     //       5 % from 2e9 on): Q8_0 128 x 4096 x 4096 29.4 / 23.1, 160 x 4096 x 4096 32.7 / 34.3, 64 x 28672 x 4096 72.1 / 83.1, 300 x 14336 x 4096 138 / 119;
     //       Q4_0 128 x 4096 x 4096 25.8 / 22.2, 260 x 4096 x 4096 41.6 / 52.7, 512 x 1024 x 4096 27.3 / 23.6.  Below 1.5e9 they are even: 256 x 1024 x
     //       4096 Q8_0 17.8 / 18.2, 256 x 4096 x 1024 14.9 / 16.4
+    // How the tiles of either kernel divide among the SMs, and short rows, decide as much as these lines: beyond them, the others keep what
+    // they look quicker at by 4 % (TQ1_0 6) with planes and results counted, since an estimate is as uncertain as that.
+    // Q4_K  68 x 8416 x 6912 26.4 / 33.2, 380 x 6158 x 4864 34.3 / 40.8, 122 x 8841 x 6912 29.6 / 34.6; of 930 sizes 47 go to fold.cuh by this, 10 %
+    //       quicker on average, two of them slower (4 and 9 %)
+    // Q5_K up to 64 tokens: 40 x 8192 x 8192 30.6 / 35.1
+    // Q4_0, Q8_0 and TQ1_0 up to 64 tokens: Q8_0 181 x 11200 x 768 17.6 / 22.8, 455 x 4689 x 768 19.0 / 22.6, Q4_0 177 x 7387 x 1280 17.9 / 21.9, TQ1_0
+    //       40 x 8192 x 8192 27.8 / 32.3, 38 x 8512 x 5376 21.3 / 28.2; of 2350 sizes 75 go to the register tiles, 5 to 13 % quicker on average, seven of
+    //       them slower (4 to 17 %, one 23)
     const double products = (double)a.m * (double)a.n * (double)a.k;
     if (a.m <= 32) return false;
-    switch (a.fmt) {
-    case F_Q6_K: if (products < 8.2e8) return false; break;
-    case F_Q5_K: if (products < 1.2e9 || (a.m <= 64 && a.k < 4096)) return false; break;
-    case F_TQ1_0: if (products < 1.2e9 || (a.m <= 40 && (a.n < 8192 || a.k < 4096))) return false; break;
-    case F_Q4_0: if (products < 1.5e9 || pair_plan(a, sm_count).cost + 5.0 > 10.0 + 7.0e-9 * products) return false; break;
-    case F_Q8_0: if (products < 1.5e9 || pair_plan(a, sm_count).cost + 5.0 > 12.0 + 7.8e-9 * products) return false; break;
-    case F_Q4_K: if (products < 1.2e9 || (a.m <= 128 ? a.n < 8192 : a.n < 2048 && a.k < 8192)) return false; break;
-    default: return false;
-    }
     // 16-byte copies of records need a 16-byte aligned matrix (of whole super-rows); extents are 32-bit in the kernel
     const long long blocks = (a.n + PR_ROWS - 1) / PR_ROWS * ((a.m + 31) / 32) * (a.k / 256);
-    return a.m < (1 << 20) && a.k % 256 == 0 && a.k < (1LL << 22) && a.n >= 8 && a.n < (1LL << 31) && blocks < (1LL << 30) && (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0;
+    if (a.m >= (1 << 20) || a.k % 256 || a.k >= (1LL << 22) || a.n < 8 || a.n >= (1LL << 31) || blocks >= (1LL << 30) || (reinterpret_cast<uintptr_t>(a.w) & 15u)) return false;
+    switch (a.fmt) {
+    case F_Q6_K: return products >= 8.2e8;
+    case F_Q5_K: return products >= 1.2e9 && (a.m > 64 || (a.k >= 4096 && pair_estimate(a, sm_count) < 1.04 * tile_estimate(a, sm_count)));
+    case F_TQ1_0: return products >= 1.2e9 && (a.m > 64 || ((a.m > 40 || (a.n >= 8192 && a.k >= 4096)) && pair_estimate(a, sm_count) < 1.06 * tile_estimate(a, sm_count)));
+    case F_Q4_K: return products >= 1.2e9 && (a.m > 128 ? a.n >= 2048 || a.k >= 8192 : a.n >= 8192) && pair_estimate(a, sm_count) < 1.04 * fold_estimate(a, sm_count);
+    case F_Q4_0: case F_Q8_0:
+        return products >= 1.5e9 && pair_plan(a, sm_count).cost + 5.0 <= (a.fmt == F_Q4_0 ? 10.0 + 7.0e-9 * products : 12.0 + 7.8e-9 * products) &&
+               pair_estimate(a, sm_count) < 1.04 * tile_estimate(a, sm_count);
+    default: return false;
+    }
 }
 
 template <int FMT>

@@ -144,6 +144,17 @@ bool tile_supported(const TileArgs &a) {
            (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0 && !by_token_rows(a);
 }
 
+// The plan's cost beside a start, the planes and the results: within 7 to 12 % (rms) of the times of 600 to 780 sizes of a format, 33 to 8192 tokens
+double tile_estimate(const TileArgs &a, int sm_count) {
+    const double planes = (double)a.m * (double)a.k * 1e-6, results = (double)a.m * (double)a.n * 1e-6;
+    switch (a.fmt) {
+    case F_Q4_0: return 2.6 + 1.33 * tile_plan<F_Q4_0>(a, sm_count).cost + 1.03 * planes + 1.32 * results;
+    case F_Q8_0: return 3.2 + 1.41 * tile_plan<F_Q8_0>(a, sm_count).cost + 1.09 * planes + 1.5 * results;
+    case F_Q5_K: return 4.3 + 1.27 * tile_plan<F_Q5_K>(a, sm_count).cost + 1.1 * planes + 1.12 * results;
+    default: return 4.4 + 1.06 * tile_plan<F_TQ1_0>(a, sm_count).cost + 1.45 * planes + 0.76 * results;
+    }
+}
+
 size_t tile_plane_bytes(const TileArgs &a) { return (size_t)((a.m + 7) / 8) * (size_t)(a.k / 256) * tile_group_bytes(a.fmt); }
 
 cudaError_t launch_tile(const TileArgs &a, uint8_t *planes, int sm_count, cudaStream_t stream) {
