@@ -10,7 +10,7 @@ UNIT_BYTES = {1: 144, 5: 272, 6: 84, 7: 110, 8: 144, 9: 176, 10: 210, 15: 66, 20
 
 class TileArgs(ctypes.Structure):               # weft::TileArgs of csrc/kernels.h
     _fields_ = [("fmt", ctypes.c_int)] + [(name, ctypes.c_void_p) for name in ("w", "x", "xq", "grid", "signs", "powers", "y")] + \
-               [(name, ctypes.c_longlong) for name in ("n", "k", "m", "ldy")]
+               [(name, ctypes.c_longlong) for name in ("n", "k", "m", "ldy")] + [("most_blocks", ctypes.c_int)]
 
 
 def library():

@@ -207,7 +207,7 @@ static cudaError_t launch_pair_format(const TileArgs &a, uint8_t *planes, int *s
     __half *mins = reinterpret_cast<__half *>(codes + s.codes + s.xd);
     PairParams p{};
     p.parts = reinterpret_cast<ulonglong2 *>(codes + s.codes + s.xd + s.mins);
-    p.w = static_cast<const uint8_t *>(a.w); p.powers = a.powers; p.xd = xd; p.y = a.y; p.n = a.n; p.ldy = a.ldy; p.pitch = s.pitch; p.status = status;
+    p.w = static_cast<const uint8_t *>(a.w); p.powers = a.powers; p.xd = xd; p.y = a.y; p.n = a.n; p.ldy = a.ldy; p.pitch = s.pitch; p.status = status; p.most_blocks = a.most_blocks;
     p.m = (int)a.m; p.nb = (int)(a.k / 256); p.chunks = plan.chunks;
     p.row_bytes = (long long)p.nb * F::UNIT;
     p.token_tiles = (int)((a.m + plan.chunks * F::CHUNK - 1) / (plan.chunks * F::CHUNK));

@@ -49,8 +49,8 @@
 //   Q8_0   512 x 14336 x 4096   247 -> 160     512 x 4096 x 14336   239 -> 161     128 x 14336 x 4096 71.3 -> 50.4   (before: register tiles)
 //   Q4_0   512 x 14336 x 4096   221 -> 156     512 x 4096 x 14336   214 -> 157     128 x 14336 x 4096 63.3 -> 48.5
 //   TQ1_0  512 x 14336 x 4096  83.2 -> 57.3    512 x 4096 x 14336  80.8 -> 66.0    512 x 28672 x 8192 217 -> 165
-// Every wait is bounded; one that runs out raises a flag in both CTAs, every role leaves its loop, copies in flight are waited for, tensor
-// memory is freed, and the host sees a status code.  Only this GPU's memory is read or written.
+// Every wait is bounded; one that runs out raises a flag in both CTAs, every role leaves its loop, copies and MMAs in flight are waited for,
+// tensor memory is freed, and the host sees a status code.  Only this GPU's memory is read or written.
 #pragma once
 
 #include "prefill_common.cuh"
@@ -88,7 +88,7 @@ template <int FMT> struct PairFormat {
     static constexpr int X_WARPS = LIMBS == 2 ? 8 : 4, WARPS = X_WARPS + PR_E_WARPS + 4, THREADS = 32 * WARPS;
     static constexpr int E_WARP0 = X_WARPS, TOKEN_WARP = E_WARP0 + PR_E_WARPS, W_WARP = TOKEN_WARP + 1, MMA_WARP = TOKEN_WARP + 2;
     // Registers a thread: at launch, and after the roles have traded (setmaxnreg).  The trade stays inside what the CTA got.
-    static constexpr int REGS = WARPS > 24 ? 72 : 80, X_REGS = WARPS > 24 ? 48 : 56, E_REGS = 96, IO_REGS = WARPS > 24 ? 24 : 40;
+    static constexpr int REGS = WARPS > 24 ? 72 : 80, X_REGS = WARPS > 24 ? 48 : 64, E_REGS = 96, IO_REGS = WARPS > 24 ? 24 : 32;
     static_assert(32 * (X_WARPS * X_REGS + PR_E_WARPS * E_REGS + 4 * IO_REGS) <= THREADS * REGS, "setmaxnreg would wait for ever");
     static constexpr int AMIN = I8 ? 4096 : 8192;                   // A operands over the sums of 32 codes: the mins, and for centred codes the scales
     static constexpr int TABLE = FMT == F_TQ1_0 ? 256 * 8 * 16 : 0;
@@ -111,6 +111,7 @@ struct PairParams {
     int pairs, rounds, rest;     // every pair has `rounds` whole tiles; the blocks of the `rest` last tiles are shared out in units
     int unit, per, extra;        // (a block, or a tile's): `per` to a pair, one more to the first `extra` pairs
     bool share;                  // units are blocks: tiles may be shared, and their parts are added behind
+    int most_blocks;             // that the record warp fetches before it gives up
     int *status;
     __device__ __forceinline__ int start_of(int pair) const { return (pair * per + min(pair, extra)) * unit; }
     __device__ __forceinline__ int pair_of(int block) const {   // where tiles are shared
@@ -120,7 +121,7 @@ struct PairParams {
 };
 
 struct PairControl {
-    uint64_t b_full[24], b_empty[24], a_full[4], a_empty[4], d_full[4], d_empty[4], scales_full[PR_RING], scales_empty[PR_RING], w_full[6], w_empty[6], turn[PR_MMA_WARPS];
+    uint64_t b_full[24], b_empty[24], a_full[4], a_empty[4], d_full[4], d_empty[4], scales_full[PR_RING], scales_empty[PR_RING], w_full[6], w_empty[6], turn[PR_MMA_WARPS], settled;
     uint32_t tmem_base;
     int abort;
 };
@@ -230,17 +231,24 @@ __device__ __forceinline__ bool pr_try(uint32_t bar, uint32_t parity) {
 }
 __device__ __forceinline__ void pr_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void pr_expect(uint32_t bar, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory"); }
-// Bounded wait of a warp.  Gives up when another role, of either CTA, has, or after the limit; then every role leaves.
-__device__ __forceinline__ bool pr_wait(uint32_t bar, uint32_t parity, uint32_t bars, int *status) {
-    const uint32_t abort = bars + (uint32_t)offsetof(PairControl, abort);
-    for (uint32_t i = 0; i < (1u << 20); ++i) {
+// Bounded wait of a whole warp: false when another role, of either CTA, has given up, or after the limit.  What follows a wait is for whole
+// warps, so its lanes must not part: those that are about to give up look once more, together, and a phase that another lane has seen
+// complete they see so too.  The role leaves, and says so behind its loop (pair_kernel): said here, at every wait, it cost registers.
+__device__ __forceinline__ bool pr_wait(uint32_t bar, uint32_t parity, uint32_t bars) {
+    for (uint32_t left = 1u << 20; left; --left) {
         if (pr_try(bar, parity)) return true;
-        if ((i & 63u) == 63u && lds_u32(abort)) return false;
+        if ((left & 7u) == 0u && lds_u32(bars + (uint32_t)offsetof(PairControl, abort))) left = 2u;
     }
-    sts_u32(abort, 1u);
-    tc::st_cluster_u32(tc::map_to_cta(abort, tc::cluster_ctarank() ^ 1u), 1u);
-    report(status, ST_WAIT_TIMEOUT);
     return false;
+}
+// Waits for the copies that a barrier counts, whichever of its phases they belong to.  Where a role has given up, a phase may lack arrivals and
+// never end: `until` (ns) is then long after its copies have landed.
+__device__ __forceinline__ void pr_settle(uint32_t bar, uint64_t until) {
+    for (uint32_t parity = 0; parity < 2; ++parity) {
+        uint64_t now;
+        do asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        while (!__all_sync(0xffffffffu, pr_try(bar, parity)) && __any_sync(0xffffffffu, now < until));
+    }
 }
 
 // ------------------------------------------------------------------ unpacking: half a block (128 elements) of one row
@@ -567,6 +575,7 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
         for (int s = 0; s < PR_RING; ++s) { mbar_init(&ctl->scales_full[s], 1 + 4); mbar_init(&ctl->scales_empty[s], PR_E_WARPS); }
         for (int s = 0; s < F::W_SLOTS; ++s) { mbar_init(&ctl->w_full[s], 1); mbar_init(&ctl->w_empty[s], F::X_WARPS); }
         for (int s = 0; s < PR_MMA_WARPS; ++s) mbar_init(&ctl->turn[s], 1);
+        mbar_init(&ctl->settled, PR_MMA_WARPS);
         ctl->abort = 0;
         ctl->tmem_base = 0xffffffffu;
         mbar_fence_init();
@@ -594,6 +603,7 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
         tc::st_cluster_u32(tc::map_to_cta(smem_addr(&ctl->abort), (uint32_t)rank ^ 1u), 1u);
         report(p.status, ST_TMEM_ALLOC);
     }
+    bool ok = tmem_ok;                                                 // of this warp's role
 
     if (warp < F::E_WARP0) {
         // ------------------------------------------------------------------ expanders: a thread per row, or per half of one
@@ -610,7 +620,7 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
         Window win{nullptr, 0u, 0u};
         PairRecord<FMT> rec;
         auto read = [&]() {
-            if (!pr_wait(PR_BAR(w_full, slot), w_phase, bars, p.status)) return false;
+            if (!pr_wait(PR_BAR(w_full, slot), w_phase, bars)) return false;
             const uint8_t *raw = s_raw + slot * (128 * F::PITCH) + record * F::PITCH;
             const uint32_t skew = F::SHIFTED ? (skew0 + (uint32_t)(b * F::UNIT)) & 15u : 0u;
             if (F::SHIFTED && tail) {                           // rows after the last whole super-row lie apart
@@ -629,7 +639,7 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
             rec.read(half, win, skew);
             return true;
         };
-        bool ok = tmem_ok && read();
+        ok = ok && read();
         if constexpr (F::GROUPED) {                             // a block is two rounds through A
             for (int it = 0; ok && it < total; ++it) {
 #pragma unroll 1
@@ -641,7 +651,7 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
                     for (int g = 0; g < 4; ++g) s_dd[ring * DD + g * 128 + l] = d[g];
                     __syncwarp();
                     if (lane == 0) pr_arrive(PR_BAR(scales_full, ring));
-                    ok = pr_wait(PR_BAR(a_empty, buf), a_phase, bars, p.status);
+                    ok = pr_wait(PR_BAR(a_empty, buf), a_phase, bars);
                     if (!ok) break;
                     tc::fence_after_sync();
                     rec.expand(h, win, 0u, lane_base + (uint32_t)(buf * F::A_COLUMNS), 0u);
@@ -669,7 +679,8 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
                 __syncwarp();
                 if (lane == 0) pr_arrive(PR_BAR(scales_full, ring));
             }
-            if (!pr_wait(PR_BAR(a_empty, buf), a_phase, bars, p.status)) break;
+            ok = pr_wait(PR_BAR(a_empty, buf), a_phase, bars);
+            if (!ok) break;
             tc::fence_after_sync();
 #pragma unroll 1
             for (int h = half; h < 2; h += F::X_WARPS / 4) {
@@ -699,7 +710,6 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
         const float *dd = s_dd + (warp & 3) * 32 + lane, *xd_base = s_xd + part * OWN;
         int tile = first_tile, b = first_b, slot = 0;
         uint32_t d_phase = 0;
-        bool ok = tmem_ok;
         // The loops are nested, and the sums set to zero in front of the inner one only: set to zero inside of it, every pair is
         // moved on every block.
         for (int it = 0; ok && it < total;) {
@@ -711,14 +721,14 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
 #pragma unroll 1
                 for (int at = 2 * it; at < 2 * tile_end; ++at) {        // half blocks
                     const int ring = at & (PR_RING - 1);
-                    if (!pr_wait(PR_BAR(scales_full, ring), (uint32_t)(at / PR_RING) & 1u, bars, p.status)) { ok = false; break; }
+                    if (!pr_wait(PR_BAR(scales_full, ring), (uint32_t)(at / PR_RING) & 1u, bars)) { ok = false; break; }
 #pragma unroll
                     for (int c = 0; c < MOST; ++c) {
                         if (c >= chunks) break;
                         const float *xd = xd_base + ring * XD + c * F::CHUNK;
 #pragma unroll
                         for (int g = 0; g < F::GROUPS; ++g, xd += F::TOKENS) {
-                            ok = pr_wait(PR_BAR(d_full, slot), d_phase, bars, p.status);
+                            ok = pr_wait(PR_BAR(d_full, slot), d_phase, bars);
                             if (!ok) break;
                             tc::fence_after_sync();
                             const uint32_t from = lane_base + (uint32_t)(F::CHUNK * slot);
@@ -753,14 +763,14 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
 #pragma unroll 1
             for (int at = it; at < tile_end; ++at) {
                 const int ring = at & (PR_RING - 1);
-                if (!pr_wait(PR_BAR(scales_full, ring), (uint32_t)(at / PR_RING) & 1u, bars, p.status)) { ok = false; break; }
+                if (!pr_wait(PR_BAR(scales_full, ring), (uint32_t)(at / PR_RING) & 1u, bars)) { ok = false; break; }
                 const float d0 = dd[ring * DD], d1 = F::MINS ? dd[ring * DD + 128] : 0.0f;
                 const uint64_t s0 = pack2(d0, d0), s1 = pack2(d1, d1);
                 const float *xd = xd_base + ring * F::TOKENS;
 #pragma unroll
                 for (int c = 0; c < MOST; ++c) {
                     if (c >= chunks) break;
-                    ok = pr_wait(PR_BAR(d_full, slot), d_phase, bars, p.status);
+                    ok = pr_wait(PR_BAR(d_full, slot), d_phase, bars);
                     if (!ok) break;
                     tc::fence_after_sync();
                     const uint32_t from = lane_base + (uint32_t)(F::SUMS * F::CHUNK * slot);
@@ -834,12 +844,11 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
             const uint32_t full_base = tc::map_to_cta(PR_BAR(b_full, 0), 0u);                  // the even CTA's, for the halves of both
             int tile = first_tile, b = first_b, s = 0;
             uint32_t phase = 1;
-            bool ok = tmem_ok;
             for (int it = 0; ok && it < total; ++it) {
                 const int t0 = (tile % p.token_tiles) * chunks * F::CHUNK;
                 for (int h = 0; ok && h < F::HALVES; ++h) {
                     const int at = F::HALVES * it + h, ring = at & (PR_RING - 1);
-                    ok = pr_wait(PR_BAR(scales_empty, ring), ((uint32_t)(at / PR_RING) & 1u) ^ 1u, bars, p.status);
+                    ok = pr_wait(PR_BAR(scales_empty, ring), ((uint32_t)(at / PR_RING) & 1u) ^ 1u, bars);
                     if (!ok) break;
                     if (elect_one()) {
                         const uint32_t bytes = (uint32_t)(chunks * F::CHUNK * 4);
@@ -849,7 +858,7 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
                     }
                     __syncwarp();
                     for (int c = 0; c < chunks; ++c) {
-                        if (!pr_wait(PR_BAR(b_empty, s), phase, bars, p.status)) { ok = false; break; }
+                        if (!pr_wait(PR_BAR(b_empty, s), phase, bars)) { ok = false; break; }
                         if (elect_one()) {
                             const int token = t0 + c * F::CHUNK + rank * (F::CHUNK / 2);
                             const uint32_t full = full_base + 8u * (uint32_t)s;
@@ -867,8 +876,9 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
             // -------------------------------------------------------------- weight records
             int tile = first_tile, b = first_b, slot = 0;
             uint32_t phase = 1;
-            for (int it = 0; tmem_ok && it < total; ++it) {
-                if (!pr_wait(PR_BAR(w_empty, slot), phase, bars, p.status)) break;
+            for (int it = 0; ok && it < total; ++it) {
+                ok = it < p.most_blocks && pr_wait(PR_BAR(w_empty, slot), phase, bars);
+                if (!ok) break;
                 if (elect_one()) {
                     uint8_t *to = s_raw + slot * (128 * F::PITCH);
                     const int row0 = (tile / p.token_tiles) * PR_ROWS + 128 * rank;
@@ -903,20 +913,21 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
             const uint64_t am0 = tc::smem_desc(base + F::AMIN_AT, 2048, 128), xm0 = tc::smem_desc(base + F::XMIN_AT, F::CHUNK * 8, 128);
             int s = 0, buf = 0, slot = 0;
             uint32_t b_phase = 0, a_phase = 0, d_phase = 1, turn = issuer ^ 1;
-            bool ok = tmem_ok, mine = issuer == 0;
+            bool mine = issuer == 0;
             if constexpr (F::GROUPED) {
                 const uint32_t floats = tc::idesc_f16_f32acc(PR_ROWS, F::CHUNK);
                 for (int at = 0; ok && at < 2 * total; ++at) {          // half blocks; a group of 32 elements a turn
-                    if (!pr_wait(PR_BAR(a_full, buf), a_phase, bars, p.status)) break;
+                    ok = pr_wait(PR_BAR(a_full, buf), a_phase, bars);
+                    if (!ok) break;
                     const uint32_t a = a_base + (uint32_t)(buf * F::A_COLUMNS);
                     for (int c = 0; ok && c < chunks; ++c) {
                         const uint64_t bs = b0 + (uint64_t)((uint32_t)(s * F::STAGE) >> 4);
-                        if (!pr_wait(PR_BAR(b_full, s), b_phase, bars, p.status)) { ok = false; break; }
+                        if (!pr_wait(PR_BAR(b_full, s), b_phase, bars)) { ok = false; break; }
 #pragma unroll 1
                         for (int g = 0; g < F::GROUPS; ++g) {
                             if ((g & 1) == issuer) {
-                                if (!pr_wait(PR_BAR(d_empty, slot), d_phase, bars, p.status)) { ok = false; break; }
-                                if (!pr_wait(PR_BAR(turn, issuer), turn, bars, p.status)) { ok = false; break; }
+                                if (!pr_wait(PR_BAR(d_empty, slot), d_phase, bars)) { ok = false; break; }
+                                if (!pr_wait(PR_BAR(turn, issuer), turn, bars)) { ok = false; break; }
                                 turn ^= 1u;
                                 tc::fence_after_sync();
                                 if (elect_one()) {
@@ -940,13 +951,14 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
                 }
             } else
             for (int it = 0; ok && it < total; ++it) {
-                if (!pr_wait(PR_BAR(a_full, buf), a_phase, bars, p.status)) break;
+                ok = pr_wait(PR_BAR(a_full, buf), a_phase, bars);
+                if (!ok) break;
                 const uint32_t a = a_base + (uint32_t)(buf * F::A_COLUMNS);
                 for (int c = 0; c < chunks; ++c) {
                     if (mine) {
-                        if (!pr_wait(PR_BAR(b_full, s), b_phase, bars, p.status)) { ok = false; break; }
-                        if (!pr_wait(PR_BAR(d_empty, slot), d_phase, bars, p.status)) { ok = false; break; }
-                        if (!pr_wait(PR_BAR(turn, issuer), turn, bars, p.status)) { ok = false; break; }
+                        if (!pr_wait(PR_BAR(b_full, s), b_phase, bars)) { ok = false; break; }
+                        if (!pr_wait(PR_BAR(d_empty, slot), d_phase, bars)) { ok = false; break; }
+                        if (!pr_wait(PR_BAR(turn, issuer), turn, bars)) { ok = false; break; }
                         turn ^= 1u;
                         tc::fence_after_sync();
                         if (elect_one()) {
@@ -980,22 +992,44 @@ pair_kernel(const __grid_constant__ PairParams p, const __grid_constant__ CUtens
         }
     }
 
-    // A CTA stays until everything addressed to it has landed: the last commits, and, when a role has given up, its loads.
+    // A CTA stays until everything addressed to it has landed: the last commits,
     __syncwarp();
-    if (*reinterpret_cast<volatile int *>(&ctl->abort)) {
-        if (warp == F::TOKEN_WARP && rank == 0)                        // the even CTA's barriers count the halves of both
-            for (int s = 0; s < F::STAGES; ++s) { mbar_wait(&ctl->b_full[s], 0u, 1u << 10); mbar_wait(&ctl->b_full[s], 1u, 1u << 10); }
-        if (warp == F::W_WARP)
-            for (int s = 0; s < F::W_SLOTS; ++s) { mbar_wait(&ctl->w_full[s], 0u, 1u << 10); mbar_wait(&ctl->w_full[s], 1u, 1u << 10); }
-    } else if (warp == F::TOKEN_WARP) {
-        const long long loads = (long long)total * F::HALVES * chunks;
-        for (long long k = max(0LL, loads - F::STAGES); k < loads; ++k) mbar_wait(&ctl->b_empty[k % F::STAGES], (uint32_t)(k / F::STAGES) & 1u, 1u << 20);
-    } else if (warp == F::MMA_WARP) {
-        for (int k = max(0, total * F::HALVES - F::A_BUFFERS); k < total * F::HALVES; ++k) mbar_wait(&ctl->a_empty[k % F::A_BUFFERS], (uint32_t)(k / F::A_BUFFERS) & 1u, 1u << 20);
+    if (ok && warp == F::TOKEN_WARP) {
+        const int loads = total * F::HALVES * chunks;
+        for (int k = max(0, loads - F::STAGES); ok && k < loads; ++k) ok = pr_wait(PR_BAR(b_empty, k % F::STAGES), (uint32_t)(k / F::STAGES) & 1u, bars);
+    } else if (ok && warp == F::MMA_WARP) {
+        for (int k = max(0, total * F::HALVES - F::A_BUFFERS); ok && k < total * F::HALVES; ++k) ok = pr_wait(PR_BAR(a_empty, k % F::A_BUFFERS), (uint32_t)(k / F::A_BUFFERS) & 1u, bars);
+    }
+    if (tmem_ok && !ok && lane == 0) {                                 // gave up, or was told: both CTAs are to leave
+        const uint32_t abort = bars + (uint32_t)offsetof(PairControl, abort);
+        sts_u32(abort, 1u);
+        tc::st_cluster_u32(tc::map_to_cta(abort, (uint32_t)rank ^ 1u), 1u);
+        report(p.status, ST_WAIT_TIMEOUT);
     }
     tc::fence_before_sync();
     __syncthreads();
     tc::cluster_sync_all();
+    if (*reinterpret_cast<volatile int *>(&ctl->abort)) {              // the same in both CTAs now
+        // or, when a role has given up, whatever has been issued: MMAs, behind which the tensor core arrives once more, and copies (a few us; a millisecond
+        // is waited for those that no complete phase counts)
+        if (warp >= F::MMA_WARP && rank == 0) {
+            if (elect_one()) commit_both(PR_BAR(settled, 0));
+            __syncwarp();
+        }
+        uint64_t until;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(until));
+        until += 1000000u;
+        if (warp == F::MMA_WARP) {
+            for (uint32_t i = 0; i < (1u << 20) && !__all_sync(0xffffffffu, pr_try(PR_BAR(settled, 0), 0u)); ++i) {}
+        } else if (warp == F::W_WARP) {
+            for (int s = 0; s < F::W_SLOTS; ++s) pr_settle(PR_BAR(w_full, s), until);
+        } else if (warp == F::TOKEN_WARP) {
+            for (int s = 0; s < PR_RING; ++s) pr_settle(PR_BAR(scales_full, s), until);
+            for (int s = 0; rank == 0 && s < F::STAGES; ++s) pr_settle(PR_BAR(b_full, s), until);      // they count the halves of both CTAs
+        }
+        __syncthreads();
+        tc::cluster_sync_all();
+    }
     if (warp == F::MMA_WARP && *reinterpret_cast<volatile uint32_t *>(&ctl->tmem_base) != 0xffffffffu) tc::tmem_free(*reinterpret_cast<volatile uint32_t *>(&ctl->tmem_base), 512);
 }
 
