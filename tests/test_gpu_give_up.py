@@ -32,7 +32,7 @@ def kernels():
 @pytest.mark.parametrize("blocks", [0, 1, 2])
 @pytest.mark.parametrize("kernel, name, mnk", [("pairs", "Q4_K", (300, 2311, 4096)), ("pairs", "Q5_K", (129, 2311, 4096)), ("pairs", "Q6_K", (129, 2311, 4096)),
                                                ("pairs", "TQ1_0", (257, 9371, 1280)), ("pairs", "Q4_0", (128, 3001, 4352)), ("pairs", "Q8_0", (255, 9371, 1280)),
-                                               ("pairs", "Q6_K", (700, 19331, 1024))])
+                                               ("pairs", "Q6_K", (700, 19331, 1024)), ("fold", "Q4_K", (33, 4099, 4096)), ("fold", "Q4_K", (100, 19000, 2048))])
 def test_a_role_that_gives_up(torch, lib, oracle, golden, kernels, kernel, name, mnk, blocks):  # noqa: F811
     problem, (launch, plane_bytes) = Problem(torch, oracle, golden, name, *mnk), kernels[kernel]
     sms, launches = torch.cuda.get_device_properties(0).multi_processor_count, ctypes.c_uint()

@@ -167,7 +167,7 @@ cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_
     float *xd = reinterpret_cast<float *>(planes + s.codes);
     __half *mins = reinterpret_cast<__half *>(planes + s.codes + s.xd);
     FoldParams p{};
-    p.xd = xd; p.ldy = a.ldy; p.pitch = s.pitch; p.status = status;
+    p.xd = xd; p.ldy = a.ldy; p.pitch = s.pitch; p.most_blocks = a.most_blocks; p.status = status;
     p.m = (int)a.m;
     p.nb = (int)(a.k / 256);
     const long long row_bytes = (long long)p.nb * FD_UNIT;

@@ -66,11 +66,12 @@ struct FoldParams {
     long long n, ldy, pitch;
     int m, nb, nt;               // tokens, blocks per row, tokens per tile (a multiple of 16)
     int token_tiles, tiles, slices, b_stages, a_buffers;
+    int most_blocks;             // that the record warp fetches before it gives up
     int *status;
 };
 
 struct FoldControl {
-    uint64_t b_full[FD_B_MAX], b_empty[FD_B_MAX], a_full[4], a_empty[4][FD_GROUPS], d_full[2], d_empty[2], xd_full[FD_SLOTS], w_full[FD_GROUPS], w_empty[FD_W_SLOTS];
+    uint64_t b_full[FD_B_MAX], b_empty[FD_B_MAX], a_full[4], a_empty[4][FD_GROUPS], d_full[2], d_empty[2], xd_full[FD_SLOTS], w_full[FD_GROUPS], w_empty[FD_W_SLOTS], settled;
     uint32_t tmem_base;
     int abort;
 };
@@ -112,14 +113,18 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32
           "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31]) : "memory");
 }
 
-// Bounded wait of one thread or a whole warp.  Gives up when another role has, or after the limit; then every role leaves.
-__device__ __forceinline__ bool fd_wait(uint64_t *bar, uint32_t parity, FoldControl *ctl, int *status) {
-    for (uint32_t i = 0; i < (1u << 20); ++i) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((i & 63u) == 63u && *reinterpret_cast<volatile int *>(&ctl->abort)) return false;
-    }
+__device__ __forceinline__ void fd_give_up(FoldControl *ctl, int *status) {
     *reinterpret_cast<volatile int *>(&ctl->abort) = 1;
     report(status, ST_WAIT_TIMEOUT);
+}
+// Bounded wait of a whole warp.  Gives up when another role has, or after the limit; then every role leaves.  What follows a wait is for whole warps,
+// so its lanes must not part: those that are about to give up look once more, and a phase that another lane has seen complete they see so too.
+__device__ __forceinline__ bool fd_wait(uint64_t *bar, uint32_t parity, FoldControl *ctl, int *status) {
+    for (uint32_t left = 1u << 20; left; --left) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((left & 7u) == 0u && *reinterpret_cast<volatile int *>(&ctl->abort)) left = 2u;
+    }
+    fd_give_up(ctl, status);
     return false;
 }
 
@@ -191,6 +196,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
         for (int s = 0; s < FD_SLOTS; ++s) mbar_init(&ctl->xd_full[s], 1);
         for (int s = 0; s < FD_GROUPS; ++s) mbar_init(&ctl->w_full[s], 1);
         for (int s = 0; s < FD_W_SLOTS; ++s) mbar_init(&ctl->w_empty[s], 4);
+        mbar_init(&ctl->settled, 1);
         ctl->abort = 0;
         ctl->tmem_base = 0xffffffffu;
         mbar_fence_init();
@@ -446,6 +452,11 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
                     mbar_wait(&ctl->a_empty[k & (abufs - 1)][block % FD_GROUPS], a_parity(block, next % FD_CHUNKS), 1u << 20);
                 }
                 for (int k = max(0, 2 * total - stages); k < 2 * total; ++k) mbar_wait(&ctl->b_empty[k % stages], (uint32_t)(k / stages) & 1u, 1u << 20);
+            } else {
+                // a role has given up: the MMAs issued so far have to be done, and their commits here, before tensor memory is freed
+                if (elect_one()) tc::commit(&ctl->settled);
+                __syncwarp();
+                mbar_wait(&ctl->settled, 0u, 1u << 20);
             }
         }
         } else if (warp == FD_W_WARP) {
@@ -454,6 +465,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
         int issued = 0;
         for (int it = 0; it < total; ++it, at.advance(begin, end, stride)) {
             const int slot = it & (w_slots - 1), row0 = (at.tile / p.token_tiles) * FD_ROWS;
+            if (it >= p.most_blocks) { fd_give_up(ctl, p.status); break; }
             if (!fd_wait(&ctl->w_empty[slot], ((uint32_t)(it >> w_shift) & 1u) ^ 1u, ctl, p.status)) break;
             if (elect_one()) {
                 uint8_t *to = s_raw + slot * (FD_ROWS * FD_UNIT);

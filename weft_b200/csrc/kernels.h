@@ -78,7 +78,7 @@ struct TileArgs {
     const uint32_t *powers;
     float *y;                // (m, ldy)
     long long n, k, m, ldy;
-    int most_blocks = 0x7fffffff;      // of weight records that a CTA of pairs.cuh fetches; fewer than it needs make its roles give up (tests)
+    int most_blocks = 0x7fffffff;      // of weight records that a CTA of pairs.cuh and fold.cuh fetches; fewer than it needs make its roles give up (tests)
 };
 bool tile_supported(const TileArgs &a);
 size_t tile_plane_bytes(const TileArgs &a);
