@@ -67,6 +67,9 @@ def test_pairs_take_whole_aligned_matrices(pair_supported, fmt):
     assert not pair_supported(fmt, 512, 14336, 4096 + 32) and not pair_supported(fmt, 512, 14336, 4096, w=(1 << 20) + 8)
     assert not pair_supported(fmt, 32, 14336, 4096) and not pair_supported(fmt, 512, 1024, 1024)
     assert not pair_supported(fmt, 1 << 19, 1 << 20, 4096)
+    for m, n, k in [(1 << 20, 4096, 2048), ((1 << 20) + 3, 5, 2048), (129, 9, (1 << 22) + 2048)]:
+        assert pair_supported(fmt, m, n, k) == (fmt == 20)                 # the only kernel for them, of this format alone
+    assert not pair_supported(fmt, 1 << 30, 8, 2048) and not pair_supported(fmt, 4096, 5, 1 << 20)
 
 
 @pytest.mark.parametrize("fmt", [1, 5])

@@ -123,3 +123,22 @@ def test_launches_are_counted_as_they_are_made(torch, lib, oracle, golden, name,
 def test_pairs_and_single_ctas_by_what_was_measured(torch, lib, pair_supported, m, n, k, pairs):  # noqa: F811
     """Q4_K at sizes where one of the two is quicker by 5 % and more.  How many clusters the device holds decides with."""
     assert pair_supported(8, m, n, k, sms=torch.cuda.get_device_properties(0).multi_processor_count) == pairs
+
+
+@pytest.mark.parametrize("m, n, k", [((1 << 20) + 3, 13, 2048), ((1 << 20) + 130, 5, 2048), (129, 9, (1 << 22) + 2048)])
+def test_ternary_batches_of_any_extent(torch, lib, oracle, golden, m, n, k):  # noqa: F811
+    """More than 2^20 tokens, fewer than eight rows of them, and rows of more than 2^22 elements: a few distinct tokens, repeated."""
+    few = Problem(torch, oracle, golden, "TQ1_0", 257 if m > 257 else 3, n, k)
+    times = -(-m // few.m)
+    x, xq, y = few.x.repeat(times, 1)[:m].contiguous(), torch.zeros((m, few.xq.shape[1]), dtype=torch.uint8, device="cuda"), torch.full((m, n), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    assert lib.weft_b200_mul_mat_shard(few.fmt, 1, few.w.data_ptr(), x.data_ptr(), xq.data_ptr(), None, None, few.powers.data_ptr(), y.data_ptr(), n, k, m, n, 0) == 0
+    torch.cuda.synchronize()
+    few.y.copy_(y[:few.m])
+    few.xq.copy_(xq[:few.m])
+    few.check()
+    assert torch.equal(xq, few.xq.repeat(times, 1)[:m])
+    # tiles that pairs share are added up in parts: up to k / 256 additions that round in another order, by 2^-24 each
+    want = few.y.repeat(times, 1)[:m].double()
+    assert float((y - want).norm() / want.norm()) <= max(8, k // 256) ** 0.5 * 2.0 ** -24
+    assert bool(((y - want).abs() <= 1e-4 + 2e-3 * want.abs()).all())

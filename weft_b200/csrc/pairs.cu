@@ -182,9 +182,12 @@ bool pair_supported(const TileArgs &a, int sm_count) {
     //       them slower (4 to 17 %, one 23)
     const double products = (double)a.m * (double)a.n * (double)a.k;
     if (a.m <= 32) return false;
-    // 16-byte copies of records need a 16-byte aligned matrix (of whole super-rows); extents are 32-bit in the kernel
-    const long long blocks = (a.n + PR_ROWS - 1) / PR_ROWS * ((a.m + 31) / 32) * (a.k / 256);
-    if (a.m >= (1 << 20) || a.k % 256 || a.k >= (1LL << 22) || a.n < 8 || a.n >= (1LL << 31) || blocks >= (1LL << 30) || (reinterpret_cast<uintptr_t>(a.w) & 15u)) return false;
+    // 16-byte copies of records need a 16-byte aligned matrix.  Blocks, bytes of a super-row and tokens are counted in 32 bits in the kernel; TQ1_0
+    // goes as far as that allows, since no other kernel takes more than 2^20 tokens
+    const long long nb = a.k / 256, blocks = (a.n + PR_ROWS - 1) / PR_ROWS * ((a.m + 31) / 32) * nb;
+    if (a.k % 256 || a.n < 1 || a.n >= (1LL << 31) || blocks >= (1LL << 30) || (reinterpret_cast<uintptr_t>(a.w) & 15u)) return false;
+    if (a.fmt == F_TQ1_0 ? a.m >= (1LL << 30) || a.m * nb >= (1LL << 33) || 8 * nb * unit_bytes(F_TQ1_0) >= (1LL << 31) || (a.n < 8 && a.m <= (1 << 20))
+                         : a.m >= (1 << 20) || a.k >= (1LL << 22) || a.n < 8) return false;
     switch (a.fmt) {
     case F_Q6_K: return products >= 8.2e8;
     case F_Q5_K: return products >= 1.2e9 && (a.m > 64 || (a.k >= 4096 && pair_estimate(a, sm_count) < 1.04 * tile_estimate(a, sm_count)));
@@ -234,11 +237,11 @@ static cudaError_t launch_pair_format(const TileArgs &a, uint8_t *planes, int *s
               : encode_piece_map(&x_codes, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, codes, 64, m, 4 * nb, F::CHUNK / 2, 4 / F::HALVES, true);
     if (e == cudaSuccess && F::MINS) e = encode_piece_map(&x_mins, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, mins, 8, m, 2 * nb, F::CHUNK / 2, 2, false);
     else x_mins = x_codes;
-    // weight records: rows of words, or super-rows of eight rows; rows after the last whole super-row are fetched by the expanders
+    // weight records: rows of words, or super-rows of eight rows; rows after the last whole super-row come by copies of their own
     if (e == cudaSuccess && !F::SHIFTED)
         e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT32, p.w, (unsigned long long)p.row_bytes / 4, (unsigned long long)a.n, (unsigned long long)p.row_bytes, F::UNIT / 4, 128, false);
     else if (e == cudaSuccess)
-        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.w, (unsigned long long)p.row_bytes * 8, (unsigned long long)a.n / 8, (unsigned long long)p.row_bytes * 8, F::PITCH, 16, false);
+        e = encode_tile_map(&w_rows, CU_TENSOR_MAP_DATA_TYPE_UINT8, p.w, (unsigned long long)p.row_bytes * std::min(a.n, 8LL), std::max(a.n / 8, 1LL), (unsigned long long)p.row_bytes * 8, F::PITCH, 16, false);
     if (e != cudaSuccess) return e;
     return launch_pair_kernel<FMT>(p, x_codes, x_mins, w_rows, plan.pairs, stream);
 }
