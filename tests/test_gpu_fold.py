@@ -1,10 +1,8 @@
-"""GPU parity of the contraction with the weights in tensor memory (larger batches of Q4_K, Q5_K, Q6_K) against the CPU oracle.
+"""GPU parity of the contractions with the weights in tensor memory against the CPU oracle: fold_kernel on every size with Q4_K, and what the
+dispatch takes for the formats that have CTA pairs (test_gpu_pairs.py has the edges of those).
 
-Sizes are the smallest that reach it (above 32 tokens and 9e8 products, Q4_K also from 25 tokens and 1.2e9, Q5_K from 65 tokens
-and 1.5e9) and sit at
-the edges of its tiles: rows that do not fill the last 128 (nor, for Q6_K, the last super-row of 8), a matrix of eight rows,
-tokens just above a tile, one block of K, blocks that do not divide among the slices of K, more tiles than SMs, a last round of
-13 rows that is a launch of its own.
+Sizes sit at the edges of fold_kernel's tiles: rows that do not fill the last 128, a matrix of eight rows, tokens just above a tile, one block
+of K, blocks that do not divide among the slices of K, more tiles than SMs, a last round of few rows that is a launch of its own.
 
 Bound: 1e-5 relative L2 and the reference harnesses' |a - e| <= 1e-4 + 2e-3 |e|.  The sums of a block are integers, held
 exactly by the accumulators; the block's sum is rounded once (Q4_K: in its last accumulation step, by at most 2^-23).
@@ -14,6 +12,7 @@ from __future__ import annotations
 import numpy as np
 import pytest
 
+from direct import run_on
 from helpers import rel_l2
 from test_gpu_batch import Problem, lib, torch  # noqa: F401  (fixtures)
 
@@ -22,37 +21,69 @@ pytestmark = pytest.mark.gpu
 FORMATS = ["Q4_K", "Q5_K", "Q6_K"]
 
 
-def check_both_sources(torch, lib, problem):  # noqa: F811
-    problem.run(lib)
+def check_both_sources(torch, lib, problem, kernel=None):  # noqa: F811
+    """With X and with the caller's records instead: the same planes, the same bits.  kernel: this one, not the dispatch's choice."""
+    def run(flags):
+        problem.y.fill_(float("nan"))
+        torch.cuda.synchronize()
+        if kernel is None:
+            problem.run(lib, flags)
+        else:
+            assert run_on(kernel, torch, problem, flags)[0] == 0
+
+    run(0)
     problem.check()
-    first = problem.y.clone()                      # the caller's records instead of X: the same planes, the same bits
-    problem.y.fill_(float("nan"))
-    torch.cuda.synchronize()
-    problem.run(lib, flags=1)
+    first = problem.y.clone()
+    run(1)
     assert torch.equal(problem.y, first)
+
+
+def check_all(torch, lib, problem, name):  # noqa: F811
+    check_both_sources(torch, lib, problem)
+    if name == "Q4_K":
+        check_both_sources(torch, lib, problem, "fold")
 
 
 @pytest.mark.parametrize("name", FORMATS)
 @pytest.mark.parametrize("mnk", [(33, 4099, 4096), (129, 1027, 4352), (300, 8, 229632), (700, 3105, 256), (58, 18949, 512), (33, 18957, 4096)])
 def test_tile_edges(torch, lib, oracle, golden, name, mnk):  # noqa: F811
-    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
+    check_all(torch, lib, Problem(torch, oracle, golden, name, *mnk), name)
 
 
 @pytest.mark.parametrize("name", FORMATS)
 @pytest.mark.parametrize("mnk", [(65, 5643, 4096), (129, 2707, 4352), (300, 24, 229632), (700, 8377, 256), (90, 32571, 512), (97, 3779, 4096), (66, 18957, 4096)])
 def test_tile_edges_further_on(torch, lib, oracle, golden, name, mnk):  # noqa: F811
-    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
+    check_all(torch, lib, Problem(torch, oracle, golden, name, *mnk), name)
 
 
 @pytest.mark.parametrize("name", ["Q4_K", "Q6_K"])
 @pytest.mark.parametrize("mnk", [(33, 6689, 4096), (48, 4587, 4096), (300, 16, 229632)])
 def test_narrow_tiles(torch, lib, oracle, golden, name, mnk):  # noqa: F811
-    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
+    check_all(torch, lib, Problem(torch, oracle, golden, name, *mnk), name)
 
 
 @pytest.mark.parametrize("name", ["Q4_K", "Q5_K"])
 def test_fewest_tokens(torch, lib, oracle, golden, name):  # noqa: F811
-    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, 25, 3190, 15360))
+    check_all(torch, lib, Problem(torch, oracle, golden, name, 25, 3190, 15360), name)
+
+
+@pytest.mark.parametrize("mnk, launches", [((32, 18945, 4096), 3), ((32, 18951, 4096), 3), ((30, 18957, 4096), 3),      # a second launch of 1, 7 and 13 rows
+                                           ((28, 9473, 6912), 2), ((30, 40001, 1280), 2)])                            # K in one slice: a tile a CTA, and several
+def test_one_slice_and_second_launches(torch, lib, oracle, golden, mnk, launches):  # noqa: F811
+    problem = Problem(torch, oracle, golden, "Q4_K", *mnk)
+    assert run_on("fold", torch, problem) == (0, launches)
+    check_both_sources(torch, lib, problem, "fold")
+    check_both_sources(torch, lib, problem)
+
+
+def check_kernels(torch, lib, problem, name, flags=0):  # noqa: F811
+    """The dispatch's choice, CTA pairs, and fold_kernel where it has the format."""
+    problem.run(lib, flags)
+    problem.check()
+    for kernel in ["pairs", "fold"][:2 if name == "Q4_K" else 1]:
+        problem.y.fill_(float("nan"))
+        assert run_on(kernel, torch, problem, flags)[0] == 0
+        problem.check()
 
 
 @pytest.mark.parametrize("name", FORMATS)
@@ -72,9 +103,7 @@ def test_largest_codes_and_scales(torch, lib, oracle, golden, name, monkeypatch)
     draw_weights = batch.weights
     monkeypatch.setattr(batch, "weights", largest)
     monkeypatch.setattr(batch, "activations", lambda rng, m, k: np.full((m, k), 0.75, dtype=np.float32))
-    problem = Problem(torch, oracle, golden, name, 66, 5700, 4096)
-    problem.run(lib)
-    problem.check()
+    check_kernels(torch, lib, Problem(torch, oracle, golden, name, 66, 5700, 4096), name)
 
 
 class Records(Problem):
@@ -112,15 +141,11 @@ def test_large_partial_sums_that_cancel(torch, lib, oracle, name, m):  # noqa: F
     codes = np.full((m, k // 256, 256), 127, np.int8)
     codes[:, :, 128:] = -127
     codes[:, :, 128:136] += rng.integers(0, 3, size=(m, k // 256, 8), dtype=np.int8)
-    problem = Records(torch, oracle, name, w.reshape(n, -1), codes.reshape(m, k), n)
-    problem.run(lib, flags=1)
-    problem.check()
+    check_kernels(torch, lib, Records(torch, oracle, name, w.reshape(n, -1), codes.reshape(m, k), n), name, flags=1)
     if name != "Q6_K":                               # the first 160 of a block against its last 96
         first = np.arange(k) % 256 < 160
         codes = np.where(first, 127 - rng.integers(0, 2, size=(m, k)), -127).astype(np.int8)
-        problem = Records(torch, oracle, name, w.reshape(n, -1), codes, n)
-        problem.run(lib, flags=1)
-        problem.check()
+        check_kernels(torch, lib, Records(torch, oracle, name, w.reshape(n, -1), codes, n), name, flags=1)
 
 
 @pytest.mark.parametrize("name", FORMATS)
@@ -135,7 +160,14 @@ def test_integer_sums_are_exact(torch, lib, oracle, name, m):  # noqa: F811
     codes = rng.integers(-127, 128, size=(m, k), dtype=np.int8)
     codes[m // 2:] = np.abs(codes[m // 2:])          # large sums of one sign
     problem = Records(torch, oracle, name, w, codes, n)
-    problem.run(lib, flags=1)
-    got, whole = problem.y.cpu().numpy(), np.abs(problem.want) < 2.0 ** 24
-    assert np.array_equal(got[whole], problem.want[whole])
-    assert rel_l2(got, problem.want) <= 2.0 ** -23
+    whole = np.abs(problem.want) < 2.0 ** 24
+    for kernel in [None, "pairs", "fold"][:3 if name == "Q4_K" else 2]:
+        problem.y.fill_(float("nan"))
+        torch.cuda.synchronize()
+        if kernel is None:
+            problem.run(lib, flags=1)
+        else:
+            assert run_on(kernel, torch, problem, flags=1)[0] == 0
+        got = problem.y.cpu().numpy()
+        assert np.array_equal(got[whole], problem.want[whole]), kernel
+        assert rel_l2(got, problem.want) <= 2.0 ** -23, kernel

@@ -1,8 +1,9 @@
 """GPU parity of the contraction on CTA pairs (larger batches of Q4_K, Q5_K, Q6_K, TQ1_0, Q4_0 and Q8_0) against the CPU oracle.
 
-Sizes are the smallest that reach it (1.2e9 products, Q4_0 and Q8_0 1.5e9; Q4_K up to 128 tokens from 8192 rows on) and sit at the edges of its tiles: rows
+The kernel is launched whatever the dispatch would choose for a size; sizes sit at the edges of its tiles: rows
 that do not fill the last 256, nor the last super-row of 8, a matrix of eight rows, tokens just above a chunk and a tile, one block of K,
-fewer tiles than pairs (each shared by several), more tiles than pairs with the rest whole or shared.
+fewer tiles than pairs (each shared by several, or all shared by all pairs so that runs span two tiles), more tiles than pairs with the rest
+whole or shared.
 
 Bound: 1e-5 relative L2 and the reference harnesses' |a - e| <= 1e-4 + 2e-3 |e|: the sums of a block are integers and exact, only the
 order of the fp32 additions over the blocks differs.
@@ -14,6 +15,7 @@ import ctypes
 import numpy as np
 import pytest
 
+from direct import run_on
 from helpers import rel_l2
 from test_gpu_batch import Problem, lib, torch  # noqa: F401  (fixtures)
 from test_gpu_fold import check_both_sources
@@ -30,17 +32,19 @@ FORMATS, GROUPED = ["Q4_K", "Q5_K", "Q6_K", "TQ1_0"], ["Q4_0", "Q8_0"]
                                  (257, 9371, 512),           # a second tile of one token
                                  (700, 6703, 256),           # one block: nothing to share
                                  (40, 14341, 2304),          # one chunk; fewer tiles than pairs, blocks that do not divide
+                                 (40, 14341, 4096),
+                                 (300, 1283, 14336),         # fewer tiles than pairs, shared by all of them
                                  (65, 19331, 1024),          # more tiles than pairs
                                  (512, 5003, 768)])
 def test_tile_edges(torch, lib, oracle, golden, name, mnk):  # noqa: F811
-    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
+    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk), "pairs")
 
 
 @pytest.mark.parametrize("name", ["Q6_K", "TQ1_0"])            # records at any even address
 @pytest.mark.parametrize("n", [3081, 3210, 3083, 3212, 3085, 3214, 3087])
 def test_rows_after_the_last_super_row(torch, lib, oracle, golden, name, n):  # noqa: F811
     """One to seven rows, in the even and in the odd CTA of a pair; the last record ends at every offset from a 16-byte boundary that there is."""
-    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, 310, n, 1280))
+    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, 310, n, 1280), "pairs")
 
 
 @pytest.mark.parametrize("name", GROUPED)                      # tiles of 128 tokens, a scale pair per 32 elements
@@ -51,7 +55,7 @@ def test_rows_after_the_last_super_row(torch, lib, oracle, golden, name, n):  # 
                                  (384, 19331, 256),          # one block: nothing to share
                                  (640, 9001, 1024)])         # more tiles than pairs, the rest shared
 def test_group_tile_edges(torch, lib, oracle, golden, name, mnk):  # noqa: F811
-    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk))
+    check_both_sources(torch, lib, Problem(torch, oracle, golden, name, *mnk), "pairs")
 
 
 @pytest.mark.parametrize("m, n, k", [(130, 2311, 4096), (300, 8203, 512)])
@@ -68,7 +72,7 @@ def test_infinite_scales_of_ternary_records(torch, lib, oracle, golden, m, n, k,
     draw_weights = batch.weights
     monkeypatch.setattr(batch, "weights", overflown)
     problem = Problem(torch, oracle, golden, "TQ1_0", m, n, k)
-    problem.run(lib)
+    assert run_on("pairs", torch, problem)[0] == 0
     got, rows = problem.y.cpu().numpy(), [5, 70, n - 9, n - 1]
     assert np.isinf(problem.want[:, rows[:2]]).any() and np.isnan(problem.want[:, n - 9]).all()
     assert np.array_equal(got[:, rows], problem.want[:, rows], equal_nan=True)
@@ -89,7 +93,7 @@ def test_infinite_scales_of_groups(torch, lib, oracle, golden, name, monkeypatch
     draw_weights = batch.weights
     monkeypatch.setattr(batch, "weights", overflown)
     problem = Problem(torch, oracle, golden, name, 250, 2311, 4096)
-    problem.run(lib)
+    assert run_on("pairs", torch, problem)[0] == 0
     got, rows = problem.y.cpu().numpy(), [5, 70, 2311 - 9, 2311 - 1]
     assert np.isinf(problem.want[:, rows[:2]]).any() and np.isnan(problem.want[:, 2311 - 9]).all()
     assert np.array_equal(got[:, rows], problem.want[:, rows], equal_nan=True)

@@ -146,8 +146,7 @@ def _run_tq1_0(torch, oracle, m, n, k, seed, column_ranges=None):
 @pytest.mark.parametrize("mnk", [(128, 128, 1024), (130, 200, 2048), (512, 384, 1024), (32, 130, 4096), (200, 1001, 3072), (512, 4736, 1024),
                                  (300, 77, 4096), (512, 1000, 2048), (256, 160, 2048), (129, 33, 6144), (700, 2000, 4096)])
 def test_prefill_tq1_0_shapes(torch, oracle, mnk):
-    """K a multiple of 1024 takes the tensor-core kernels (above 128 tokens and with K a multiple of 2048 the CTA-pair
-    kernel, whose tiles are 32 to 160 weights wide); odd N exercises 2-byte-aligned weight rows and ragged last tiles."""
+    """Register tiles, and CTA pairs for the larger products; odd N exercises 2-byte-aligned weight rows and ragged last tiles."""
     m, n, k = mnk
     _run_tq1_0(torch, oracle, m, n, k, seed=sum(mnk))
 
@@ -159,7 +158,7 @@ def test_prefill_tq1_0_benchmark_shape(torch, oracle):
 
 
 def test_prefill_tq1_0_given_records_and_plane_reuse(torch, oracle):
-    """The CTA-pair kernel reads planes that a kernel of its own makes of the Q8_K records.  With flags bit 0 the records
+    """The kernels for batches read planes that a kernel of their own makes of the Q8_K records.  With flags bit 0 the records
     are the caller's (X is not read); a small call after a large one reuses the larger plane allocation.  Every result
     must equal, bit for bit, what the same call computes when it quantizes X itself."""
     import ctypes
@@ -171,7 +170,7 @@ def test_prefill_tq1_0_given_records_and_plane_reuse(torch, oracle):
     fn = lib.weft_b200_mul_mat_shard
     fn.argtypes = [ctypes.c_int, ctypes.c_int] + [ctypes.c_void_p] * 7 + [ctypes.c_size_t] * 4 + [ctypes.c_uint]
     powers = torch.tensor([1, 3, 9, 27, 81], dtype=torch.int32, device="cuda")
-    for m, n, k in [(512, 640, 4096), (130, 96, 2048), (300, 333, 2048)]:
+    for m, n, k in [(512, 640, 4096), (512, 5003, 768), (200, 520, 12288), (130, 96, 2048), (300, 333, 2048)]:      # CTA pairs with shared tiles, without, with; register tiles
         rng = np.random.default_rng(m + n + k)
         w = torch.from_numpy(weights(oracle.TQ1_0, rng, n, k)).cuda()
         x_host = activations(rng, m, k)

@@ -69,8 +69,8 @@ def grow_and_leave(torch, lib, problem):
             lib.weft_b200_set_stream(None)
 
 
-# a contraction in tensor memory with K in slices, one with a launch for its last rows, the CTA-pair kernel, two limbs
-@pytest.mark.parametrize("name, mnk", [("Q4_K", (64, 3450, 4096)), ("Q4_K", (33, 18957, 4096)), ("TQ1_0", (200, 520, 2048)), ("Q6_K", (129, 1611, 4352)), ("Q5_K", (97, 3779, 4096))])
+# single CTAs with K in slices, and with a launch for the last rows; register tiles; CTA pairs that share tiles
+@pytest.mark.parametrize("name, mnk", [("Q4_K", (64, 3450, 4096)), ("Q4_K", (32, 18957, 4096)), ("TQ1_0", (200, 520, 2048)), ("TQ1_0", (200, 520, 12288)), ("Q6_K", (129, 1611, 4352)), ("Q5_K", (97, 3779, 4096))])
 def test_repeated_batch_follows_its_inputs(torch, lib, oracle, golden, name, mnk):  # noqa: F811
     from test_gpu_batch import Problem
 
