@@ -507,7 +507,7 @@ __global__ void __launch_bounds__(FD_THREADS, 1) fold_kernel(const __grid_consta
     }
 }
 
-// ------------------------------------------------------------------ launch (fold_*.cu instantiate one family each)
+// ------------------------------------------------------------------ launch
 
 struct FoldPlan { int nt, slices, stages, a_buffers; double cost; };
 

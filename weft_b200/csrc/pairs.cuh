@@ -43,12 +43,12 @@
 // What bounds it: instructions and their latency.  A block of 256 tokens takes 3400 (Q4_K), 4500 (Q6_K), 2500 (TQ1_0) clocks against 2304,
 // 2048 and 1024 of tensor work; issue slots are 50 to 65 % busy and every barrier operation takes 100 to 250 clocks.
 // Measured on B200 (us, device time with the kernels before and behind it; before: fold.cuh, TQ1_0 CTA pairs with the tokens as rows):
-//   Q4_K   512 x 14336 x 4096  84.2 -> 64.9    512 x 4096 x 14336  83.4 -> 70.5    512 x 28672 x 8192 274 -> 215
-//   Q5_K   512 x 14336 x 4096   146 -> 94.7    512 x 4096 x 14336   159 -> 105     128 x 14336 x 4096 50.8 -> 37.5
-//   Q6_K   512 x 14336 x 4096   141 -> 76.8    512 x 4096 x 14336   150 -> 83.5    512 x 28672 x 8192 495 -> 248
-//   Q8_0   512 x 14336 x 4096   247 -> 160     512 x 4096 x 14336   239 -> 161     128 x 14336 x 4096 71.3 -> 50.4   (before: register tiles)
-//   Q4_0   512 x 14336 x 4096   221 -> 156     512 x 4096 x 14336   214 -> 157     128 x 14336 x 4096 63.3 -> 48.5
-//   TQ1_0  512 x 14336 x 4096  83.2 -> 57.3    512 x 4096 x 14336  80.8 -> 66.0    512 x 28672 x 8192 217 -> 165
+//   Q4_K   512 x 14336 x 4096  84.2 -> 66.2    512 x 4096 x 14336  83.4 -> 69.7    512 x 28672 x 8192 274 -> 215
+//   Q5_K   512 x 14336 x 4096   146 -> 95.9    512 x 4096 x 14336   159 -> 99.0    128 x 14336 x 4096 50.8 -> 37.1
+//   Q6_K   512 x 14336 x 4096   141 -> 76.3    512 x 4096 x 14336   150 -> 78.4    512 x 28672 x 8192 495 -> 244
+//   Q8_0   512 x 14336 x 4096   247 -> 146     512 x 4096 x 14336   239 -> 148     128 x 14336 x 4096 71.3 -> 46.9   (before: register tiles)
+//   Q4_0   512 x 14336 x 4096   221 -> 143     512 x 4096 x 14336   214 -> 146     128 x 14336 x 4096 63.3 -> 45.7
+//   TQ1_0  512 x 14336 x 4096  83.2 -> 57.3    512 x 4096 x 14336  80.8 -> 64.3    512 x 28672 x 8192 217 -> 165
 // Every wait is bounded; one that runs out raises a flag in both CTAs, every role leaves its loop, copies and MMAs in flight are waited for,
 // tensor memory is freed, and the host sees a status code.  Only this GPU's memory is read or written.
 #pragma once
@@ -233,7 +233,8 @@ __device__ __forceinline__ void pr_arrive(uint32_t bar) { asm volatile("mbarrier
 __device__ __forceinline__ void pr_expect(uint32_t bar, uint32_t bytes) { asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory"); }
 // Bounded wait of a whole warp: false when another role, of either CTA, has given up, or after the limit.  What follows a wait is for whole
 // warps, so its lanes must not part: those that are about to give up look once more, together, and a phase that another lane has seen
-// complete they see so too.  The role leaves, and says so behind its loop (pair_kernel): said here, at every wait, it cost registers.
+// complete they see so too.  The role leaves, and says so behind its loop (pair_kernel): said here, at every wait, it cost registers (512 x 14336 x
+// 4096 Q8_0 160 us, now 146; Q6_K 78.5, now 76.3).
 __device__ __forceinline__ bool pr_wait(uint32_t bar, uint32_t parity, uint32_t bars) {
     for (uint32_t left = 1u << 20; left; --left) {
         if (pr_try(bar, parity)) return true;
