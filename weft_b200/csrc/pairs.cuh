@@ -88,6 +88,7 @@ template <int FMT> struct PairFormat {
     static constexpr int X_WARPS = LIMBS == 2 ? 8 : 4, WARPS = X_WARPS + PR_E_WARPS + 4, THREADS = 32 * WARPS;
     static constexpr int E_WARP0 = X_WARPS, TOKEN_WARP = E_WARP0 + PR_E_WARPS, W_WARP = TOKEN_WARP + 1, MMA_WARP = TOKEN_WARP + 2;
     // Registers a thread: at launch, and after the roles have traded (setmaxnreg).  The trade stays inside what the CTA got.
+    // 24 warps: expanders with 64 and copies and MMAs with 32 take 2 % less than with 56 and 40 (Q8_0, TQ1_0; Q4_K and Q4_0 even).
     static constexpr int REGS = WARPS > 24 ? 72 : 80, X_REGS = WARPS > 24 ? 48 : 64, E_REGS = 96, IO_REGS = WARPS > 24 ? 24 : 32;
     static_assert(32 * (X_WARPS * X_REGS + PR_E_WARPS * E_REGS + 4 * IO_REGS) <= THREADS * REGS, "setmaxnreg would wait for ever");
     static constexpr int AMIN = I8 ? 4096 : 8192;                   // A operands over the sums of 32 codes: the mins, and for centred codes the scales
