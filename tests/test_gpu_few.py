@@ -1,0 +1,90 @@
+"""GPU parity of the streaming kernel for a few tokens (3 to 32, every format of the batch path) against the CPU oracle.
+
+The kernel is launched whatever the dispatch would choose for a size; sizes sit at the edges of its tiles of 16 rows, its token groups of
+eight, its chunks of K (one for a tile, an odd number, blocks that do not divide) and its grid (fewer tiles than SMs, just above once and twice as many).
+
+Bound: 1e-5 relative L2 and the reference harnesses' |a - e| <= 1e-4 + 2e-3 |e|: the sums of a block are integers and exact, only the
+order of the fp32 additions over the blocks differs.
+"""
+from __future__ import annotations
+
+import ctypes
+
+import numpy as np
+import pytest
+
+from helpers import rel_l2
+from test_dispatch_bounds import TileArgs, library
+from test_gpu_batch import FORMATS, Problem, torch  # noqa: F401  (fixture)
+
+pytestmark = pytest.mark.gpu
+
+WAIT_RAN_OUT = 1
+
+
+def run(torch, problem, flags=0, stages=2 ** 31 - 1):  # noqa: F811
+    """Planes and kernel; the device status."""
+    built = library()
+    launch, plane_bytes = built["_ZN4weft10launch_fewERKNS_8TileArgsEPhPiiP11CUstream_st"], built["_ZN4weft16tile_plane_bytesERKNS_8TileArgsE"]
+    launch.argtypes, plane_bytes.restype = [ctypes.POINTER(TileArgs), ctypes.c_void_p, ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p], ctypes.c_size_t
+    p = problem
+    args = TileArgs(p.fmt, p.w.data_ptr(), None if flags else p.x.data_ptr(), p.xq.data_ptr(), p.grid.data_ptr(), p.signs.data_ptr(), p.powers.data_ptr(), p.y.data_ptr(), p.n, p.k, p.m, p.n, stages)
+    planes, status = torch.empty(plane_bytes(ctypes.byref(args)), dtype=torch.uint8, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    p.y.fill_(float("nan"))
+    assert launch(ctypes.byref(args), planes.data_ptr(), status.data_ptr(), torch.cuda.get_device_properties(0).multi_processor_count, torch.cuda.current_stream().cuda_stream) == 0
+    return int(status)
+
+
+def check_both_sources(torch, problem):  # noqa: F811
+    """With X and with the caller's records instead: the same planes, the same bits."""
+    assert run(torch, problem) == 0
+    problem.check()
+    first = problem.y.clone()
+    assert run(torch, problem, flags=1) == 0
+    assert torch.equal(problem.y, first)
+
+
+@pytest.mark.parametrize("name", FORMATS)
+@pytest.mark.parametrize("mnk", [(3, 1, 2048), (8, 17, 4096), (9, 2369, 4096), (17, 4753, 2048), (24, 300, 4096), (32, 2383, 2048), (5, 2390, 6144), (8, 330, 14336)])
+def test_tile_edges(torch, oracle, golden, name, mnk):  # noqa: F811
+    if name in ("Q8_0", "Q2_K") and mnk[2] == 14336:
+        mnk = (*mnk[:2], 10240)                    # the planes of longer rows leave no room for the ring
+    check_both_sources(torch, Problem(torch, oracle, golden, name, *mnk))
+
+
+@pytest.mark.parametrize("name", ["Q4_0", "Q8_0", "Q4_K", "Q5_K"])             # records that are multiples of 16 bytes: any number of blocks
+@pytest.mark.parametrize("mnk", [(7, 1000, 768), (16, 515, 2304), (8, 5000, 256), (20, 2400, 4352)])
+def test_blocks_that_do_not_divide(torch, oracle, golden, name, mnk):  # noqa: F811
+    check_both_sources(torch, Problem(torch, oracle, golden, name, *mnk))
+
+
+@pytest.mark.parametrize("name", ["Q4_0", "Q8_0"])
+def test_infinite_scales_of_groups(torch, oracle, golden, name, monkeypatch):  # noqa: F811
+    """Records of 32 elements whose f16 scale is infinite or NaN: the rows are what the oracle gives, NaN where its sums are."""
+    import test_gpu_batch as batch
+
+    def overflown(fmt, rng, n, k):
+        w = draw_weights(fmt, rng, n, k)
+        d = w.reshape(n, k // 32, -1)[:, :, :2]
+        d[5, 0], d[70, -1], d[n - 1, 3], d[n - 9, 1] = [0, 0x7c], [0, 0xfc], [0, 0x7c], [0, 0x7e]
+        return w
+
+    draw_weights = batch.weights
+    monkeypatch.setattr(batch, "weights", overflown)
+    problem = Problem(torch, oracle, golden, name, 12, 2500, 4096)
+    assert run(torch, problem) == 0
+    got, rows = problem.y.cpu().numpy(), [5, 70, 2500 - 9, 2500 - 1]
+    assert np.isinf(problem.want[:, rows[:2]]).any() and np.isnan(problem.want[:, 2500 - 9]).all()
+    assert np.array_equal(got[:, rows], problem.want[:, rows], equal_nan=True)
+    assert rel_l2(np.delete(got, rows, axis=1), np.delete(problem.want, rows, axis=1)) <= 1e-5
+
+
+@pytest.mark.parametrize("name, mnk", [("Q4_K", (8, 5000, 4096)), ("Q8_0", (20, 2400, 4352)), ("IQ2_XXS", (9, 300, 2048))])
+@pytest.mark.parametrize("stages", [0, 1, 5])
+def test_roles_that_give_up(torch, oracle, golden, name, mnk, stages):  # noqa: F811
+    """Stages that nobody fetches: the call ends with a status, and the next one is not affected."""
+    problem = Problem(torch, oracle, golden, name, *mnk)
+    if stages < -(-mnk[2] // 256 // (4 if name == "Q8_0" else 8)):
+        assert run(torch, problem, stages=stages) == WAIT_RAN_OUT
+    assert run(torch, problem) == 0
+    problem.check()

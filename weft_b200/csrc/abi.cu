@@ -506,7 +506,7 @@ struct MulMat {
         bool gathered = false;
         if (path == NOTHING) return 0;
         if (path == TILES) {          // their first kernel quantizes X
-            if (launched(launch_tile(tile_args(), planes, sms, stream), "batched mul_mat", 2)) return 1;
+            if (launched(launch_tile(tile_args(), planes, g.status_dev, sms, stream), "batched mul_mat", 2)) return 1;
         } else if (path == PAIRS) {
             unsigned kernels = 0;
             const cudaError_t e = launch_pair(tile_args(), planes, g.status_dev, sms, stream, &kernels);

@@ -120,12 +120,12 @@ extern "C" int production_mul_mat_q4_k_decode_noalloc(const uint8_t *W, const fl
     cudaError_t e = cudaMemsetAsync(status, 0, kControlBytes, stream);            // the one thing that must start at zero
     if (e == cudaSuccess && x_staged) e = cudaMemcpyAsync(x, X, x_bytes, cudaMemcpyHostToDevice, stream);
     if (e == cudaSuccess) {
-        // A batch takes the register tiles (the regular entry point's kernel up to 24 tokens and for smaller products) while its
+        // A batch takes the register tiles or the kernel for a few tokens (the regular entry point's up to 24 tokens and for smaller products) while its
         // activation planes fit behind the staged arguments; beyond that a GEMV per token row needs no workspace.
         const TileArgs batch{F_Q4_K, W, x, xq, nullptr, nullptr, nullptr, y, (long long)N, (long long)K, (long long)M, (long long)N};
         const bool tiles = tile_supported(batch) && used + tile_plane_bytes(batch) <= WEFT_B200_NOALLOC_BYTES;
         GemvArgs args{F_Q4_K, W, xq, x, nullptr, nullptr, nullptr, y, (long long)N, (long long)K, (long long)M, (long long)N, status};
-        e = tiles ? launch_tile(batch, base + used, g_sm_count[device], stream) : launch_gemv(args, g_sm_count[device], stream);
+        e = tiles ? launch_tile(batch, base + used, status, g_sm_count[device], stream) : launch_gemv(args, g_sm_count[device], stream);
     }
     int device_status = 0;
     if (e == cudaSuccess && xq_staged) e = cudaMemcpyAsync(Xq, xq, xq_bytes, cudaMemcpyDeviceToHost, stream);

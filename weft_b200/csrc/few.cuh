@@ -1,0 +1,305 @@
+// mul_mat for a few token rows (3 to 32): the tensor-core tiles of tile.cuh behind the streaming scheme of the decode GEMVs.
+// (Same functions; examples/kernels/mul_mat/*.py of the reference.)
+//
+// What it is for: up to 32 tokens the matrix is the traffic, as for one, and the register tiles reached half of the GEMVs' rate
+// (8 x 14336 x 4096 Q4_K: 16.4 us where one token takes 7.3).  Their warps fetch everything themselves: 500 to 1000 clocks of
+// issuing 16-byte copies for every 16 rows and block, as long as the arithmetic, and the planes of the tokens, as many bytes as the weights, with
+// every step; a finer cut or more warps gave nothing.  Here a persistent CTA per SM keeps the planes of all tokens in shared memory for the whole
+// launch, and one thread brings the weights: a stage is a tensor-map box of 16 rows x up to eight blocks.  Two teams of eight warps
+// take the stages in turn, a block for each warp; a collector adds the sixteen sums of a tile in the order of the blocks and stores the results while the next
+// tile runs.  8 x 14336 x 4096, us, register tiles and this: Q4_K 16.4, 11.2; Q5_K 18.0, 13.1; Q6_K 24.5, 16.2; Q3_K 29.3, 16.3; IQ2_XXS 24.2, 18.6; TQ1_0 16.1,
+// 13.4; with 32 tokens Q6_K 38.5, 31.7; Q3_K 43.8, 27.6; TQ1_0 25.6, 19.6.
+//
+// A box takes a few bytes of the next chunk along, so that rows start 32 (16) bytes apart in the banks; whole rows by bulk copies would start all in the
+// same one.  Built and slower: a bulk copy for each row (60 ns each, whoever issues them: 13.5 us), 16-byte copies by three loader warps (17.8) or by each
+// warp for itself (14.5), K split over a cluster (22 and more), three teams (12.2).  Two or three stages in flight are best, as for the GEMVs (six: 13.2).
+// What bounds it now (ncu, Q4_K at this size): 2.9 us until the planes are there, then issue slots at 0.6 and the logic pipe at 0.55 of their rates with four
+// warps a scheduler, and the seventh tile of a few CTAs where the others have six; DRAM runs at 0.31 over the whole launch.
+#pragma once
+
+#include "ring.cuh"
+#include "tensormap.cuh"
+#include "tile.cuh"
+
+namespace weft {
+
+constexpr int FW_WARPS = 16, FW_PRODUCER = FW_WARPS, FW_COLLECTOR = FW_WARPS + 1, FW_THREADS = (FW_WARPS + 2) * 32;
+// A team of warps takes a stage, a block each: a box of a tensor map has at most 256 elements (of 8 bytes) a row, less than eight blocks of Q8_0
+__host__ __device__ constexpr int fw_members(int fmt) { return fmt == F_Q8_0 ? 4 : 8; }
+constexpr int FW_ROWS = 16, FW_MAX_SLOTS = 16;
+constexpr int FW_SMEM = 227 * 1024;
+constexpr uint32_t FW_LIMIT = 1u << 20;                      // polls of a wait before a role gives up
+
+struct FewParams {
+    const uint8_t *w;
+    const uint8_t *planes;       // [token groups][nb] groups, as tile.cuh reads them
+    const uint8_t *xq;
+    const int8_t *grid, *signs;
+    const uint32_t *powers;
+    float *y;
+    long long n, ldy, row_bytes;
+    int m, nb;
+    int chunk, chunks;           // blocks of a stage, stages of a tile
+    int slots, pitch;            // of the ring (as many for each team); bytes from row to row in a slot
+    int inflight;                // stages that the producer keeps outstanding
+    int tiles;                   // of FW_ROWS rows
+    int most;                    // stages that the producer fetches: all, or fewer, so that the others give up (TileArgs::most_blocks)
+    int *status;
+};
+
+// shared memory: barriers, tables, planes, partial sums, ring
+constexpr int FW_FULL = 0, FW_EMPTY = FW_FULL + 8 * FW_MAX_SLOTS, FW_SUMS_FULL = FW_EMPTY + 8 * FW_MAX_SLOTS, FW_SUMS_EMPTY = FW_SUMS_FULL + 16,
+              FW_TOKENS_FULL = FW_SUMS_EMPTY + 16, FW_FIXED = 384;
+static_assert(FW_TOKENS_FULL + 8 <= FW_FIXED, "barriers");
+__host__ __device__ constexpr int fw_sum_buffers(int nt) { return nt == 1 ? 2 : 1; }
+__host__ __device__ constexpr int fw_sum_bytes(int nt) { return FW_WARPS * fw_sum_buffers(nt) * nt * 512; }
+__host__ __device__ constexpr int fw_token_bytes(int nt, int nb, int group) { return (nt * nb * group + 127) & ~127; }
+
+template <int FMT, int NT>
+__global__ void __launch_bounds__(FW_THREADS, 1) few_kernel(const __grid_constant__ FewParams p, const __grid_constant__ CUtensorMap weights) {
+    using F = TileFormat<FMT>;
+    constexpr int BUFS = fw_sum_buffers(NT), MEMBERS = fw_members(FMT), TEAMS = FW_WARPS / MEMBERS;
+    extern __shared__ __align__(128) uint8_t smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2;
+    const int nb = p.nb, chunks = p.chunks, stride = gridDim.x;
+    const int count = (p.tiles - (int)blockIdx.x + stride - 1) / stride, total = count * chunks;      // tiles blockIdx.x, + stride, ... and their stages
+
+    const uint32_t bars = smem_addr(smem);
+    uint8_t *s_tables = smem + FW_FIXED;
+    uint8_t *s_tokens = s_tables + F::TABLES;
+    float4 *s_sums = reinterpret_cast<float4 *>(s_tokens + fw_token_bytes(NT, nb, F::GROUP));
+    uint8_t *s_ring = reinterpret_cast<uint8_t *>(s_sums) + fw_sum_bytes(NT);
+    const uint32_t slot_bytes = (uint32_t)(FW_ROWS * p.pitch);
+
+    asm volatile("griddepcontrol.launch_dependents;");
+    if (warp == FW_PRODUCER) {
+        if (lane < p.slots) {
+            mbar_init(reinterpret_cast<uint64_t *>(smem + FW_FULL) + lane, 1);
+            mbar_init(reinterpret_cast<uint64_t *>(smem + FW_EMPTY) + lane, MEMBERS);
+        }
+        if (lane < BUFS) {
+            mbar_init(reinterpret_cast<uint64_t *>(smem + FW_SUMS_FULL) + lane, FW_WARPS);
+            mbar_init(reinterpret_cast<uint64_t *>(smem + FW_SUMS_EMPTY) + lane, 1);
+        }
+        if (lane == 0) mbar_init(reinterpret_cast<uint64_t *>(smem + FW_TOKENS_FULL), 1);
+        mbar_fence_init();
+    }
+    __syncthreads();
+
+    // ---- producer: stage s holds chunk s % chunks of the CTA's tile s / chunks
+    int tile = blockIdx.x, chunk = 0, slot = 0;
+    const auto issue = [&]() {
+        const uint32_t bar = bars + FW_FULL + 8 * slot;
+        mbar_expect_tx_a(bar, slot_bytes);
+        tma_load_2d(s_ring + (size_t)slot * slot_bytes, &weights, chunk * p.chunk * (F::UNIT / 2) / 4, tile * FW_ROWS, reinterpret_cast<uint64_t *>(smem + FW_FULL) + slot);
+        if (++slot == p.slots) slot = 0;
+        if (++chunk == chunks) { chunk = 0; tile += stride; }
+    };
+    const int wanted = min(total, p.most), ahead = min(p.inflight, wanted);
+    if (warp == FW_PRODUCER && lane == 0)
+        for (int s = 0; s < ahead; ++s) issue();
+
+    // What precedes in the stream is the kernel that makes the planes, which started behind everything before it: weights and
+    // tables are there, planes and outputs are once it has ended.
+    if constexpr (F::TABLES > 0) {
+        stage_iq2_tables_striped(p.grid, p.signs, s_tables, s_tables + 256 * 128);
+        __syncthreads();
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+
+    if (warp == FW_PRODUCER) {
+        if (lane == 0) {
+            mbar_expect_tx_a(bars + FW_TOKENS_FULL, (uint32_t)(NT * nb * F::GROUP));
+            bulk_g2s_a(smem_addr(s_tokens), p.planes, (uint32_t)(NT * nb * F::GROUP), bars + FW_TOKENS_FULL);
+            int s = ahead;
+            for (int fill = 0, landed = 0, parity = 0; s < wanted; ++s) {    // fill: of the slot; landed: slot of the stage that has to be there
+                if (s >= p.slots) {
+                    if (slot == 0 || s == p.slots) fill = s / p.slots;
+                    if (!mbar_wait_a(bars + FW_EMPTY + 8 * slot, (uint32_t)(fill - 1) & 1u, FW_LIMIT)) break;
+                    fence_proxy_async();
+                }
+                if (!mbar_wait_a(bars + FW_FULL + 8 * landed, (uint32_t)parity, FW_LIMIT)) break;
+                if (++landed == p.slots) { landed = 0; parity ^= 1; }
+                issue();
+            }
+            if (s < wanted) report(p.status, ST_WAIT_TIMEOUT);
+            // the CTA stays until its copies have landed
+            for (int i = max(0, s - p.slots); i < s; ++i) mbar_wait_a(bars + FW_FULL + 8 * (i % p.slots), (uint32_t)(i / p.slots) & 1u, FW_LIMIT);
+            mbar_wait_a(bars + FW_TOKENS_FULL, 0, FW_LIMIT);
+        }
+        return;
+    }
+
+    if (warp == FW_COLLECTOR) {
+        // ---- collector: adds the sums of a tile, in the order of the blocks, and stores the results
+        for (int i = 0; i < count; ++i) {
+            const int buf = BUFS == 2 ? i & 1 : 0;
+            if (!mbar_wait_a(bars + FW_SUMS_FULL + 8 * buf, (uint32_t)(i / BUFS) & 1u, FW_LIMIT)) { if (lane == 0) report(p.status, ST_WAIT_TIMEOUT); return; }
+            float4 sum[NT];
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) sum[nt] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int c = 0; c < min(chunks, TEAMS); ++c) {     // the teams in the order of their first chunks
+                const float4 *v = s_sums + (size_t)(buf * FW_WARPS + (i * chunks + c) % TEAMS * MEMBERS) * NT * 32 + lane;
+                for (int k = min(p.chunk, nb - c * p.chunk); k > 0; --k, v += NT * 32)
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) {
+                        const float4 a = v[nt * 32];
+                        sum[nt].x += a.x; sum[nt].y += a.y; sum[nt].z += a.z; sum[nt].w += a.w;
+                    }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive_a(bars + FW_SUMS_EMPTY + 8 * buf);
+            const long long n0 = (long long)((int)blockIdx.x + stride * i) * FW_ROWS + r;
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) {
+                const float v[4] = {sum[nt].x, sum[nt].y, sum[nt].z, sum[nt].w};
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int token = 8 * nt + 2 * (lane & 3) + (c & 1);
+                    const long long n = n0 + 8 * (c >> 1);
+                    if (token >= p.m || n >= p.n) continue;
+                    float result = v[c];
+                    if constexpr (F::PAIR32)                   // infinite scales: tile_half
+                        if (result != result) result = pair32_dot<FMT>(p.w + n * p.row_bytes, p.xq + (long long)token * nb * 272, nb);
+                    p.y[(long long)token * p.ldy + n] = result;
+                }
+            }
+        }
+        return;
+    }
+
+    // ---- the teams take the stages in turn, a block of it for each member
+    uint32_t powers[5] = {1, 3, 9, 27, 81};
+    bool plain_powers = true;
+    if constexpr (FMT == F_TQ1_0) {
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+            const uint32_t v = p.powers[i] & 255u;
+            plain_powers &= v == powers[i];
+            powers[i] = v;
+        }
+    }
+    const int team = warp / MEMBERS, self = warp - team * MEMBERS;
+    bool ok = mbar_wait_a(bars + FW_TOKENS_FULL, 0, FW_LIMIT);
+    uint32_t phase = 0;
+    slot = team;                                               // as many slots for each team: it always meets the same ones
+    for (int i = 0, next = team; ok && i < count; ++i, next -= chunks) {       // next: this team's next chunk, counted from the tile's first
+        float acc[NT][1][4];
+#pragma unroll
+        for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[nt][0][c] = 0.f;
+        const bool any = next < chunks;
+        for (; next < chunks; next += TEAMS) {
+            if (!mbar_wait_a(bars + FW_FULL + 8 * slot, phase, FW_LIMIT)) { ok = false; break; }
+            const int block = next * p.chunk + self;
+            if (self < p.chunk && block < nb) {
+                const uint8_t *at = s_ring + (size_t)slot * slot_bytes + self * F::UNIT + r * p.pitch;
+                const uint8_t *const rows[1][2] = {{at, at + 8 * p.pitch}};
+                tile_block<FMT, NT, 1, NT <= 2>(rows, s_tokens + block * F::GROUP, nb * F::GROUP, lane, s_tables, plain_powers, powers, acc);
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive_a(bars + FW_EMPTY + 8 * slot);
+            slot += TEAMS;
+            if (slot >= p.slots) { slot = team; phase ^= 1u; }
+        }
+        if (!ok) break;
+        const int buf = BUFS == 2 ? i & 1 : 0;
+        if (i >= BUFS) ok = mbar_wait_a(bars + FW_SUMS_EMPTY + 8 * buf, (uint32_t)(i / BUFS - 1) & 1u, FW_LIMIT);
+        if (any) {
+            float4 *to = s_sums + (size_t)(buf * FW_WARPS + warp) * NT * 32 + lane;
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt) to[nt * 32] = make_float4(acc[nt][0][0], acc[nt][0][1], acc[nt][0][2], acc[nt][0][3]);
+        }
+        __syncwarp();
+        if (lane == 0) mbar_arrive_a(bars + FW_SUMS_FULL + 8 * buf);
+    }
+    if (!ok && lane == 0) report(p.status, ST_WAIT_TIMEOUT);
+}
+
+// ------------------------------------------------------------------ launch
+
+struct FewPlan { int chunk, slots, pitch, smem; };
+
+// Rows whose lanes read side by side start in different banks: the box takes some bytes of the next chunk along
+template <int FMT> int few_pitch(int chunk) {
+    using F = TileFormat<FMT>;
+    const int bytes = (chunk * F::UNIT + 15) & ~15;
+    if (F::ORDER == ORDER_NATURAL && FMT != F_IQ2_XXS) return bytes + ((32 - bytes) & 63);      // 32 bytes of a row side by side, four rows
+    return bytes + ((16 - bytes) & 31);                                                          // 16 bytes, eight rows
+}
+
+// false: the planes leave no room for a slot of every team, or rows are no multiple of 16 bytes
+template <int FMT>
+bool few_plan(FewPlan &plan, int nt, long long nb) {
+    using F = TileFormat<FMT>;
+    constexpr int MEMBERS = fw_members(FMT), TEAMS = FW_WARPS / MEMBERS;
+    if (nb * F::UNIT % 16 || nb > FW_SMEM / F::GROUP) return false;
+    constexpr int STEP = 16 / tl_gcd(F::UNIT, 16);             // chunks start on 16-byte boundaries
+    const int chunks = ((int)nb + MEMBERS - 1) / MEMBERS;
+    plan.chunk = (((int)nb + chunks - 1) / chunks + STEP - 1) / STEP * STEP;
+    if (plan.chunk > MEMBERS) return false;
+    plan.pitch = few_pitch<FMT>(plan.chunk);
+    const int fixed = FW_FIXED + F::TABLES + fw_token_bytes(nt, (int)nb, F::GROUP) + fw_sum_bytes(nt) + 16;   // 16: unaligned words are read with the next one
+    plan.slots = fixed < FW_SMEM ? std::min(FW_MAX_SLOTS, (FW_SMEM - fixed) / (FW_ROWS * plan.pitch)) / TEAMS * TEAMS : 0;
+    plan.smem = fixed + plan.slots * FW_ROWS * plan.pitch;
+    return plan.slots > 0;
+}
+
+template <int FMT, int NT>
+cudaError_t launch_few_plan(const TileArgs &a, const uint8_t *planes, const FewPlan &plan, int *status, int sm_count, cudaStream_t stream) {
+    using F = TileFormat<FMT>;
+    FewParams p{};
+    p.w = static_cast<const uint8_t *>(a.w);
+    p.planes = planes;
+    p.xq = static_cast<const uint8_t *>(a.xq);
+    p.grid = a.grid; p.signs = a.signs; p.powers = a.powers;
+    p.y = a.y;
+    p.n = a.n; p.ldy = a.ldy;
+    p.nb = (int)(a.k / 256);
+    p.row_bytes = (long long)p.nb * F::UNIT;
+    p.m = (int)a.m;
+    p.chunk = plan.chunk; p.chunks = (p.nb + plan.chunk - 1) / plan.chunk;
+    p.slots = plan.slots; p.pitch = plan.pitch;
+    const int stage = FW_ROWS * plan.pitch;
+    p.inflight = std::max(1, std::min(plan.slots, (40 * 1024 + stage / 2) / stage));
+    p.tiles = (int)((a.n + FW_ROWS - 1) / FW_ROWS);
+    p.most = a.most_blocks;
+    p.status = status;
+    CUtensorMap weights;
+    cudaError_t e = encode_tile_map(&weights, CU_TENSOR_MAP_DATA_TYPE_INT64, a.w, (unsigned long long)p.row_bytes / 8, (unsigned long long)a.n, (unsigned long long)p.row_bytes, (unsigned)plan.pitch / 8, FW_ROWS);
+    if (e == cudaSuccess) e = grant_dynamic_smem(reinterpret_cast<const void *>(few_kernel<FMT, NT>), plan.smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)std::min(sm_count, p.tiles));
+    cfg.blockDim = dim3(FW_THREADS);
+    cfg.dynamicSmemBytes = (size_t)plan.smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, few_kernel<FMT, NT>, p, weights);
+}
+
+template <int FMT>
+cudaError_t launch_few_kernel(const TileArgs &a, const uint8_t *planes, int *status, int sm_count, cudaStream_t stream) {
+    FewPlan plan;
+    const int nt = (int)((a.m + 7) / 8);
+    if (!few_plan<FMT>(plan, nt, a.k / 256)) return cudaErrorNotSupported;
+    switch (nt) {
+    case 1: return launch_few_plan<FMT, 1>(a, planes, plan, status, sm_count, stream);
+    case 2: return launch_few_plan<FMT, 2>(a, planes, plan, status, sm_count, stream);
+    case 3: return launch_few_plan<FMT, 3>(a, planes, plan, status, sm_count, stream);
+    case 4: return launch_few_plan<FMT, 4>(a, planes, plan, status, sm_count, stream);
+    default: return cudaErrorNotSupported;
+    }
+}
+
+// One translation unit per family instantiates its kernels (few_*.cu).
+#define FW_ELSEWHERE(FMT) extern template cudaError_t launch_few_kernel<FMT>(const TileArgs &, const uint8_t *, int *, int, cudaStream_t);
+TL_EACH_FORMAT(FW_ELSEWHERE)
+#undef FW_ELSEWHERE
+
+}  // namespace weft

@@ -78,12 +78,17 @@ struct TileArgs {
     const uint32_t *powers;
     float *y;                // (m, ldy)
     long long n, k, m, ldy;
-    int most_blocks = 0x7fffffff;      // of weight records that a CTA of pairs.cuh and fold.cuh fetches; fewer than it needs make its roles give up (tests)
+    int most_blocks = 0x7fffffff;      // of weight records that a CTA of pairs.cuh and fold.cuh fetches (few.cuh: stages); fewer than it needs make its roles give up (tests)
 };
 bool tile_supported(const TileArgs &a);
 size_t tile_plane_bytes(const TileArgs &a);
 double tile_estimate(const TileArgs &a, int sm_count);      // us on the device, with the kernel that makes the planes: Q4_0, Q8_0, Q5_K and TQ1_0
-cudaError_t launch_tile(const TileArgs &a, uint8_t *planes, int sm_count, cudaStream_t stream);   // two kernels
+cudaError_t launch_tile(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream);   // two kernels
+// A few token rows (3 to 32): the same tiles behind a producer that streams the weights (few.cuh), on the same planes; launch_tile takes it by itself.
+bool few_supported(const TileArgs &a);
+cudaError_t launch_few(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream);
+template <int FMT> cudaError_t launch_few_kernel(const TileArgs &a, const uint8_t *planes, int *status, int sm_count, cudaStream_t stream);
+cudaError_t launch_tile_planes(const TileArgs &a, uint8_t *planes, cudaStream_t stream);      // the first of the two
 template <int FMT> cudaError_t launch_tile_kernel(const TileArgs &a, const uint8_t *planes, int sm_count, cudaStream_t stream);
 
 // tcgen05 contraction with the weights expanded into tensor memory (fold.cuh), behind the kernel that makes its planes.

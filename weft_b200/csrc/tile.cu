@@ -157,17 +157,21 @@ double tile_estimate(const TileArgs &a, int sm_count) {
 
 size_t tile_plane_bytes(const TileArgs &a) { return (size_t)((a.m + 7) / 8) * (size_t)(a.k / 256) * tile_group_bytes(a.fmt); }
 
-cudaError_t launch_tile(const TileArgs &a, uint8_t *planes, int sm_count, cudaStream_t stream) {
-    cudaError_t e;
+cudaError_t launch_tile_planes(const TileArgs &a, uint8_t *planes, cudaStream_t stream) {
     switch (a.fmt) {
-    case F_Q4_0: e = launch_planes<F_Q4_0>(a, planes, stream); break;
-    case F_Q8_0: e = launch_planes<F_Q8_0>(a, planes, stream); break;
-    case F_Q4_K: case F_Q5_K: e = launch_planes<F_Q4_K>(a, planes, stream); break;
-    case F_Q2_K: e = launch_planes<F_Q2_K>(a, planes, stream); break;
-    case F_Q3_K: case F_Q6_K: e = launch_planes<F_Q6_K>(a, planes, stream); break;
-    case F_IQ2_XXS: e = launch_planes<F_IQ2_XXS>(a, planes, stream); break;
-    default: e = launch_planes<F_TQ1_0>(a, planes, stream); break;
+    case F_Q4_0: return launch_planes<F_Q4_0>(a, planes, stream);
+    case F_Q8_0: return launch_planes<F_Q8_0>(a, planes, stream);
+    case F_Q4_K: case F_Q5_K: return launch_planes<F_Q4_K>(a, planes, stream);
+    case F_Q2_K: return launch_planes<F_Q2_K>(a, planes, stream);
+    case F_Q3_K: case F_Q6_K: return launch_planes<F_Q6_K>(a, planes, stream);
+    case F_IQ2_XXS: return launch_planes<F_IQ2_XXS>(a, planes, stream);
+    default: return launch_planes<F_TQ1_0>(a, planes, stream);
     }
+}
+
+cudaError_t launch_tile(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream) {
+    if (few_supported(a)) return launch_few(a, planes, status, sm_count, stream);
+    const cudaError_t e = launch_tile_planes(a, planes, stream);
     if (e != cudaSuccess) return e;
     switch (a.fmt) {
     case F_Q4_0: return launch_tile_kernel<F_Q4_0>(a, planes, sm_count, stream);

@@ -83,6 +83,11 @@ __device__ __forceinline__ void mma_k32(int (&d)[4], const uint32_t (&a)[4], uin
     asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%10,%11,%10,%11};"
         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(c0), "r"(c1));
 }
+// A unsigned
+__device__ __forceinline__ void mma_k32_u8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%10,%10,%10,%10};"
+        : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(0));
+}
 __device__ __forceinline__ void mma_k32_add(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3},{%4,%5,%6,%7},{%8,%9},{%0,%1,%2,%3};"
         : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
@@ -195,7 +200,9 @@ __device__ __forceinline__ void unpack_half(const uint8_t *p, int t, const uint8
             const uint2 q = *reinterpret_cast<const uint2 *>(p + QS + 32 * (2 * H + j) + 8 * t);
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                uint32_t l = (q.x >> (4 * e)) & 0x0f0f0f0fu, h = (q.y >> (4 * e)) & 0x0f0f0f0fu;
+                // Q4_K: the upper codes stay where they are, sixteenfold, and the lower ones' scales make up for it
+                uint32_t l = FMT == F_Q4_K ? q.x & (0x0f0f0f0fu << (4 * e)) : (q.x >> (4 * e)) & 0x0f0f0f0fu;
+                uint32_t h = FMT == F_Q4_K ? q.y & (0x0f0f0f0fu << (4 * e)) : (q.y >> (4 * e)) & 0x0f0f0f0fu;
                 if constexpr (FMT == F_Q5_K) {
                     const int g = 4 * H + 2 * j + e;
                     l |= (g <= 4 ? fifth.x << (4 - g) : fifth.x >> (g - 4)) & 0x10101010u;
@@ -207,8 +214,9 @@ __device__ __forceinline__ void unpack_half(const uint8_t *p, int t, const uint8
         }
         const uint4 head = *reinterpret_cast<const uint4 *>(p);
         const uint32_t s = H == 0 ? head.y & 0x3f3f3f3fu : (head.w & 0x0f0f0f0fu) | (((head.y >> 6) & 0x03030303u) << 4);
+        const uint32_t even = (s & 0x00ff00ffu) << 4;
 #pragma unroll
-        for (int g = 0; g < 4; ++g) sc[g] = (int)byte_of(s, g);
+        for (int g = 0; g < 4; ++g) sc[g] = FMT == F_Q4_K && !(g & 1) ? (int)__byte_perm(even, 0, 0x4400 + 0x11 * g + 0x10) : (int)__byte_perm(s, 0, 0x4440 + g);
     } else if constexpr (FMT == F_Q6_K) {
         const EvenWords w(p);
         const uint32_t s0 = w.at(192 + 8 * H), s1 = w.at(196 + 8 * H);
@@ -321,7 +329,7 @@ __device__ __forceinline__ void unpack_block(const uint8_t *p, int t, float &d, 
                                              uint32_t (&high)[TileFormat<FMT>::MINS ? TileFormat<FMT>::MINS : 1]) {
     if constexpr (FMT == F_Q4_K || FMT == F_Q5_K) {
         const uint4 head = *reinterpret_cast<const uint4 *>(p);
-        d = half_bits_to_float(head.x);
+        d = half_bits_to_float(head.x) * (FMT == F_Q4_K ? 0.0625f : 1.0f);       // the sums come sixteenfold (unpack_half)
         dmin = half_bits_to_float(head.x >> 16);
         const uint32_t m = t < 2 ? head.z & 0x3f3f3f3fu : ((head.w >> 4) & 0x0f0f0f0fu) | (((head.z >> 6) & 0x03030303u) << 4);
         low[0] = bytes_to_half2(m, 16 * (t & 1));
@@ -358,15 +366,16 @@ __device__ __forceinline__ TilePlace tile_place(const TileParams &p, int index, 
     return r;
 }
 
-// One half of a block for every token group of the tile.  `stage` is the (eight tokens, block) groups in shared memory.
-template <int FMT, int NT, int MT, int H>
-__device__ __forceinline__ void tile_half(const uint8_t *stage, int lane, const TileHalf<FMT, MT> &wt, const TileBlock<FMT, MT> &blk, float (&acc)[NT][MT][4]) {
+// One half of a block for every token group of the tile.  `stage` is the (eight tokens, block) groups in shared memory, `next` bytes apart.
+// WHOLE: the integer sums of a block stay in one piece (`sums`, below 2^29 in every format), else results are formed by halves.
+template <int FMT, int NT, int MT, int H, bool WHOLE>
+__device__ __forceinline__ void tile_half(const uint8_t *stage, int next, int lane, const TileHalf<FMT, MT> &wt, const TileBlock<FMT, MT> &blk, int (&sums)[NT][MT][4], float (&acc)[NT][MT][4]) {
     using F = TileFormat<FMT>;
     constexpr int MAGIC = 0x4b400000;                        // 1.5 * 2^23 as bits: integer accumulators that start here are floats
     const int t = lane & 3;
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-        const uint8_t *group = stage + nt * F::GROUP;
+        const uint8_t *group = stage + nt * next;
         const uint4 q0 = *reinterpret_cast<const uint4 *>(group + 1024 * H + 16 * lane), q1 = *reinterpret_cast<const uint4 *>(group + 1024 * H + 512 + 16 * lane);
         const uint32_t b[4][2] = {{q0.x, q0.y}, {q0.z, q0.w}, {q1.x, q1.y}, {q1.z, q1.w}};
         if constexpr (F::PAIR32) {
@@ -405,9 +414,13 @@ __device__ __forceinline__ void tile_half(const uint8_t *stage, int lane, const 
             }
 #pragma unroll
             for (int mt = 0; mt < MT; ++mt) {
-                int isum[4] = {0, 0, 0, 0};
+                int (&isum)[4] = sums[nt][mt];
+                if (!WHOLE)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) isum[c] = 0;
                 if constexpr (FMT == F_TQ1_0) {              // one scale per block: the groups accumulate on the tensor core
-                    mma_k32(isum, wt.a[mt][0], b[0][0], b[0][1], bias.x, bias.y);
+                    if (WHOLE && H == 1) mma_k32_add(isum, wt.a[mt][0], b[0][0], b[0][1]);
+                    else mma_k32(isum, wt.a[mt][0], b[0][0], b[0][1], bias.x, bias.y);
 #pragma unroll
                     for (int g = 1; g < 4; ++g) mma_k32_add(isum, wt.a[mt][g], b[g][0], b[g][1]);
                 } else {
@@ -422,14 +435,15 @@ __device__ __forceinline__ void tile_half(const uint8_t *stage, int lane, const 
                                 for (int c = 0; c < 4; ++c) isum[c] += wt.sc[mt][c >> 1][2 * g + s] * d[c];
                             }
                         } else {
-                            mma_k32(d, wt.a[mt][g], b[g][0], b[g][1], 0, 0);
+                            if constexpr (FMT == F_Q4_K) mma_k32_u8(d, wt.a[mt][g], b[g][0], b[g][1]);
+                            else mma_k32(d, wt.a[mt][g], b[g][0], b[g][1], 0, 0);
 #pragma unroll
                             for (int c = 0; c < 4; ++c) isum[c] += wt.sc[mt][c >> 1][g] * d[c];
                         }
                     }
                 }
 #pragma unroll
-                for (int e = 0; e < 2; ++e) {                 // rows r and r + 8, the lane's two tokens side by side
+                for (int e = 0; e < (WHOLE && H == 0 ? 0 : 2); ++e) {     // rows r and r + 8, the lane's two tokens side by side
                     float2 v = mul2(make_float2((float)isum[2 * e], (float)isum[2 * e + 1]), make_float2(blk.d[mt][e], blk.d[mt][e]));
                     if constexpr (F::MINS > 0 && H == 1)
                         v = fma2(make_float2(msum[mt][2 * e], msum[mt][2 * e + 1]), make_float2(-blk.dmin[mt][e], -blk.dmin[mt][e]), v);
@@ -440,13 +454,48 @@ __device__ __forceinline__ void tile_half(const uint8_t *stage, int lane, const 
     }
 }
 
+// One block of a warp's rows against the token groups: rows r and r + 8 of every m16 tile lie at `rows`.
+template <int FMT, int NT, int MT, bool WHOLE = false>
+__device__ __forceinline__ void tile_block(const uint8_t *const (&rows)[MT][2], const uint8_t *tokens, int next, int lane, const uint8_t *s_tables, bool plain_powers,
+                                           const uint32_t (&powers)[5], float (&acc)[NT][MT][4]) {
+    using F = TileFormat<FMT>;
+    const int t = lane & 3;
+    TileBlock<FMT, MT> blk;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            constexpr int Q = F::MINS ? F::MINS : 1;
+            uint32_t low[Q] = {}, high[Q] = {};
+            if constexpr (!F::PAIR32) unpack_block<FMT>(rows[mt][e], t, blk.d[mt][e], blk.dmin[mt][e], low, high);
+#pragma unroll
+            for (int q = 0; q < Q; ++q) { blk.mins[mt][q][e] = low[q]; blk.mins[mt][q][2 + e] = high[q]; }
+        }
+    int sums[NT][MT][4] = {};
+    auto half = [&](auto h) {
+        constexpr int H = decltype(h)::value;
+        TileHalf<FMT, MT> wt;
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                uint32_t lo[4], hi[4];
+                unpack_half<FMT, H>(rows[mt][e], t, s_tables, s_tables + 256 * 128, lane & 15, plain_powers, powers, lo, hi, wt.sc[mt][e], wt.dw[mt][e]);
+#pragma unroll
+                for (int g = 0; g < 4; ++g) { wt.a[mt][g][e] = lo[g]; wt.a[mt][g][2 + e] = hi[g]; }
+            }
+        tile_half<FMT, NT, MT, H, WHOLE>(tokens, next, lane, wt, blk, sums, acc);
+    };
+    half(std::integral_constant<int, 0>{});
+    half(std::integral_constant<int, 1>{});
+}
+
 // PAIR32: one result by itself, infinite scales included.
 template <int FMT>
-__device__ float pair32_dot(const TileParams &p, int token, long long n) {
-    const uint8_t *w = p.w + n * p.row_bytes, *x = p.xq + (long long)token * p.nb * 272;
+__device__ float pair32_dot(const uint8_t *w, const uint8_t *x, int nb) {
     float acc = 0.0f;
 #pragma unroll 1
-    for (int record = 0; record < 8 * p.nb; ++record, w += record_bytes(FMT), x += 34) {
+    for (int record = 0; record < 8 * nb; ++record, w += record_bytes(FMT), x += 34) {
         int isum = 0;
 #pragma unroll 1
         for (int i = 2; i < 18; ++i) {
@@ -631,33 +680,7 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
                     rows[mt][e] = stage + own_rows + (16 * mt + 8 * e + r) * F::PITCH;
                     if (F::SHIFTED) rows[mt][e] += (skew[mt][e] + (uint32_t)block * (uint32_t)F::UNIT) & 15u;
                 }
-            TileBlock<FMT, MT> blk;
-#pragma unroll
-            for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                for (int e = 0; e < 2; ++e) {
-                    constexpr int Q = F::MINS ? F::MINS : 1;
-                    uint32_t low[Q] = {}, high[Q] = {};
-                    if constexpr (!F::PAIR32) unpack_block<FMT>(rows[mt][e], t, blk.d[mt][e], blk.dmin[mt][e], low, high);
-#pragma unroll
-                    for (int q = 0; q < Q; ++q) { blk.mins[mt][q][e] = low[q]; blk.mins[mt][q][2 + e] = high[q]; }
-                }
-            auto half = [&](auto h) {
-                constexpr int H = decltype(h)::value;
-                TileHalf<FMT, MT> wt;
-#pragma unroll
-                for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        uint32_t lo[4], hi[4];
-                        unpack_half<FMT, H>(rows[mt][e], t, s_tables, s_tables + 256 * 128, lane & 15, plain_powers, powers, lo, hi, wt.sc[mt][e], wt.dw[mt][e]);
-#pragma unroll
-                        for (int g = 0; g < 4; ++g) { wt.a[mt][g][e] = lo[g]; wt.a[mt][g][2 + e] = hi[g]; }
-                    }
-                tile_half<FMT, NT, MT, H>(tokens, lane, wt, blk, acc);
-            };
-            half(std::integral_constant<int, 0>{});
-            half(std::integral_constant<int, 1>{});
+            tile_block<FMT, NT, MT>(rows, tokens, F::GROUP, lane, s_tables, plain_powers, powers, acc);
         }
 
         // ---- the slices' sums meet in shared memory, two token groups at a time: [slice][token][row]
@@ -733,7 +756,7 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
                     const long long n = place.row0 + row;
                     if (token >= p.m || n >= p.n) continue;
                     float *y = p.y + (long long)token * p.ldy + n;
-                    if (*y != *y) *y = pair32_dot<FMT>(p, token, n);
+                    if (*y != *y) *y = pair32_dot<FMT>(p.w + n * p.row_bytes, p.xq + (long long)token * p.nb * 272, p.nb);
                 }
             }
     }
