@@ -1,4 +1,4 @@
-"""GPU parity of the streaming kernel for a few tokens (3 to 32, every format of the batch path) against the CPU oracle.
+"""GPU parity of the streaming kernel for a few tokens (3 to 32, every format of the batch path but Q8_0) against the CPU oracle.
 
 The kernel is launched whatever the dispatch would choose for a size; sizes sit at the edges of its tiles of 16 rows, its token groups of
 eight, its chunks of K (one for a tile, an odd number, blocks that do not divide) and its grid (fewer tiles than SMs, just above once and twice as many).
@@ -15,11 +15,12 @@ import pytest
 
 from helpers import rel_l2
 from test_dispatch_bounds import TileArgs, library
-from test_gpu_batch import FORMATS, Problem, torch  # noqa: F401  (fixture)
+from test_gpu_batch import FORMATS as BATCH_FORMATS, Problem, torch  # noqa: F401  (fixture)
 
 pytestmark = pytest.mark.gpu
 
 WAIT_RAN_OUT = 1
+FORMATS = [name for name in BATCH_FORMATS if name != "Q8_0"]
 
 
 def run(torch, problem, flags=0, stages=2 ** 31 - 1):  # noqa: F811
@@ -47,19 +48,18 @@ def check_both_sources(torch, problem):  # noqa: F811
 @pytest.mark.parametrize("name", FORMATS)
 @pytest.mark.parametrize("mnk", [(3, 1, 2048), (8, 17, 4096), (9, 2369, 4096), (17, 4753, 2048), (24, 300, 4096), (32, 2383, 2048), (5, 2390, 6144), (8, 330, 14336)])
 def test_tile_edges(torch, oracle, golden, name, mnk):  # noqa: F811
-    if name in ("Q8_0", "Q2_K") and mnk[2] == 14336:
+    if name == "Q2_K" and mnk[2] == 14336:
         mnk = (*mnk[:2], 10240)                    # the planes of longer rows leave no room for the ring
     check_both_sources(torch, Problem(torch, oracle, golden, name, *mnk))
 
 
-@pytest.mark.parametrize("name", ["Q4_0", "Q8_0", "Q4_K", "Q5_K"])             # records that are multiples of 16 bytes: any number of blocks
+@pytest.mark.parametrize("name", ["Q4_0", "Q4_K", "Q5_K"])             # records that are multiples of 16 bytes: any number of blocks
 @pytest.mark.parametrize("mnk", [(7, 1000, 768), (16, 515, 2304), (8, 5000, 256), (20, 2400, 4352)])
 def test_blocks_that_do_not_divide(torch, oracle, golden, name, mnk):  # noqa: F811
     check_both_sources(torch, Problem(torch, oracle, golden, name, *mnk))
 
 
-@pytest.mark.parametrize("name", ["Q4_0", "Q8_0"])
-def test_infinite_scales_of_groups(torch, oracle, golden, name, monkeypatch):  # noqa: F811
+def test_infinite_scales_of_groups(torch, oracle, golden, monkeypatch):  # noqa: F811
     """Records of 32 elements whose f16 scale is infinite or NaN: the rows are what the oracle gives, NaN where its sums are."""
     import test_gpu_batch as batch
 
@@ -71,7 +71,7 @@ def test_infinite_scales_of_groups(torch, oracle, golden, name, monkeypatch):  #
 
     draw_weights = batch.weights
     monkeypatch.setattr(batch, "weights", overflown)
-    problem = Problem(torch, oracle, golden, name, 12, 2500, 4096)
+    problem = Problem(torch, oracle, golden, "Q4_0", 12, 2500, 4096)
     assert run(torch, problem) == 0
     got, rows = problem.y.cpu().numpy(), [5, 70, 2500 - 9, 2500 - 1]
     assert np.isinf(problem.want[:, rows[:2]]).any() and np.isnan(problem.want[:, 2500 - 9]).all()
@@ -79,12 +79,11 @@ def test_infinite_scales_of_groups(torch, oracle, golden, name, monkeypatch):  #
     assert rel_l2(np.delete(got, rows, axis=1), np.delete(problem.want, rows, axis=1)) <= 1e-5
 
 
-@pytest.mark.parametrize("name, mnk", [("Q4_K", (8, 5000, 4096)), ("Q8_0", (20, 2400, 4352)), ("IQ2_XXS", (9, 300, 2048))])
-@pytest.mark.parametrize("stages", [0, 1, 5])
+@pytest.mark.parametrize("name, mnk", [("Q4_K", (8, 5000, 4096)), ("Q6_K", (20, 2400, 4096)), ("IQ2_XXS", (9, 5000, 2048))])
+@pytest.mark.parametrize("stages", [0, 1])
 def test_roles_that_give_up(torch, oracle, golden, name, mnk, stages):  # noqa: F811
     """Stages that nobody fetches: the call ends with a status, and the next one is not affected."""
     problem = Problem(torch, oracle, golden, name, *mnk)
-    if stages < -(-mnk[2] // 256 // (4 if name == "Q8_0" else 8)):
-        assert run(torch, problem, stages=stages) == WAIT_RAN_OUT
+    assert run(torch, problem, stages=stages) == WAIT_RAN_OUT
     assert run(torch, problem) == 0
     problem.check()

@@ -426,8 +426,9 @@ struct Route { Path path; size_t plane_bytes; };
 
 Route find_route(const TileArgs &a) {
     const int sms = g.prop.multiProcessorCount;
-    if (pair_supported(a, sms)) return Route{PAIRS, pair_plane_bytes(a, sms)};
-    if (fold_supported(a)) return Route{FOLD, fold_plane_bytes(a)};
+    if (pair_supported(a, sms)) {
+        if (!tiles_quicker(a, pair_estimate(a, sms), sms)) return Route{PAIRS, pair_plane_bytes(a, sms)};
+    } else if (fold_supported(a) && !tiles_quicker(a, fold_estimate(a, sms), sms)) return Route{FOLD, fold_plane_bytes(a)};
     if (tile_supported(a)) return Route{TILES, tile_plane_bytes(a)};
     return Route{GEMV, 0};
 }

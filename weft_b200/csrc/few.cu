@@ -7,38 +7,38 @@ static bool plan_of(const TileArgs &a, FewPlan &plan) {
     const int nt = (int)((a.m + 7) / 8);
     switch (a.fmt) {
 #define FW_PLAN(FMT) case FMT: return few_plan<FMT>(plan, nt, a.k / 256);
-    TL_EACH_FORMAT(FW_PLAN)
+    FW_EACH_FORMAT(FW_PLAN)
 #undef FW_PLAN
     default: return false;
     }
 }
 
-// Where the streaming kernel is the quicker one.  Measured at 3400 sizes (3 to 32 tokens, 256 to 32768 rows, K 512 to 14336, all formats) against
-// the register tiles: 2300 of them are taken, with 0.83 of their time in the median; 1.5 % of those are more than 2 % slower, none more than 7 %.
-// What is not, with streaming / tiles in us:
-// * Q4_0 and Q8_0, with an epilogue for every 32 elements, gain where the tiles' grid is more than one round and rows are long
-//   (16 x 14336 x 4096 Q8_0 18.7 / 23.0, Q4_0 17.3 / 19.8; 16 x 8192 x 2048 Q4_0 9.6 / 8.2);
-// * a ring with one slot for each team only (the planes take the rest) leaves nothing to hide the copies behind, which the formats with
-//   little arithmetic feel (8 x 4096 x 14336 Q5_K 18.1 / 15.7; Q6_K 6144 rows 29.7 / 37.4);
-// * tiles of few rows: more than eight tokens on fewer rows than SMs take K in slices there (16 x 512 x 4096 Q4_K 5.4 / 5.1, 24 x 512 Q6_K 7.0 / 6.4);
-// * short rows: the collector's turn for a tile is as long as the tile (32 x 28672 x 1024 Q5_K 17.6 / 14.7).
+// Where the streaming kernel is the quicker one.  Measured at 2200 sizes (3 to 32 tokens, 256 to 32768 rows, K 512 to 14336, all formats) against
+// the register tiles: the choice is 0.1 (Q3_K) to 1.8 % (Q2_K) slower than the better one on average, the tiles alone would be 3 (Q4_0) to 39 % (Q3_K).
+// What is not taken, with streaming / tiles in us:
+// * Q8_0, and Q4_0 with more than eight tokens or short rows, whose epilogue for every 32 elements is the larger part (16 x 14336 x 4096 Q4_0 17.3 / 16.9);
+// * a ring with one slot for each team only (the planes take the rest): nothing hides the copies then, which formats with little arithmetic feel
+//   (8 x 4096 x 14336 Q5_K 18.1 / 15.7; Q6_K 6144 rows 29.7 / 37.4), others with many tokens (20 x 8771 x 6144 Q6_K 30.9 / 25.5);
+// * chunks that leave members of a team idle, with many tokens (29 x 4032 x 3072 Q4_K 10.4 / 8.9);
+// * more tokens on fewer rows than SMs have warps for, where the tiles take K in slices (24 x 512 x 4096 Q6_K 7.0 / 6.3);
+// * short rows, where the collector's turn for a tile is as long as the tile (32 x 28672 x 1024 Q5_K 17.6 / 13.9).
 bool few_supported(const TileArgs &a) {
     FewPlan plan;
     if (a.m < 3 || a.m > 32 || a.k % 256 || a.k < 256 || a.n > (1LL << 30) || (reinterpret_cast<uintptr_t>(a.w) & 15u) || !plan_of(a, plan)) return false;
-    const bool tight = plan.slots < 2 * FW_WARPS / fw_members(a.fmt);
+    const bool tight = plan.slots < 2 * FW_WARPS / FW_MEMBERS, full = plan.chunk >= FW_MEMBERS - 1;
     switch (a.fmt) {
-    case F_Q4_0: return !tight && (a.m <= 8 ? a.k >= 8192 : a.k >= 4096 && (a.m <= 16 ? a.n >= 6144 : a.m <= 24 && a.n >= 9472));
-    case F_Q8_0: return a.m > 8 && a.m <= 24 && a.n >= 6144 && a.k >= (a.m <= 16 ? 2048 : 4096);
-    case F_Q4_K: case F_Q5_K: if (tight) return a.n >= 24576; break;
-    case F_Q2_K: if (a.m > 24 || a.k < 2048) return false; break;
-    case F_IQ2_XXS: break;
-    case F_Q3_K: return a.m <= 16 || a.n >= 512;
-    case F_TQ1_0: if (a.m <= 8 && a.k <= 4096 && a.n >= 2048 && a.n <= 5120) return false; break;      // a tile and three quarters for a CTA
-    default: break;
+    case F_Q4_0: return a.m <= 8 && !tight && (a.k >= 8192 || (a.k >= 4096 && a.n >= 9472));
+    case F_Q4_K: case F_Q5_K: if (tight || a.m > 24 || (a.m > 8 && !full)) return false; break;
+    case F_Q2_K: if (a.m > 16 || a.k < 2048) return false; break;
+    case F_Q3_K: return a.m <= 16 || a.n >= 1024;
+    case F_IQ2_XXS: return a.m <= 8 || !tight || a.n < 7168;
+    case F_Q6_K: if ((tight && a.m > 8) || (a.m > 16 && (!full || (a.m > 24 && a.n >= 8192)))) return false; break;
+    default:                                                   // TQ1_0; 2048 to 5120 rows are a tile and three quarters for a CTA
+        if ((a.m <= 8 && a.k <= 4096 && a.n >= 2048 && a.n <= 5120) || (a.m > 16 && (tight || !full || (a.m > 24 && a.n >= 8192)))) return false;
     }
     if (a.m <= 8) return true;
-    if (a.fmt != F_IQ2_XXS && a.n < (a.m <= 16 && a.k >= 4096 ? 1024 : 1536)) return false;
-    return a.k >= 2048 || a.n <= 16384;
+    if (a.n < (a.m <= 16 && a.k >= 4096 ? 1024 : 1536)) return false;
+    return a.k >= 2048 || a.n <= (a.m <= 16 ? 16384 : 8192);
 }
 
 cudaError_t launch_few(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream) {
@@ -46,7 +46,7 @@ cudaError_t launch_few(const TileArgs &a, uint8_t *planes, int *status, int sm_c
     if (e != cudaSuccess) return e;
     switch (a.fmt) {
 #define FW_LAUNCH(FMT) case FMT: return launch_few_kernel<FMT>(a, planes, status, sm_count, stream);
-    TL_EACH_FORMAT(FW_LAUNCH)
+    FW_EACH_FORMAT(FW_LAUNCH)
 #undef FW_LAUNCH
     default: return cudaErrorNotSupported;
     }

@@ -24,15 +24,14 @@
 namespace weft {
 
 constexpr int FW_WARPS = 16, FW_PRODUCER = FW_WARPS, FW_COLLECTOR = FW_WARPS + 1, FW_THREADS = (FW_WARPS + 2) * 32;
-// A team of warps takes a stage, a block each: a box of a tensor map has at most 256 elements (of 8 bytes) a row, less than eight blocks of Q8_0
-__host__ __device__ constexpr int fw_members(int fmt) { return fmt == F_Q8_0 ? 4 : 8; }
+constexpr int FW_MEMBERS = 8, FW_TEAMS = FW_WARPS / FW_MEMBERS;      // a team of warps takes a stage, a block each
 constexpr int FW_ROWS = 16, FW_MAX_SLOTS = 16;
 constexpr int FW_SMEM = 227 * 1024;
 constexpr uint32_t FW_LIMIT = 1u << 20;                      // polls of a wait before a role gives up
 
 struct FewParams {
     const uint8_t *w;
-    const uint8_t *planes;       // [token groups][nb] groups, as tile.cuh reads them
+    const uint8_t *planes;       // [nb][token groups] groups, as tile.cuh reads them
     const uint8_t *xq;
     const int8_t *grid, *signs;
     const uint32_t *powers;
@@ -58,7 +57,7 @@ __host__ __device__ constexpr int fw_token_bytes(int nt, int nb, int group) { re
 template <int FMT, int NT>
 __global__ void __launch_bounds__(FW_THREADS, 1) few_kernel(const __grid_constant__ FewParams p, const __grid_constant__ CUtensorMap weights) {
     using F = TileFormat<FMT>;
-    constexpr int BUFS = fw_sum_buffers(NT), MEMBERS = fw_members(FMT), TEAMS = FW_WARPS / MEMBERS;
+    constexpr int BUFS = fw_sum_buffers(NT), MEMBERS = FW_MEMBERS, TEAMS = FW_TEAMS;
     extern __shared__ __align__(128) uint8_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, r = lane >> 2;
     const int nb = p.nb, chunks = p.chunks, stride = gridDim.x;
@@ -196,7 +195,7 @@ __global__ void __launch_bounds__(FW_THREADS, 1) few_kernel(const __grid_constan
             if (self < p.chunk && block < nb) {
                 const uint8_t *at = s_ring + (size_t)slot * slot_bytes + self * F::UNIT + r * p.pitch;
                 const uint8_t *const rows[1][2] = {{at, at + 8 * p.pitch}};
-                tile_block<FMT, NT, 1, NT <= 2>(rows, s_tokens + block * F::GROUP, nb * F::GROUP, lane, s_tables, plain_powers, powers, acc);
+                tile_block<FMT, NT, 1, NT <= 2>(rows, s_tokens + block * NT * F::GROUP, F::GROUP, lane, s_tables, plain_powers, powers, acc);
             }
             __syncwarp();
             if (lane == 0) mbar_arrive_a(bars + FW_EMPTY + 8 * slot);
@@ -233,7 +232,7 @@ template <int FMT> int few_pitch(int chunk) {
 template <int FMT>
 bool few_plan(FewPlan &plan, int nt, long long nb) {
     using F = TileFormat<FMT>;
-    constexpr int MEMBERS = fw_members(FMT), TEAMS = FW_WARPS / MEMBERS;
+    constexpr int MEMBERS = FW_MEMBERS, TEAMS = FW_TEAMS;
     if (nb * F::UNIT % 16 || nb > FW_SMEM / F::GROUP) return false;
     constexpr int STEP = 16 / tl_gcd(F::UNIT, 16);             // chunks start on 16-byte boundaries
     const int chunks = ((int)nb + MEMBERS - 1) / MEMBERS;
@@ -299,7 +298,8 @@ cudaError_t launch_few_kernel(const TileArgs &a, const uint8_t *planes, int *sta
 
 // One translation unit per family instantiates its kernels (few_*.cu).
 #define FW_ELSEWHERE(FMT) extern template cudaError_t launch_few_kernel<FMT>(const TileArgs &, const uint8_t *, int *, int, cudaStream_t);
-TL_EACH_FORMAT(FW_ELSEWHERE)
+#define FW_EACH_FORMAT(DO) DO(F_Q4_0) DO(F_Q2_K) DO(F_Q3_K) DO(F_Q4_K) DO(F_Q5_K) DO(F_Q6_K) DO(F_IQ2_XXS) DO(F_TQ1_0)
+FW_EACH_FORMAT(FW_ELSEWHERE)
 #undef FW_ELSEWHERE
 
 }  // namespace weft

@@ -2,6 +2,7 @@
 #include "few.cuh"
 
 namespace weft {
+template cudaError_t launch_few_kernel<F_Q4_0>(const TileArgs &, const uint8_t *, int *, int, cudaStream_t);
 template cudaError_t launch_few_kernel<F_Q4_K>(const TileArgs &, const uint8_t *, int *, int, cudaStream_t);
 template cudaError_t launch_few_kernel<F_Q5_K>(const TileArgs &, const uint8_t *, int *, int, cudaStream_t);
 }  // namespace weft

@@ -82,14 +82,14 @@ struct TileArgs {
 };
 bool tile_supported(const TileArgs &a);
 size_t tile_plane_bytes(const TileArgs &a);
-double tile_estimate(const TileArgs &a, int sm_count);      // us on the device, with the kernel that makes the planes: Q4_0, Q8_0, Q5_K and TQ1_0
+bool tiles_quicker(const TileArgs &a, double other, int sm_count);      // than a kernel that takes `other` us on the device, planes included
 cudaError_t launch_tile(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream);   // two kernels
 // A few token rows (3 to 32): the same tiles behind a producer that streams the weights (few.cuh), on the same planes; launch_tile takes it by itself.
 bool few_supported(const TileArgs &a);
 cudaError_t launch_few(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream);
 template <int FMT> cudaError_t launch_few_kernel(const TileArgs &a, const uint8_t *planes, int *status, int sm_count, cudaStream_t stream);
 cudaError_t launch_tile_planes(const TileArgs &a, uint8_t *planes, cudaStream_t stream);      // the first of the two
-template <int FMT> cudaError_t launch_tile_kernel(const TileArgs &a, const uint8_t *planes, int sm_count, cudaStream_t stream);
+template <int FMT> cudaError_t launch_tile_kernel(const TileArgs &a, const uint8_t *planes, int *status, int sm_count, cudaStream_t stream);
 
 // tcgen05 contraction with the weights expanded into tensor memory (fold.cuh), behind the kernel that makes its planes.
 bool fold_supported(const TileArgs &a);
@@ -101,6 +101,7 @@ cudaError_t launch_fold(const TileArgs &a, uint8_t *planes, int *status, int sm_
 struct PairPlan { int chunks, pairs; bool share; long long tiles; double cost; };      // chunks of tokens of a tile, pairs, whether they share the tiles, and the estimated time (us) of that
 PairPlan pair_plan(const TileArgs &a, int sm_count);
 bool pair_supported(const TileArgs &a, int sm_count);
+double pair_estimate(const TileArgs &a, int sm_count);      // us on the device, with the kernel that makes the planes
 size_t pair_plane_bytes(const TileArgs &a, int sm_count);
 cudaError_t launch_pair(const TileArgs &a, uint8_t *planes, int *status, int sm_count, cudaStream_t stream, unsigned *launches);   // two or three kernels
 

@@ -145,7 +145,7 @@ size_t pair_plane_bytes(const TileArgs &a, int sm_count) {
 
 // The plan's cost beside a start, the planes and the results: within 3 (Q4_0, Q8_0) to 6 % (TQ1_0) rms of the times of 600 to 930 sizes of a
 // format.  A tile of many parts takes 0.16 us longer for each.
-static double pair_estimate(const TileArgs &a, int sm_count) {
+double pair_estimate(const TileArgs &a, int sm_count) {
     const PairPlan plan = pair_plan(a, sm_count);
     const double planes = (double)a.m * (double)a.k * 1e-6, results = (double)a.m * (double)a.n * 1e-6, parts = plan.share ? std::max(0.0, (double)plan.pairs / (double)plan.tiles - 1.0) : 0.0;
     switch (a.fmt) {
@@ -158,28 +158,15 @@ static double pair_estimate(const TileArgs &a, int sm_count) {
 }
 
 bool pair_supported(const TileArgs &a, int sm_count) {
-    // Where this kernel is the quickest, us on the device of what runs otherwise (register tiles, for Q4_K fold.cuh) / this:
-    // Q6_K  from 33 tokens and 8.2e8 products on: 48 x 4096 x 4096 (8.1e8) 18.4 / 18.9, 200 x 1024 x 4096 (8.4e8) 19.0 / 17.9, 256 x 2048 x
-    //       2048 (1.1e9) 22.3 / 16.8, 64 x 4096 x 4096 21.7 / 19.2
-    // Q5_K  1.2e9: 64 x 4096 x 4096 (1.1e9) 16.5 / 17.8, 384 x 4096 x 768 (1.2e9) 14.0 / 12.5, 96 x 4096 x 4096 21.5 / 19.0; short rows from 65
-    //       tokens: 40 x 32000 x 2048 27.3 / 30.4, 64 35.8 / 31
-    // TQ1_0 1.2e9: 256 x 2048 x 2048 (1.1e9) 15.3 / 16.9, 384 x 4096 x 768 13.3 / 12.9, 384 x 1024 x 4096 20.4 / 19.5; up to 40 tokens the tiles
-    //       of 8 are quicker unless there are many long rows: 40 x 4096 x 14336 27.4 / 29.3, 40 x 14336 x 4096 29.1 / 27.0
-    // Q4_K  1.2e9 and more than 128 tokens: 160 x 4096 x 2048 (1.3e9) 15.4 / 14.6, 160 x 4096 x 4096 20.9 / 19.0, 128 x 4096 x 4096 16.4 / 17.1; but few
-    //       short rows leave too little for every pair: 512 x 1024 x 4096 17.7 / 18.9, 256 x 1024 x 14336 27.4 / 25.2.  Fewer tokens where
-    //       there are many rows: 40 x 14336 x 4096 25.1 / 23.1, 128 x 4096 x 14336 31.0 / 31.5
-    // Q4_0, Q8_0: tiles of 128 tokens, so by the plan's own estimate against that of the register tiles, which is linear in the products (within
-    //       5 % from 2e9 on): Q8_0 128 x 4096 x 4096 29.4 / 23.1, 160 x 4096 x 4096 32.7 / 34.3, 64 x 28672 x 4096 72.1 / 83.1, 300 x 14336 x 4096 138 / 119;
-    //       Q4_0 128 x 4096 x 4096 25.8 / 22.2, 260 x 4096 x 4096 41.6 / 52.7, 512 x 1024 x 4096 27.3 / 23.6.  Below 1.5e9 they are even: 256 x 1024 x
-    //       4096 Q8_0 17.8 / 18.2, 256 x 4096 x 1024 14.9 / 16.4
-    // How the tiles of either kernel divide among the SMs, and short rows, decide as much as these lines: beyond them, the others keep what
-    // they look quicker at by 4 % (TQ1_0 6) with planes and results counted, since an estimate is as uncertain as that.
-    // Q4_K  68 x 8416 x 6912 26.4 / 33.2, 380 x 6158 x 4864 34.3 / 40.8, 122 x 8841 x 6912 29.6 / 34.6; of 930 sizes 47 go to fold.cuh by this, 10 %
-    //       quicker on average, two of them slower (4 and 9 %)
-    // Q5_K up to 64 tokens: 40 x 8192 x 8192 30.6 / 35.1
-    // Q4_0, Q8_0 and TQ1_0 up to 64 tokens: Q8_0 181 x 11200 x 768 17.6 / 22.8, 455 x 4689 x 768 19.0 / 22.6, Q4_0 177 x 7387 x 1280 17.9 / 21.9, TQ1_0
-    //       40 x 8192 x 8192 27.8 / 32.3, 38 x 8512 x 5376 21.3 / 28.2; of 2350 sizes 75 go to the register tiles, 5 to 13 % quicker on average, seven of
-    //       them slower (4 to 17 %, one 23)
+    // Where this kernel may be the quickest; the register tiles keep what they look quicker at all the same (tiles_quicker).  The lines are
+    // where it never was: us of the register tiles, for Q4_K of fold.cuh / this:
+    // Q6_K  below 8.2e8 products: 200 x 1024 x 4096 (8.4e8) 15.7 / 17.9, 64 x 4096 x 4096 18.0 / 19.2
+    // Q5_K, TQ1_0 below 1.2e9 and, up to 50 tokens, unless there are many long rows: Q5_K 40 x 8192 x 8192 24.8 / 35.7, TQ1_0 50 x 4722 x 5888 16.6 / 24.7
+    // Q4_K  below 1.2e9; 512 x 1024 x 4096 17.7 / 18.9, 256 x 1024 x 14336 27.4 / 25.2; fewer tokens only where there are many rows: 40 x 14336 x 4096
+    //       25.1 / 23.1, 128 x 4096 x 14336 31.0 / 31.5; and where fold.cuh looks quicker by 4 %, since an estimate is as uncertain as that:
+    //       68 x 8416 x 6912 26.4 / 33.2, 380 x 6158 x 4864 34.3 / 40.8, 122 x 8841 x 6912 29.6 / 34.6
+    // Q4_0, Q8_0: tiles of 128 tokens, so by the plan's own estimate against what is linear in the products, and short rows never: Q8_0 181 x 11200 x 768
+    //       14.8 / 22.1, 455 x 4689 x 768 17.0 / 21.5, Q4_0 177 x 7387 x 1280 16.3 / 20.8
     const double products = (double)a.m * (double)a.n * (double)a.k;
     if (a.m <= 32) return false;
     // 16-byte copies of records need a 16-byte aligned matrix.  Blocks, bytes of a super-row and tokens are counted in 32 bits in the kernel; TQ1_0
@@ -190,12 +177,9 @@ bool pair_supported(const TileArgs &a, int sm_count) {
                          : a.m >= (1 << 20) || a.k >= (1LL << 22) || a.n < 8) return false;
     switch (a.fmt) {
     case F_Q6_K: return products >= 8.2e8;
-    case F_Q5_K: return products >= 1.2e9 && (a.m > 64 || (a.k >= 4096 && pair_estimate(a, sm_count) < 1.04 * tile_estimate(a, sm_count)));
-    case F_TQ1_0: return products >= 1.2e9 && (a.m > 64 || ((a.m > 40 || (a.n >= 8192 && a.k >= 4096)) && pair_estimate(a, sm_count) < 1.06 * tile_estimate(a, sm_count)));
+    case F_Q5_K: case F_TQ1_0: return products >= 1.2e9 && (a.m > 50 || (a.k >= 4096 && (a.n >= 12288 || products >= 4e9)));
     case F_Q4_K: return products >= 1.2e9 && (a.m > 128 ? a.n >= 2048 || a.k >= 8192 : a.n >= 8192) && pair_estimate(a, sm_count) < 1.04 * fold_estimate(a, sm_count);
-    case F_Q4_0: case F_Q8_0:
-        return products >= 1.5e9 && pair_plan(a, sm_count).cost + 5.0 <= (a.fmt == F_Q4_0 ? 10.0 + 7.0e-9 * products : 12.0 + 7.8e-9 * products) &&
-               pair_estimate(a, sm_count) < 1.04 * tile_estimate(a, sm_count);
+    case F_Q4_0: case F_Q8_0: return products >= 1.5e9 && (a.k >= 2048 || (a.k >= 1024 && products >= 1.8e9)) && pair_plan(a, sm_count).cost + 5.0 <= (a.fmt == F_Q4_0 ? 10.0 + 7.0e-9 * products : 12.0 + 7.8e-9 * products);
     default: return false;
     }
 }

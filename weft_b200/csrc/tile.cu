@@ -18,7 +18,7 @@ __global__ void __launch_bounds__(256) tile_planes_kernel(const float *__restric
     const long long unit = (long long)blockIdx.x * 8 + warp;
     if (unit >= (long long)m * nb) return;
     const int token = (int)(unit / nb), block = (int)(unit - (long long)token * nb), n = token & 7;
-    uint8_t *group = planes + ((long long)(token >> 3) * nb + block) * F::GROUP;
+    uint8_t *group = planes + ((long long)block * ((m + 7) / 8) + (token >> 3)) * F::GROUP;
     uint32_t q0, q1;
     int sum = 0;                                  // Q8_K: of the lane pair's 16 codes (the record's bsum)
     float d;
@@ -144,15 +144,29 @@ bool tile_supported(const TileArgs &a) {
            (reinterpret_cast<uintptr_t>(a.w) & 15u) == 0 && !by_token_rows(a);
 }
 
-// The plan's cost beside a start, the planes and the results: within 7 to 12 % (rms) of the times of 600 to 780 sizes of a format, 33 to 8192 tokens
-double tile_estimate(const TileArgs &a, int sm_count) {
+// The plan's cost beside a start, the planes and the results: within 3 (Q4_0) to 7 % (Q4_K, rms) of the times of 230 to 270 sizes of a format, 33 to 512 tokens:
+// Q4_0, Q8_0, Q4_K and TQ1_0
+static double tile_estimate(const TileArgs &a, int sm_count) {
     const double planes = (double)a.m * (double)a.k * 1e-6, results = (double)a.m * (double)a.n * 1e-6;
     switch (a.fmt) {
-    case F_Q4_0: return 2.6 + 1.33 * tile_plan<F_Q4_0>(a, sm_count).cost + 1.03 * planes + 1.32 * results;
-    case F_Q8_0: return 3.2 + 1.41 * tile_plan<F_Q8_0>(a, sm_count).cost + 1.09 * planes + 1.5 * results;
-    case F_Q5_K: return 4.3 + 1.27 * tile_plan<F_Q5_K>(a, sm_count).cost + 1.1 * planes + 1.12 * results;
-    default: return 4.4 + 1.06 * tile_plan<F_TQ1_0>(a, sm_count).cost + 1.45 * planes + 0.76 * results;
+    case F_Q4_0: return 3.8 + 0.471 * tile_plan<F_Q4_0>(a, sm_count).cost + 0.384 * planes + 0.675 * results;
+    case F_Q8_0: return 3.9 + 0.451 * tile_plan<F_Q8_0>(a, sm_count).cost + 0.566 * planes + 0.911 * results;
+    case F_Q4_K: return 2.5 + 0.904 * tile_plan<F_Q4_K>(a, sm_count).cost + 0.744 * planes + 2.696 * results;
+    default: return 3.9 + 0.706 * tile_plan<F_TQ1_0>(a, sm_count).cost + 1.441 * planes + 1.889 * results;
     }
+}
+
+// Whether the register tiles look quicker than `other` (us on the device, pairs.cuh or fold.cuh).  How the tiles of either kernel divide among the
+// SMs decides, so it goes by the estimates of both; those of Q4_0 and Q8_0 on CTA pairs run 5 % high.  Of 1000 sizes of 4e8 products and more
+// (33 to 512 tokens) the choice is 0.1 (Q4_0, Q8_0) to 0.3 % slower than the better one on average.  Tiles / pairs, us:
+// Q8_0 128 x 4096 x 4096 18.5 / 22.3, 512 x 14336 x 4096 170 / 146; TQ1_0 384 x 1024 x 4096 16.0 / 19.5, 512 x 28672 x 8192 581 / 166; Q4_K 160 x 4096 x
+// 4096 21.6 / 18.9; tiles / fold.cuh, Q4_K: 202 x 1216 x 4096 11.7 / 15.2, 209 x 1984 x 6144 27.4 / 19.1.
+// Not Q5_K and Q6_K: the tiles form results by half blocks, whose sums of those formats may pass 2^24 and are rounded there, where the pairs keep
+// those of whole blocks exact.
+bool tiles_quicker(const TileArgs &a, double other, int sm_count) {
+    if (a.fmt == F_Q5_K || a.fmt == F_Q6_K) return false;
+    if (a.fmt == F_TQ1_0 && a.m > 128 && a.n >= 2048) return false;              // 5 of 64 sizes there: 142 x 5766 x 2048 14.7 / 19.1, 180 x 6144 x 4096 27.8 / 25.0
+    return tile_supported(a) && tile_estimate(a, sm_count) < (a.fmt == F_Q4_0 || a.fmt == F_Q8_0 ? 0.94 : 1.0) * other;
 }
 
 size_t tile_plane_bytes(const TileArgs &a) { return (size_t)((a.m + 7) / 8) * (size_t)(a.k / 256) * tile_group_bytes(a.fmt); }
@@ -174,15 +188,15 @@ cudaError_t launch_tile(const TileArgs &a, uint8_t *planes, int *status, int sm_
     const cudaError_t e = launch_tile_planes(a, planes, stream);
     if (e != cudaSuccess) return e;
     switch (a.fmt) {
-    case F_Q4_0: return launch_tile_kernel<F_Q4_0>(a, planes, sm_count, stream);
-    case F_Q8_0: return launch_tile_kernel<F_Q8_0>(a, planes, sm_count, stream);
-    case F_Q2_K: return launch_tile_kernel<F_Q2_K>(a, planes, sm_count, stream);
-    case F_Q3_K: return launch_tile_kernel<F_Q3_K>(a, planes, sm_count, stream);
-    case F_Q4_K: return launch_tile_kernel<F_Q4_K>(a, planes, sm_count, stream);
-    case F_Q5_K: return launch_tile_kernel<F_Q5_K>(a, planes, sm_count, stream);
-    case F_Q6_K: return launch_tile_kernel<F_Q6_K>(a, planes, sm_count, stream);
-    case F_IQ2_XXS: return launch_tile_kernel<F_IQ2_XXS>(a, planes, sm_count, stream);
-    default: return launch_tile_kernel<F_TQ1_0>(a, planes, sm_count, stream);
+    case F_Q4_0: return launch_tile_kernel<F_Q4_0>(a, planes, status, sm_count, stream);
+    case F_Q8_0: return launch_tile_kernel<F_Q8_0>(a, planes, status, sm_count, stream);
+    case F_Q2_K: return launch_tile_kernel<F_Q2_K>(a, planes, status, sm_count, stream);
+    case F_Q3_K: return launch_tile_kernel<F_Q3_K>(a, planes, status, sm_count, stream);
+    case F_Q4_K: return launch_tile_kernel<F_Q4_K>(a, planes, status, sm_count, stream);
+    case F_Q5_K: return launch_tile_kernel<F_Q5_K>(a, planes, status, sm_count, stream);
+    case F_Q6_K: return launch_tile_kernel<F_Q6_K>(a, planes, status, sm_count, stream);
+    case F_IQ2_XXS: return launch_tile_kernel<F_IQ2_XXS>(a, planes, status, sm_count, stream);
+    default: return launch_tile_kernel<F_TQ1_0>(a, planes, status, sm_count, stream);
     }
 }
 

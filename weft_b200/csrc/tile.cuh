@@ -13,15 +13,25 @@
 // of a CTA are `wr` row groups times `wk` slices of K (blocks are dealt to the slices in turn; the slices' sums meet in
 // shared memory at the end of a tile): few tokens or few rows leave the chip idle unless K is cut as well.
 //
-// Weights are read once per token tile by 16-byte cp.async into a ring of stages.  Rows of formats whose record is not a
-// multiple of 16 bytes start at any even address: the copy takes the 16-byte window around the record and the reader
-// shifts.  Activations come from planes in fragment order that tile_planes_kernel writes while it quantizes: 2048 bytes
-// of codes per (eight tokens, block) plus the scales and the operand of the min term, so a fragment is one 16-byte
-// shared-memory load for two 32-element groups.
+// Weights are read once per token tile into a ring of stages.  Where rows are multiples of 16 bytes a slice's part of a step is one box of a
+// tensor map, and the token groups of a block, which follow each other in the planes, are one bulk copy; each arrives on the stage's barrier, and as
+// many warps issue as there are copies.  Other rows (records of 210, 110, 84, 66 and 54 bytes) start at any even address: 16-byte cp.async takes
+// the window around the record and the reader shifts, in boxes too, since a block starts there as rows do.  Everything by cp.async
+// held the warps up for as long as their arithmetic took (77 x 4096 x 4096 Q8_0: a step of 3200 clocks, 1100 of them copies; one thread that
+// issued all boxes of a step: 900), and the slices' sums went through an epilogue of 6000 clocks a tile where it is 1700 now.
+// us: 77 x 4096 x 4096 Q8_0 22.0 -> 16.4, 77 x 14336 x 4096 52.8 -> 38.9, 256 x 2048 x 2048 Q5_K 17.9 -> 12.9, 512 x 4096 x 4096 Q3_K 111 -> 97.
+// What bounds it now (ncu, 77 x 14336 x 4096 Q8_0): two warps a scheduler that wait for their own MMAs and multiply-adds (0.38 of the issue
+// slots, MMA pipe 0.30); four, with 16 rows each, read the tokens twice as often and are no quicker.
+//
+// A single token group keeps its copies to each warp (PRIVATE in the kernel).  Activations come from planes in fragment order that
+// tile_planes_kernel writes while it quantizes: for each block the groups of eight tokens, 2048 bytes of codes plus the scales and the operand of the
+// min term each, so a fragment is one 16-byte shared-memory load for two 32-element groups.
 #pragma once
 
 #include "gemv_units.cuh"
 #include "kernels.h"
+#include "prefill_common.cuh"
+#include "ring.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -29,7 +39,8 @@
 namespace weft {
 
 constexpr int TL_WARPS = 8, TL_THREADS = TL_WARPS * 32;
-constexpr int TL_SMEM = 227 * 1024;
+constexpr int TL_SMEM = 227 * 1024, TL_BARRIERS = 128;
+constexpr uint32_t TL_LIMIT = 1u << 20;                      // polls of a wait before the kernel gives up
 
 constexpr int tl_gcd(int a, int b) { return b ? tl_gcd(b, a % b) : a; }
 
@@ -55,20 +66,29 @@ template <int FMT> struct TileFormat {
     static constexpr int TABLES = FMT == F_IQ2_XXS ? (256 + 128) * 128 : 0;   // shared-memory bytes of the striped codebooks
 };
 
+template <int FMT> __host__ __device__ constexpr int tl_stage_bytes(int nt, int mt, int wk) {      // a box starts on 128 bytes
+    return (TL_WARPS * 16 * mt * TileFormat<FMT>::PITCH + (nt == 1 ? TL_WARPS : wk * nt) * TileFormat<FMT>::GROUP + 127) & ~127;
+}
+
+// token groups whose sums over the slices of K meet in one go
+__host__ __device__ constexpr int tl_at_once(int nt) { return nt < 4 ? nt : 4; }
+
 // CTAs per SM: narrow tiles have few independent MMAs per step, so a second CTA hides what one waits for
 constexpr int tl_ctas(int nt, int mt) { return mt == 2 ? 1 : nt == 1 ? 3 : 2; }
 
 struct TileParams {
     const uint8_t *w;
-    const uint8_t *planes;       // [(m + 7) / 8][nb] groups
+    const uint8_t *planes;       // [nb][(m + 7) / 8] groups
+    int *status;
     const uint8_t *xq;           // the caller's records
     const int8_t *grid, *signs;  // IQ2_XXS
     const uint32_t *powers;      // TQ1_0
     float *y;
     long long n, ldy, row_bytes, w_bytes;
-    int m, nb;                   // tokens, blocks per row
+    int m, nb, groups;           // tokens, blocks per row, groups of eight tokens
     int wk;                      // slices of K (1, 2, 4, 8); 8 / wk row groups
     int row_tiles, token_tiles, tiles, steps, stages;
+    bool boxes;                  // weights come as boxes of the tensor map: rows are multiples of 16 bytes
 };
 
 // Word i (0..15) of lane t in ORDER_TERNARY: the element of its first code, and the stride to the next three.
@@ -508,24 +528,32 @@ __device__ float pair32_dot(const uint8_t *w, const uint8_t *x, int nb) {
 }
 
 template <int FMT, int NT, int MT>
-__global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const TileParams p) {
+__global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const __grid_constant__ TileParams p, const __grid_constant__ CUtensorMap weights) {
     using F = TileFormat<FMT>;
     constexpr int TL_ROWS = 16 * MT;
     extern __shared__ __align__(128) uint8_t smem[];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, r = lane >> 2, t = lane & 3;
     const int wk = p.wk, wr = TL_WARPS / wk, slice = warp / wr, row_group = warp - slice * wr;
     const int tile_rows = wr * TL_ROWS;
-    uint8_t *s_tables = smem;
-    uint8_t *ring = smem + F::TABLES;
+    uint8_t *s_tables = smem + TL_BARRIERS;
+    uint8_t *ring = s_tables + F::TABLES;
     // With one token group every warp keeps its own copy of the slice's group behind its rows and never meets the others
     // before the end of a tile: the step's barrier was a fifth of the time at eight tokens, the second copy comes from L2.
     constexpr bool PRIVATE = NT == 1;
     constexpr int OWN = TL_ROWS * F::PITCH + F::GROUP;         // PRIVATE: bytes of a stage per warp
-    const int w_stage = TL_WARPS * TL_ROWS * F::PITCH, stage_bytes = PRIVATE ? TL_WARPS * OWN : w_stage + wk * NT * F::GROUP;
+    const int w_stage = TL_WARPS * TL_ROWS * F::PITCH, stage_bytes = tl_stage_bytes<FMT>(NT, MT, wk);
     const int own_rows = warp * (PRIVATE ? OWN : TL_ROWS * F::PITCH);
     uint8_t *s_sums = ring + (size_t)p.stages * stage_bytes;   // only with wk > 1
 
+    // boxes and token groups arrive on the stage's barrier: for each slice an arrival with their bytes
+    const uint32_t full = smem_addr(smem);
+    const bool boxes = !PRIVATE && p.boxes;
     asm volatile("griddepcontrol.launch_dependents;");
+    if (!PRIVATE) {
+        if (tid < p.stages) mbar_init(reinterpret_cast<uint64_t *>(smem) + tid, boxes ? 2 * wk : wk);
+        mbar_fence_init();
+        __syncthreads();
+    }
 
     // ---- copies of one step of a tile.  A warp brings its own 32 rows: piece i * 32 + lane of them, in the order in which they
     // lie in shared memory, so that the destination is an immediate offset
@@ -549,7 +577,19 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
                 offsets[i] = (uint32_t)min(row, w_last) * row_bytes + 16u * (uint32_t)(piece - row * F::PIECES);
             }
     };
-    auto copy_weights = [&](int step, uint8_t *stage) {
+    auto copy_weights = [&](const TilePlace &place, int step, int slot) {
+        uint8_t *stage = ring + (size_t)slot * stage_bytes;
+        if (boxes) {                                           // warp w brings slice w: one warp for all of them held the others up for 900 clocks a step
+            if (warp < wk && elect_one()) {
+                const int block = step * wk + warp;
+                if (block < p.nb) {
+                    fence_proxy_async();
+                    mbar_expect_tx_a(full + 8 * slot, (uint32_t)(tile_rows * F::PITCH));
+                    tma_load_2d(stage + warp * tile_rows * F::PITCH, &weights, (int)((uint32_t)(block * F::UNIT) & ~15u) / 8, (int)place.row0, reinterpret_cast<uint64_t *>(smem) + slot);
+                } else mbar_arrive_a(full + 8 * slot);
+            }
+            return;
+        }
         const int block = step * wk + slice;
         if (block >= p.nb) return;
         const uint32_t dst = smem_addr(stage + own_rows) + 16 * lane;
@@ -575,26 +615,24 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
             }
         }
     };
-    auto copy_tokens = [&](const TilePlace &place, int step, uint8_t *stage) {
-        constexpr int PIECES = F::GROUP / 16;
+    auto copy_tokens = [&](const TilePlace &place, int step, int slot) {
+        uint8_t *stage = ring + (size_t)slot * stage_bytes;
         if constexpr (PRIVATE) {
+            constexpr int PIECES = F::GROUP / 16;
             const int block = step * wk + slice;
             if (block >= p.nb) return;
             const uint32_t dst = smem_addr(stage + own_rows + TL_ROWS * F::PITCH) + 16 * lane;
-            const uint8_t *src = p.planes + ((long long)place.group0 * p.nb + block) * F::GROUP + 16 * lane;
+            const uint8_t *src = p.planes + ((long long)block * p.groups + place.group0) * F::GROUP + 16 * lane;
 #pragma unroll
             for (int i = 0; i < (PIECES + 31) / 32; ++i)
                 if ((i + 1) * 32 <= PIECES || i * 32 + lane < PIECES) cp16(dst + 512 * i, src + 512 * i);
-        } else {
-        for (int unit = warp; unit < wk * place.live; unit += TL_WARPS) {        // (slice, token group): GROUP contiguous bytes
-            const int kg = unit / place.live, nt = unit - kg * place.live, block = step * wk + kg;
-            if (block >= p.nb) break;
-            const uint32_t dst = smem_addr(stage + w_stage + (kg * NT + nt) * F::GROUP) + 16 * lane;
-            const uint8_t *src = p.planes + ((long long)(place.group0 + nt) * p.nb + block) * F::GROUP + 16 * lane;
-#pragma unroll
-            for (int i = 0; i < (PIECES + 31) / 32; ++i)
-                if ((i + 1) * 32 <= PIECES || i * 32 + lane < PIECES) cp16(dst + 512 * i, src + 512 * i);
-        }
+        } else if (TL_WARPS - 1 - warp < wk && elect_one()) {    // the token groups of a block follow each other
+            const int kg = TL_WARPS - 1 - warp, block = step * wk + kg;
+            if (block < p.nb) {
+                fence_proxy_async();
+                mbar_expect_tx_a(full + 8 * slot, (uint32_t)(place.live * F::GROUP));
+                bulk_g2s_a(smem_addr(stage + w_stage + kg * NT * F::GROUP), p.planes + ((long long)block * p.groups + place.group0) * F::GROUP, (uint32_t)(place.live * F::GROUP), full + 8 * slot);
+            } else mbar_arrive_a(full + 8 * slot);
         }
     };
 
@@ -605,7 +643,7 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
         int tile = fill_tile, step = 0;
         enter_tile(tile_place<NT>(p, tile, tile_rows));
         for (int s = 0; s < ahead && tile < p.tiles; ++s) {
-            copy_weights(step, ring + (size_t)s * stage_bytes);
+            copy_weights(tile_place<NT>(p, tile, tile_rows), step, s);
             if (++step == p.steps) { step = 0; tile += gridDim.x; if (tile < p.tiles) enter_tile(tile_place<NT>(p, tile, tile_rows)); }
         }
     }
@@ -627,7 +665,7 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
     TilePlace fill_place = tile_place<NT>(p, fill_tile, tile_rows);
     for (int s = 0; s < ahead; ++s) {
         if (fill_tile < p.tiles) {
-            copy_tokens(fill_place, fill_step, ring + (size_t)s * stage_bytes);
+            copy_tokens(fill_place, fill_step, s);
             if (++fill_step == p.steps) { fill_step = 0; fill_tile += gridDim.x; if (fill_tile < p.tiles) fill_place = tile_place<NT>(p, fill_tile, tile_rows); }
         }
         cp_commit();
@@ -642,6 +680,8 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
             for (int c = 0; c < 4; ++c) acc[nt][mt][c] = 0.0f;
 
     int slot = 0, fill_slot = ahead;
+    uint32_t phase = 0;
+    bool ok = true;
     for (int tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
         const TilePlace place = tile_place<NT>(p, tile, tile_rows);
         uint32_t skew[MT][2];                                   // SHIFTED: low bits of the rows' byte offsets
@@ -653,12 +693,11 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
                 skew[mt][e] = (uint32_t)(n >= p.n ? p.n - 1 : n) * row_bytes;
             }
         for (int step = 0; step < p.steps; ++step) {
-            if (p.stages == 2) cp_wait<0>(); else if (p.stages == 3) cp_wait<1>(); else if (p.stages == 4) cp_wait<2>(); else cp_wait<4>();
-            if constexpr (PRIVATE) __syncwarp(); else __syncthreads();   // this step has landed for all its readers; the oldest slot is free
+            if (!boxes) { if (p.stages == 2) cp_wait<0>(); else if (p.stages == 3) cp_wait<1>(); else if (p.stages == 4) cp_wait<2>(); else cp_wait<4>(); }
+            if constexpr (PRIVATE) __syncwarp(); else __syncthreads();   // the warp's rows of this step have landed; the oldest slot is free
             if (fill_tile < p.tiles) {
-                uint8_t *stage = ring + (size_t)fill_slot * stage_bytes;
-                copy_weights(fill_step, stage);
-                copy_tokens(fill_place, fill_step, stage);
+                copy_weights(fill_place, fill_step, fill_slot);
+                copy_tokens(fill_place, fill_step, fill_slot);
                 if (++fill_step == p.steps) {
                     fill_step = 0;
                     fill_tile += gridDim.x;
@@ -666,9 +705,10 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
                 }
             }
             cp_commit();
+            if (!PRIVATE) ok = ok && mbar_wait_a(full + 8 * slot, phase, TL_LIMIT);
             if (++fill_slot == p.stages) fill_slot = 0;
             const uint8_t *stage = ring + (size_t)slot * stage_bytes;
-            if (++slot == p.stages) slot = 0;
+            if (++slot == p.stages) { slot = 0; phase ^= 1u; }
             const int block = step * wk + slice;
             if (block >= p.nb) continue;
             const uint8_t *tokens = PRIVATE ? stage + own_rows + TL_ROWS * F::PITCH : stage + w_stage + slice * NT * F::GROUP;
@@ -683,12 +723,22 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
             tile_block<FMT, NT, MT>(rows, tokens, F::GROUP, lane, s_tables, plain_powers, powers, acc);
         }
 
-        // ---- the slices' sums meet in shared memory, two token groups at a time: [slice][token][row]
-        constexpr int AT_ONCE = NT > 1 ? 2 : 1;
+        // ---- the slices' sums meet in shared memory, a few token groups at a time, each lane's values side by side: [slice][row group][group][m16 tile][lane].
+        // Slice k adds up, in the order of the slices, and stores group nt where nt % wk is k.
+        constexpr int AT_ONCE = tl_at_once(NT);
         bool again = false;                                    // PAIR32: a result of this thread is NaN
+        const auto store = [&](int nt, int mt, const float (&v)[4]) {
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int token = (place.group0 + nt) * 8 + 2 * t + (c & 1);
+                const long long n = place.row0 + row_group * TL_ROWS + 16 * mt + 8 * (c >> 1) + r;
+                if (token >= p.m || n >= p.n) continue;
+                p.y[(long long)token * p.ldy + n] = v[c];
+                if (F::PAIR32) again |= v[c] != v[c];
+            }
+        };
         if (wk > 1) {
-            const int pitch = tile_rows + 4;                   // the four quads of a row of lanes store to different banks
-            float *sums = reinterpret_cast<float *>(s_sums);
+            float4 *sums = reinterpret_cast<float4 *>(s_sums) + lane;
 #pragma unroll
             for (int nt0 = 0; nt0 < NT; nt0 += AT_ONCE) {
 #pragma unroll
@@ -696,40 +746,25 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
                     if (nt0 + i < NT)
 #pragma unroll
                         for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                            for (int c = 0; c < 4; ++c)
-                                sums[((slice * AT_ONCE + i) * 8 + 2 * t + (c & 1)) * pitch + row_group * TL_ROWS + 16 * mt + 8 * (c >> 1) + r] = acc[nt0 + i][mt][c];
+                            sums[(((slice * wr + row_group) * AT_ONCE + i) * MT + mt) * 32] = make_float4(acc[nt0 + i][mt][0], acc[nt0 + i][mt][1], acc[nt0 + i][mt][2], acc[nt0 + i][mt][3]);
                 __syncthreads();
-                for (int i = tid; i < AT_ONCE * 8 * tile_rows; i += TL_THREADS) {
-                    const int token_in = i / tile_rows, row = i - token_in * tile_rows, token = (place.group0 + nt0) * 8 + token_in;
-                    const long long n = place.row0 + row;
-                    if (token >= p.m || n >= p.n || nt0 * 8 + token_in >= NT * 8) continue;
-                    float total = 0.0f;
-                    for (int k = 0; k < wk; ++k) total += sums[(k * AT_ONCE * 8 + token_in) * pitch + row];
-                    p.y[(long long)token * p.ldy + n] = total;
-                    if (F::PAIR32) again |= total != total;
-                }
-                __syncthreads();
-            }
-        } else
-        {
+                for (int i = (slice - nt0) & (wk - 1); i < AT_ONCE && nt0 + i < NT; i += wk)
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt) {
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const int token = (place.group0 + nt) * 8 + 2 * t + c;
-                    if (token >= p.m) continue;
-                    float *y = p.y + (long long)token * p.ldy;
-#pragma unroll
-                    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-                        for (int e = 0; e < 2; ++e) {
-                            const long long n = place.row0 + row_group * TL_ROWS + 16 * mt + 8 * e + r;
-                            if (n < p.n) y[n] = acc[nt][mt][2 * e + c];
-                            if (F::PAIR32) again |= acc[nt][mt][2 * e + c] != acc[nt][mt][2 * e + c];
+                    for (int mt = 0; mt < MT; ++mt) {
+                        float total[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+                        for (int k = 0; k < wk; ++k) {
+                            const float4 v = sums[(((k * wr + row_group) * AT_ONCE + i) * MT + mt) * 32];
+                            total[0] += v.x; total[1] += v.y; total[2] += v.z; total[3] += v.w;
                         }
-                }
+                        store(nt0 + i, mt, total);
+                    }
+                __syncthreads();
             }
+        } else {
+#pragma unroll
+            for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                for (int mt = 0; mt < MT; ++mt) store(nt, mt, acc[nt][mt]);
         }
 #pragma unroll
         for (int nt = 0; nt < NT; ++nt)
@@ -738,29 +773,26 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
 #pragma unroll
                 for (int c = 0; c < 4; ++c) acc[nt][mt][c] = 0.0f;
         if constexpr (F::PAIR32)
-            if (again) {                                       // the thread's results in the order above
-                const int sums = AT_ONCE * 8 * tile_rows, per = (sums + TL_THREADS - 1) / TL_THREADS;
-                const int results = wk > 1 ? (NT + AT_ONCE - 1) / AT_ONCE * per : NT * MT * 4;
+            if (again)                                         // the thread's results once more
 #pragma unroll 1
-                for (int i = 0; i < results; ++i) {
-                    int token, row;
-                    if (wk > 1) {
-                        const int at = (i % per) * TL_THREADS + tid;
-                        token = (place.group0 + i / per * AT_ONCE) * 8 + at / tile_rows;
-                        row = at % tile_rows;
-                        if (at >= sums || token >= (place.group0 + NT) * 8) continue;
-                    } else {
-                        token = (place.group0 + i / (4 * MT)) * 8 + 2 * t + (i & 1);
-                        row = row_group * TL_ROWS + 16 * (i / 4 % MT) + 8 * (i / 2 & 1) + r;
+                for (int nt = wk > 1 ? slice : 0; nt < NT; nt += wk)
+#pragma unroll 1
+                    for (int i = 0; i < 4 * MT; ++i) {
+                        const int token = (place.group0 + nt) * 8 + 2 * t + (i & 1);
+                        const long long n = place.row0 + row_group * TL_ROWS + 16 * (i >> 2) + 8 * (i >> 1 & 1) + r;
+                        if (token >= p.m || n >= p.n) continue;
+                        float *y = p.y + (long long)token * p.ldy + n;
+                        if (*y != *y) *y = pair32_dot<FMT>(p.w + n * p.row_bytes, p.xq + (long long)token * p.nb * 272, p.nb);
                     }
-                    const long long n = place.row0 + row;
-                    if (token >= p.m || n >= p.n) continue;
-                    float *y = p.y + (long long)token * p.ldy + n;
-                    if (*y != *y) *y = pair32_dot<FMT>(p.w + n * p.row_bytes, p.xq + (long long)token * p.nb * 272, p.nb);
-                }
-            }
     }
     cp_wait<0>();
+    if (!ok) {                                                    // the warps stay together all the same; a millisecond is long after the last copy has landed
+        report(p.status, ST_WAIT_TIMEOUT);
+        unsigned long long now, until;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+        until = now + 1000000;
+        while (now < until) asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    }
 }
 
 // ------------------------------------------------------------------ launch
@@ -768,11 +800,10 @@ __global__ void __launch_bounds__(TL_THREADS, tl_ctas(NT, MT)) tile_kernel(const
 // How a launch is cut: token groups per tile, slices of K per CTA, ring stages.
 struct TilePlan { int nt, mt, wk, stages; double cost; };
 
-constexpr int tl_sum_bytes(int nt, int mt, int wk) { return wk > 1 ? wk * (nt > 1 ? 16 : 8) * (TL_WARPS / wk * 16 * mt + 4) * 4 : 0; }
-template <int FMT> constexpr int tl_stage_bytes(int nt, int mt, int wk) { return TL_WARPS * 16 * mt * TileFormat<FMT>::PITCH + (nt == 1 ? TL_WARPS : wk * nt) * TileFormat<FMT>::GROUP; }
+constexpr int tl_sum_bytes(int nt, int mt, int wk) { return wk > 1 ? TL_WARPS * tl_at_once(nt) * mt * 512 : 0; }
 
 template <int FMT, int NT, int MT>
-cudaError_t launch_tile_plan(const TileArgs &a, const uint8_t *planes, const TilePlan &plan, int sm_count, cudaStream_t stream) {
+cudaError_t launch_tile_plan(const TileArgs &a, const uint8_t *planes, const TilePlan &plan, int *status, int sm_count, cudaStream_t stream) {
     using F = TileFormat<FMT>;
     TileParams p{};
     p.w = static_cast<const uint8_t *>(a.w);
@@ -785,6 +816,9 @@ cudaError_t launch_tile_plan(const TileArgs &a, const uint8_t *planes, const Til
     p.row_bytes = (long long)p.nb * F::UNIT;
     p.w_bytes = p.row_bytes * a.n;
     p.m = (int)a.m;
+    p.groups = (int)((a.m + 7) / 8);
+    p.status = status;
+    p.boxes = p.row_bytes % 16 == 0 && a.n < (1LL << 30);
     p.wk = plan.wk;
     p.stages = plan.stages;
     const int tile_rows = TL_WARPS / plan.wk * 16 * MT;
@@ -792,8 +826,12 @@ cudaError_t launch_tile_plan(const TileArgs &a, const uint8_t *planes, const Til
     p.token_tiles = (int)(((a.m + 7) / 8 + NT - 1) / NT);
     p.tiles = p.row_tiles * p.token_tiles;
     p.steps = (p.nb + plan.wk - 1) / plan.wk;
-    const int smem = F::TABLES + plan.stages * tl_stage_bytes<FMT>(NT, MT, plan.wk) + tl_sum_bytes(NT, MT, plan.wk);
-    cudaError_t e = grant_dynamic_smem(reinterpret_cast<const void *>(tile_kernel<FMT, NT, MT>), smem);
+    const int smem = TL_BARRIERS + F::TABLES + plan.stages * tl_stage_bytes<FMT>(NT, MT, plan.wk) + tl_sum_bytes(NT, MT, plan.wk);
+    CUtensorMap weights{};
+    cudaError_t e = cudaSuccess;
+    if (NT > 1 && p.boxes)
+        e = encode_tile_map(&weights, CU_TENSOR_MAP_DATA_TYPE_INT64, a.w, (unsigned long long)p.row_bytes / 8, (unsigned long long)a.n, (unsigned long long)p.row_bytes, F::PITCH / 8, (unsigned)tile_rows);
+    if (e == cudaSuccess) e = grant_dynamic_smem(reinterpret_cast<const void *>(tile_kernel<FMT, NT, MT>), smem);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)std::min(p.tiles, sm_count * std::max(1, std::min(tl_ctas(NT, MT), 228 * 1024 / (smem + 1024)))));
@@ -805,26 +843,25 @@ cudaError_t launch_tile_plan(const TileArgs &a, const uint8_t *planes, const Til
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, tile_kernel<FMT, NT, MT>, p);
+    return cudaLaunchKernelEx(&cfg, tile_kernel<FMT, NT, MT>, p, weights);
 }
 
 // What a step costs, in units of a step's fixed part with 16 rows per warp (mt = 1): the MMAs of a token group, the same two with
-// 32 rows, a tile's own part, the slices' sums per token group; how much a further CTA on the SM adds to one alone, and how much
-// a ring of only two stages loses.
-struct TileCosts { double group1, fixed2, group2, tile, sums, beside, shallow; };
+// 32 rows, a tile's own part (Q4_0: not of one token group), the slices' sums per token group; how much a further CTA on the SM adds to one alone, how much
+// a ring of only two stages loses, and a whole step of one token group (its warps fetch for themselves) with 16 and with 32 rows.
+struct TileCosts { double group1, fixed2, group2, tile, sums, beside, shallow, one1, one2; };
 template <int FMT> constexpr TileCosts tile_costs() {
     using F = TileFormat<FMT>;
-    if (F::SUB16) return {0.147, 1.466, 0.206, 0.96, 0.182, 0.583, 0.075};
-    if (F::PAIR32) return {0.116, 1.741, 0.150, 0.0, 0.211, 0.267, 0.033};
-    if (FMT == F_IQ2_XXS) return {0.166, 1.754, 0.171, 0.0, 0.423, 0.729, 0.036};
-    if (FMT == F_TQ1_0) return {0.175, 1.438, 0.220, 0.267, 0.071, 0.224, 0.227};
-    return {0.127, 1.540, 0.153, 0.0, 0.150, 0.492, 0.090};
+    if (F::SUB16) return {0.330, 1.504, 0.573, 0.557, 0.058, 0.616, 0.022, 1.665, 2.490};
+    if (F::PAIR32) return {0.416, 1.595, 0.579, 1.112, 0.121, 0.513, 0.046, 1.951, 3.326};
+    if (FMT == F_IQ2_XXS) return {0.210, 1.927, 0.269, 0.364, 0.125, 0.666, 0.021, 1.463, 2.423};
+    if (FMT == F_TQ1_0) return {0.161, 1.521, 0.253, 0.453, 0.080, 0.549, 0.053, 1.339, 2.059};
+    return {0.127, 1.540, 0.153, 0.0, 0.150, 0.492, 0.090, 1.127, 1.693};
 }
 
 // Picks the cut with the least estimated time: what decides is how full the last round of the grid is, how long K is kept in one
-// piece and whether CTAs share an SM.  The costs were fitted to the times of every cut at 780 sizes (3 to 512 tokens, 256 to
-// 32768 rows, K 256 to 14336, all formats): the cut picked is 2 % slower than the best one on average (an estimate in
-// microseconds from a few sizes of Q4_K: 5.5 %, some sizes 20 to 30 %).
+// piece and whether CTAs share an SM.  The costs were fitted to the times of every cut at 980 sizes (3 to 600 tokens,
+// 256 to 32768 rows, K 512 to 14336, all formats): the cut picked is 0.7 (IQ2_XXS) to 2.1 % (Q6_K) slower than the best one on average.
 template <int FMT>
 TilePlan tile_plan(const TileArgs &a, int sm_count) {
     using F = TileFormat<FMT>;
@@ -834,27 +871,28 @@ TilePlan tile_plan(const TileArgs &a, int sm_count) {
     for (int mt = 1; mt <= 2; ++mt)
         for (int nt = 1; nt <= 8 && nt <= groups; ++nt)
             for (int wk : {1, 2, 4, 8}) {
-                const int stage = tl_stage_bytes<FMT>(nt, mt, wk), fixed = F::TABLES + tl_sum_bytes(nt, mt, wk);
+                const int tile_rows = TL_WARPS / wk * 16 * mt, stage = tl_stage_bytes<FMT>(nt, mt, wk), fixed = TL_BARRIERS + F::TABLES + tl_sum_bytes(nt, mt, wk);
+                const long long tiles = ((a.n + tile_rows - 1) / tile_rows) * ((groups + nt - 1) / nt), steps = (nb + wk - 1) / wk;
+                const long long on_sm = (tiles + sm_count - 1) / sm_count;      // tiles of the busiest SM
                 int ctas = tl_ctas(nt, mt), stages = 0;
+                if (nt > 1) ctas = (int)std::min<long long>(ctas, on_sm);         // a CTA that has an SM to itself takes all of its shared memory, unless its warps would fill it
                 for (; ctas > 0 && stages < 2; --ctas) stages = (TL_SMEM / ctas - 1024 - fixed) / stage;
                 ++ctas;
                 stages = stages >= 6 ? 6 : stages >= 4 ? 4 : stages;
                 if (stages < 2 || (wk > nb && wk > 1)) continue;
-                const int tile_rows = TL_WARPS / wk * 16 * mt;
-                const long long tiles = ((a.n + tile_rows - 1) / tile_rows) * ((groups + nt - 1) / nt), steps = (nb + wk - 1) / wk;
-                const long long on_sm = (tiles + sm_count - 1) / sm_count, rounds = on_sm / ctas, rest = on_sm - rounds * ctas;   // tiles of the busiest SM
-                const double step = (mt == 2 ? C.fixed2 + C.group2 * nt : 1.0 + C.group1 * nt) * (stages == 2 ? 1.0 + C.shallow : 1.0);
+                const long long rounds = on_sm / ctas, rest = on_sm - rounds * ctas;
+                const double step = (nt == 1 ? (mt == 2 ? C.one2 : C.one1) : mt == 2 ? C.fixed2 + C.group2 * nt : 1.0 + C.group1 * nt) * (stages == 2 ? 1.0 + C.shallow : 1.0);
                 const double times = rounds * (1.0 + C.beside * (ctas - 1)) + (rest ? 1.0 + C.beside * (rest - 1) : 0.0);
-                const double cost = times * (steps * step + C.tile) + (wk > 1 ? C.sums * nt * on_sm : 0.0);
+                const double cost = times * (steps * step + (nt > 1 || FMT != F_Q4_0 ? C.tile : 0.0)) + (wk > 1 ? C.sums * nt * on_sm : 0.0);
                 if (!best.nt || cost < best.cost) best = TilePlan{nt, mt, wk, stages, cost};
             }
     return best;
 }
 
 template <int FMT>
-cudaError_t launch_tile_kernel(const TileArgs &a, const uint8_t *planes, int sm_count, cudaStream_t stream) {
+cudaError_t launch_tile_kernel(const TileArgs &a, const uint8_t *planes, int *status, int sm_count, cudaStream_t stream) {
     const TilePlan plan = tile_plan<FMT>(a, sm_count);
-#define TL_CASE(NT, MT) case (NT) * 4 + (MT): return launch_tile_plan<FMT, NT, MT>(a, planes, plan, sm_count, stream)
+#define TL_CASE(NT, MT) case (NT) * 4 + (MT): return launch_tile_plan<FMT, NT, MT>(a, planes, plan, status, sm_count, stream)
     switch (plan.nt * 4 + plan.mt) {
     TL_CASE(1, 1); TL_CASE(2, 1); TL_CASE(3, 1); TL_CASE(4, 1); TL_CASE(5, 1); TL_CASE(6, 1); TL_CASE(7, 1); TL_CASE(8, 1);
     TL_CASE(1, 2); TL_CASE(2, 2); TL_CASE(3, 2); TL_CASE(4, 2); TL_CASE(5, 2); TL_CASE(6, 2); TL_CASE(7, 2); TL_CASE(8, 2);
@@ -865,7 +903,7 @@ cudaError_t launch_tile_kernel(const TileArgs &a, const uint8_t *planes, int sm_
 
 // One translation unit per family instantiates its kernels (tile_*.cu).
 #define TL_EACH_FORMAT(DO) DO(F_Q4_0) DO(F_Q8_0) DO(F_Q2_K) DO(F_Q3_K) DO(F_Q4_K) DO(F_Q5_K) DO(F_Q6_K) DO(F_IQ2_XXS) DO(F_TQ1_0)
-#define TL_ELSEWHERE(FMT) extern template cudaError_t launch_tile_kernel<FMT>(const TileArgs &, const uint8_t *, int, cudaStream_t);
+#define TL_ELSEWHERE(FMT) extern template cudaError_t launch_tile_kernel<FMT>(const TileArgs &, const uint8_t *, int *, int, cudaStream_t);
 TL_EACH_FORMAT(TL_ELSEWHERE)
 #undef TL_ELSEWHERE
 

@@ -2,6 +2,6 @@
 #include "tile.cuh"
 
 namespace weft {
-template cudaError_t launch_tile_kernel<F_Q4_0>(const TileArgs &, const uint8_t *, int, cudaStream_t);
-template cudaError_t launch_tile_kernel<F_Q8_0>(const TileArgs &, const uint8_t *, int, cudaStream_t);
+template cudaError_t launch_tile_kernel<F_Q4_0>(const TileArgs &, const uint8_t *, int *, int, cudaStream_t);
+template cudaError_t launch_tile_kernel<F_Q8_0>(const TileArgs &, const uint8_t *, int *, int, cudaStream_t);
 }  // namespace weft
