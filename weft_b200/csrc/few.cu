@@ -21,10 +21,10 @@ static bool plan_of(const TileArgs &a, FewPlan &plan) {
 //   (8 x 4096 x 14336 Q5_K 18.1 / 15.7; Q6_K 6144 rows 29.7 / 37.4), others with many tokens (20 x 8771 x 6144 Q6_K 30.9 / 25.5);
 // * chunks that leave members of a team idle, with many tokens (29 x 4032 x 3072 Q4_K 10.4 / 8.9);
 // * more tokens on fewer rows than SMs have warps for, where the tiles take K in slices (24 x 512 x 4096 Q6_K 7.0 / 6.3);
-// * short rows, where the collector's turn for a tile is as long as the tile (32 x 28672 x 1024 Q5_K 17.6 / 13.9).
+// * short rows, where the collector's turn for a tile is as long as the tile (32 x 28672 x 1024 Q5_K 17.6 / 13.9), and fewer than four blocks for a team of eight.
 bool few_supported(const TileArgs &a) {
     FewPlan plan;
-    if (a.m < 3 || a.m > 32 || a.k % 256 || a.k < 256 || a.n > (1LL << 30) || (reinterpret_cast<uintptr_t>(a.w) & 15u) || !plan_of(a, plan)) return false;
+    if (a.m < 3 || a.m > 32 || a.k % 256 || a.k < 1024 || a.n > (1LL << 30) || (reinterpret_cast<uintptr_t>(a.w) & 15u) || !plan_of(a, plan)) return false;
     const bool tight = plan.slots < 2 * FW_WARPS / FW_MEMBERS, full = plan.chunk >= FW_MEMBERS - 1;
     switch (a.fmt) {
     case F_Q4_0: return a.m <= 8 && !tight && (a.k >= 8192 || (a.k >= 4096 && a.n >= 9472));

@@ -13,8 +13,9 @@
 // A box takes a few bytes of the next chunk along, so that rows start 32 (16) bytes apart in the banks; whole rows by bulk copies would start all in the
 // same one.  Built and slower: a bulk copy for each row (60 ns each, whoever issues them: 13.5 us), 16-byte copies by three loader warps (17.8) or by each
 // warp for itself (14.5), K split over a cluster (22 and more), three teams (12.2).  Two or three stages in flight are best, as for the GEMVs (six: 13.2).
-// What bounds it now (ncu, Q4_K at this size): 2.9 us until the planes are there, then issue slots at 0.6 and the logic pipe at 0.55 of their rates with four
-// warps a scheduler, and the seventh tile of a few CTAs where the others have six; DRAM runs at 0.31 over the whole launch.
+// What bounds it now (ncu, Q4_K at this size): 2.9 us until the planes are there, then instructions: issue slots at 0.45 and the logic pipe at 0.37 of
+// their rates over the whole launch, a half more while it multiplies, four warps a scheduler; and the seventh tile of a few CTAs where the others have
+// six.  DRAM delivers 2.5 TB/s over the whole launch.
 #pragma once
 
 #include "ring.cuh"
@@ -267,7 +268,7 @@ cudaError_t launch_few_plan(const TileArgs &a, const uint8_t *planes, const FewP
     p.status = status;
     CUtensorMap weights;
     cudaError_t e = encode_tile_map(&weights, CU_TENSOR_MAP_DATA_TYPE_INT64, a.w, (unsigned long long)p.row_bytes / 8, (unsigned long long)a.n, (unsigned long long)p.row_bytes, (unsigned)plan.pitch / 8, FW_ROWS);
-    if (e == cudaSuccess) e = grant_dynamic_smem(reinterpret_cast<const void *>(few_kernel<FMT, NT>), plan.smem);
+    if (e == cudaSuccess) e = grant_dynamic_smem(reinterpret_cast<const void *>(few_kernel<FMT, NT>), FW_SMEM);      // once for all sizes
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)std::min(sm_count, p.tiles));

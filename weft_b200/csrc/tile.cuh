@@ -831,7 +831,7 @@ cudaError_t launch_tile_plan(const TileArgs &a, const uint8_t *planes, const Til
     cudaError_t e = cudaSuccess;
     if (NT > 1 && p.boxes)
         e = encode_tile_map(&weights, CU_TENSOR_MAP_DATA_TYPE_INT64, a.w, (unsigned long long)p.row_bytes / 8, (unsigned long long)a.n, (unsigned long long)p.row_bytes, F::PITCH / 8, (unsigned)tile_rows);
-    if (e == cudaSuccess) e = grant_dynamic_smem(reinterpret_cast<const void *>(tile_kernel<FMT, NT, MT>), smem);
+    if (e == cudaSuccess) e = grant_dynamic_smem(reinterpret_cast<const void *>(tile_kernel<FMT, NT, MT>), TL_SMEM);     // once for all sizes
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)std::min(p.tiles, sm_count * std::max(1, std::min(tl_ctas(NT, MT), 228 * 1024 / (smem + 1024)))));
